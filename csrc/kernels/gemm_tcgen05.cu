@@ -648,6 +648,9 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         if (col0 >= p.N) break;  // warp-uniform
         uint32_t r[32];
         tmem_ld_32x32b_x32(t_row + c, r);
+        Bias32 bias;
+        const bool bias_vec = bias32_vec_ok(p.bias, p.bias_f32, col0, p.N);
+        if (bias_vec) bias32_load(bias, p.bias, col0);
         tmem_ld_wait();
         if (row < p.M) {
           float v[32];
@@ -666,18 +669,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 #pragma unroll
           for (int i = 0; i < 32; ++i) v[i] *= p.alpha;
           const bool full_chunk = (col0 + 32 <= p.N);
-          if (p.bias) {
-#pragma unroll
-            for (int i = 0; i < 32; ++i) {
-              if (full_chunk || col0 + i < p.N) {
-                float b = p.bias_f32
-                              ? reinterpret_cast<const float*>(p.bias)[col0 + i]
-                              : __bfloat162float(
-                                    reinterpret_cast<const __nv_bfloat16*>(p.bias)[col0 + i]);
-                v[i] += b;
-              }
-            }
-          }
+          if (bias_vec) bias32_add(v, bias);
+          else if (p.bias) bias32_add_any(v, p.bias, p.bias_f32, col0, p.N);
           if (p.rs_mode && rs_coalesce) {
             // bf16 partial into the warp's staging rows; flushed below in 128-byte row segments
             uint8_t* srow = out_stage + lane * 144 + (c & 32) * 2;
