@@ -229,17 +229,96 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __
   }
 }
 
-// out[c] = sum_r part[r, c]; one thread per column, coalesced across the warp.
-__global__ void colsum_kernel(const float* __restrict__ part, int nrows, int H,
-                              float* __restrict__ out_f32, __nv_bfloat16* __restrict__ out_bf16,
-                              int accumulate) {
-  int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= H) return;
+// out[c] = sum_r part[r, c] for one or two (blockIdx.y) fp32 matrices [nrows, H] that a kernel before left as
+// per-block partial rows. A few hundred rows are too few bytes to matter and many dependent steps if one thread
+// walks a column (30 us at 592 x 4096): here a block owns 32 columns and its 32 warps take every 32nd row, eight
+// loads in flight each, so a column is three round trips deep (4 us).
+struct ColsumArgs {
+  const float* part[2];
+  float* out_f32[2];
+  __nv_bfloat16* out_bf16[2];
+};
+constexpr int kColsumThreads = 1024;
+__global__ void __launch_bounds__(kColsumThreads)
+colsum_kernel(const ColsumArgs a, int nrows, int H, int accumulate) {
+  __shared__ float sm[32][33];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const float* __restrict__ part = a.part[blockIdx.y];
+  const int c = blockIdx.x * 32 + lane;
   float s = 0.f;
-  for (int r = 0; r < nrows; ++r) s += part[(size_t)r * H + c];
-  if (out_f32) out_f32[c] = accumulate ? out_f32[c] + s : s;
-  if (out_bf16)
-    out_bf16[c] = __float2bfloat16(accumulate ? __bfloat162float(out_bf16[c]) + s : s);
+  if (c < H) {
+    for (int r0 = warp; r0 < nrows; r0 += 32 * 8) {
+      float v[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[j] = (r0 + 32 * j < nrows) ? part[(size_t)(r0 + 32 * j) * H + c] : 0.f;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) s += v[j];
+    }
+  }
+  sm[warp][lane] = s;
+  __syncthreads();
+  // warp w sums column w of the block
+  float t = sm[lane][warp];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+  const int co = blockIdx.x * 32 + warp;
+  if (lane == 0 && co < H) {
+    float* of = a.out_f32[blockIdx.y];
+    __nv_bfloat16* ob = a.out_bf16[blockIdx.y];
+    if (of) of[co] = accumulate ? of[co] + t : t;
+    if (ob) ob[co] = __float2bfloat16(accumulate ? __bfloat162float(ob[co]) + t : t);
+  }
+}
+static void launch_colsum(const ColsumArgs& a, int n, int nrows, int H, int accumulate, cudaStream_t stream) {
+  colsum_kernel<<<dim3((H + 31) / 32, n), kColsumThreads, 0, stream>>>(a, nrows, H, accumulate);
+}
+
+// Column sums of a bf16 matrix [rows, N] (the gradient of a bias): one partial row of fp32 sums per block, then
+// colsum_kernel. Bound by reading the matrix once; a block is 256 columns (16 bytes a lane) by a slice of rows.
+constexpr int kBiasRowsMin = 32;   // rows per block below which more blocks no longer pay
+__global__ void __launch_bounds__(256)
+bias_grad_kernel(const __nv_bfloat16* __restrict__ x, float* __restrict__ part, int rows, int N, long long ld,
+                 int rows_per_block) {
+  __shared__ float sm[8][256 + 8];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int c = blockIdx.x * 256 + lane * 8;
+  const int r1 = min(rows, ((int)blockIdx.y + 1) * rows_per_block);
+  float acc[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) acc[j] = 0.f;
+  if (c < N) {
+    for (int r = blockIdx.y * rows_per_block + warp; r < r1; r += 32) {
+      uint4 v[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        v[u] = (r + 8 * u < r1) ? __ldg(reinterpret_cast<const uint4*>(x + (size_t)(r + 8 * u) * ld + c))
+                                : make_uint4(0, 0, 0, 0);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        float f[8];
+        unpack8(v[u], f);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc[j] += f[j];
+      }
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < 8; ++j) sm[warp][lane * 8 + j] = acc[j];
+  __syncthreads();
+  const int co = blockIdx.x * 256 + threadIdx.x;
+  if (co < N) {
+    float s = 0.f;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) s += sm[w][threadIdx.x];
+    part[(size_t)blockIdx.y * N + co] = s;
+  }
+}
+static int bias_grad_chunks(int rows, int N) {
+  const int cols = (N + 255) / 256;
+  int n = (sm_count() * 8 + cols - 1) / cols;
+  const int most = (rows + kBiasRowsMin - 1) / kBiasRowsMin;
+  if (n > most) n = most;
+  return n < 1 ? 1 : n;
 }
 
 // ------------------------------------------------------------------ LayerNorm
@@ -735,8 +814,8 @@ extern "C" int tpb_rmsnorm_bwd(const void* dy, const void* x, const void* w, con
                           (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x,
                           (const __nv_bfloat16*)w, rstd, (const __nv_bfloat16*)dres,
                           (__nv_bfloat16*)dx, dw_part, rows, H, x_stride, dy_stride, dx_stride)));
-  colsum_kernel<<<(H + 255) / 256, 256, 0, (cudaStream_t)stream>>>(
-      dw_part, grid, H, dw_f32, (__nv_bfloat16*)dw_bf16, dw_accumulate);
+  launch_colsum({{dw_part, nullptr}, {dw_f32, nullptr}, {(__nv_bfloat16*)dw_bf16, nullptr}}, 1, grid, H, dw_accumulate,
+                (cudaStream_t)stream);
   return (int)cudaGetLastError();
 }
 
@@ -767,10 +846,22 @@ extern "C" int tpb_layernorm_bwd(const void* dy, const void* x, const void* w, c
                           (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x,
                           (const __nv_bfloat16*)w, mean, rstd, (__nv_bfloat16*)dx, dw_part, db_part,
                           rows, H)));
-  colsum_kernel<<<(H + 255) / 256, 256, 0, (cudaStream_t)stream>>>(
-      dw_part, grid, H, dw_f32, (__nv_bfloat16*)dw_bf16, accumulate);
-  colsum_kernel<<<(H + 255) / 256, 256, 0, (cudaStream_t)stream>>>(
-      db_part, grid, H, db_f32, (__nv_bfloat16*)db_bf16, accumulate);
+  launch_colsum({{dw_part, db_part}, {dw_f32, db_f32}, {(__nv_bfloat16*)dw_bf16, (__nv_bfloat16*)db_bf16}}, 2, grid, H,
+                accumulate, (cudaStream_t)stream);
+  return (int)cudaGetLastError();
+}
+
+// Column sums of a bf16 matrix: `part` holds tpb_bias_grad_chunks(rows, N) * N floats.
+extern "C" int tpb_bias_grad_chunks(int rows, int N) { return bias_grad_chunks(rows, N); }
+extern "C" int tpb_bias_grad(const void* x, float* part, void* out_bf16, int rows, int N, long long ld, void* stream) {
+  TPB_NVTX("tpb_bias_grad");
+  if (N % 8 || ld % 8 || (reinterpret_cast<uintptr_t>(x) & 15)) return -2;
+  if (rows <= 0 || N <= 0) return 0;
+  const int chunks = bias_grad_chunks(rows, N);
+  bias_grad_kernel<<<dim3((N + 255) / 256, chunks), 256, 0, (cudaStream_t)stream>>>(
+      (const __nv_bfloat16*)x, part, rows, N, ld, (rows + chunks - 1) / chunks);
+  launch_colsum({{part, nullptr}, {nullptr, nullptr}, {(__nv_bfloat16*)out_bf16, nullptr}}, 1, chunks, N, 0,
+                (cudaStream_t)stream);
   return (int)cudaGetLastError();
 }
 
@@ -938,7 +1029,7 @@ extern "C" int tpb_rmsnorm_bwd_noalloc(const void* dy, const void* x, const void
                           (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x,
                           (const __nv_bfloat16*)w, rstd, (const __nv_bfloat16*)dres,
                           (__nv_bfloat16*)dx, scratch, rows, H, x_stride, dy_stride, dx_stride)));
-  colsum_kernel<<<(H + 255) / 256, 256, 0, (cudaStream_t)stream>>>(
-      scratch, grid, H, dw_f32, (__nv_bfloat16*)dw_bf16, dw_accumulate);
+  launch_colsum({{scratch, nullptr}, {dw_f32, nullptr}, {(__nv_bfloat16*)dw_bf16, nullptr}}, 1, grid, H, dw_accumulate,
+                (cudaStream_t)stream);
   return (int)cudaGetLastError();
 }

@@ -86,6 +86,8 @@ int tpb_layernorm_bwd(const void* dy, const void* x, const void* w, const float*
                       const float* rstd, void* dx, float* dw_part, float* db_part, float* dw_f32,
                       void* dw_bf16, float* db_f32, void* db_bf16, int accumulate, int rows, int H,
                       void* stream);
+int tpb_bias_grad_chunks(int rows, int N);
+int tpb_bias_grad(const void* x, float* part, void* out_bf16, int rows, int N, long long ld, void* stream);
 int tpb_rope(void* x, const float* cos_t, const float* sin_t, const long long* pos,
              long long tokens, int heads, int D, long long tok_stride, long long head_stride,
              int seq_len, int interleaved, int backward, void* stream);

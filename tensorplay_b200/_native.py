@@ -41,6 +41,8 @@ _KERNEL_SIGS = {
     "tpb_rmsnorm_bwd": [P, P, P, P, P, P, P, P, P, I, I, I, LL, LL, LL, P],
     "tpb_layernorm_fwd": [P, P, P, P, P, P, I, I, F, P],
     "tpb_layernorm_bwd": [P, P, P, P, P, P, P, P, P, P, P, P, I, I, I, P],
+    "tpb_bias_grad_chunks": [I, I],
+    "tpb_bias_grad": [P, P, P, I, I, LL, P],
     "tpb_rope": [P, P, P, P, LL, I, I, LL, LL, I, I, I, P],
     "tpb_rope_out": [P, P, P, P, P, LL, I, I, LL, LL, LL, LL, I, I, I, P],
     "tpb_swiglu_fwd": [P, P, P, LL, I, LL, P],
@@ -109,7 +111,7 @@ def _load(name: str):
 
 
 # kernel launches issued by one call of each entry point (for launch accounting)
-_LAUNCHES = {"tpb_rmsnorm_bwd": 2, "tpb_layernorm_bwd": 3, "tpb_flash_bwd": 3, "tpb_rmsnorm_bwd_grid": 0,
+_LAUNCHES = {"tpb_rmsnorm_bwd": 2, "tpb_layernorm_bwd": 2, "tpb_bias_grad": 2, "tpb_bias_grad_chunks": 0, "tpb_flash_bwd": 3, "tpb_rmsnorm_bwd_grid": 0,
              "tpb_grouped_workspace_ints": 0, "tpb_adamw_set_overlap": 0, "tpb_flash_fwd_config": 0, "tpb_gemm_set_splitk_workspace": 0, "tpb_grouped_gemm": 2}
 launch_count = 0
 

@@ -99,6 +99,20 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
     return out
 
 
+def _bias_grad(dy: torch.Tensor) -> torch.Tensor:
+    """Column sums of ``dy [rows, N]`` in fp32, rounded once to its dtype."""
+    rows, N = dy.shape
+    if not (rows and N and dy.dtype == torch.bfloat16 and N % 8 == 0 and dy.data_ptr() % 16 == 0
+            and dy.is_contiguous() and use_native(dy)):
+        return dy.float().sum(0).to(dy.dtype)
+    L = lib()
+    part = torch.empty((L.tpb_bias_grad_chunks(rows, N), N), dtype=torch.float32, device=dy.device)
+    out = torch.empty(N, dtype=dy.dtype, device=dy.device)
+    _native.check(L.tpb_bias_grad(dy.data_ptr(), part.data_ptr(), out.data_ptr(), rows, N, N, stream_ptr()),
+                  "tpb_bias_grad")
+    return out
+
+
 class _LinearFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, weight, bias):
@@ -135,7 +149,7 @@ class _LinearFn(torch.autograd.Function):
             else:
                 dw = gemm(dy2, x2, a_mn=True, b_mn=True, out_dtype=weight.dtype)
         if ctx.has_bias and ctx.needs_input_grad[2]:
-            db = dy2.float().sum(0).to(dy.dtype)
+            db = _bias_grad(dy2)
         return dx, dw, db
 
 
