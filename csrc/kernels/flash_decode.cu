@@ -1,0 +1,369 @@
+// Attention of a few query rows over a long key/value sequence (decoding, speculative verification) for sm_100a.
+//
+// The work is reading K and V once: 2 * Tk * D * Hkv values per sequence against 4 * R flops a value, R = query rows
+// that share a KV head (Tq * Hq / Hkv). The 128-row tiles of flash_fwd_kernel read every KV head once per QUERY head
+// and leave all but B * Hq CTAs idle: 437 us at B = 8, Tk = 16381, 32/8 heads of 128 (0.54 GB). Here
+//   * all query rows of a KV head form the 16-row operand of one warp MMA (m16n8k16), so K and V are read once per
+//     16 rows; with at most 16 rows there is no tile that would amortise TMEM and a shared-memory operand pipeline;
+//   * K and V go from global memory straight into the B fragments. The sum over d (and over keys) is free of order,
+//     so a lane takes whole 16-byte pieces of a row and the query fragments are permuted alike: no shared memory, no
+//     ldmatrix, 8 KB in flight per warp (one 16-key step of K and one of V ahead);
+//   * the keys are split over CTAs until the chip is full; partial sums stay fp32 and a second kernel merges them.
+// The same case takes 117 us (4.6 TB/s).
+// Scores, running maximum, sums and output accumulate in fp32; probabilities are rounded to bf16 for the second
+// product, as in flash_fwd_kernel.
+#include "sm100.cuh"
+#include "tpb_api.h"
+
+namespace tpb {
+
+constexpr int kDecWarps = 4;
+constexpr int kDecRows = 16;   // query rows per CTA
+constexpr int kDecKeys = 16;   // keys per warp and step
+
+struct DecodeParams {
+  const __nv_bfloat16 *q, *k, *v;
+  __nv_bfloat16* o;
+  float* lse;
+  float* part_o;    // [n_splits][B * Hkv * R][D], null when n_splits == 1
+  float* part_lse;  // [n_splits][B * Hkv * R], log2 domain
+  int B, Tq, Tk, Hq, Hkv, group, R, row_tiles, causal, window, lse_stride, n_splits, keys_per_split;
+  float scale_log2e;
+  long long q_tok, q_head, q_batch, k_tok, k_head, k_batch, v_tok, v_head, v_batch, o_tok, o_head, o_batch;
+};
+
+__device__ __forceinline__ void mma_bf16_16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
+                                               uint32_t b0, uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
+      "{%0, %1, %2, %3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ float dec_exp2(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ uint32_t dec_pack(float lo, float hi) {
+  uint32_t d;
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(hi), "f"(lo));
+  return d;
+}
+// K and V are read once: keep them from pushing the next layer's weights out of L1.
+__device__ __forceinline__ uint4 dec_ld(const __nv_bfloat16* p) {
+  uint4 r;
+  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w)
+               : "l"(p));
+  return r;
+}
+
+template <int D>
+__global__ void __launch_bounds__(kDecWarps * 32)
+flash_decode_kernel(const DecodeParams p) {
+  constexpr int NP = D / 32;   // 16-byte pieces of a K row per lane
+  constexpr int VP = D / 64;   // 16-byte pieces of a V row per lane
+  __shared__ float sm_o[kDecWarps][kDecRows][D];
+  __shared__ float sm_m[kDecWarps][kDecRows], sm_l[kDecWarps][kDecRows];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int gq = lane >> 2, t = lane & 3;
+  const int split = blockIdx.x, hk = blockIdx.y / p.row_tiles, rt = blockIdx.y % p.row_tiles, b = blockIdx.z;
+
+  // this lane's two rows: r0 (fragment row gq) and r0 + 8
+  const int r0 = rt * kDecRows + gq;
+  int lim[2], low[2];
+  uint4 qf[2][NP];
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const int r = r0 + 8 * i;
+    const int tq = r / p.group, h = hk * p.group + r % p.group;
+    const bool in = r < p.R;
+    lim[i] = in ? (p.causal ? min(p.Tk - 1, tq + p.Tk - p.Tq) : p.Tk - 1) : -1;
+    low[i] = p.window > 0 ? tq + p.Tk - p.Tq - p.window + 1 : 0;
+    const __nv_bfloat16* qr = p.q + b * p.q_batch + (long long)tq * p.q_tok + (long long)h * p.q_head;
+#pragma unroll
+    for (int c = 0; c < NP; ++c)
+      qf[i][c] = in ? *reinterpret_cast<const uint4*>(qr + (t + 4 * c) * 8) : make_uint4(0, 0, 0, 0);
+  }
+
+  int k_begin = split * p.keys_per_split;
+  const int k_end = min(p.Tk, k_begin + p.keys_per_split);
+  if (p.window > 0) {
+    // the CTA's first row has the lowest bound
+    const int first = (rt * kDecRows) / p.group + p.Tk - p.Tq - p.window + 1;
+    if (first > k_begin) k_begin += (first - k_begin) / kDecKeys * kDecKeys;
+  }
+  const __nv_bfloat16* kb = p.k + b * p.k_batch + (long long)hk * p.k_head;
+  const __nv_bfloat16* vb = p.v + b * p.v_batch + (long long)hk * p.v_head;
+
+  uint4 kf[2][NP], vf[4][VP];
+  auto load_k = [&](int base) {
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int key = base + u * 8 + gq;
+#pragma unroll
+      for (int c = 0; c < NP; ++c)
+        kf[u][c] = key < k_end ? dec_ld(kb + (long long)key * p.k_tok + (t + 4 * c) * 8) : make_uint4(0, 0, 0, 0);
+    }
+  };
+  // keys past the end are zero-filled: their probability is zero, but zero times whatever lies there need not be
+  auto load_v = [&](int base) {
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int key = base + (u >> 1) * 8 + 2 * t + (u & 1);
+#pragma unroll
+      for (int c = 0; c < VP; ++c)
+        vf[u][c] = key < k_end ? dec_ld(vb + (long long)key * p.v_tok + (gq + 8 * c) * 8) : make_uint4(0, 0, 0, 0);
+    }
+  };
+
+  float acc[VP * 8][4];
+#pragma unroll
+  for (int n = 0; n < VP * 8; ++n)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[n][j] = 0.f;
+  float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
+
+  int base = k_begin + warp * kDecKeys;
+  if (base < k_end) {
+    load_k(base);
+    load_v(base);
+  }
+  for (; base < k_end; base += kDecWarps * kDecKeys) {
+    const int next = base + kDecWarps * kDecKeys;
+    float s[2][4];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) s[u][j] = 0.f;
+#pragma unroll
+      for (int c = 0; c < NP; ++c) {
+        mma_bf16_16816(s[u], qf[0][c].x, qf[1][c].x, qf[0][c].y, qf[1][c].y, kf[u][c].x, kf[u][c].y);
+        mma_bf16_16816(s[u], qf[0][c].z, qf[1][c].z, qf[0][c].w, qf[1][c].w, kf[u][c].z, kf[u][c].w);
+      }
+    }
+    if (next < k_end) load_k(next);
+    // s[u][2 i + j]: row i, key base + 8 u + 2 t + j
+    float mx[2] = {-INFINITY, -INFINITY};
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          const int key = base + u * 8 + 2 * t + j;
+          float& x = s[u][2 * i + j];
+          x = (key <= lim[i] && key >= low[i] && key < k_end) ? x * p.scale_log2e : -INFINITY;
+          mx[i] = fmaxf(mx[i], x);
+        }
+    float alpha[2], mu[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      mx[i] = fmaxf(mx[i], __shfl_xor_sync(0xffffffffu, mx[i], 1));
+      mx[i] = fmaxf(mx[i], __shfl_xor_sync(0xffffffffu, mx[i], 2));
+      const float mn = fmaxf(m[i], mx[i]);
+      mu[i] = mn == -INFINITY ? 0.f : mn;   // no key yet: every exponent below is -inf
+      alpha[i] = dec_exp2(m[i] - mu[i]);
+      m[i] = mn;
+      l[i] *= alpha[i];
+    }
+    if (__any_sync(0xffffffffu, alpha[0] != 1.f || alpha[1] != 1.f)) {
+#pragma unroll
+      for (int n = 0; n < VP * 8; ++n) {
+        acc[n][0] *= alpha[0]; acc[n][1] *= alpha[0];
+        acc[n][2] *= alpha[1]; acc[n][3] *= alpha[1];
+      }
+    }
+    uint32_t pa[4];   // A fragment of the second product: (row, key half)
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const float e0 = dec_exp2(s[u][2 * i] - mu[i]), e1 = dec_exp2(s[u][2 * i + 1] - mu[i]);
+        l[i] += e0 + e1;
+        pa[2 * u + i] = dec_pack(e0, e1);
+      }
+#pragma unroll
+    for (int c = 0; c < VP; ++c) {
+      const uint32_t* w0 = reinterpret_cast<const uint32_t*>(&vf[0][c]);
+      const uint32_t* w1 = reinterpret_cast<const uint32_t*>(&vf[1][c]);
+      const uint32_t* w2 = reinterpret_cast<const uint32_t*>(&vf[2][c]);
+      const uint32_t* w3 = reinterpret_cast<const uint32_t*>(&vf[3][c]);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const uint32_t sel = (e & 1) ? 0x7632u : 0x5410u;
+        mma_bf16_16816(acc[c * 8 + e], pa[0], pa[1], pa[2], pa[3], __byte_perm(w0[e >> 1], w1[e >> 1], sel),
+                       __byte_perm(w2[e >> 1], w3[e >> 1], sel));
+      }
+    }
+    if (next < k_end) load_v(next);
+  }
+
+  // ---- the four warps' partial rows
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    l[i] += __shfl_xor_sync(0xffffffffu, l[i], 1);
+    l[i] += __shfl_xor_sync(0xffffffffu, l[i], 2);
+    if (t == 0) { sm_m[warp][gq + 8 * i] = m[i]; sm_l[warp][gq + 8 * i] = l[i]; }
+#pragma unroll
+    for (int c = 0; c < VP; ++c)
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        float* dst = &sm_o[warp][gq + 8 * i][(2 * t + j + 8 * c) * 8];
+        *reinterpret_cast<float4*>(dst) = make_float4(acc[c * 8][2 * i + j], acc[c * 8 + 1][2 * i + j],
+                                                      acc[c * 8 + 2][2 * i + j], acc[c * 8 + 3][2 * i + j]);
+        *reinterpret_cast<float4*>(dst + 4) = make_float4(acc[c * 8 + 4][2 * i + j], acc[c * 8 + 5][2 * i + j],
+                                                          acc[c * 8 + 6][2 * i + j], acc[c * 8 + 7][2 * i + j]);
+      }
+  }
+  __syncthreads();
+  constexpr int VEC = D / 4;   // float4 per row
+  for (int x = threadIdx.x; x < kDecRows * VEC; x += kDecWarps * 32) {
+    const int rr = x / VEC, d = (x % VEC) * 4;
+    const int r = rt * kDecRows + rr;
+    if (r >= p.R) break;
+    float M = -INFINITY;
+#pragma unroll
+    for (int w = 0; w < kDecWarps; ++w) M = fmaxf(M, sm_m[w][rr]);
+    float L = 0.f;
+    float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (M != -INFINITY) {
+#pragma unroll
+      for (int w = 0; w < kDecWarps; ++w) {
+        const float f = dec_exp2(sm_m[w][rr] - M);
+        L += f * sm_l[w][rr];
+        const float4 a = *reinterpret_cast<const float4*>(&sm_o[w][rr][d]);
+        o.x += f * a.x; o.y += f * a.y; o.z += f * a.z; o.w += f * a.w;
+      }
+    }
+    const float inv = L > 0.f ? 1.f / L : 0.f;
+    o.x *= inv; o.y *= inv; o.z *= inv; o.w *= inv;
+    const float lse2 = L > 0.f ? M + log2f(L) : -INFINITY;
+    if (p.n_splits > 1) {
+      const long long row = (long long)(b * p.Hkv + hk) * p.R + r;
+      const long long at = (long long)split * p.B * p.Hkv * p.R + row;
+      *reinterpret_cast<float4*>(p.part_o + at * D + d) = o;
+      if (d == 0) p.part_lse[at] = lse2;
+    } else {
+      const int tq = r / p.group, h = hk * p.group + r % p.group;
+      uint2 w;
+      w.x = dec_pack(o.x, o.y);
+      w.y = dec_pack(o.z, o.w);
+      *reinterpret_cast<uint2*>(p.o + b * p.o_batch + (long long)tq * p.o_tok + (long long)h * p.o_head + d) = w;
+      if (d == 0) p.lse[((long long)b * p.Hq + h) * p.lse_stride + tq] = lse2 * 0.6931471805599453f;
+    }
+  }
+}
+
+// o = sum_s w_s o_s / sum_s w_s with w_s = 2^(lse_s - max); one warp per row, the splits' rows requested eight at a time.
+template <int D>
+__global__ void __launch_bounds__(128)
+flash_decode_merge_kernel(const DecodeParams p) {
+  constexpr int E = D / 32;   // floats per lane
+  const int lane = threadIdx.x & 31;
+  const long long rows = (long long)p.B * p.Hkv * p.R;
+  const long long row = (long long)blockIdx.x * 4 + (threadIdx.x >> 5);
+  if (row >= rows) return;
+  float M = -INFINITY;
+  for (int s = lane; s < p.n_splits; s += 32) M = fmaxf(M, p.part_lse[s * rows + row]);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
+  const float mu = M == -INFINITY ? 0.f : M;
+  float acc[E], den = 0.f;
+#pragma unroll
+  for (int e = 0; e < E; ++e) acc[e] = 0.f;
+  for (int s0 = 0; s0 < p.n_splits; s0 += 8) {
+    float v[8][E], w[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const bool in = s0 + j < p.n_splits;
+      const long long at = (s0 + j) * rows + row;
+      w[j] = in ? p.part_lse[at] : -INFINITY;
+#pragma unroll
+      for (int e = 0; e < E; ++e) v[j][e] = in ? p.part_o[at * D + lane + 32 * e] : 0.f;
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const float f = dec_exp2(w[j] - mu);
+      den += f;
+#pragma unroll
+      for (int e = 0; e < E; ++e) acc[e] += f * v[j][e];
+    }
+  }
+  const float inv = den > 0.f ? 1.f / den : 0.f;
+  const int r = (int)(row % p.R);
+  const int hk = (int)(row / p.R % p.Hkv), b = (int)(row / p.R / p.Hkv);
+  const int tq = r / p.group, h = hk * p.group + r % p.group;
+  __nv_bfloat16* o = p.o + b * p.o_batch + (long long)tq * p.o_tok + (long long)h * p.o_head;
+#pragma unroll
+  for (int e = 0; e < E; ++e) o[lane + 32 * e] = __float2bfloat16(acc[e] * inv);
+  if (lane == 0)
+    p.lse[((long long)b * p.Hq + h) * p.lse_stride + tq] = den > 0.f ? (M + log2f(den)) * 0.6931471805599453f : -INFINITY;
+}
+
+// Splits of the keys: the rounds of resident CTAs times the keys of one split is what a launch takes; a second kernel
+// and its partial rows cost about as much as 256 keys. Two CTAs of 128 threads fit an SM (registers).
+static int decode_splits(int B, int Hkv, int row_tiles, int Tk) {
+  const long long ctas = (long long)B * Hkv * row_tiles, slots = 2LL * sm_count();
+  int best = 1;
+  long long best_cost = -1;
+  for (int n = 1; n <= 64 && (n == 1 || (Tk + n - 1) / n >= 128); ++n) {
+    const long long rounds = (ctas * n + slots - 1) / slots;
+    const long long cost = rounds * ((Tk + n - 1) / n + 64) + (n > 1 ? 256 : 0);
+    if (best_cost < 0 || cost < best_cost) { best = n; best_cost = cost; }
+  }
+  return best;
+}
+
+}  // namespace tpb
+
+using namespace tpb;
+
+// Number of key splits tpb_flash_decode uses: with more than one, part_o holds n * B * Hq * Tq * D floats and part_lse
+// n * B * Hq * Tq.
+extern "C" int tpb_flash_decode_splits(int B, int Tq, int Tk, int Hq, int Hkv) {
+  if (B <= 0 || Tq <= 0 || Tk <= 0 || Hkv <= 0) return 1;
+  const int R = Tq * (Hq / Hkv);
+  return decode_splits(B, Hkv, (R + kDecRows - 1) / kDecRows, Tk);
+}
+
+// Arguments as in tpb_flash_fwd_ex; lse [B, Hq, lse_stride].
+extern "C" int tpb_flash_decode(const void* q, const void* k, const void* v, void* o, float* lse, float* part_o,
+                                float* part_lse, int B, int Tq, int Tk, int Hq, int Hkv, int D, long long q_tok,
+                                long long q_head, long long q_batch, long long k_tok, long long k_head,
+                                long long k_batch, long long v_tok, long long v_head, long long v_batch,
+                                long long o_tok, long long o_head, long long o_batch, int lse_stride, int causal,
+                                float scale, int window, int n_splits, void* stream) {
+  TPB_NVTX("tpb_flash_decode");
+  if (B <= 0 || Tq <= 0 || Hq <= 0) return 0;
+  if ((D != 64 && D != 128) || Hkv <= 0 || Hq % Hkv || Tk <= 0 || n_splits < 1 || B > 65535) return -2;
+  if ((q_tok | q_head | q_batch | k_tok | k_head | k_batch | v_tok | v_head | v_batch | o_tok | o_head | o_batch) % 8)
+    return -2;
+  if ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v) |
+       reinterpret_cast<uintptr_t>(o)) & 15)
+    return -2;
+  if (n_splits > 1 && (!part_o || !part_lse)) return -2;
+  DecodeParams p;
+  p.q = (const __nv_bfloat16*)q; p.k = (const __nv_bfloat16*)k; p.v = (const __nv_bfloat16*)v;
+  p.o = (__nv_bfloat16*)o; p.lse = lse; p.part_o = part_o; p.part_lse = part_lse;
+  p.B = B; p.Tq = Tq; p.Tk = Tk; p.Hq = Hq; p.Hkv = Hkv; p.group = Hq / Hkv; p.R = Tq * p.group;
+  p.row_tiles = (p.R + kDecRows - 1) / kDecRows;
+  p.causal = causal; p.window = window > 0 ? window : 0; p.lse_stride = lse_stride; p.n_splits = n_splits;
+  const int per = (Tk + n_splits - 1) / n_splits;
+  p.keys_per_split = (per + kDecKeys - 1) / kDecKeys * kDecKeys;
+  p.scale_log2e = scale * 1.4426950408889634f;
+  p.q_tok = q_tok; p.q_head = q_head; p.q_batch = q_batch; p.k_tok = k_tok; p.k_head = k_head; p.k_batch = k_batch;
+  p.v_tok = v_tok; p.v_head = v_head; p.v_batch = v_batch; p.o_tok = o_tok; p.o_head = o_head; p.o_batch = o_batch;
+  if ((long long)Hkv * p.row_tiles > 65535) return -2;
+  const dim3 grid(n_splits, Hkv * p.row_tiles, B);
+  if (D == 128) flash_decode_kernel<128><<<grid, kDecWarps * 32, 0, (cudaStream_t)stream>>>(p);
+  else flash_decode_kernel<64><<<grid, kDecWarps * 32, 0, (cudaStream_t)stream>>>(p);
+  if (n_splits > 1) {
+    const long long rows = (long long)B * Hkv * p.R;
+    const unsigned blocks = (unsigned)((rows + 3) / 4);
+    if (D == 128) flash_decode_merge_kernel<128><<<blocks, 128, 0, (cudaStream_t)stream>>>(p);
+    else flash_decode_merge_kernel<64><<<blocks, 128, 0, (cudaStream_t)stream>>>(p);
+  }
+  return (int)cudaGetLastError();
+}

@@ -86,6 +86,12 @@ int tpb_layernorm_bwd(const void* dy, const void* x, const void* w, const float*
                       const float* rstd, void* dx, float* dw_part, float* db_part, float* dw_f32,
                       void* dw_bf16, float* db_f32, void* db_bf16, int accumulate, int rows, int H,
                       void* stream);
+int tpb_flash_decode_splits(int B, int Tq, int Tk, int Hq, int Hkv);
+int tpb_flash_decode(const void* q, const void* k, const void* v, void* o, float* lse, float* part_o, float* part_lse,
+                     int B, int Tq, int Tk, int Hq, int Hkv, int D, long long q_tok, long long q_head,
+                     long long q_batch, long long k_tok, long long k_head, long long k_batch, long long v_tok,
+                     long long v_head, long long v_batch, long long o_tok, long long o_head, long long o_batch,
+                     int lse_stride, int causal, float scale, int window, int n_splits, void* stream);
 int tpb_bias_grad_chunks(int rows, int N);
 int tpb_bias_grad(const void* x, float* part, void* out_bf16, int rows, int N, long long ld, void* stream);
 int tpb_rope(void* x, const float* cos_t, const float* sin_t, const long long* pos,

@@ -18,7 +18,7 @@ import torch
 
 from .. import _native
 from . import _ckpt
-from ._common import lib, status_word, stream_ptr, use_native
+from ._common import lib, ptr, status_word, stream_ptr, use_native
 
 
 def _strides_ok(t: torch.Tensor) -> bool:
@@ -63,6 +63,38 @@ def attention_reference(q, k, v, causal: bool = True, scale: Optional[float] = N
     return o.permute(0, 2, 1, 3).to(q.dtype)
 
 
+def _few_rows(q, k, v) -> bool:
+    """Whether the rows that share a KV head (``Tq * Hq / Hkv``) are few enough for the kernel that streams K and V
+    through the warp MMA. It reads them once per 16 rows while the 128-row tiles read them once per query head, and it
+    splits the keys over the chip; at 64 rows (Tq = 8, groups of 8) the four reads through L2 are still half of those,
+    and beyond 16 tokens the tensor-core tiles fill up."""
+    rows = q.shape[1] * (q.shape[2] // k.shape[2])
+    return (q.shape[1] <= 16 and rows <= 64 and q.shape[3] in (64, 128) and q.dtype == torch.bfloat16
+            and q.shape[2] % k.shape[2] == 0 and 0 < q.shape[0] <= 65535 and k.shape[2] * ((rows + 15) // 16) <= 65535
+            and rows > 0 and k.shape[1] > 0 and _strides_ok(q) and _strides_ok(k) and _strides_ok(v))
+
+
+def _flash_decode(q, k, v, o, lse, causal: bool, scale: float, window: int) -> None:
+    B, Tq, Hq, D = q.shape
+    Tk, Hkv = k.shape[1], k.shape[2]
+    L = lib()
+    n = L.tpb_flash_decode_splits(B, Tq, Tk, Hq, Hkv)
+    part_o = part_lse = None
+    if n > 1:   # fp32 partial rows, merged by a second launch
+        part_o = torch.empty((n, B * Hq * Tq, D), dtype=torch.float32, device=q.device)
+        part_lse = torch.empty((n, B * Hq * Tq), dtype=torch.float32, device=q.device)
+    code = L.tpb_flash_decode(
+        q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr(), ptr(part_o), ptr(part_lse), B, Tq, Tk,
+        Hq, Hkv, D, q.stride(1), q.stride(2), q.stride(0), k.stride(1), k.stride(2), k.stride(0), v.stride(1),
+        v.stride(2), v.stride(0), o.stride(1), o.stride(2), o.stride(0), lse.shape[2], int(causal), float(scale),
+        int(window or 0), n, stream_ptr())
+    _native.check(code, "tpb_flash_decode")
+    if n > 1:
+        _native.launch_count += 1
+    if _native.flop_sinks:
+        _native.add_flops("tpb.flash_attention_forward", 4 * B * Hq * Tq * Tk * D // (2 if causal and Tq == Tk else 1))
+
+
 def flash_fwd(q, k, v, causal: bool, scale: float, kv_len: Optional[torch.Tensor] = None, n_splits: int = 1,
               window: int = 0, seg_start: Optional[torch.Tensor] = None, seg_end: Optional[torch.Tensor] = None,
               out: Optional[torch.Tensor] = None):
@@ -85,6 +117,9 @@ def flash_fwd(q, k, v, causal: bool, scale: float, kv_len: Optional[torch.Tensor
     lse_stride = (Tq + 127) // 128 * 128
     lse = torch.empty((B, Hq, lse_stride), dtype=torch.float32, device=q.device)
     n_splits = max(1, min(int(n_splits), (Tk + 127) // 128)) if not causal else 1
+    if n_splits == 1 and kv_len is None and seg_start is None and seg_end is None and _few_rows(q, k, v):
+        _flash_decode(q, k, v, o, lse, causal, scale, window)
+        return o, lse
     if n_splits > 1:
         part = torch.empty((n_splits, B, Tq, Hq, D), dtype=q.dtype, device=q.device)
         lse_part = torch.empty((n_splits, B, Hq, lse_stride), dtype=torch.float32, device=q.device)
