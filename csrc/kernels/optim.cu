@@ -27,6 +27,59 @@ __device__ __forceinline__ void adamw_one(float& p, float& m, float& v, float g,
   p -= (h.lr / h.bias_c1) * (m / denom);
 }
 
+// Four consecutive elements (element index 4 i): the vector body of both forms.
+template <typename GradT, typename ModelT>
+__device__ __forceinline__ void adamw_vec4(float* __restrict__ master, float* __restrict__ m, float* __restrict__ v,
+                                           const GradT* __restrict__ grad, ModelT* __restrict__ model, long long i,
+                                           float gs, const AdamHyper& h) {
+  float4 p4 = reinterpret_cast<float4*>(master)[i];
+  float4 m4 = reinterpret_cast<float4*>(m)[i];
+  float4 v4 = reinterpret_cast<float4*>(v)[i];
+  float g[4];
+  if constexpr (sizeof(GradT) == 2) {
+    uint2 raw = reinterpret_cast<const uint2*>(grad)[i];
+    float2 a = __bfloat1622float2(*reinterpret_cast<__nv_bfloat162*>(&raw.x));
+    float2 b = __bfloat1622float2(*reinterpret_cast<__nv_bfloat162*>(&raw.y));
+    g[0] = a.x; g[1] = a.y; g[2] = b.x; g[3] = b.y;
+  } else {
+    float4 g4 = reinterpret_cast<const float4*>(grad)[i];
+    g[0] = g4.x; g[1] = g4.y; g[2] = g4.z; g[3] = g4.w;
+  }
+  float pp[4] = {p4.x, p4.y, p4.z, p4.w};
+  float mm[4] = {m4.x, m4.y, m4.z, m4.w};
+  float vv[4] = {v4.x, v4.y, v4.z, v4.w};
+#pragma unroll
+  for (int j = 0; j < 4; ++j) adamw_one(pp[j], mm[j], vv[j], g[j] * gs, h);
+  reinterpret_cast<float4*>(master)[i] = make_float4(pp[0], pp[1], pp[2], pp[3]);
+  reinterpret_cast<float4*>(m)[i] = make_float4(mm[0], mm[1], mm[2], mm[3]);
+  reinterpret_cast<float4*>(v)[i] = make_float4(vv[0], vv[1], vv[2], vv[3]);
+  if (model) {
+    if constexpr (sizeof(ModelT) == 2) {
+      uint2 o;
+      *reinterpret_cast<__nv_bfloat162*>(&o.x) = __floats2bfloat162_rn(pp[0], pp[1]);
+      *reinterpret_cast<__nv_bfloat162*>(&o.y) = __floats2bfloat162_rn(pp[2], pp[3]);
+      reinterpret_cast<uint2*>(model)[i] = o;
+    } else {
+      reinterpret_cast<float4*>(model)[i] = make_float4(pp[0], pp[1], pp[2], pp[3]);
+    }
+  }
+}
+template <typename GradT, typename ModelT>
+__device__ __forceinline__ void adamw_scalar(float* __restrict__ master, float* __restrict__ m, float* __restrict__ v,
+                                             const GradT* __restrict__ grad, ModelT* __restrict__ model, long long i,
+                                             float gs, const AdamHyper& h) {
+  float p = master[i], mm = m[i], vv = v[i];
+  float g;
+  if constexpr (sizeof(GradT) == 2) g = __bfloat162float(grad[i]);
+  else g = grad[i];
+  adamw_one(p, mm, vv, g * gs, h);
+  master[i] = p; m[i] = mm; v[i] = vv;
+  if (model) {
+    if constexpr (sizeof(ModelT) == 2) model[i] = __float2bfloat16(p);
+    else model[i] = p;
+  }
+}
+
 // clip_coef (device, optional): grads are additionally multiplied by *clip_coef.
 // found_inf (device, optional): if *found_inf != 0 the step is skipped.
 template <typename GradT, typename ModelT>
@@ -39,59 +92,20 @@ adamw_flat_kernel(float* __restrict__ master, float* __restrict__ m, float* __re
   const float gs = h.grad_scale * (clip_coef ? *clip_coef : 1.f);
   const long long nvec = n / 4;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < nvec;
-       i += (long long)gridDim.x * blockDim.x) {
-    float4 p4 = reinterpret_cast<float4*>(master)[i];
-    float4 m4 = reinterpret_cast<float4*>(m)[i];
-    float4 v4 = reinterpret_cast<float4*>(v)[i];
-    float g[4];
-    if constexpr (sizeof(GradT) == 2) {
-      uint2 raw = reinterpret_cast<const uint2*>(grad)[i];
-      float2 a = __bfloat1622float2(*reinterpret_cast<__nv_bfloat162*>(&raw.x));
-      float2 b = __bfloat1622float2(*reinterpret_cast<__nv_bfloat162*>(&raw.y));
-      g[0] = a.x; g[1] = a.y; g[2] = b.x; g[3] = b.y;
-    } else {
-      float4 g4 = reinterpret_cast<const float4*>(grad)[i];
-      g[0] = g4.x; g[1] = g4.y; g[2] = g4.z; g[3] = g4.w;
-    }
-    float pp[4] = {p4.x, p4.y, p4.z, p4.w};
-    float mm[4] = {m4.x, m4.y, m4.z, m4.w};
-    float vv[4] = {v4.x, v4.y, v4.z, v4.w};
-#pragma unroll
-    for (int j = 0; j < 4; ++j) adamw_one(pp[j], mm[j], vv[j], g[j] * gs, h);
-    reinterpret_cast<float4*>(master)[i] = make_float4(pp[0], pp[1], pp[2], pp[3]);
-    reinterpret_cast<float4*>(m)[i] = make_float4(mm[0], mm[1], mm[2], mm[3]);
-    reinterpret_cast<float4*>(v)[i] = make_float4(vv[0], vv[1], vv[2], vv[3]);
-    if (model) {
-      if constexpr (sizeof(ModelT) == 2) {
-        uint2 o;
-        *reinterpret_cast<__nv_bfloat162*>(&o.x) = __floats2bfloat162_rn(pp[0], pp[1]);
-        *reinterpret_cast<__nv_bfloat162*>(&o.y) = __floats2bfloat162_rn(pp[2], pp[3]);
-        reinterpret_cast<uint2*>(model)[i] = o;
-      } else {
-        reinterpret_cast<float4*>(model)[i] = make_float4(pp[0], pp[1], pp[2], pp[3]);
-      }
-    }
-  }
+       i += (long long)gridDim.x * blockDim.x)
+    adamw_vec4(master, m, v, grad, model, i, gs, h);
   // tail (n not a multiple of 4)
   long long t0 = nvec * 4 + (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t0 < n) {
-    float p = master[t0], mm = m[t0], vv = v[t0];
-    float g;
-    if constexpr (sizeof(GradT) == 2) g = __bfloat162float(grad[t0]);
-    else g = grad[t0];
-    adamw_one(p, mm, vv, g * gs, h);
-    master[t0] = p; m[t0] = mm; v[t0] = vv;
-    if (model) {
-      if constexpr (sizeof(ModelT) == 2) model[t0] = __float2bfloat16(p);
-      else model[t0] = p;
-    }
-  }
+  if (t0 < n) adamw_scalar(master, m, v, grad, model, t0, gs, h);
 }
 
-// ---- multi-tensor form: up to kMtaTensors tensors and kMtaBlocks (tensor, chunk) pairs per launch
+// ---- multi-tensor form: up to kMtaTensors tensors per launch, cut into chunks of kMtaChunk elements.
+// Bound by memory (28 bytes per parameter with bf16 gradients and weights). A block finds the tensor of its chunk in
+// a table of first chunks and walks the chunk in 16-byte accesses, so one launch covers any amount of data with the
+// access pattern of the flat form: 240 M parameters in 15 tensors took 1.70 ms (3.95 TB/s) with scalar accesses and
+// launches of 640 blocks, and takes 1.10 ms now (6.1 TB/s).
 constexpr int kMtaTensors = 48;
-constexpr int kMtaBlocks = 640;
-constexpr int kMtaChunk = 65536;
+constexpr int kMtaChunk = 8192;
 struct MtaArgs {
   void* master[kMtaTensors];
   void* m[kMtaTensors];
@@ -99,36 +113,32 @@ struct MtaArgs {
   const void* grad[kMtaTensors];
   void* model[kMtaTensors];
   long long numel[kMtaTensors];
-  unsigned char block_tensor[kMtaBlocks];
-  int block_chunk[kMtaBlocks];
+  int first_chunk[kMtaTensors + 1];   // of tensor t; [count] = number of chunks
+  unsigned char vec[kMtaTensors];     // every pointer of the tensor allows the vector accesses
+  int count;
 };
 
 template <typename GradT, typename ModelT>
-__global__ void __launch_bounds__(512)
+__global__ void __launch_bounds__(256)
 adamw_mta_kernel(const __grid_constant__ MtaArgs a, AdamHyper h,
                  const float* __restrict__ clip_coef, const float* __restrict__ found_inf) {
   if (found_inf && *found_inf != 0.f) return;
   const float gs = h.grad_scale * (clip_coef ? *clip_coef : 1.f);
-  const int t = a.block_tensor[blockIdx.x];
-  const long long start = (long long)a.block_chunk[blockIdx.x] * kMtaChunk;
-  const long long n = a.numel[t];
-  const long long end = start + kMtaChunk < n ? start + kMtaChunk : n;
-  float* master = reinterpret_cast<float*>(a.master[t]);
-  float* m = reinterpret_cast<float*>(a.m[t]);
-  float* v = reinterpret_cast<float*>(a.v[t]);
-  const GradT* grad = reinterpret_cast<const GradT*>(a.grad[t]);
-  ModelT* model = reinterpret_cast<ModelT*>(a.model[t]);
-  for (long long i = start + threadIdx.x; i < end; i += blockDim.x) {
-    float p = master[i], mm = m[i], vv = v[i];
-    float g;
-    if constexpr (sizeof(GradT) == 2) g = __bfloat162float(grad[i]);
-    else g = grad[i];
-    adamw_one(p, mm, vv, g * gs, h);
-    master[i] = p; m[i] = mm; v[i] = vv;
-    if (model) {
-      if constexpr (sizeof(ModelT) == 2) model[i] = __float2bfloat16(p);
-      else model[i] = p;
-    }
+  const int chunks = a.first_chunk[a.count];
+  int t = 0;
+  for (int c = blockIdx.x; c < chunks; c += gridDim.x) {
+    while (a.first_chunk[t + 1] <= c) ++t;   // chunks only grow: the search goes on where it stopped
+    const long long start = (long long)(c - a.first_chunk[t]) * kMtaChunk;
+    const long long left = a.numel[t] - start;
+    const int n = left < kMtaChunk ? (int)left : kMtaChunk;
+    float* master = reinterpret_cast<float*>(a.master[t]) + start;
+    float* m = reinterpret_cast<float*>(a.m[t]) + start;
+    float* v = reinterpret_cast<float*>(a.v[t]) + start;
+    const GradT* grad = reinterpret_cast<const GradT*>(a.grad[t]) + start;
+    ModelT* model = a.model[t] ? reinterpret_cast<ModelT*>(a.model[t]) + start : nullptr;
+    const int nvec = a.vec[t] ? n / 4 : 0;
+    for (int i = threadIdx.x; i < nvec; i += 256) adamw_vec4(master, m, v, grad, model, i, gs, h);
+    for (int i = nvec * 4 + threadIdx.x; i < n; i += 256) adamw_scalar(master, m, v, grad, model, i, gs, h);
   }
 }
 
@@ -247,34 +257,39 @@ extern "C" int tpb_adamw_multi(int count, void* const* master, void* const* m, v
   AdamHyper h = make_hyper(lr, beta1, beta2, eps, wd, step, grad_scale, maximize);
   cudaStream_t s = (cudaStream_t)stream;
   MtaArgs a;
-  int nt = 0, nb = 0;
+  a.count = 0;
+  a.first_chunk[0] = 0;
+  const uintptr_t gmask = grad_bf16 ? 7 : 15, wmask = model_bf16 ? 7 : 15;
   auto flush = [&]() -> int {
-    if (nb == 0) { nt = 0; return 0; }
-#define LAUNCH(GT, MT) adamw_mta_kernel<GT, MT><<<nb, 512, 0, s>>>(a, h, clip_coef, found_inf)
+    if (a.count == 0) return 0;
+    const int chunks = a.first_chunk[a.count], cap = sm_count() * 16;
+    const int grid = chunks < cap ? chunks : cap;
+#define LAUNCH(GT, MT) adamw_mta_kernel<GT, MT><<<grid, 256, 0, s>>>(a, h, clip_coef, found_inf)
     if (grad_bf16 && model_bf16) LAUNCH(__nv_bfloat16, __nv_bfloat16);
     else if (grad_bf16) LAUNCH(__nv_bfloat16, float);
     else if (model_bf16) LAUNCH(float, __nv_bfloat16);
     else LAUNCH(float, float);
 #undef LAUNCH
-    nt = 0; nb = 0;
+    a.count = 0;
     return (int)cudaGetLastError();
   };
   for (int i = 0; i < count; ++i) {
-    long long n = numel[i];
+    const long long n = numel[i];
     if (n <= 0) continue;
-    int chunks = (int)((n + kMtaChunk - 1) / kMtaChunk);
-    int c = 0;
-    while (c < chunks) {
-      if (nt == kMtaTensors || nb == kMtaBlocks) { int r = flush(); if (r) return r; }
-      int t = nt++;
-      a.master[t] = master[i]; a.m[t] = m[i]; a.v[t] = v[i]; a.grad[t] = grad[i];
-      a.model[t] = model ? model[i] : nullptr; a.numel[t] = n;
-      while (c < chunks && nb < kMtaBlocks) {
-        a.block_tensor[nb] = (unsigned char)t;
-        a.block_chunk[nb] = c++;
-        ++nb;
-      }
+    const long long chunks = (n + kMtaChunk - 1) / kMtaChunk;
+    if (chunks > 0x3fffffff) return -2;
+    if (a.count == kMtaTensors || (a.count > 0 && a.first_chunk[a.count] + chunks > 0x3fffffff)) {
+      const int r = flush();
+      if (r) return r;
     }
+    const int t = a.count++;
+    a.master[t] = master[i]; a.m[t] = m[i]; a.v[t] = v[i]; a.grad[t] = grad[i];
+    a.model[t] = model ? model[i] : nullptr; a.numel[t] = n;
+    const uintptr_t state = reinterpret_cast<uintptr_t>(master[i]) | reinterpret_cast<uintptr_t>(m[i]) |
+                            reinterpret_cast<uintptr_t>(v[i]);
+    a.vec[t] = !(state & 15) && !(reinterpret_cast<uintptr_t>(grad[i]) & gmask) &&
+               !(reinterpret_cast<uintptr_t>(a.model[t]) & wmask);
+    a.first_chunk[t + 1] = a.first_chunk[t] + (int)chunks;
   }
   return flush();
 }
