@@ -1,0 +1,342 @@
+// bf16 GEMM for few rows of A (M <= 128, K-major: decoding, small batches) on clusters that split the reduction:
+//   C[m, n] (+)= alpha * sum_k A(m, k) * B(n, k)  (+ bias[n])
+// The product is bound by streaming B once. The weight rows are the 128-row operand of the MMA and the NT = 16..128
+// rows of A its column operand, so a stage is 16 KB of weights plus 2..16 KB, and the two CTAs of an SM keep about
+// 190 KB in flight. (With A as the 128-row operand, as in the one-CTA kernel, most rows of its tiles are empty and only
+// N / 128 CTAs work.) A cluster of up to eight CTAs shares the k-blocks of one 128-column tile: every CTA drains its
+// fp32 partial tile into its own shared memory, and after a cluster barrier each sums a slice of the tile over the
+// cluster through distributed shared memory, in rank order, and stores it. The reduction needs no workspace, no flags
+// and no second launch, so it is safe on any stream and under graph capture, and its result does not depend on timing.
+//
+// Measured against the other two kernels (operands beyond L2): M = 1, N = 4096, K = 14336: 70 -> 22 us; M = 16,
+// N = K = 4096: 25 -> 11 us, N = 28672: 52 -> 41 us (5.7 TB/s), N = 128256: 190 -> 165 us (6.4 TB/s).
+#include "sm100.cuh"
+#include "tpb_api.h"
+
+namespace tpb {
+
+constexpr int kRowsThreads = 192;   // warp 0 TMA, warp 1 TMEM owner + MMA issue, warps 2..5 drain
+constexpr int kRowsK = 64;
+constexpr int kRowsBBytes = 128 * kRowsK * 2;
+
+template <int NT>
+struct RowsCfg {
+  static constexpr int kStageBytes = kRowsBBytes + NT * kRowsK * 2;
+  static constexpr int kStages = NT <= 32 ? 5 : (NT == 64 ? 4 : 3);
+  static constexpr int kTmemCols = NT < 32 ? 32 : NT;
+  static constexpr int kTileBytes = NT * 132 * 4;   // the partial tile reuses the ring: [NT][128 + 4] floats
+  static_assert(kTileBytes <= kStages * kStageBytes, "the partial tile must fit the ring");
+  static constexpr int kSmem = kStages * kStageBytes + 1024 + 256;   // two CTAs per SM
+};
+
+struct RowsParams {
+  int M, N, K, ldc;
+  void* C;
+  const void* bias;
+  int bias_f32, out_f32, accumulate;
+  float alpha;
+  uint32_t* status;
+  unsigned long long wait_ns;
+};
+
+__device__ __forceinline__ uint32_t rows_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ uint32_t rows_size() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void rows_cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ float4 rows_ld_remote(uint32_t saddr, uint32_t rank) {
+  float4 v;
+  asm volatile(
+      "{\n\t.reg .b32 ra;\n\t"
+      "mapa.shared::cluster.u32 ra, %4, %5;\n\t"
+      "ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [ra];\n\t}"
+      : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+      : "r"(saddr), "r"(rank)
+      : "memory");
+  return v;
+}
+
+template <int NT, bool B_MN>
+__global__ void __launch_bounds__(kRowsThreads, 2)
+gemm_rows_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmA,
+                   const RowsParams p) {
+  using Cfg = RowsCfg<NT>;
+  constexpr int S = Cfg::kStages;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + S * Cfg::kStageBytes);
+  uint64_t* empty = full + S;
+  uint64_t* done = empty + S;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
+  volatile uint32_t* abort_w = tmem_slot + 1;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rank = (int)rows_rank(), csize = (int)rows_size();
+  const int tile = blockIdx.x / csize;
+  const int n0 = tile * 128;
+  const int k_blocks = (p.K + kRowsK - 1) / kRowsK;
+  const int per = k_blocks / csize, rem = k_blocks % csize;
+  const int kb0 = rank * per + min(rank, rem);
+  const int n_kb = per + (rank < rem ? 1 : 0);   // the host keeps csize <= k_blocks
+
+  if (threadIdx.x == 0) {
+    *abort_w = 0;
+    for (int i = 0; i < S; ++i) {
+      mbar_init(&full[i], 1);
+      mbar_init(&empty[i], 1);
+    }
+    mbar_init(done, 1);
+    fence_barrier_init();
+    prefetch_tmap(&tmB);
+    prefetch_tmap(&tmA);
+  }
+  if (warp == 1) {
+    tmem_alloc(tmem_slot, Cfg::kTmemCols);
+    tmem_relinquish();
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  const uint32_t tmem = *tmem_slot;
+  WaitCtx wc{abort_w, p.status, p.wait_ns};
+
+  if (warp == 0) {
+    if (lane == 0) {
+      for (int it = 0; it < n_kb; ++it) {
+        const int s = it % S;
+        if (!mbar_wait_relaxed(&empty[s], ((it / S) & 1) ^ 1, wc, 1)) break;
+        uint8_t* sp = smem + s * Cfg::kStageBytes;
+        uint8_t* sq = sp + kRowsBBytes;
+        const int k = (kb0 + it) * kRowsK;
+        mbar_arrive_expect_tx(&full[s], Cfg::kStageBytes);
+        if (!B_MN) {
+          tma_load_2d(sp, &tmB, &full[s], k, n0);
+        } else {
+#pragma unroll
+          for (int c = 0; c < 2; ++c) tma_load_2d(sp + c * (kRowsK * 128), &tmB, &full[s], n0 + c * 64, k);
+        }
+        tma_load_2d(sq, &tmA, &full[s], k, 0);
+      }
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    // warp-uniform control flow, one elected lane issues (tcgen05 operands live in uniform registers)
+    constexpr uint32_t idesc = make_idesc_f16(128, NT, 1, B_MN ? 1 : 0, 0);
+    constexpr uint32_t hi = smem_desc_hi(1024);
+    const uint32_t p_lo0 = smem_desc_lo(smem_u32(smem), B_MN ? kRowsK * 128 : 16);
+    const uint32_t q_lo0 = smem_desc_lo(smem_u32(smem + kRowsBBytes), 16);
+    for (int it = 0; it < n_kb; ++it) {
+      const int s = it % S;
+      if (!mbar_wait_warp(&full[s], (it / S) & 1, wc, 2)) break;
+      tc_fence_after_sync();
+      const uint32_t p_lo = p_lo0 + s * (Cfg::kStageBytes >> 4), q_lo = q_lo0 + s * (Cfg::kStageBytes >> 4);
+      if (elect_one()) {
+#pragma unroll
+        for (int j = 0; j < kRowsK / 16; ++j) {
+          const uint32_t po = B_MN ? j * (2048 >> 4) : j * (32 >> 4);
+          umma_f16_ss_w(tmem, p_lo + po, hi, q_lo + j * (32 >> 4), hi, idesc, (it | j) != 0);
+        }
+        umma_commit(&empty[s]);
+        if (it == n_kb - 1) umma_commit(done);
+      }
+      __syncwarp();
+    }
+  } else {
+    // drain the accumulator into the ring (every load has landed and every MMA has read it once `done` completes)
+    const int q = warp & 3;
+    if (mbar_wait_warp(done, 0, wc, 3)) {
+      tc_fence_after_sync();
+      const int row = q * 32 + lane;
+      const uint32_t t_row = tmem + ((uint32_t)(q * 32) << 16);
+      float* tile_s = reinterpret_cast<float*>(smem);
+      constexpr int STEP = NT < 32 ? 16 : 32;
+#pragma unroll 1
+      for (int c = 0; c < NT; c += STEP) {
+        uint32_t r[32];
+        if constexpr (STEP == 16) {
+          uint32_t r16[16];
+          tmem_ld_32x32b_x16(t_row + c, r16);
+          tmem_ld_wait();
+#pragma unroll
+          for (int i = 0; i < 16; ++i) r[i] = r16[i];
+        } else {
+          tmem_ld_32x32b_x32(t_row + c, r);
+          tmem_ld_wait();
+        }
+#pragma unroll
+        for (int i = 0; i < STEP; ++i) tile_s[(c + i) * 132 + row] = __uint_as_float(r[i]);
+      }
+    }
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  if (*abort_w) {
+    // copies of this CTA may still be in flight: give them time before memory is read or goes away
+    const unsigned long long t0 = globaltimer_ns();
+    while (globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
+    __syncthreads();
+  }
+  rows_cluster_sync();   // every partial tile of the cluster is in shared memory
+  if (!*abort_w) {
+    const uint32_t base = smem_u32(smem);
+    for (int u = rank * kRowsThreads + (int)threadIdx.x; u < p.M * 32; u += csize * kRowsThreads) {
+      const int r = u >> 5, c = (u & 31) * 4;   // row of C, column of the tile
+      const int col = n0 + c;
+      if (col >= p.N) continue;
+      const uint32_t at = base + (uint32_t)(r * 132 + c) * 4;
+      float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+      for (int h0 = 0; h0 < csize; h0 += 4) {
+        float4 t[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          t[j] = h0 + j < csize ? rows_ld_remote(at, h0 + j) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) { acc.x += t[j].x; acc.y += t[j].y; acc.z += t[j].z; acc.w += t[j].w; }
+      }
+      float v[4] = {acc.x * p.alpha, acc.y * p.alpha, acc.z * p.alpha, acc.w * p.alpha};
+      const bool whole = col + 4 <= p.N;
+      if (p.bias) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          if (col + i < p.N)
+            v[i] += p.bias_f32 ? reinterpret_cast<const float*>(p.bias)[col + i]
+                               : __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(p.bias)[col + i]);
+      }
+      const size_t off = (size_t)r * p.ldc + col;
+      if (p.out_f32) {
+        float* o = reinterpret_cast<float*>(p.C) + off;
+        if (whole && (reinterpret_cast<uintptr_t>(o) & 15) == 0) {
+          float4 w = make_float4(v[0], v[1], v[2], v[3]);
+          if (p.accumulate) {
+            const float4 old = *reinterpret_cast<const float4*>(o);
+            w.x += old.x; w.y += old.y; w.z += old.z; w.w += old.w;
+          }
+          *reinterpret_cast<float4*>(o) = w;
+        } else {
+          for (int i = 0; i < 4 && col + i < p.N; ++i) o[i] = p.accumulate ? o[i] + v[i] : v[i];
+        }
+      } else {
+        __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(p.C) + off;
+        if (whole && (reinterpret_cast<uintptr_t>(o) & 7) == 0) {
+          if (p.accumulate) {
+            const uint2 old = *reinterpret_cast<const uint2*>(o);
+            const float2 f0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&old.x));
+            const float2 f1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&old.y));
+            v[0] += f0.x; v[1] += f0.y; v[2] += f1.x; v[3] += f1.y;
+          }
+          uint2 w;
+          *reinterpret_cast<__nv_bfloat162*>(&w.x) = __floats2bfloat162_rn(v[0], v[1]);
+          *reinterpret_cast<__nv_bfloat162*>(&w.y) = __floats2bfloat162_rn(v[2], v[3]);
+          *reinterpret_cast<uint2*>(o) = w;
+        } else {
+          for (int i = 0; i < 4 && col + i < p.N; ++i)
+            o[i] = __float2bfloat16(p.accumulate ? __bfloat162float(o[i]) + v[i] : v[i]);
+        }
+      }
+    }
+  }
+  rows_cluster_sync();   // nobody leaves while a peer may read its tile
+  if (warp == 1) {
+    tc_fence_after_sync();
+    tmem_dealloc(tmem, Cfg::kTmemCols);
+  }
+}
+
+template <int NT, bool B_MN>
+static cudaError_t rows_config(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attr, int csize, unsigned tiles) {
+  static bool configured = false;
+  if (!configured) {
+    cudaError_t e = cudaFuncSetAttribute(gemm_rows_kernel<NT, B_MN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         RowsCfg<NT>::kSmem);
+    if (e != cudaSuccess) return e;
+    configured = true;
+  }
+  attr->id = cudaLaunchAttributeClusterDimension;
+  attr->val.clusterDim.x = csize;
+  attr->val.clusterDim.y = 1;
+  attr->val.clusterDim.z = 1;
+  cfg->gridDim = dim3(tiles * csize);
+  cfg->blockDim = dim3(kRowsThreads);
+  cfg->dynamicSmemBytes = RowsCfg<NT>::kSmem;
+  cfg->attrs = attr;
+  cfg->numAttrs = 1;
+  return cudaSuccess;
+}
+
+// Cluster size for `tiles` tiles of `kb` k-blocks: rounds of resident clusters times the k-blocks of one CTA, plus
+// six k-blocks a round for prologue and drain and two for the cluster's barriers and reduction. How many clusters of
+// a size fit at once depends on how many SMs the device's GPCs have left (48 clusters of 6 do not, although 288 CTAs
+// would: N = 6144 took 17 us with 6 against 10 us for N = 4096 with 8), so it is asked of the runtime, once per size.
+template <int NT, bool B_MN>
+static int rows_cluster(int tiles, int kb) {
+  static int resident[9] = {0};
+  long long best_cost = -1;
+  int best = 1;
+  for (int c = 1; c <= 8 && c <= kb; ++c) {
+    if (resident[c] == 0) {
+      cudaLaunchConfig_t cfg = {};
+      cudaLaunchAttribute attr[1];
+      int n = 0;
+      if (rows_config<NT, B_MN>(&cfg, attr, c, 2 * sm_count()) != cudaSuccess ||
+          cudaOccupancyMaxActiveClusters(&n, gemm_rows_kernel<NT, B_MN>, &cfg) != cudaSuccess || n <= 0)
+        n = -1;
+      resident[c] = n;
+    }
+    if (resident[c] < 0) continue;
+    const long long rounds = (tiles + resident[c] - 1) / resident[c];
+    const long long cost = rounds * ((kb + c - 1) / c + 6 + (c > 1 ? 2 : 0));
+    if (best_cost < 0 || cost < best_cost) { best = c; best_cost = cost; }
+  }
+  return best;
+}
+
+template <int NT, bool B_MN>
+static int launch_rows(const CUtensorMap& tb, const CUtensorMap& ta, const RowsParams& p, cudaStream_t stream) {
+  const int tiles = (p.N + 127) / 128;
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  cudaError_t e = rows_config<NT, B_MN>(&cfg, attr, rows_cluster<NT, B_MN>(tiles, (p.K + kRowsK - 1) / kRowsK), tiles);
+  if (e != cudaSuccess) return (int)e;
+  cfg.stream = stream;
+  return (int)cudaLaunchKernelEx(&cfg, gemm_rows_kernel<NT, B_MN>, tb, ta, p);
+}
+
+bool gemm_rows_takes(int M, int a_mn) {
+  return M <= 128 && !a_mn;
+}
+
+// Same contract as gemm_bf16_dispatch for the plain product with a K-major A of at most 128 rows.
+int gemm_rows_dispatch(const void* A, const void* B, void* C, const void* bias, int M, int N, int K, int lda, int ldb,
+                       int ldc, int b_mn, int out_f32, int bias_f32, int accumulate, float alpha, uint32_t* status,
+                       cudaStream_t stream) {
+  if (M <= 0 || N <= 0) return 0;
+  if (M > 128 || K <= 0 || (lda % 8) || (ldb % 8) || (reinterpret_cast<uintptr_t>(A) & 15) ||
+      (reinterpret_cast<uintptr_t>(B) & 15))
+    return -2;
+  const int nt = M <= 16 ? 16 : (M <= 32 ? 32 : (M <= 64 ? 64 : 128));
+  CUtensorMap tb, ta;
+  int r = !b_mn ? make_tmap_2d_bf16(&tb, B, K, N, ldb, 128) : make_tmap_2d_bf16(&tb, B, N, K, ldb, kRowsK);
+  if (r) return r;
+  if ((r = make_tmap_2d_bf16(&ta, A, K, M, lda, nt))) return r;
+  RowsParams p;
+  p.M = M; p.N = N; p.K = K; p.ldc = ldc;
+  p.C = C; p.bias = bias; p.bias_f32 = bias_f32; p.out_f32 = out_f32; p.accumulate = accumulate; p.alpha = alpha;
+  p.status = status; p.wait_ns = kDefaultWaitNs;
+#define TPB_ROWS_CASE(NT) \
+  if (nt == NT) return b_mn ? launch_rows<NT, true>(tb, ta, p, stream) : launch_rows<NT, false>(tb, ta, p, stream);
+  TPB_ROWS_CASE(16)
+  TPB_ROWS_CASE(32)
+  TPB_ROWS_CASE(64)
+  TPB_ROWS_CASE(128)
+#undef TPB_ROWS_CASE
+  return -3;
+}
+
+}  // namespace tpb

@@ -1,0 +1,42 @@
+"""Products with few rows: every tile width of the kernel, edges of its tiles and of its reduction split."""
+import pytest
+import torch
+
+import tensorplay_b200.ops as O
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def _check(M, N, K, a_mn, b_mn, out_dtype=torch.bfloat16, bias=None, accumulate=False, alpha=1.0, pad=0):
+    torch.manual_seed(M * 7 + N * 3 + K)
+    a = torch.randn((K, M + (-M) % 8 + pad) if a_mn else (M, K + pad), device=DEV).bfloat16()
+    b = torch.randn((K, N + (-N) % 8 + pad) if b_mn else (N, K + pad), device=DEV).bfloat16()
+    a, b = (a[:, :M] if a_mn else a[:, :K]), (b[:, :N] if b_mn else b[:, :K])
+    out = torch.randn(M, N, device=DEV).to(out_dtype)
+    ref = alpha * ((a.t() if a_mn else a).double() @ (b if b_mn else b.t()).double())
+    if bias is not None:
+        bias = torch.randn(N, device=DEV).to(bias)
+        ref = ref + bias.double()
+    if accumulate:
+        ref = ref + out.double()
+    O.gemm(a, b, a_mn=a_mn, b_mn=b_mn, out=out, bias=bias, accumulate=accumulate, alpha=alpha)
+    O.check_status()
+    # one rounding to the output, and the fp32 accumulator: K / 16 steps that each cut at most an ulp (2^-23) of a
+    # partial sum of K unit-variance products (below 2 sqrt(K) but for outliers)
+    tol = 2.0 ** -8 * ref.abs() * (out_dtype == torch.bfloat16) + (K / 16 + 1) * 2.0 ** -23 * 2 * K ** 0.5 + 1e-6
+    assert ((out.double() - ref).abs() <= tol).all()
+
+
+@pytest.mark.parametrize("b_mn", [False, True])
+@pytest.mark.parametrize("M", [1, 16, 17, 32, 33, 64, 65, 128])
+@pytest.mark.parametrize("N,K", [(8, 8), (136, 72), (1000, 512), (4096, 4104)])
+def test_few_rows(M, N, K, b_mn):
+    _check(M, N, K, False, b_mn, pad=8)
+
+
+@pytest.mark.parametrize("kw", [dict(out_dtype=torch.float32, bias=torch.float32, accumulate=True, alpha=0.5),
+                                dict(bias=torch.bfloat16, accumulate=True), dict(bias=torch.float32)])
+@pytest.mark.parametrize("M,N,K", [(5, 264, 2048), (100, 1036, 1024)])
+def test_few_rows_epilogue(M, N, K, kw):
+    _check(M, N, K, False, False, **kw)
