@@ -107,12 +107,13 @@ __device__ __forceinline__ void umma_pair_f16_ss(uint32_t d_tmem, uint32_t a_lo,
       "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-// All MMAs issued so far by this thread complete -> one arrival on `bar` in BOTH CTAs of the pair.
-__device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
+// All MMAs issued so far by this thread complete -> one arrival on `bar` in BOTH CTAs of the pair (`mask`: their
+// ranks in the cluster).
+__device__ __forceinline__ void umma_commit_pair(uint64_t* bar, uint16_t mask = 3) {
   asm volatile(
       "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(
           smem_u32(bar)),
-      "h"((uint16_t)3)
+      "h"(mask)
       : "memory");
 }
 
@@ -508,6 +509,331 @@ static int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const PairP
   if (pairs <= 0) return 0;
   cfg.gridDim = dim3(2 * pairs);
   return (int)cudaLaunchKernelEx(&cfg, kern, ta, tb, p);
+}
+
+// ------------------------------------------------------------------ few tiles, long reduction
+// The same pair pipeline for products with fewer tiles than CTA pairs and a long reduction (weight gradients): a
+// cluster of 2 c CTAs holds c pairs that share the k-blocks of ONE tile. Every CTA drains its 128 rows of the fp32
+// partial tile into its ring; after a cluster barrier the c CTAs that hold the same rows each sum a slice over the
+// others' shared memory, in pair order, and store it. No workspace, no flags, no second launch.
+// One-CTA tiles of 128 x 128 were what these products ran on: a k-block of such a tile brings 32 KB into an SM for 64
+// cycles x 4 of MMA, and at ~100 GB/s per SM the loads take 0.33 us of it: 85 us for 2304 x 768 x 16384.
+template <int BN>
+struct PairSplitCfg {
+  static constexpr int kLd = BN + 4;
+  static_assert(128 * kLd * 4 <= PairCfg<BN>::kStages * PairCfg<BN>::kStageBytes, "the partial tile must fit the ring");
+};
+
+__device__ __forceinline__ uint32_t cluster_nctas() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ float4 ld_cluster_f4(uint32_t saddr, uint32_t rank) {
+  float4 v;
+  asm volatile(
+      "{\n\t.reg .b32 ra;\n\t"
+      "mapa.shared::cluster.u32 ra, %4, %5;\n\t"
+      "ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [ra];\n\t}"
+      : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+      : "r"(saddr), "r"(rank)
+      : "memory");
+  return v;
+}
+
+template <int BN, bool A_MN, bool B_MN>
+__global__ void __launch_bounds__(kPairThreads, 1)
+gemm_pair_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+                       const PairParams p) {
+  using Cfg = PairCfg<BN>;
+  constexpr int S = Cfg::kStages, LD = PairSplitCfg<BN>::kLd;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + S * Cfg::kStageBytes);   // leader only
+  uint64_t* empty = full + S;
+  uint64_t* done = empty + S;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
+  volatile uint32_t* abort_w = tmem_slot + 1;
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rank = (int)cluster_ctarank(), csize = (int)cluster_nctas();
+  const int half = rank & 1, lead = rank & ~1, pair = rank >> 1, c = csize >> 1;
+  const int tiles_m = (p.M + kPairM - 1) / kPairM;
+  const int tile = blockIdx.x / csize;
+  const int tm = tile % tiles_m, tn = tile / tiles_m;
+  const int k_blocks = (p.K + kPairK - 1) / kPairK;
+  const int per = k_blocks / c, rem = k_blocks % c;
+  const int kb0 = pair * per + min(pair, rem), n_kb = per + (pair < rem ? 1 : 0);   // the host keeps c <= k_blocks
+  const uint16_t mask = (uint16_t)(3u << lead);
+
+  if (threadIdx.x == 0) {
+    *abort_w = 0;
+    for (int i = 0; i < S; ++i) {
+      mbar_init(&full[i], 1);
+      mbar_init(&empty[i], 1);
+    }
+    mbar_init(done, 1);
+    fence_barrier_init();
+    prefetch_tmap(&tmA);
+    prefetch_tmap(&tmB);
+  }
+  __syncthreads();
+  if (warp == 1) {
+    tmem_alloc_pair(tmem_slot, BN);
+    tmem_relinquish_pair();
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  cluster_sync_all();
+  tc_fence_after_sync();
+  const uint32_t tmem = *tmem_slot;
+  WaitCtx wc{abort_w, p.status, p.wait_ns};
+
+  if (warp == 0) {
+    if (lane == 0) {
+      const int row0 = tm * kPairM + half * 128, col0 = tn * BN + half * Cfg::kHalfN;
+      bool ok = true;
+      for (int it = 0; it < n_kb; ++it) {
+        const int s = it % S;
+        if (!mbar_wait_relaxed(&empty[s], ((it / S) & 1) ^ 1, wc, 1)) { ok = false; break; }
+        uint8_t* sa = smem + s * Cfg::kStageBytes;
+        uint8_t* sb = sa + kPairABytes;
+        const int k = (kb0 + it) * kPairK;
+        if (half == 0) mbar_arrive_expect_tx(&full[s], 2 * Cfg::kStageBytes);
+        const uint32_t fb = mapa_u32(&full[s], lead);
+        if (!A_MN) {
+          tma_load_2d_pair(sa, &tmA, fb, k, row0);
+        } else {
+#pragma unroll
+          for (int j = 0; j < 2; ++j) tma_load_2d_pair(sa + j * (kPairK * 128), &tmA, fb, row0 + j * 64, k);
+        }
+        if (!B_MN) {
+          tma_load_2d_pair(sb, &tmB, fb, k, col0);
+        } else {
+#pragma unroll
+          for (int j = 0; j < Cfg::kHalfN / 64; ++j)
+            tma_load_2d_pair(sb + j * (kPairK * 128), &tmB, fb, col0 + j * 64, k);
+        }
+      }
+      // the last commits of every slot arrive on this CTA's `empty` barriers, from the other SM for the peer
+      for (int it = n_kb; it < n_kb + S && ok; ++it) {
+        if (it < S) continue;   // this slot was never filled
+        ok = mbar_wait_relaxed(&empty[it % S], ((it / S) & 1) ^ 1, wc, 7);
+      }
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    if (half == 0) {
+      constexpr uint32_t idesc = make_idesc_f16(kPairM, BN, 1, A_MN ? 1 : 0, B_MN ? 1 : 0);
+      constexpr uint32_t hi = smem_desc_hi(1024);
+      const uint32_t a_lo0 = smem_desc_lo(smem_u32(smem), A_MN ? kPairK * 128 : 16);
+      const uint32_t b_lo0 = smem_desc_lo(smem_u32(smem + kPairABytes), B_MN ? kPairK * 128 : 16);
+      for (int it = 0; it < n_kb; ++it) {
+        const int s = it % S;
+        if (!mbar_wait_warp(&full[s], (it / S) & 1, wc, 4)) break;
+        tc_fence_after_sync();
+        const uint32_t a_lo = a_lo0 + s * (Cfg::kStageBytes >> 4), b_lo = b_lo0 + s * (Cfg::kStageBytes >> 4);
+        if (elect_one()) {
+#pragma unroll
+          for (int j = 0; j < kPairK / 16; ++j) {
+            const uint32_t ao = A_MN ? j * (2048 >> 4) : j * (32 >> 4);
+            const uint32_t bo = B_MN ? j * (2048 >> 4) : j * (32 >> 4);
+            umma_pair_f16_ss(tmem, a_lo + ao, hi, b_lo + bo, hi, idesc, (it | j) != 0);
+          }
+          umma_commit_pair(&empty[s], mask);
+          if (it == n_kb - 1) umma_commit_pair(done, mask);
+        }
+        __syncwarp();
+      }
+    }
+  } else {
+    const int q = warp & 3;
+    if (mbar_wait_warp(done, 0, wc, 6)) {
+      tc_fence_after_sync();
+      const uint32_t t_row = tmem + ((uint32_t)(q * 32) << 16);
+      float* dst = reinterpret_cast<float*>(smem) + (q * 32 + lane) * LD;
+#pragma unroll 1
+      for (int col = 0; col < BN; col += 32) {
+        uint32_t r[32];
+        tmem_ld_32x32b_x32(t_row + col, r);
+        tmem_ld_wait();
+#pragma unroll
+        for (int i = 0; i < 32; i += 4)
+          *reinterpret_cast<float4*>(dst + col + i) = make_float4(__uint_as_float(r[i]), __uint_as_float(r[i + 1]),
+                                                                  __uint_as_float(r[i + 2]), __uint_as_float(r[i + 3]));
+      }
+    }
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  if (*abort_w) {
+    // copies or MMAs of this pair may still be in flight: give them time before memory is read or goes away
+    const unsigned long long t0 = globaltimer_ns();
+    while (globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
+    __syncthreads();
+  }
+  cluster_sync_all();   // every partial tile is in shared memory, and the MMAs are done with the peers' operands
+  if (!*abort_w) {
+    const int row0 = tm * kPairM + half * 128;
+    const int rows = min(128, p.M - row0);
+    const uint32_t base = smem_u32(smem);
+    for (int u = pair * kPairThreads + (int)threadIdx.x; u < rows * (BN / 4); u += c * kPairThreads) {
+      const int r = u / (BN / 4), j4 = (u % (BN / 4)) * 4;
+      const int col = tn * BN + j4;
+      if (col >= p.N) continue;
+      const uint32_t at = base + (uint32_t)(r * LD + j4) * 4;
+      float4 t[4];
+#pragma unroll
+      for (int h = 0; h < 4; ++h) t[h] = h < c ? ld_cluster_f4(at, 2 * h + half) : make_float4(0.f, 0.f, 0.f, 0.f);
+      float v[4] = {t[0].x, t[0].y, t[0].z, t[0].w};
+#pragma unroll
+      for (int h = 1; h < 4; ++h) { v[0] += t[h].x; v[1] += t[h].y; v[2] += t[h].z; v[3] += t[h].w; }
+      const bool whole = col + 4 <= p.N;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        v[i] *= p.alpha;
+        if (p.bias && col + i < p.N)
+          v[i] += p.bias_f32 ? reinterpret_cast<const float*>(p.bias)[col + i]
+                             : __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(p.bias)[col + i]);
+      }
+      const size_t off = (size_t)(row0 + r) * p.ldc + col;
+      if (p.out_f32) {
+        float* o = reinterpret_cast<float*>(p.C) + off;
+        if (whole && (reinterpret_cast<uintptr_t>(o) & 15) == 0) {
+          float4 w = make_float4(v[0], v[1], v[2], v[3]);
+          if (p.accumulate) {
+            const float4 old = *reinterpret_cast<const float4*>(o);
+            w.x += old.x; w.y += old.y; w.z += old.z; w.w += old.w;
+          }
+          *reinterpret_cast<float4*>(o) = w;
+        } else {
+          for (int i = 0; i < 4 && col + i < p.N; ++i) o[i] = p.accumulate ? o[i] + v[i] : v[i];
+        }
+      } else {
+        __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(p.C) + off;
+        if (whole && (reinterpret_cast<uintptr_t>(o) & 7) == 0) {
+          if (p.accumulate) {
+            const uint2 old = *reinterpret_cast<const uint2*>(o);
+            const float2 f0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&old.x));
+            const float2 f1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&old.y));
+            v[0] += f0.x; v[1] += f0.y; v[2] += f1.x; v[3] += f1.y;
+          }
+          uint2 w;
+          *reinterpret_cast<__nv_bfloat162*>(&w.x) = __floats2bfloat162_rn(v[0], v[1]);
+          *reinterpret_cast<__nv_bfloat162*>(&w.y) = __floats2bfloat162_rn(v[2], v[3]);
+          *reinterpret_cast<uint2*>(o) = w;
+        } else {
+          for (int i = 0; i < 4 && col + i < p.N; ++i)
+            o[i] = __float2bfloat16(p.accumulate ? __bfloat162float(o[i]) + v[i] : v[i]);
+        }
+      }
+    }
+  }
+  cluster_sync_all();   // nobody leaves while a peer may read its tile
+  if (warp == 1) {
+    tc_fence_after_sync();
+    tmem_dealloc_pair(tmem, BN);
+  }
+}
+
+template <int BN, bool A_MN, bool B_MN>
+static cudaError_t pair_split_config(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attr, int c, unsigned tiles) {
+  static bool configured = false;
+  if (!configured) {
+    cudaError_t e = cudaFuncSetAttribute(gemm_pair_split_kernel<BN, A_MN, B_MN>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, PairCfg<BN>::kSmem);
+    if (e != cudaSuccess) return e;
+    configured = true;
+  }
+  attr->id = cudaLaunchAttributeClusterDimension;
+  attr->val.clusterDim.x = 2 * c;
+  attr->val.clusterDim.y = 1;
+  attr->val.clusterDim.z = 1;
+  cfg->gridDim = dim3(tiles * 2 * c);
+  cfg->blockDim = dim3(kPairThreads);
+  cfg->dynamicSmemBytes = PairCfg<BN>::kSmem;
+  cfg->attrs = attr;
+  cfg->numAttrs = 1;
+  return cudaSuccess;
+}
+// Clusters of c pairs that fit the device at once (asked of the runtime once per size; every form has the same
+// resources, so one stands for all).
+template <int BN>
+static int pair_split_resident(int c) {
+  static int resident[5] = {0};
+  if (resident[c] == 0) {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    int n = 0;
+    if (pair_split_config<BN, true, true>(&cfg, attr, c, sm_count()) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, gemm_pair_split_kernel<BN, true, true>, &cfg) != cudaSuccess || n <= 0)
+      n = -1;
+    resident[c] = n;
+  }
+  return resident[c];
+}
+
+template <int BN, bool A_MN, bool B_MN>
+static int launch_pair_split(const CUtensorMap& ta, const CUtensorMap& tb, const PairParams& p, int c, cudaStream_t stream) {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  const unsigned tiles = (unsigned)(((p.M + kPairM - 1) / kPairM) * ((p.N + BN - 1) / BN));
+  cudaError_t e = pair_split_config<BN, A_MN, B_MN>(&cfg, attr, c, tiles);
+  if (e != cudaSuccess) return (int)e;
+  cfg.stream = stream;
+  return (int)cudaLaunchKernelEx(&cfg, gemm_pair_split_kernel<BN, A_MN, B_MN>, ta, tb, p);
+}
+
+// Whether a product with fewer tiles than one wave of CTA pairs goes to the split form, and with which tile width and
+// how many pairs per tile. Estimated times in units of 10 ns, from measurements on one B200: a k-block takes 0.44 us in
+// a 256 x 256 pair tile and 0.28 us in a 256 x 128 one, 0.55 and 0.33 us in the one-CTA tiles of 128 x 256 and
+// 128 x 128; a launch costs about 5 us beside its k-blocks and the cluster reduction 3 us a round.
+bool gemm_pair_split_plan(int M, int N, int K, int* bn, int* c) {
+  if (M <= 128 || N <= 64 || K <= 0) return false;
+  const long long kb = (K + kPairK - 1) / kPairK, sms = sm_count();
+  const long long tm1 = (M + 127) / 128;
+  const long long t256 = tm1 * ((N + 255) / 256), t128 = tm1 * ((N + 127) / 128);
+  const long long single = (t256 * 2 > sms ? (t256 + sms - 1) / sms * kb * 55 : (t128 + sms - 1) / sms * kb * 33) + 500;
+  long long best = single * 9 / 10;
+  bool found = false;
+  for (int width = 256; width >= 128; width -= 128) {
+    const long long tiles = (long long)((M + kPairM - 1) / kPairM) * ((N + width - 1) / width);
+    for (int n = 1; n <= 4 && n <= kb; ++n) {
+      const int fit = width == 256 ? pair_split_resident<256>(n) : pair_split_resident<128>(n);
+      if (fit <= 0) continue;
+      const long long cost = (tiles + fit - 1) / fit * ((kb + n - 1) / n * (width == 256 ? 44 : 28) + 300) + 500;
+      if (cost < best) { best = cost; *bn = width; *c = n; found = true; }
+    }
+  }
+  return found;
+}
+
+int gemm_pair_split_dispatch(const void* A, const void* B, void* C, const void* bias, int M, int N, int K, int lda,
+                             int ldb, int ldc, int a_mn, int b_mn, int out_f32, int bias_f32, int accumulate,
+                             float alpha, uint32_t* status, cudaStream_t stream, int bn, int c) {
+  if (M <= 0 || N <= 0) return 0;
+  if (K <= 0 || (lda % 8) || (ldb % 8) || (reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15))
+    return -2;
+  CUtensorMap ta, tb;
+  int r = !a_mn ? make_tmap_2d_bf16(&ta, A, K, M, lda, 128) : make_tmap_2d_bf16(&ta, A, M, K, lda, kPairK);
+  if (r) return r;
+  r = !b_mn ? make_tmap_2d_bf16(&tb, B, K, N, ldb, bn / 2) : make_tmap_2d_bf16(&tb, B, N, K, ldb, kPairK);
+  if (r) return r;
+  PairParams p = {};
+  p.M = M; p.N = N; p.K = K; p.ldc = ldc; p.C = C; p.bias = bias; p.bias_f32 = bias_f32; p.out_f32 = out_f32;
+  p.accumulate = accumulate; p.alpha = alpha; p.status = status; p.wait_ns = kDefaultWaitNs;
+#define TPB_SPLIT_CASE(BN, AM, BM) \
+  if (bn == BN && (bool)a_mn == AM && (bool)b_mn == BM) return launch_pair_split<BN, AM, BM>(ta, tb, p, c, stream);
+  TPB_SPLIT_CASE(256, false, false)
+  TPB_SPLIT_CASE(256, false, true)
+  TPB_SPLIT_CASE(256, true, false)
+  TPB_SPLIT_CASE(256, true, true)
+  TPB_SPLIT_CASE(128, false, false)
+  TPB_SPLIT_CASE(128, false, true)
+  TPB_SPLIT_CASE(128, true, false)
+  TPB_SPLIT_CASE(128, true, true)
+#undef TPB_SPLIT_CASE
+  return -3;
 }
 
 // Same contract as gemm_bf16_dispatch for the plain product (no flags, no fused collective).

@@ -1061,6 +1061,10 @@ extern "C" int tpb_gemm_bf16(const void* A, const void* B, void* C, const void* 
   if (g_pair_min_tiles > 0 && (long long)((M + 255) / 256) * ((N + 255) / 256) >= g_pair_min_tiles)
     return tpb::gemm_pair_dispatch(A, B, C, bias, M, N, K, lda, ldb, ldc, a_mn, b_mn, out_f32, bias_f32,
                                    accumulate, alpha, 0, status, static_cast<cudaStream_t>(stream));
+  int bn, c;
+  if (g_pair_min_tiles > 0 && tpb::gemm_pair_split_plan(M, N, K, &bn, &c))
+    return tpb::gemm_pair_split_dispatch(A, B, C, bias, M, N, K, lda, ldb, ldc, a_mn, b_mn, out_f32, bias_f32, accumulate,
+                                         alpha, status, static_cast<cudaStream_t>(stream), bn, c);
   return tpb::gemm_bf16_dispatch(A, B, C, bias, M, N, K, lda, ldb, ldc, a_mn, b_mn, out_f32,
                                  bias_f32, accumulate, alpha, nullptr, 0, 0, 0, status,
                                  static_cast<cudaStream_t>(stream), nullptr);
