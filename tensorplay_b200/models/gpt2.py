@@ -71,9 +71,10 @@ class GPT2Block(nn.Module):
         B, T, d = x.shape
         H = cfg.n_heads
         h = ops.layer_norm(x, self.ln1_w, self.ln1_b, cfg.ln_eps)
-        qkv = ops.linear(h, self.w_qkv, self.b_qkv).view(B, T, 3, H, d // H)
-        a = ops.flash_attention(qkv[:, :, 0], qkv[:, :, 1], qkv[:, :, 2], causal=True)
-        x = x + ops.linear(a.reshape(B, T, d), self.w_o, self.b_o)
+        # one op over the packed projection: its backward writes dq, dk and dv into one buffer, where slices of the
+        # projection would each be padded to its size and added (four passes over it, 0.2 ms at 16 x 1024 x 768)
+        a = ops.qkv_attention(ops.linear(h, self.w_qkv, self.b_qkv), None, None, None, H, H, d // H, causal=True)
+        x = x + ops.linear(a, self.w_o, self.b_o)
         h = ops.layer_norm(x, self.ln2_w, self.ln2_b, cfg.ln_eps)
         h = ops.gelu(ops.linear(h, self.w_fc, self.b_fc), cfg.gelu_approximate)
         return x + ops.linear(h, self.w_proj, self.b_proj)

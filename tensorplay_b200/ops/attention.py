@@ -235,11 +235,10 @@ def flash_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, causal: b
 
 
 class _QKVAttnFn(torch.autograd.Function):
-    """RoPE + flash attention on a packed QKV projection ``[B, T, (Hq + 2 Hkv) * D]``.
+    """Flash attention on a packed QKV projection ``[B, T, (Hq + 2 Hkv) * D]``, with RoPE unless ``cos`` is None.
 
-    Forward rotates q and k out of the packed buffer into a fresh ``[B, T, Hq + Hkv, D]`` one with one launch
-    (no copy before the rotation) and
-    attends with v read in place from the packed buffer. Backward has the flash kernels
+    Without rotation q, k and v are all read in place. Forward rotates q and k out of the packed buffer into a fresh
+    ``[B, T, Hq + Hkv, D]`` one with one launch (no copy before the rotation) and attends with v read in place from the packed buffer. Backward has the flash kernels
     write dq, dk and dv straight into the slices of one packed gradient buffer and un-rotates
     its q/k part in place, so that no concatenation or copy is needed around the projection.
     """
@@ -250,43 +249,51 @@ class _QKVAttnFn(torch.autograd.Function):
         B, T, _ = qkv.shape
         tot = Hq + 2 * Hkv
         packed = qkv.view(B, T, tot, D)
-        qk = torch.empty((B, T, Hq + Hkv, D), device=qkv.device, dtype=qkv.dtype)
-        _rope_native_out(packed[:, :, : Hq + Hkv], qk, cos, sin, pos, interleaved, False)
-        q, k, v = qk[:, :, :Hq], qk[:, :, Hq:], packed[:, :, Hq + Hkv:]
+        if cos is None:
+            qk = packed
+        else:
+            qk = torch.empty((B, T, Hq + Hkv, D), device=qkv.device, dtype=qkv.dtype)
+            _rope_native_out(packed[:, :, : Hq + Hkv], qk, cos, sin, pos, interleaved, False)
+        q, k, v = qk[:, :, :Hq], qk[:, :, Hq:Hq + Hkv], packed[:, :, Hq + Hkv:]
         kept = _ckpt.take()  # selective checkpointing: output and LSE of the first forward pass
         if kept is not None:
             o, lse = kept
         else:
             o, lse = flash_fwd(q, k, v, causal, scale)
             _ckpt.stash(o, lse)
-        ctx.save_for_backward(qk, qkv, o, lse, cos, sin, pos if pos is not None else torch.empty(0))
+        rot = (None, None, None, None) if cos is None else (qk, cos, sin, pos if pos is not None else torch.empty(0))
+        ctx.save_for_backward(qkv, o, lse, *rot)
         ctx.cfg = (Hq, Hkv, D, causal, scale, interleaved, pos is not None)
         return o.view(B, T, Hq * D)
 
     @staticmethod
     def backward(ctx, do):
         from .rope import _rope_native_
-        qk, qkv, o, lse, cos, sin, pos = ctx.saved_tensors
+        qkv, o, lse, qk, cos, sin, pos = ctx.saved_tensors
         Hq, Hkv, D, causal, scale, interleaved, has_pos = ctx.cfg
         B, T, _ = qkv.shape
         tot = Hq + 2 * Hkv
         packed = qkv.view(B, T, tot, D)
+        if qk is None:
+            qk = packed
         dqkv = torch.empty_like(qkv)
         dp = dqkv.view(B, T, tot, D)
         do4 = do.reshape(B, T, Hq, D)
         if not _strides_ok(do4):
             do4 = do4.contiguous()
-        flash_bwd(do4, qk[:, :, :Hq], qk[:, :, Hq:], packed[:, :, Hq + Hkv:], o, lse, causal, scale,
+        flash_bwd(do4, qk[:, :, :Hq], qk[:, :, Hq:Hq + Hkv], packed[:, :, Hq + Hkv:], o, lse, causal, scale,
                   dq=dp[:, :, :Hq], dk=dp[:, :, Hq:Hq + Hkv], dv=dp[:, :, Hq + Hkv:])
-        _rope_native_(dp[:, :, : Hq + Hkv], cos, sin, pos if has_pos else None, interleaved, True)
+        if cos is not None:
+            _rope_native_(dp[:, :, : Hq + Hkv], cos, sin, pos if has_pos else None, interleaved, True)
         return dqkv, None, None, None, None, None, None, None, None, None
 
 
-def qkv_attention(qkv: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor,
+def qkv_attention(qkv: torch.Tensor, cos: Optional[torch.Tensor], sin: Optional[torch.Tensor],
                   position_ids: Optional[torch.Tensor], num_heads: int, num_kv_heads: int,
                   head_dim: int, causal: bool = True, scale: Optional[float] = None,
                   interleaved: bool = False) -> torch.Tensor:
-    """Attention over a packed QKV projection; returns ``[B, T, num_heads * head_dim]``."""
+    """Attention over a packed QKV projection; returns ``[B, T, num_heads * head_dim]``. ``cos`` / ``sin`` None: no
+    rotation (absolute positions)."""
     scale = scale if scale is not None else 1.0 / math.sqrt(head_dim)
     B, T, _ = qkv.shape
     native = (qkv.is_cuda and qkv.dtype == torch.bfloat16 and head_dim in (64, 128)
@@ -299,6 +306,10 @@ def qkv_attention(qkv: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor,
                                 interleaved)
     from .rope import _rope_ref
     packed = qkv.view(B, T, num_heads + 2 * num_kv_heads, head_dim)
+    if cos is None:
+        o = flash_attention(packed[:, :, :num_heads], packed[:, :, num_heads:num_heads + num_kv_heads],
+                            packed[:, :, num_heads + num_kv_heads:], causal, scale)
+        return o.reshape(B, T, num_heads * head_dim)
     qk = _rope_ref(packed[:, :, : num_heads + num_kv_heads], cos, sin, position_ids, interleaved, 1.0)
     o = attention_reference(qk[:, :, :num_heads], qk[:, :, num_heads:],
                             packed[:, :, num_heads + num_kv_heads:], causal, scale)
