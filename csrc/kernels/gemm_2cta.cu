@@ -32,7 +32,9 @@ struct PairCfg {
   static constexpr int kBBytes = kHalfN * kPairK * 2;
   static constexpr int kStageBytes = kPairABytes + kBBytes;
   static constexpr int kStages = BN == 256 ? 6 : 8;
-  static constexpr int kSmem = kStages * kStageBytes + 1024 + 512;
+  // staging of the bf16 epilogue: per warp 32 rows of 64 columns, padded to 144 bytes (conflict-free both ways)
+  static constexpr int kOutOff = kStages * kStageBytes + 512;
+  static constexpr int kSmem = kOutOff + 4 * 32 * 144 + 1024;
 };
 constexpr int kPairGroupM = 8;
 
@@ -314,7 +316,12 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     }
   } else {
     // ------------------------------------------------------------ epilogue (4 warps per CTA, own 128 rows)
+    // A lane holds 32 columns of one row. Stored from there, an instruction touches 32 rows by 16 bytes and takes 32
+    // passes of the load/store unit: 4096 of the ~6000 cycles that the MMAs of a tile take at K = 768. Plain bf16
+    // results therefore go through shared memory and leave as 4 rows by 128 contiguous bytes.
     const int q = warp & 3;
+    uint8_t* out_stage = smem + Cfg::kOutOff + q * (32 * 144);
+    const bool staged = !p.out_f32 && !p.accumulate && p.ldc % 8 == 0 && (reinterpret_cast<uintptr_t>(p.C) & 15) == 0;
     uint32_t lt = 0;
     for (int wi = 0; pair_work(sc, pair, wi, w); ++wi, ++lt) {
       int tm, tn;
@@ -368,8 +375,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         Bias32 bias;
         const bool bias_vec = bias32_vec_ok(p.bias, p.bias_f32, col0, p.N);
         if (bias_vec) bias32_load(bias, p.bias, col0);
+        const bool stage_it = staged && (c & ~32) + tn * kPairN + 64 <= p.N;   // warp-uniform, both halves of 64 columns
         tmem_ld_wait();
-        if (row < p.M) {
+        if (row < p.M || stage_it) {
           float v[32];
 #pragma unroll
           for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
@@ -388,7 +396,17 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           const bool full_chunk = (col0 + 32 <= p.N);
           if (bias_vec) bias32_add(v, bias);
           else if (p.bias) bias32_add_any(v, p.bias, p.bias_f32, col0, p.N);
-          if (p.out_f32) {
+          if (stage_it) {
+            uint8_t* srow = out_stage + lane * 144 + (c & 32) * 2;
+#pragma unroll
+            for (int i = 0; i < 32; i += 8) {
+              uint4 o;
+              __nv_bfloat162* ob2 = reinterpret_cast<__nv_bfloat162*>(&o);
+#pragma unroll
+              for (int j = 0; j < 4; ++j) ob2[j] = __floats2bfloat162_rn(v[i + 2 * j], v[i + 2 * j + 1]);
+              *reinterpret_cast<uint4*>(srow + i * 2) = o;
+            }
+          } else if (p.out_f32) {
             float* crow = reinterpret_cast<float*>(p.C) + (size_t)row * p.ldc + col0;
             if (full_chunk && ((reinterpret_cast<uintptr_t>(crow) & 15) == 0)) {
 #pragma unroll
@@ -433,6 +451,17 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                 }
             }
           }
+        }
+        if (stage_it && (c & 32)) {
+          __syncwarp();
+          const int row8 = tm * kPairM + (int)crank * 128 + q * 32 + (lane >> 3);
+          __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(p.C) + (size_t)row8 * p.ldc + (col0 - 32) + (lane & 7) * 8;
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const uint4 val = *reinterpret_cast<const uint4*>(out_stage + (i * 4 + (lane >> 3)) * 144 + (lane & 7) * 16);
+            if (row8 + i * 4 < p.M) *reinterpret_cast<uint4*>(dst + (size_t)(i * 4) * p.ldc) = val;
+          }
+          __syncwarp();
         }
       }
       tc_fence_before_sync();

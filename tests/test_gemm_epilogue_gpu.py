@@ -25,6 +25,25 @@ def test_bias_columns(impl, dtype, M, N, shift):
     assert (y.double() - ref).abs().max().item() < 64 * 2.0 ** -22
 
 
+@pytest.mark.parametrize("M,N", [(256, 256), (130, 264), (513, 64), (129, 40), (300, 328)])
+@pytest.mark.parametrize("pad,shift", [(0, 0), (8, 8), (8, 4), (3, 0)])
+def test_bf16_stores(M, N, pad, shift):
+    """Rows that leave as whole lines and those that cannot (last columns, unaligned output), and nothing beside them."""
+    torch.manual_seed(M + N)
+    a = torch.randn(M, 192, device=DEV, dtype=torch.bfloat16)
+    b = torch.randn(N, 192, device=DEV, dtype=torch.bfloat16)
+    bias = torch.randn(N, device=DEV, dtype=torch.bfloat16)
+    ref = (a.double() @ b.double().t() + bias.double())
+    buf = torch.full((M + 2, N + pad + shift), 7.0, device=DEV, dtype=torch.bfloat16)
+    out = buf[:M, shift:shift + N]
+    O.gemm(a, b, bias=bias, out=out, impl="pair")
+    O.check_status()
+    assert ((out.double() - ref).abs() <= ref.abs() * 2.0 ** -8 + 192 * 2.0 ** -20).all()
+    rest = buf.clone()
+    rest[:M, shift:shift + N] = 7.0
+    assert (rest == 7.0).all()
+
+
 @pytest.mark.parametrize("rows,N", [(1, 8), (7, 264), (33, 768), (4096, 40), (16384, 2304)])
 def test_bias_gradient(rows, N):
     torch.manual_seed(rows)
