@@ -65,7 +65,9 @@ struct KvAppendParams {
   long long d_b, d_t, d_h;        // destination strides: batch (or block), token, head
 };
 
-__global__ void __launch_bounds__(256) kv_append_kernel(const KvAppendParams p) {
+// blockIdx.y selects one of two appends (keys and values of a step in one launch).
+__global__ void __launch_bounds__(256) kv_append_kernel(const KvAppendParams p0, const KvAppendParams p1) {
+  const KvAppendParams& p = blockIdx.y ? p1 : p0;
   const int vec = p.D / 8;
   const long long total = (long long)p.B * p.T * p.H * vec;
   for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < total; i += (long long)gridDim.x * 256) {
@@ -365,11 +367,9 @@ int tpb_embedding_bwd(const long long* ids, const void* dy, void* dw, long long 
   return (int)cudaGetLastError();
 }
 
-int tpb_kv_append(const void* src, void* dst, const int* pos, const int* block_table, int pos0,
-                  int B, int T, int H, int D, int block, int max_blocks, long long s_b,
-                  long long s_t, long long s_h, long long d_b, long long d_t, long long d_h,
-                  void* stream) {
-  if (B <= 0 || T <= 0) return 0;
+static int kv_append_params(KvAppendParams* out, const void* src, void* dst, const int* pos, const int* block_table,
+                            int pos0, int B, int T, int H, int D, int block, int max_blocks, long long s_b,
+                            long long s_t, long long s_h, long long d_b, long long d_t, long long d_h) {
   if (D <= 0 || (D & 7) || ((s_b | s_t | s_h | d_b | d_t | d_h) & 7)) return -1;
   if (block_table && (block <= 0 || max_blocks <= 0)) return -2;
   KvAppendParams p;
@@ -377,10 +377,39 @@ int tpb_kv_append(const void* src, void* dst, const int* pos, const int* block_t
   p.block_table = block_table; p.pos0 = pos0; p.B = B; p.T = T; p.H = H; p.D = D;
   p.block = block; p.max_blocks = max_blocks;
   p.s_b = s_b; p.s_t = s_t; p.s_h = s_h; p.d_b = d_b; p.d_t = d_t; p.d_h = d_h;
-  const long long total = (long long)B * T * H * (D / 8);
+  *out = p;
+  return 0;
+}
+static int kv_append_launch(const KvAppendParams& a, const KvAppendParams& b, int n, void* stream) {
+  const long long total = (long long)a.B * a.T * a.H * (a.D / 8);
   const int grid = (int)((total + 255) / 256 < 148 * 16 ? (total + 255) / 256 : 148 * 16);
-  kv_append_kernel<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(p);
+  kv_append_kernel<<<dim3(grid, n), 256, 0, static_cast<cudaStream_t>(stream)>>>(a, b);
   return (int)cudaGetLastError();
+}
+
+// Keys and values of the same shape into contiguous caches of the same strides at token pos0, in one launch.
+int tpb_kv_append2(const void* k, const void* v, void* k_cache, void* v_cache, int pos0, int B, int T, int H, int D,
+                   long long k_b, long long k_t, long long k_h, long long v_b, long long v_t, long long v_h,
+                   long long c_b, long long c_t, long long c_h, void* stream) {
+  if (B <= 0 || T <= 0) return 0;
+  if ((reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v) | reinterpret_cast<uintptr_t>(k_cache) |
+       reinterpret_cast<uintptr_t>(v_cache)) & 15)
+    return -1;
+  KvAppendParams pk, pv;
+  int r = kv_append_params(&pk, k, k_cache, nullptr, nullptr, pos0, B, T, H, D, 0, 0, k_b, k_t, k_h, c_b, c_t, c_h);
+  if (!r) r = kv_append_params(&pv, v, v_cache, nullptr, nullptr, pos0, B, T, H, D, 0, 0, v_b, v_t, v_h, c_b, c_t, c_h);
+  return r ? r : kv_append_launch(pk, pv, 2, stream);
+}
+
+int tpb_kv_append(const void* src, void* dst, const int* pos, const int* block_table, int pos0,
+                  int B, int T, int H, int D, int block, int max_blocks, long long s_b,
+                  long long s_t, long long s_h, long long d_b, long long d_t, long long d_h,
+                  void* stream) {
+  if (B <= 0 || T <= 0) return 0;
+  KvAppendParams p;
+  const int r = kv_append_params(&p, src, dst, pos, block_table, pos0, B, T, H, D, block, max_blocks, s_b, s_t, s_h, d_b,
+                                 d_t, d_h);
+  return r ? r : kv_append_launch(p, p, 1, stream);
 }
 
 // qkv [B, Hq + 2 Hkv, D] (batch stride qkv_b); q_out [B, Hq, D] contiguous; caches addressed as

@@ -96,6 +96,12 @@ int tpb_layernorm_bwd(const void* dy, const void* x, const void* w, const float*
                       const float* rstd, void* dx, float* dw_part, float* db_part, float* dw_f32,
                       void* dw_bf16, float* db_f32, void* db_bf16, int accumulate, int rows, int H,
                       void* stream);
+int tpb_block_pre(const void* x, const void* norm_w, float eps, const void* w_qkv, void* h, void* qkv, void* qk,
+                  const float* cos_t, const float* sin_t, const long long* pos, long long pos0, int rows, int T,
+                  int hidden, int Hq, int Hkv, int D, uint32_t* status, void* stream);
+int tpb_block_post(const void* attn, const void* w_o, void* o, const void* x, const void* norm_w, float eps, void* x2,
+                   void* h, const void* w_gu, void* gu, void* act, const void* w_down, void* y, int accumulate,
+                   int rows, int hidden, int attn_width, int inter, uint32_t* status, void* stream);
 int tpb_flash_decode_splits(int B, int Tq, int Tk, int Hq, int Hkv);
 int tpb_flash_decode(const void* q, const void* k, const void* v, void* o, float* lse, float* part_o, float* part_lse,
                      int B, int Tq, int Tk, int Hq, int Hkv, int D, long long q_tok, long long q_head,

@@ -87,6 +87,9 @@ _KERNEL_SIGS = {
     "tpb_nms": [P, P, I, F, P, P, P, P],
     "tpb_roi_align_fwd": [P, P, P, I, I, I, I, I, I, I, I, F, I, I, P],
     "tpb_roi_align_bwd": [P, P, P, I, I, I, I, I, I, I, I, F, I, I, P],
+    "tpb_kv_append2": [P, P, P, P, I, I, I, I, I, LL, LL, LL, LL, LL, LL, LL, LL, LL, P],
+    "tpb_block_pre": [P, P, F, P, P, P, P, P, P, P, LL, I, I, I, I, I, I, P, P],
+    "tpb_block_post": [P, P, P, P, P, F, P, P, P, P, P, P, P, I, I, I, I, I, P, P],
     "tpb_decode_qkv_prep": [P, P, P, P, P, P, P, I, I, I, I, I, I, LL, LL, LL, LL, P],
     "tpb_sample": [P, P, P, P, I, I, LL, I, F, I, F, P],
 }
@@ -113,7 +116,7 @@ def _load(name: str):
 
 
 # kernel launches issued by one call of each entry point (for launch accounting)
-_LAUNCHES = {"tpb_rmsnorm_bwd": 2, "tpb_layernorm_bwd": 2, "tpb_bias_grad": 2, "tpb_bias_grad_chunks": 0, "tpb_flash_decode_splits": 0, "tpb_flash_bwd": 3, "tpb_rmsnorm_bwd_grid": 0,
+_LAUNCHES = {"tpb_rmsnorm_bwd": 2, "tpb_layernorm_bwd": 2, "tpb_bias_grad": 2, "tpb_bias_grad_chunks": 0, "tpb_flash_decode_splits": 0, "tpb_block_pre": 3, "tpb_block_post": 5, "tpb_flash_bwd": 3, "tpb_rmsnorm_bwd_grid": 0,
              "tpb_grouped_workspace_ints": 0, "tpb_adamw_set_overlap": 0, "tpb_flash_fwd_config": 0, "tpb_gemm_set_splitk_workspace": 0, "tpb_grouped_gemm": 2}
 launch_count = 0
 
@@ -147,6 +150,7 @@ class _Counting:
                 return _raw(*a)
 
             self._cache[name] = fn
+            setattr(self, name, fn)   # the next look-up does not come through here
         return fn
 
 

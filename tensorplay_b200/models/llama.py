@@ -15,7 +15,9 @@ from typing import Optional
 import torch
 from torch import Tensor, nn
 
-from .. import ops
+from .. import _native, ops
+from ..ops import _ckpt
+from ..ops._common import lib, status_word, stream_ptr, use_native
 
 
 @dataclass
@@ -88,6 +90,8 @@ class LlamaBlock(nn.Module):
     def forward(self, x: Tensor, cos: Tensor, sin: Tensor, position_ids: Optional[Tensor] = None,
                 past_key_values=None) -> Tensor:
         cfg = self.cfg
+        if past_key_values is not None and self._plain_inference(x, cos, sin):
+            return self._infer_cached(x, cos, sin, position_ids, past_key_values)
         h = ops.rms_norm(x, self.attn_norm, cfg.rms_eps)
         qkv = ops.linear(h, self.wqkv)
         if past_key_values is None:
@@ -99,6 +103,62 @@ class LlamaBlock(nn.Module):
         h, x = ops.rms_norm(a, self.ffn_norm, cfg.rms_eps, residual=x)
         gu = ops.linear(h, self.w_gate_up)
         return x + ops.linear(ops.swiglu_packed(gu), self.w_down)
+
+    def _plain_inference(self, x: Tensor, cos: Tensor, sin: Tensor) -> bool:
+        """Whether a forward pass with a cache may go to the native halves of the block: plain CUDA bf16 tensors, no
+        gradient, and nothing that watches or transforms single operators."""
+        if torch.is_grad_enabled() or type(x) is not Tensor or not x.is_cuda or x.dtype != torch.bfloat16 \
+                or not x.is_contiguous() or x.data_ptr() % 16 or x.numel() == 0 or self.cfg.head_dim not in (64, 128):
+            return False
+        if _native.flop_sinks or _ckpt.active() or torch._C._are_functorch_transforms_active() \
+                or torch._C._len_torch_dispatch_stack() or torch._C._is_torch_function_mode_enabled() \
+                or torch.autograd.forward_ad._current_level >= 0 or torch.jit.is_tracing():
+            return False
+        dev = x.device
+        for w in (self.attn_norm, self.wqkv, self.wo, self.ffn_norm, self.w_gate_up, self.w_down):
+            if type(w) is not nn.Parameter or w.dtype != torch.bfloat16 or w.device != dev or not w.is_contiguous() \
+                    or w.data_ptr() % 16 or w.shape[-1] % 8:
+                return False
+        for t in (cos, sin):
+            if type(t) is not Tensor or t.dtype != torch.float32 or t.device != dev or not t.is_contiguous() \
+                    or t.data_ptr() % 16:
+                return False
+        return dev.index == torch._C._cuda_getDevice() and use_native(x)
+
+    def _infer_cached(self, x: Tensor, cos: Tensor, sin: Tensor, position_ids: Optional[Tensor], cache) -> Tensor:
+        """The block as two native calls around the cache and the attention. Of at most 128 rows the last product is
+        accumulated into the residual stream."""
+        cfg = self.cfg
+        B, T, H = x.shape
+        Hq, Hkv, D, I = cfg.num_heads, cfg.num_kv_heads, cfg.head_dim, cfg.ffn_size
+        off = cache.get_seq_length(self.layer_idx)
+        pos = None
+        if position_ids is not None:
+            pos = position_ids.reshape(-1).to(torch.int64).contiguous()
+        elif off + T > cos.shape[0]:
+            raise IndexError(f"rotary tables of {cos.shape[0]} positions are too short for position {off + T - 1}")
+        rows, tot, L = B * T, Hq + 2 * Hkv, lib()
+        st, stream = status_word(x.device).data_ptr(), stream_ptr()
+        qkv, qk = x.new_empty(B, T, tot, D), x.new_empty(B, T, Hq + Hkv, D)
+        scratch = x.new_empty(rows * (2 * H + 3 * I))
+        h = scratch.data_ptr()
+        o, gu = h + 2 * rows * H, h + 4 * rows * H
+        act = gu + 4 * rows * I
+        _native.check(L.tpb_block_pre(
+            x.data_ptr(), self.attn_norm.data_ptr(), cfg.rms_eps, self.wqkv.data_ptr(), h, qkv.data_ptr(), qk.data_ptr(),
+            cos.data_ptr(), sin.data_ptr(), None if pos is None else pos.data_ptr(), off, rows, T, H, Hq, Hkv, D, st,
+            stream), "tpb_block_pre")
+        k, v = cache.update(qk[:, :, Hq:].transpose(1, 2), qkv[:, :, Hq + Hkv:].transpose(1, 2), self.layer_idx)
+        a = ops.flash_attention(qk[:, :, :Hq], k.transpose(1, 2), v.transpose(1, 2), causal=True)
+        if not a.is_contiguous():
+            a = a.contiguous()
+        x2 = torch.empty_like(x)
+        y = x2 if rows <= 128 else torch.empty_like(x)
+        _native.check(L.tpb_block_post(
+            a.data_ptr(), self.wo.data_ptr(), o, x.data_ptr(), self.ffn_norm.data_ptr(), cfg.rms_eps, x2.data_ptr(), h,
+            self.w_gate_up.data_ptr(), gu, act, self.w_down.data_ptr(), y.data_ptr(), int(y is x2), rows, H, Hq * D, I, st,
+            stream), "tpb_block_post")
+        return x2 if y is x2 else x2 + y
 
     def _attend_cached(self, qkv, cos, sin, position_ids, cache):
         cfg = self.cfg

@@ -10,6 +10,8 @@ from typing import Dict, List, Optional, Tuple
 import torch
 from torch import Tensor
 
+from ..ops.decode import kv_append_pair
+
 
 class Cache:
     def update(self, key: Tensor, value: Tensor, layer_idx: int = 0) -> Tuple[Tensor, Tensor]:
@@ -40,9 +42,7 @@ class DynamicCache(Cache):
                 nv[:, :, :n] = self._v[layer_idx][:, :, :n]
             self._k[layer_idx], self._v[layer_idx] = nk, nv
         if key.is_cuda and key.dtype == torch.bfloat16:
-            from ..ops import kv_append
-            kv_append(self._k[layer_idx], key, n)
-            kv_append(self._v[layer_idx], value, n)
+            kv_append_pair(self._k[layer_idx], self._v[layer_idx], key, value, n)
         else:
             self._k[layer_idx][:, :, n:n + t] = key
             self._v[layer_idx][:, :, n:n + t] = value
@@ -72,9 +72,7 @@ class StaticCache(Cache):
             self._k[layer_idx] = key.new_zeros(shape)
             self._v[layer_idx] = value.new_zeros(shape)
         if key.is_cuda and key.dtype == torch.bfloat16:
-            from ..ops import kv_append
-            kv_append(self._k[layer_idx], key, n)
-            kv_append(self._v[layer_idx], value, n)
+            kv_append_pair(self._k[layer_idx], self._v[layer_idx], key, value, n)
         else:
             self._k[layer_idx][:, :, n:n + t] = key
             self._v[layer_idx][:, :, n:n + t] = value

@@ -12,8 +12,11 @@ def use_native(*tensors: torch.Tensor) -> bool:
     A CUDA tensor never falls back to PyTorch: if the kernel library cannot be loaded the
     call raises, so that a silent library fallback cannot pass for the native path.
     """
-    if not tensors or not all(t is None or t.is_cuda for t in tensors):
+    if not tensors:
         return False
+    for t in tensors:
+        if t is not None and not t.is_cuda:
+            return False
     _native.kernels()  # raises NativeUnavailable with a clear message
     return True
 
@@ -23,7 +26,9 @@ def lib():
 
 
 def stream_ptr() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    """Handle of the current stream of the current device (without building a ``torch.cuda.Stream``: 0.3 instead of
+    2.5 us, paid by every launch)."""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def ptr(t):

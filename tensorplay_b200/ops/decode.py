@@ -105,6 +105,23 @@ def kv_append(cache: Tensor, new: Tensor, pos, block_table: Optional[Tensor] = N
     return cache
 
 
+def kv_append_pair(k_cache: Tensor, v_cache: Tensor, k: Tensor, v: Tensor, pos: int) -> None:
+    """``kv_append`` of keys and values ``[B, H, T, D]`` at token ``pos`` of two contiguous-layout caches, in one launch
+    where shapes and strides allow."""
+    ks, vs, cs = k.stride(), v.stride(), k_cache.stride()
+    if (k.shape == v.shape and cs == v_cache.stride() and k.dtype == v.dtype == k_cache.dtype == v_cache.dtype == torch.bfloat16
+            and ks[3] == vs[3] == cs[3] == 1 and not k.shape[3] % 8
+            and not (ks[0] | ks[1] | ks[2] | vs[0] | vs[1] | vs[2] | cs[0] | cs[1] | cs[2]) % 8
+            and not (k.data_ptr() | v.data_ptr() | k_cache.data_ptr() | v_cache.data_ptr()) % 16 and use_native(k, v, k_cache)):
+        B, H, T, D = k.shape
+        _native.check(lib().tpb_kv_append2(
+            k.data_ptr(), v.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), int(pos), B, T, H, D, ks[0], ks[2], ks[1],
+            vs[0], vs[2], vs[1], cs[0], cs[2], cs[1], stream_ptr()), "tpb_kv_append2")
+        return
+    kv_append(k_cache, k, pos)
+    kv_append(v_cache, v, pos)
+
+
 def decode_qkv_prep(qkv: Tensor, cos: Tensor, sin: Tensor, pos: Tensor, num_heads: int, num_kv_heads: int,
                     k_cache: Tensor, v_cache: Tensor) -> Tensor:
     """One decode step's QKV projection ``[B, Hq + 2 Hkv, D]`` -> rotated queries ``[B, Hq, D]``; the rotated keys
