@@ -574,20 +574,20 @@ __global__ void swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ dy,
   reinterpret_cast<uint4*>(dup + r * out_stride)[v] = pack8(du);
 }
 
-// GELU; approx = 1 selects the tanh form.
+// GELU; approx = 1 selects the tanh form, evaluated as x * sigmoid(2u) with u = sqrt(2/pi) (x + 0.044715 x^3): the
+// same function as 0.5 x (1 + tanh u), without the cancellation of 1 + tanh for negative u, and one exponential and one
+// division where tanhf takes some thirty instructions. The pass was bound by those: 54 us forward and 68 us backward at
+// 16384 x 3072 against 30 and 45 us of memory time.
+__device__ __forceinline__ float sigmoid_2u(float u) { return __fdividef(1.f, 1.f + __expf(-2.f * u)); }
 __device__ __forceinline__ float gelu_f(float x, int approx) {
-  if (approx) {
-    float t = tanhf(0.7978845608028654f * (x + 0.044715f * x * x * x));
-    return 0.5f * x * (1.f + t);
-  }
+  if (approx) return x * sigmoid_2u(0.7978845608028654f * (x + 0.044715f * x * x * x));
   return 0.5f * x * (1.f + erff(x * 0.7071067811865476f));
 }
 __device__ __forceinline__ float gelu_grad_f(float x, int approx) {
   if (approx) {
-    float u = 0.7978845608028654f * (x + 0.044715f * x * x * x);
-    float t = tanhf(u);
-    float du = 0.7978845608028654f * (1.f + 3.f * 0.044715f * x * x);
-    return 0.5f * (1.f + t) + 0.5f * x * (1.f - t * t) * du;
+    const float s = sigmoid_2u(0.7978845608028654f * (x + 0.044715f * x * x * x));
+    const float du2 = 2.f * 0.7978845608028654f * (1.f + 3.f * 0.044715f * x * x);
+    return s + x * (s * (1.f - s)) * du2;
   }
   float cdf = 0.5f * (1.f + erff(x * 0.7071067811865476f));
   float pdf = 0.3989422804014327f * __expf(-0.5f * x * x);
