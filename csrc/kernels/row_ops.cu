@@ -75,6 +75,35 @@ __device__ __forceinline__ float row_max(float v, float* scratch) {
   return v;
 }
 
+// One partial row per CTA from the column sums of its RPB row groups: [sub][H] through shared memory, added in order.
+template <int TPR, int VPT>
+__device__ __forceinline__ void fold_row_groups(const float (&acc)[VPT][8], float* __restrict__ out, int H, float* sm) {
+  constexpr int RPB = kRowThreads / TPR;
+  const int t = threadIdx.x % TPR, sub = threadIdx.x / TPR, nvec = H / 8;
+#pragma unroll
+  for (int i = 0; i < VPT; ++i) {
+    const int v = t + i * TPR;
+    if (v < nvec) {
+      float4* d = reinterpret_cast<float4*>((RPB == 1 ? out : sm + sub * H) + v * 8);
+      d[0] = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+      d[1] = make_float4(acc[i][4], acc[i][5], acc[i][6], acc[i][7]);
+    }
+  }
+  if constexpr (RPB > 1) {
+    __syncthreads();
+    for (int c = threadIdx.x; c < H; c += kRowThreads) {
+      float s = 0.f;
+#pragma unroll
+      for (int r = 0; r < RPB; ++r) s += sm[r * H + c];
+      out[c] = s;
+    }
+    __syncthreads();
+  }
+}
+// Floats of shared memory that fold_row_groups needs: RPB groups of at most TPR * VPT vectors of 8.
+template <int TPR, int VPT>
+constexpr int fold_floats() { return TPR == kRowThreads ? 4 : kRowThreads * VPT * 8; }
+
 // ------------------------------------------------------------------ RMSNorm forward
 // y = (x [+ res]) * rstd * w ; optionally writes the summed residual stream back (res_out).
 template <int TPR, int VPT>
@@ -197,36 +226,8 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __
       }
     }
   }
-  // Fold the RPB sub-rows of this CTA, then write one partial row per CTA.
-  float* out = dw_part + (size_t)blockIdx.x * H;
-  if constexpr (RPB == 1) {
-#pragma unroll
-    for (int i = 0; i < VPT; ++i) {
-      int v = t + i * TPR;
-      if (v < nvec) {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) out[v * 8 + j] = dwacc[i][j];
-      }
-    }
-  } else {
-    // Several rows per CTA (small H): serialise the sub-row groups through global memory adds.
-    for (int s = 0; s < RPB; ++s) {
-      if (sub == s) {
-#pragma unroll
-        for (int i = 0; i < VPT; ++i) {
-          int v = t + i * TPR;
-          if (v < nvec) {
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-              if (s == 0) out[v * 8 + j] = dwacc[i][j];
-              else out[v * 8 + j] += dwacc[i][j];
-            }
-          }
-        }
-      }
-      __syncthreads();
-    }
-  }
+  __shared__ __align__(16) float fold[fold_floats<TPR, VPT>()];
+  fold_row_groups<TPR, VPT>(dwacc, dw_part + (size_t)blockIdx.x * H, H, fold);
 }
 
 // out[c] = sum_r part[r, c] for one or two (blockIdx.y) fp32 matrices [nrows, H] that a kernel before left as
@@ -390,7 +391,6 @@ layernorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* 
                      float* __restrict__ dw_part, float* __restrict__ db_part, int rows, int H) {
   __shared__ float scratch[kRowThreads / 32];
   constexpr int RPB = kRowThreads / TPR;
-  static_assert(RPB == 1 || TPR <= 128, "");
   const int t = threadIdx.x % TPR;
   const int sub = threadIdx.x / TPR;
   const int nvec = H / 8;
@@ -446,24 +446,9 @@ layernorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* 
       }
     }
   }
-  float* ow = dw_part + (size_t)blockIdx.x * H;
-  float* ob = db_part + (size_t)blockIdx.x * H;
-  for (int s = 0; s < RPB; ++s) {
-    if (sub == s) {
-#pragma unroll
-      for (int i = 0; i < VPT; ++i) {
-        int v = t + i * TPR;
-        if (v < nvec) {
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            if (s == 0) { ow[v * 8 + j] = dwacc[i][j]; ob[v * 8 + j] = dbacc[i][j]; }
-            else { ow[v * 8 + j] += dwacc[i][j]; ob[v * 8 + j] += dbacc[i][j]; }
-          }
-        }
-      }
-    }
-    if (RPB > 1) __syncthreads();
-  }
+  __shared__ __align__(16) float fold[fold_floats<TPR, VPT>()];
+  fold_row_groups<TPR, VPT>(dwacc, dw_part + (size_t)blockIdx.x * H, H, fold);
+  fold_row_groups<TPR, VPT>(dbacc, db_part + (size_t)blockIdx.x * H, H, fold);
 }
 
 // ------------------------------------------------------------------ RoPE (in place capable)
@@ -761,12 +746,16 @@ cross_entropy_bwd_kernel(const __nv_bfloat16* __restrict__ logits,
 }
 
 // ------------------------------------------------------------------ launch helpers
+// Threads per row. Rows of up to 1024 take one warp each: the row sums are shuffles only, so the eight rows of a CTA run
+// without a block barrier (with 128 threads per row, 768 columns left a quarter of them idle and every row paid two to
+// four barriers: LayerNorm 21 us forward and 30 us backward at 16384 x 768).
 static int pick_tpr(int H) {
   int nvec = H / 8;
-  return nvec <= 16 ? 16 : (nvec <= 256 ? 128 : 256);
+  return nvec <= 16 ? 16 : (nvec <= 128 ? 32 : (nvec <= 256 ? 128 : 256));
 }
 static int pick_vpt(int H, int tpr) {
   int need = (H / 8 + tpr - 1) / tpr;
+  if (tpr == 32) return need;   // 1..4
   int v = 1;
   while (v < need) v <<= 1;
   return v;
@@ -788,8 +777,21 @@ int row_grid(int rows, int tpr) {
   }
 #define TPB_ROW_SWITCH(tpr, vpt, ...)                                          \
   switch (tpr) {                                                               \
-    case 16: { constexpr int TPR = 16; TPB_VPT_SWITCH(vpt, __VA_ARGS__) } break;   \
-    case 128: { constexpr int TPR = 128; TPB_VPT_SWITCH(vpt, __VA_ARGS__) } break; \
+    case 16: { constexpr int TPR = 16; constexpr int VPT = 1; __VA_ARGS__; } break; \
+    case 32: {                                                                 \
+      constexpr int TPR = 32;                                                  \
+      switch (vpt) {                                                           \
+        case 1: { constexpr int VPT = 1; __VA_ARGS__; } break;                 \
+        case 2: { constexpr int VPT = 2; __VA_ARGS__; } break;                 \
+        case 3: { constexpr int VPT = 3; __VA_ARGS__; } break;                 \
+        default: { constexpr int VPT = 4; __VA_ARGS__; } break;                \
+      }                                                                        \
+    } break;                                                                   \
+    case 128: {                                                                \
+      constexpr int TPR = 128;                                                 \
+      constexpr int VPT = 2;                                                   \
+      __VA_ARGS__;                                                             \
+    } break;                                                                   \
     case 256: { constexpr int TPR = 256; TPB_VPT_SWITCH(vpt, __VA_ARGS__) } break; \
     default: return -2;                                                        \
   }
