@@ -31,7 +31,9 @@ struct GCfg {
   static constexpr int kABytes = kGBlockM * kGBlockK * 2;
   static constexpr int kBBytes = BLOCK_N * kGBlockK * 2;
   static constexpr int kStageBytes = kABytes + kBBytes;
-  static constexpr int kSmemBytes = kStages * kStageBytes + 1024 + 256;
+  // staging of the bf16 epilogue: per warp 32 rows of 64 columns, padded to 144 bytes (conflict-free both ways)
+  static constexpr int kOutOff = kStages * kStageBytes + 256;
+  static constexpr int kSmemBytes = kOutOff + 4 * 32 * 144 + 1024;
   static constexpr int kTmemCols = 2 * BLOCK_N;
 };
 
@@ -181,46 +183,53 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      const uint32_t idesc = (p.mode == 0)
-                                 ? make_idesc_f16(kGBlockM, BLOCK_N, 1, 0, B_MN ? 1 : 0)
-                                 : make_idesc_f16(kGBlockM, BLOCK_N, 1, 1, 1);
-      uint32_t it = 0, lt = 0;
-      bool ok = true;
-      for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
-        int e, row0, c0, kb0, kb1;
-        decode(tile, e, row0, c0, kb0, kb1);
-        if (kb1 <= kb0) continue;  // expert without rows: nothing to accumulate (lt counts used tiles)
-        const int as = lt & 1;
-        const uint32_t aph = (lt >> 1) & 1;
-        ++lt;
-        if (!mbar_wait(&tempty[as], aph ^ 1, wc, 2)) break;
+    // warp-uniform control flow, one elected lane issues: tcgen05 operands live in uniform registers, and an MMA issued
+    // from a divergent branch with its descriptors rebuilt costs about as long as a quarter of its execution
+    const bool a_mn = p.mode == 1, b_mn = p.mode == 1 || B_MN;
+    const uint32_t idesc = make_idesc_f16(kGBlockM, BLOCK_N, 1, a_mn ? 1 : 0, b_mn ? 1 : 0);
+    constexpr uint32_t hi = smem_desc_hi(1024);
+    const uint32_t a_lo0 = smem_desc_lo(smem_u32(smem), a_mn ? kGBlockK * 128 : 16);
+    const uint32_t b_lo0 = smem_desc_lo(smem_u32(smem + Cfg::kABytes), b_mn ? kGBlockK * 128 : 16);
+    const uint32_t a_step = a_mn ? 2048 >> 4 : 32 >> 4, b_step = b_mn ? 2048 >> 4 : 32 >> 4;
+    uint32_t it = 0, lt = 0;
+    bool ok = true;
+    for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
+      int e, row0, c0, kb0, kb1;
+      decode(tile, e, row0, c0, kb0, kb1);
+      if (kb1 <= kb0) continue;  // expert without rows: nothing to accumulate (lt counts used tiles)
+      const int as = lt & 1;
+      const uint32_t aph = (lt >> 1) & 1;
+      ++lt;
+      if (!mbar_wait_warp(&tempty[as], aph ^ 1, wc, 2)) break;
+      tc_fence_after_sync();
+      const uint32_t d_tmem = tmem_base + as * BLOCK_N;
+      for (int kb = kb0; kb < kb1; ++kb, ++it) {
+        const int s = it % Cfg::kStages;
+        const uint32_t ph = (it / Cfg::kStages) & 1;
+        if (!mbar_wait_warp(&full[s], ph, wc, 3)) { ok = false; break; }
         tc_fence_after_sync();
-        const uint32_t d_tmem = tmem_base + as * BLOCK_N;
-        for (int kb = kb0; kb < kb1; ++kb, ++it) {
-          const int s = it % Cfg::kStages;
-          const uint32_t ph = (it / Cfg::kStages) & 1;
-          if (!mbar_wait(&full[s], ph, wc, 3)) { ok = false; break; }
-          tc_fence_after_sync();
-          const uint32_t sa = smem_u32(smem + s * Cfg::kStageBytes);
-          const uint32_t sb = sa + Cfg::kABytes;
-          const bool a_mn = p.mode == 1;
-          const bool b_mn = p.mode == 1 || B_MN;
+        const uint32_t a_lo = a_lo0 + s * (Cfg::kStageBytes >> 4), b_lo = b_lo0 + s * (Cfg::kStageBytes >> 4);
+        if (elect_one()) {
 #pragma unroll
-          for (int j = 0; j < kGBlockK / 16; ++j) {
-            uint64_t da = a_mn ? make_smem_desc_sw128(sa + j * 2048, kGBlockK * 128, 1024)
-                               : make_smem_desc_sw128(sa + j * 32, 16, 1024);
-            uint64_t db = b_mn ? make_smem_desc_sw128(sb + j * 2048, kGBlockK * 128, 1024)
-                               : make_smem_desc_sw128(sb + j * 32, 16, 1024);
-            umma_f16_ss(d_tmem, da, db, idesc, (kb != kb0) || (j != 0));
-          }
+          for (int j = 0; j < kGBlockK / 16; ++j)
+            umma_f16_ss_w(d_tmem, a_lo + j * a_step, hi, b_lo + j * b_step, hi, idesc, (kb != kb0) || (j != 0));
           umma_commit(&empty[s]);
         }
-        if (ok) umma_commit(&tfull[as]);
+        __syncwarp();
+      }
+      if (ok) {
+        if (elect_one()) umma_commit(&tfull[as]);
+        __syncwarp();
       }
     }
   } else {
+    // Plain bf16 results go through shared memory and leave as 4 rows by 128 contiguous bytes: stored from the lane that
+    // holds 32 columns of a row, an instruction touches 32 rows by 16 bytes, and a weight gradient over the ~256 rows of
+    // an expert has four k-blocks per tile to hide that behind.
     const int q = warp & 3;
+    uint8_t* out_stage = smem + Cfg::kOutOff + q * (32 * 144);
+    const bool staged = !p.out_f32 && !p.accumulate && p.ldc % 8 == 0 && (p.mode == 0 || p.c_expert_stride % 8 == 0) &&
+                        (reinterpret_cast<uintptr_t>(p.C) & 15) == 0;
     uint32_t lt = 0;
     for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
       int e, row0, c0, kb0, kb1;
@@ -249,7 +258,30 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
 #pragma unroll
           for (int i = 0; i < 32; ++i) r[i] = 0;
         }
-        if (row < row_lim) {
+        if (staged && (c0 + (c & ~32)) + 64 <= col_lim) {   // warp-uniform, both halves of 64 columns
+          uint8_t* srow = out_stage + lane * 144 + (c & 32) * 2;
+#pragma unroll
+          for (int i = 0; i < 32; i += 8) {
+            uint4 o;
+            __nv_bfloat162* ob2 = reinterpret_cast<__nv_bfloat162*>(&o);
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+              ob2[j] = __floats2bfloat162_rn(__uint_as_float(r[i + 2 * j]), __uint_as_float(r[i + 2 * j + 1]));
+            *reinterpret_cast<uint4*>(srow + i * 2) = o;
+          }
+          if (c & 32) {
+            __syncwarp();
+            const int row8 = row0 + q * 32 + (lane >> 3);
+            __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(p.C) + (p.mode == 0 ? (size_t)0 : (size_t)e * p.c_expert_stride) +
+                                 (size_t)row8 * p.ldc + (col0 - 32) + (lane & 7) * 8;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              const uint4 val = *reinterpret_cast<const uint4*>(out_stage + (i * 4 + (lane >> 3)) * 144 + (lane & 7) * 16);
+              if (row8 + i * 4 < row_lim) *reinterpret_cast<uint4*>(dst + (size_t)(i * 4) * p.ldc) = val;
+            }
+            __syncwarp();
+          }
+        } else if (row < row_lim) {
           const bool full_chunk = col0 + 32 <= col_lim;
           const size_t base = (p.mode == 0) ? (size_t)row * p.ldc + col0
                                             : (size_t)e * p.c_expert_stride + (size_t)row * p.ldc + col0;
