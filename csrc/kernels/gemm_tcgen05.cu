@@ -1012,7 +1012,16 @@ int gemm_bf16_dispatch(const void* A, const void* B, void* C, const void* bias, 
 // operands MN-major (weight gradients) the two kernels time the same in isolation, but the pair
 // kernel moves a third less through shared memory and the training step, which runs at the power
 // cap, is 1.2 % shorter with it. 0 = never.
+// Among those, the one-CTA kernel (128 x 256 tiles, one per SM) where it needs clearly fewer rounds: a round of either
+// kernel takes about the same time (256 x 256 on two SMs against 128 x 256 on one; the one-CTA kernel 5-12 % longer), and
+// a product whose rows just exceed a multiple of 256 pays a nearly empty row of pair tiles: M = 777, N = 14336 has 224
+// pair tiles, four rounds of 74, and 392 one-CTA tiles, three rounds of 148.
 static int g_pair_min_tiles = 74;
+static bool single_has_fewer_rounds(int M, int N) {
+  const long long sms = tpb::sm_count(), pairs = sms / 2;
+  const long long tp = (long long)((M + 255) / 256) * ((N + 255) / 256), ts = (long long)((M + 127) / 128) * ((N + 255) / 256);
+  return ((ts + sms - 1) / sms) * 112 < ((tp + pairs - 1) / pairs) * 100;
+}
 extern "C" void tpb_gemm_set_pair_min_tiles(int tiles) { g_pair_min_tiles = tiles; }
 
 namespace tpb { int g_nvtx_on = 0; }
@@ -1058,9 +1067,13 @@ extern "C" int tpb_gemm_bf16(const void* A, const void* B, void* C, const void* 
   if (tpb::gemm_rows_takes(M, a_mn))
     return tpb::gemm_rows_dispatch(A, B, C, bias, M, N, K, lda, ldb, ldc, b_mn, out_f32, bias_f32, accumulate, alpha,
                                    status, static_cast<cudaStream_t>(stream));
-  if (g_pair_min_tiles > 0 && (long long)((M + 255) / 256) * ((N + 255) / 256) >= g_pair_min_tiles)
+  if (g_pair_min_tiles > 0 && (long long)((M + 255) / 256) * ((N + 255) / 256) >= g_pair_min_tiles) {
+    if (single_has_fewer_rounds(M, N))
+      return tpb::gemm_bf16_dispatch(A, B, C, bias, M, N, K, lda, ldb, ldc, a_mn, b_mn, out_f32, bias_f32, accumulate,
+                                     alpha, nullptr, 0, 0, 0, status, static_cast<cudaStream_t>(stream), nullptr);
     return tpb::gemm_pair_dispatch(A, B, C, bias, M, N, K, lda, ldb, ldc, a_mn, b_mn, out_f32, bias_f32,
                                    accumulate, alpha, 0, status, static_cast<cudaStream_t>(stream));
+  }
   int bn, c;
   if (g_pair_min_tiles > 0 && tpb::gemm_pair_split_plan(M, N, K, &bn, &c))
     return tpb::gemm_pair_split_dispatch(A, B, C, bias, M, N, K, lda, ldb, ldc, a_mn, b_mn, out_f32, bias_f32, accumulate,
