@@ -455,21 +455,26 @@ layernorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* 
 // x viewed as [tokens, heads, D] with explicit token/head strides (elements), y likewise with its
 // own strides (y == x rotates in place: each thread reads all it needs before it writes). cos/sin
 // tables are fp32 [max_pos, D/2]; pos[token] optional (else token % seq_len). sign = -1 for backward.
-__global__ void rope_kernel(const __nv_bfloat16* x, __nv_bfloat16* y, const float* __restrict__ cos_t,
+// Idx: 32-bit indices wherever they suffice; the three divisions that take an index apart were most of the kernel's
+// instructions in 64 bits.
+template <typename Idx>
+__global__ void __launch_bounds__(256)
+rope_kernel(const __nv_bfloat16* x, __nv_bfloat16* y, const float* __restrict__ cos_t,
                             const float* __restrict__ sin_t, const long long* __restrict__ pos,
                             long long tokens, int heads, int D, long long tok_stride,
                             long long head_stride, long long y_tok_stride, long long y_head_stride,
                             int seq_len, int interleaved, float sign) {
   const int half = D / 2;
   const int vec_per_head = half / 8;  // NeoX: 8 pairs per thread from both halves
-  long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  long long total = tokens * heads * vec_per_head;
+  const Idx idx = (Idx)blockIdx.x * 256 + threadIdx.x;
+  const Idx total = (Idx)tokens * heads * vec_per_head;
   if (idx >= total) return;
-  int v = idx % vec_per_head;
-  long long th = idx / vec_per_head;
-  int h = th % heads;
-  long long tok = th / heads;
-  long long p = pos ? pos[tok] : (tok % seq_len);
+  const Idx th = idx / (Idx)vec_per_head;
+  const int v = (int)(idx - th * vec_per_head);
+  const Idx tk = th / (Idx)heads;
+  const int h = (int)(th - tk * heads);
+  const long long tok = (long long)tk;
+  const long long p = pos ? pos[tok] : (long long)(tk % (Idx)seq_len);
   const __nv_bfloat16* base = x + tok * tok_stride + (long long)h * head_stride;
   __nv_bfloat16* obase = y + tok * y_tok_stride + (long long)h * y_head_stride;
   const float* c = cos_t + p * half;
@@ -515,48 +520,82 @@ __global__ void rope_kernel(const __nv_bfloat16* x, __nv_bfloat16* y, const floa
 
 // ------------------------------------------------------------------ SwiGLU / GELU
 // out[r, i] = silu(gate[r, i]) * up[r, i]; gate/up given with a common row stride.
-__global__ void swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gate,
-                                  const __nv_bfloat16* __restrict__ up,
-                                  __nv_bfloat16* __restrict__ out, long long rows, int I,
-                                  long long in_stride, const int* __restrict__ rows_dev) {
-  const int nvec = I / 8;
-  long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+// Bound by memory. A thread takes kActVecs vectors of eight elements, one block's width apart, with all their loads in
+// flight together; the vector index is 32 bits wide wherever that suffices (Idx), since the division that splits it into
+// row and column costs some ninety instructions in 64 bits, more than the arithmetic of the eight elements.
+constexpr int kActVecs = 2;
+template <typename Idx>
+__global__ void __launch_bounds__(256)
+swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gate, const __nv_bfloat16* __restrict__ up,
+                  __nv_bfloat16* __restrict__ out, long long rows, int I, long long in_stride,
+                  const int* __restrict__ rows_dev) {
+  const Idx nvec = I / 8;
   if (rows_dev) rows = min(rows, (long long)*rows_dev);  // row count known only on the device (ragged buffers)
-  if (idx >= rows * nvec) return;
-  long long r = idx / nvec;
-  int v = idx % nvec;
-  float g[8], u[8], o[8];
-  unpack8(reinterpret_cast<const uint4*>(gate + r * in_stride)[v], g);
-  unpack8(reinterpret_cast<const uint4*>(up + r * in_stride)[v], u);
+  const Idx total = (Idx)rows * nvec;
+  const Idx i0 = (Idx)blockIdx.x * (256 * kActVecs) + threadIdx.x;
+  uint4 gv[kActVecs], uv[kActVecs];
 #pragma unroll
-  for (int j = 0; j < 8; ++j) o[j] = g[j] / (1.f + __expf(-g[j])) * u[j];
-  reinterpret_cast<uint4*>(out + r * (long long)I)[v] = pack8(o);
-}
-__global__ void swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ dy,
-                                  const __nv_bfloat16* __restrict__ gate,
-                                  const __nv_bfloat16* __restrict__ up,
-                                  __nv_bfloat16* __restrict__ dgate, __nv_bfloat16* __restrict__ dup,
-                                  long long rows, int I, long long in_stride,
-                                  long long out_stride, const int* __restrict__ rows_dev) {
-  const int nvec = I / 8;
-  long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (rows_dev) rows = min(rows, (long long)*rows_dev);
-  if (idx >= rows * nvec) return;
-  long long r = idx / nvec;
-  int v = idx % nvec;
-  float g[8], u[8], d[8], dg[8], du[8];
-  unpack8(reinterpret_cast<const uint4*>(gate + r * in_stride)[v], g);
-  unpack8(reinterpret_cast<const uint4*>(up + r * in_stride)[v], u);
-  unpack8(reinterpret_cast<const uint4*>(dy + r * (long long)I)[v], d);
-#pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    float sg = 1.f / (1.f + __expf(-g[j]));
-    float silu = g[j] * sg;
-    du[j] = d[j] * silu;
-    dg[j] = d[j] * u[j] * (sg + silu * (1.f - sg));
+  for (int k = 0; k < kActVecs; ++k) {
+    const Idx idx = i0 + k * 256;
+    if (idx >= total) break;
+    const Idx r = idx / nvec;
+    const int v = (int)(idx - r * nvec);
+    gv[k] = reinterpret_cast<const uint4*>(gate + (long long)r * in_stride)[v];
+    uv[k] = reinterpret_cast<const uint4*>(up + (long long)r * in_stride)[v];
   }
-  reinterpret_cast<uint4*>(dgate + r * out_stride)[v] = pack8(dg);
-  reinterpret_cast<uint4*>(dup + r * out_stride)[v] = pack8(du);
+#pragma unroll
+  for (int k = 0; k < kActVecs; ++k) {
+    const Idx idx = i0 + k * 256;
+    if (idx >= total) break;
+    float g[8], u[8], o[8];
+    unpack8(gv[k], g);
+    unpack8(uv[k], u);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) o[j] = g[j] / (1.f + __expf(-g[j])) * u[j];
+    reinterpret_cast<uint4*>(out)[idx] = pack8(o);   // rows of out are contiguous
+  }
+}
+template <typename Idx>
+__global__ void __launch_bounds__(256)
+swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ gate,
+                  const __nv_bfloat16* __restrict__ up, __nv_bfloat16* __restrict__ dgate,
+                  __nv_bfloat16* __restrict__ dup, long long rows, int I, long long in_stride, long long out_stride,
+                  const int* __restrict__ rows_dev) {
+  const Idx nvec = I / 8;
+  if (rows_dev) rows = min(rows, (long long)*rows_dev);
+  const Idx total = (Idx)rows * nvec;
+  const Idx i0 = (Idx)blockIdx.x * (256 * kActVecs) + threadIdx.x;
+  uint4 gv[kActVecs], uv[kActVecs], dv[kActVecs];
+  Idx row[kActVecs];
+  int col[kActVecs];
+#pragma unroll
+  for (int k = 0; k < kActVecs; ++k) {
+    const Idx idx = i0 + k * 256;
+    if (idx >= total) break;
+    row[k] = idx / nvec;
+    col[k] = (int)(idx - row[k] * nvec);
+    gv[k] = reinterpret_cast<const uint4*>(gate + (long long)row[k] * in_stride)[col[k]];
+    uv[k] = reinterpret_cast<const uint4*>(up + (long long)row[k] * in_stride)[col[k]];
+    dv[k] = reinterpret_cast<const uint4*>(dy)[idx];
+  }
+#pragma unroll
+  for (int k = 0; k < kActVecs; ++k) {
+    const Idx idx = i0 + k * 256;
+    if (idx >= total) break;
+    float g[8], u[8], d[8], dg[8], du[8];
+    unpack8(gv[k], g);
+    unpack8(uv[k], u);
+    unpack8(dv[k], d);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      float sg = 1.f / (1.f + __expf(-g[j]));
+      float silu = g[j] * sg;
+      du[j] = d[j] * silu;
+      dg[j] = d[j] * u[j] * (sg + silu * (1.f - sg));
+    }
+    reinterpret_cast<uint4*>(dgate + (long long)row[k] * out_stride)[col[k]] = pack8(dg);
+    reinterpret_cast<uint4*>(dup + (long long)row[k] * out_stride)[col[k]] = pack8(du);
+  }
 }
 
 // GELU; approx = 1 selects the tanh form, evaluated as x * sigmoid(2u) with u = sqrt(2/pi) (x + 0.044715 x^3): the
@@ -904,7 +943,8 @@ extern "C" int tpb_rope_out(const void* x, void* y, const float* cos_t, const fl
   long long total = tokens * heads * (D / 16);
   if (total <= 0) return 0;
   int grid = (int)((total + 255) / 256);
-  rope_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(
+  auto kern = total < 0x7ff00000LL ? rope_kernel<unsigned> : rope_kernel<unsigned long long>;
+  kern<<<grid, 256, 0, (cudaStream_t)stream>>>(
       (const __nv_bfloat16*)x, (__nv_bfloat16*)y, cos_t, sin_t, pos, tokens, heads, D, tok_stride,
       head_stride, y_tok_stride, y_head_stride, seq_len, interleaved, backward ? -1.f : 1.f);
   return (int)cudaGetLastError();
@@ -927,7 +967,8 @@ extern "C" int tpb_swiglu_fwd_n(const void* gate, const void* up, void* out, lon
   if (I % 8 || in_stride % 8) return -2;
   long long total = rows * (I / 8);
   if (total <= 0) return 0;
-  swiglu_fwd_kernel<<<(unsigned)((total + 255) / 256), 256, 0, (cudaStream_t)stream>>>(
+  auto kern = total < 0x7ff00000LL ? swiglu_fwd_kernel<unsigned> : swiglu_fwd_kernel<unsigned long long>;
+  kern<<<(unsigned)((total + 256 * kActVecs - 1) / (256 * kActVecs)), 256, 0, (cudaStream_t)stream>>>(
       (const __nv_bfloat16*)gate, (const __nv_bfloat16*)up, (__nv_bfloat16*)out, rows, I,
       in_stride, rows_dev);
   return (int)cudaGetLastError();
@@ -944,7 +985,8 @@ extern "C" int tpb_swiglu_bwd_n(const void* dy, const void* gate, const void* up
   if (I % 8 || in_stride % 8 || out_stride % 8) return -2;
   long long total = rows * (I / 8);
   if (total <= 0) return 0;
-  swiglu_bwd_kernel<<<(unsigned)((total + 255) / 256), 256, 0, (cudaStream_t)stream>>>(
+  auto kern = total < 0x7ff00000LL ? swiglu_bwd_kernel<unsigned> : swiglu_bwd_kernel<unsigned long long>;
+  kern<<<(unsigned)((total + 256 * kActVecs - 1) / (256 * kActVecs)), 256, 0, (cudaStream_t)stream>>>(
       (const __nv_bfloat16*)dy, (const __nv_bfloat16*)gate, (const __nv_bfloat16*)up,
       (__nv_bfloat16*)dgate, (__nv_bfloat16*)dup, rows, I, in_stride, out_stride, rows_dev);
   return (int)cudaGetLastError();
