@@ -8,67 +8,21 @@
 //     group happens inside the accumulator (no expanded K/V, no atomics).
 //   * dQ pass: a CTA owns 128 queries of one query head, keeps Q and dO resident and streams
 //     64-key tiles of K and V; dQ += dS K in TMEM (deterministic, no atomics).
-// Per streamed tile: S = X0 Y0^T and dP = X1 Y1^T (tcgen05.mma, TMEM double-buffered), the four
-// "softmax" warps turn them into P and dS = P (dP - delta) * scale, write them as bf16 into
-// 128-byte-swizzled tiles, and the accumulating MMAs read those tiles.
+// Two forms share the passes. Here, for head dimension 64 with few CTAs: per streamed tile S = X0 Y0^T and
+// dP = X1 Y1^T go to TMEM (two tiles at a time), eight warps turn both into P and dS = P (dP - delta) * scale in one step
+// and write them as bf16 over the same columns, from where the accumulating MMAs take them. The other form, for head
+// dimension 128 and for 64 with many CTAs, is in flash_bwd_wide.cu.
 //
 // Counterpart in the reference: FlashAttention-2 sm80 backward
 // (p10/src/backend/cuda/transformers/AttentionKernels.cu:2286-2543), which has no GQA path
 // (:2459-2461) and accumulates dQ with fp32 atomics.
-#include "sm100.cuh"
+#include "flash_bwd.cuh"
 #include "tpb_api.h"
 
 namespace tpb {
 
-int make_tmap_bthd(CUtensorMap* out, const void* base, int B, int T, int H, int D,
-                   long long tok_stride, long long head_stride, long long batch_stride, int rows);
-
-constexpr int kBwdThreads = 320;  // TMA warp, MMA warp, 8 P/dS warps (two per TMEM lane quarter)
-constexpr int kSoftThreads = 256;
-constexpr int kStat = 128;   // rows of the stationary tiles
 constexpr int kStream = 64;  // rows of the streamed tiles
 constexpr int kYStages = 4;  // streamed-tile ring: loads run three tiles ahead of the MMAs
-
-struct AttnBwdParams {
-  int B, Tq, Tk, Hq, Hkv;
-  int causal, kv_offset;
-  // optional key bounds of a query, as in the forward: window > 0 = local attention; seg_start / seg_end
-  // [B * Tq] = keys [start, end) of every query, which with Tq == Tk (packed self-attention, the only form
-  // that takes them) are also the queries [start, end) of every key
-  int window;
-  const int* seg_start;
-  const int* seg_end;
-  float scale, scale_log2e;
-  const float* lse;    // [B, Hq, lse_stride]
-  const float* delta;  // [B, Hq, lse_stride]
-  int lse_stride;
-  __nv_bfloat16* out0;  // dKV: dV ; dQ: unused
-  __nv_bfloat16* out1;  // dKV: dK ; dQ: dQ
-  long long out_tok, out_head, out_batch;
-  uint32_t* status;
-  unsigned long long wait_ns;
-  unsigned long long* trace;  // optional: timestamps of CTA (0,0,0), see tpb_flash_bwd_set_trace
-  int trace_cap;
-};
-
-// Debug aid: records (role, iteration, phase, globaltimer) tuples of block (0,0,0).
-__device__ __forceinline__ void trace_pt(const AttnBwdParams& p, int role, int it, int phase) {
-  if (p.trace && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0) {
-    unsigned long long idx = atomicAdd(p.trace, 1ull);
-    if ((int)idx < p.trace_cap) {
-      unsigned long long t;
-      asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-      p.trace[1 + idx * 2] = ((unsigned long long)role << 48) | ((unsigned long long)(it & 0xffffff) << 16) | (unsigned)phase;
-      p.trace[2 + idx * 2] = t;
-    }
-  }
-}
-
-__device__ __forceinline__ float bwd_exp2(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));  // pure: let the compiler schedule it
-  return y;
-}
 
 template <int D>
 struct BwdSmem {
@@ -78,7 +32,7 @@ struct BwdSmem {
   static constexpr int kX0 = 0;
   static constexpr int kX1 = kX0 + kStatBytes;
   static constexpr int kY = kX1 + kStatBytes;  // kYStages x (Y0, Y1)
-  static constexpr int kStats = kY + 2 * kYStages * kStreamBytes;  // per Y stage: lse[64] then delta[64] (fp32)
+  static constexpr int kStats = kY + 2 * kYStages * kStreamBytes;  // per Y stage: -lse * log2e [64] then -delta * scale [64]
   static constexpr int kBar = kStats + kYStages * 2 * kStream * 4;
   static constexpr int kTotal = kBar + 256 + 1024;
   static_assert(kTotal <= 227 * 1024, "attention backward exceeds the shared memory of one CTA");
@@ -86,26 +40,27 @@ struct BwdSmem {
 
 // P = exp2(S * scale_log2e - lse2) and dS = P * (dP * scale - delta * scale) for 32 columns of
 // one row, packed to bf16 pairs. Straight-line code: the masked variant selects, it never branches.
-//   DKV: per-column statistics (lse, delta of the streamed queries) come from shared memory;
-//   dQ : the row's own statistics (already scaled) are in registers.
+//   DKV: per-column statistics of the streamed queries come from shared memory;
+//   dQ : the row's own statistics are in registers.
+// Both come negated and scaled from the pass that computes delta: scaling them here cost two of the ~eight instructions
+// per element of the dK/dV pass.
 template <bool DKV, bool MASKED>
 __device__ __forceinline__ void pds_math(const uint32_t (&sr)[32], const uint32_t (&dr)[32],
-                                         uint32_t stats_sa, float lse2_row, float dsc_row, int y0i,
+                                         uint32_t stats_sa, float nlse2_row, float ndsc_row, int y0i,
                                          int y_lo, int y_hi, float scale_log2e, float scale,
                                          uint32_t (&pw)[16], uint32_t (&dw)[16]) {
-  constexpr float kLog2e = 1.4426950408889634f;
 #pragma unroll
   for (int c = 0; c < 32; c += 4) {
     float l4[4], d4[4];
     if (DKV) {
       float4 a, d;
-      asm("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w) : "r"(stats_sa + c * 4));
-      asm("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(d.x), "=f"(d.y), "=f"(d.z), "=f"(d.w) : "r"(stats_sa + (kStream + c) * 4));
-      l4[0] = a.x * kLog2e; l4[1] = a.y * kLog2e; l4[2] = a.z * kLog2e; l4[3] = a.w * kLog2e;
-      d4[0] = d.x * scale; d4[1] = d.y * scale; d4[2] = d.z * scale; d4[3] = d.w * scale;
+      asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w) : "r"(stats_sa + c * 4));
+      asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(d.x), "=f"(d.y), "=f"(d.z), "=f"(d.w) : "r"(stats_sa + (kStream + c) * 4));
+      l4[0] = a.x; l4[1] = a.y; l4[2] = a.z; l4[3] = a.w;
+      d4[0] = d.x; d4[1] = d.y; d4[2] = d.z; d4[3] = d.w;
     } else {
-      l4[0] = l4[1] = l4[2] = l4[3] = lse2_row;
-      d4[0] = d4[1] = d4[2] = d4[3] = dsc_row;
+      l4[0] = l4[1] = l4[2] = l4[3] = nlse2_row;
+      d4[0] = d4[1] = d4[2] = d4[3] = ndsc_row;
     }
     float pr[4], ds[4];
     const float2 sc2 = make_float2(scale_log2e, scale_log2e), s2 = make_float2(scale, scale);
@@ -113,9 +68,9 @@ __device__ __forceinline__ void pds_math(const uint32_t (&sr)[32], const uint32_
     for (int i = 0; i < 4; i += 2) {
       // packed fp32x2 arithmetic: two elements per FMA / MUL
       const float2 x = __ffma2_rn(make_float2(__uint_as_float(sr[c + i]), __uint_as_float(sr[c + i + 1])), sc2,
-                                  make_float2(-l4[i], -l4[i + 1]));
+                                  make_float2(l4[i], l4[i + 1]));
       const float2 t = __ffma2_rn(make_float2(__uint_as_float(dr[c + i]), __uint_as_float(dr[c + i + 1])), s2,
-                                  make_float2(-d4[i], -d4[i + 1]));
+                                  make_float2(d4[i], d4[i + 1]));
       float2 e = make_float2(bwd_exp2(x.x), bwd_exp2(x.y));
       float2 g = __fmul2_rn(e, t);
       if (MASKED) {
@@ -152,7 +107,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmX0, const __grid_constant
   uint64_t* y_full = bars + 1;                    // kYStages
   uint64_t* y_empty = y_full + kYStages;          // kYStages
   uint64_t* sdp_full = y_empty + kYStages;        // 2
-  uint64_t* pds_full = sdp_full + 2;              // 1 (256 arrivals)
+  uint64_t* pds_full = sdp_full + 2;              // 1 (one arrival per P/dS warp)
   uint64_t* acc_done = pds_full + 1;              // 1
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_done + 1);
   volatile uint32_t* abort_w = tmem_slot + 1;
@@ -222,7 +177,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmX0, const __grid_constant
     for (int i = 0; i < 2; ++i) {
       mbar_init(&sdp_full[i], 1);
     }
-    mbar_init(pds_full, kSoftThreads);
+    mbar_init(pds_full, kSoftThreads / 32);
     mbar_init(acc_done, 1);
     fence_barrier_init();
     prefetch_tmap(&tmX0);
@@ -265,10 +220,10 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmX0, const __grid_constant
         mbar_arrive_expect_tx(&y_full[s], 2 * L::kStreamBytes + (DKV ? 2 * kStream * 4 : 0));
         if (DKV) {
           // the per-query statistics of the streamed tile ride along with it
-          const long long so = ((long long)b * p.Hq + hy) * p.lse_stride + (long long)yb * kStream;
+          const long long so = ((long long)b * p.Hq + hy) * p.stat_stride + (long long)yb * kStream;
           float* st = reinterpret_cast<float*>(smem + L::kStats) + s * 2 * kStream;
-          bulk_load_1d(st, p.lse + so, kStream * 4, &y_full[s]);
-          bulk_load_1d(st + kStream, p.delta + so, kStream * 4, &y_full[s]);
+          bulk_load_1d(st, p.nlse2 + so, kStream * 4, &y_full[s]);
+          bulk_load_1d(st + kStream, p.ndsc + so, kStream * 4, &y_full[s]);
         }
 #pragma unroll
         for (int c = 0; c < L::kChunks; ++c) {
@@ -360,13 +315,12 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmX0, const __grid_constant
     const int row = qd * 32 + lane;
     const int xi = x0 + row;  // key index (DKV) or query index (dQ)
     const uint32_t t_lane = ((uint32_t)(qd * 32) << 16);
-    const float log2e = 1.4426950408889634f;
     float lse_row = 0.f, delta_row = 0.f;
     if (!DKV) {
       if (xi < p.Tq) {
-        long long o = ((long long)b * p.Hq + hx) * p.lse_stride + xi;
-        lse_row = p.lse[o];
-        delta_row = p.delta[o];
+        long long o = ((long long)b * p.Hq + hx) * p.stat_stride + xi;
+        lse_row = p.nlse2[o];
+        delta_row = p.ndsc[o];
       }
     }
     // streamed indices (queries for dKV, keys for dQ) that this row may pair with
@@ -388,8 +342,6 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmX0, const __grid_constant
         if (p.seg_end) y_hi = min(y_hi, p.seg_end[seg_base + xi]);
       }
     }
-    lse_row *= log2e;
-    delta_row *= p.scale;
     bool ok = true;
     for (int it = 0; it < n_it; ++it) {
       const int s = it & 1;
@@ -426,7 +378,8 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmX0, const __grid_constant
       tmem_st_32x32b_x16(tmem_base + t_lane + s * 128 + 64 + half * 32, dw);
       tmem_st_wait();
       tc_fence_before_sync();
-      mbar_arrive(pds_full);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(pds_full);   // one arrival per warp: 32 on one barrier are served one after the other
       if (threadIdx.x == 64) trace_pt(p, 2, it, 5);
     }
     if (ok && n_it > 0) ok = mbar_wait_warp(acc_done, 0, wc, 8);
@@ -486,15 +439,17 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmX0, const __grid_constant
   }
 }
 
-// delta[b, h, t] = sum_d O[b, t, h, d] * dO[b, t, h, d].
+// ndsc[b, h, t] = -scale * sum_d O[b, t, h, d] * dO[b, t, h, d] and nlse2[b, h, t] = -log2(e) * lse[b, h, t].
 // Reads O and dO once, so a lane takes whole 16-byte pieces (16 lanes per row of 128, 8 per row of 64) and a warp
 // several rows; with 4-byte loads and a warp per row the pass took 40 us at T = 4096, 32 heads of 128 (10 us of
 // memory time). O whose rows are not 16-byte aligned is read two elements at a time.
 template <int D>
 __global__ void __launch_bounds__(256)
 attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ dout,
-                  float* __restrict__ delta, int B, int T, int H, long long o_tok, long long o_head, long long o_batch,
-                  long long d_tok, long long d_head, long long d_batch, int lse_stride, int o_vec) {
+                  const float* __restrict__ lse, float* __restrict__ nlse2, float* __restrict__ ndsc, float scale, int B,
+                  int T, int H, long long o_tok, long long o_head, long long o_batch,
+                  long long d_tok, long long d_head, long long d_batch, int lse_stride, int stat_stride,
+                  int o_vec) {
   constexpr int LPR = D / 8;   // lanes per row
   const long long w = ((long long)blockIdx.x * 256 + threadIdx.x) / LPR;
   const int i = (threadIdx.x % LPR) * 8;
@@ -525,7 +480,11 @@ attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __re
   }
 #pragma unroll
   for (int off = LPR / 2; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
-  if (live && i == 0) delta[((long long)b * H + h) * lse_stride + t] = s;
+  if (live && i == 0) {
+    const long long at = ((long long)b * H + h) * stat_stride + t;
+    ndsc[at] = -(s * scale);
+    nlse2[at] = -(lse[((long long)b * H + h) * lse_stride + t] * 1.4426950408889634f);
+  }
 }
 
 static unsigned long long* g_bwd_trace = nullptr;
@@ -551,8 +510,8 @@ static int launch_bwd(const CUtensorMap& x0, const CUtensorMap& x1, const CUtens
 
 using namespace tpb;
 
-// lse / delta: [B, Hq, lse_stride] fp32 with lse_stride a multiple of 64 and >= Tq rounded up
-// to 64 (the dKV pass reads whole 64-query vectors). delta is scratch written here.
+// lse: [B, Hq, lse_stride] fp32 with lse_stride a multiple of 64 and >= Tq rounded up to 64. delta: scratch of two
+// arrays [B, Hq, Tq rounded up to 128], written here (the dKV pass reads whole streamed tiles).
 // window / seg_start / seg_end as in tpb_flash_fwd_ex; segment bounds need Tq == Tk.
 extern "C" int tpb_flash_bwd_ex(const void* dout, const void* q, const void* k, const void* v,
                                 const void* o, const float* lse, float* delta, void* dq, void* dk,
@@ -575,20 +534,26 @@ extern "C" int tpb_flash_bwd_ex(const void* dout, const void* q, const void* k, 
   if ((q_tok | q_head | q_batch | k_tok | k_head | k_batch | v_tok | v_head | v_batch | do_tok |
        do_head | do_batch | dq_tok | dq_head | dq_batch | dkv_tok | dkv_head | dkv_batch) % 8)
     return -2;
-  // delta
+  const int stat_stride = (Tq + kStatPad - 1) / kStatPad * kStatPad;
+  float *ndsc = delta, *nlse2 = delta + (size_t)B * Hq * stat_stride;
+  // Which form (measured on one B200, D = 64, dKV / dQ pass in us, this file's form against the wide one): 16 x 1024
+  // tokens, 12 heads (1536 CTAs) 138 / 99 against 118 / 91; 8190 tokens, 32/8 heads (512 / 2048 CTAs) 733 / 610 against
+  // 853 / 553; 2 x 2048 tokens, 16 heads (512 CTAs) 68 / 53 against 72 / 56; 8 x 309 tokens, 16/4 heads (96 / 384 CTAs)
+  // 22 / 17 against 32 / 18. Two CTAs per SM pay from some six CTAs per SM on.
+  auto wide = [&](long long ctas) { return D == 128 || ctas >= 6LL * sm_count(); };
   {
     if (reinterpret_cast<uintptr_t>(dout) & 15) return -2;
     const long long threads = (long long)B * Tq * Hq * (D / 8);
     const int o_vec = !((o_tok | o_head | o_batch) % 8) && !(reinterpret_cast<uintptr_t>(o) & 15);
     const unsigned blocks = (unsigned)((threads + 255) / 256);
     auto kern = D == 128 ? attn_delta_kernel<128> : attn_delta_kernel<64>;
-    kern<<<blocks, 256, 0, stream>>>((const __nv_bfloat16*)o, (const __nv_bfloat16*)dout, delta, B, Tq, Hq, o_tok, o_head,
-                                     o_batch, do_tok, do_head, do_batch, lse_stride, o_vec);
+    kern<<<blocks, 256, 0, stream>>>((const __nv_bfloat16*)o, (const __nv_bfloat16*)dout, lse, nlse2, ndsc, scale, B, Tq, Hq, o_tok, o_head,
+                                     o_batch, do_tok, do_head, do_batch, lse_stride, stat_stride, o_vec);
   }
   AttnBwdParams p;
   p.B = B; p.Tq = Tq; p.Tk = Tk; p.Hq = Hq; p.Hkv = Hkv; p.causal = causal;
   p.kv_offset = Tk - Tq; p.scale = scale; p.scale_log2e = scale * 1.4426950408889634f;
-  p.lse = lse; p.delta = delta; p.lse_stride = lse_stride; p.status = status;
+  p.nlse2 = nlse2; p.ndsc = ndsc; p.stat_stride = stat_stride; p.status = status;
   p.wait_ns = kDefaultWaitNs;
   p.trace = g_bwd_trace; p.trace_cap = g_bwd_trace_cap;
   p.window = window > 0 ? window : 0; p.seg_start = seg_start; p.seg_end = seg_end;
@@ -596,29 +561,33 @@ extern "C" int tpb_flash_bwd_ex(const void* dout, const void* q, const void* k, 
   // ---- dK / dV: [B, Tk, Hkv, D] by the dkv strides (dk and dv share them)
   {
     CUtensorMap tk, tv, tq, tdo;
+    const dim3 grid((Tk + kStat - 1) / kStat, Hkv, B);
+    const bool w = wide((long long)grid.x * grid.y * grid.z);
+    const int rows = w ? bwd_wide_rows(D) : kStream;
     if ((r = make_tmap_bthd(&tk, k, B, Tk, Hkv, D, k_tok, k_head, k_batch, kStat))) return r;
     if ((r = make_tmap_bthd(&tv, v, B, Tk, Hkv, D, v_tok, v_head, v_batch, kStat))) return r;
-    if ((r = make_tmap_bthd(&tq, q, B, Tq, Hq, D, q_tok, q_head, q_batch, kStream))) return r;
-    if ((r = make_tmap_bthd(&tdo, dout, B, Tq, Hq, D, do_tok, do_head, do_batch, kStream))) return r;
+    if ((r = make_tmap_bthd(&tq, q, B, Tq, Hq, D, q_tok, q_head, q_batch, rows))) return r;
+    if ((r = make_tmap_bthd(&tdo, dout, B, Tq, Hq, D, do_tok, do_head, do_batch, rows))) return r;
     p.out0 = (__nv_bfloat16*)dv; p.out1 = (__nv_bfloat16*)dk;
     p.out_tok = dkv_tok; p.out_head = dkv_head; p.out_batch = dkv_batch;
-    dim3 grid((Tk + kStat - 1) / kStat, Hkv, B);
-    r = (D == 128) ? launch_bwd<128, true>(tk, tv, tq, tdo, p, grid, stream)
-                   : launch_bwd<64, true>(tk, tv, tq, tdo, p, grid, stream);
+    r = w ? launch_bwd_wide(D, true, tk, tv, tq, tdo, p, grid, stream)
+          : launch_bwd<64, true>(tk, tv, tq, tdo, p, grid, stream);
     if (r) return r;
   }
   // ---- dQ: [B, Tq, Hq, D] by the dq strides
   {
     CUtensorMap tq, tdo, tk, tv;
+    const dim3 grid((Tq + kStat - 1) / kStat, Hq, B);
+    const bool w = wide((long long)grid.x * grid.y * grid.z);
+    const int rows = w ? bwd_wide_rows(D) : kStream;
     if ((r = make_tmap_bthd(&tq, q, B, Tq, Hq, D, q_tok, q_head, q_batch, kStat))) return r;
     if ((r = make_tmap_bthd(&tdo, dout, B, Tq, Hq, D, do_tok, do_head, do_batch, kStat))) return r;
-    if ((r = make_tmap_bthd(&tk, k, B, Tk, Hkv, D, k_tok, k_head, k_batch, kStream))) return r;
-    if ((r = make_tmap_bthd(&tv, v, B, Tk, Hkv, D, v_tok, v_head, v_batch, kStream))) return r;
+    if ((r = make_tmap_bthd(&tk, k, B, Tk, Hkv, D, k_tok, k_head, k_batch, rows))) return r;
+    if ((r = make_tmap_bthd(&tv, v, B, Tk, Hkv, D, v_tok, v_head, v_batch, rows))) return r;
     p.out0 = nullptr; p.out1 = (__nv_bfloat16*)dq;
     p.out_tok = dq_tok; p.out_head = dq_head; p.out_batch = dq_batch;
-    dim3 grid((Tq + kStat - 1) / kStat, Hq, B);
-    r = (D == 128) ? launch_bwd<128, false>(tq, tdo, tk, tv, p, grid, stream)
-                   : launch_bwd<64, false>(tq, tdo, tk, tv, p, grid, stream);
+    r = w ? launch_bwd_wide(D, false, tq, tdo, tk, tv, p, grid, stream)
+          : launch_bwd<64, false>(tq, tdo, tk, tv, p, grid, stream);
     if (r) return r;
   }
   return 0;

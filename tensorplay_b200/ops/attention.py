@@ -158,7 +158,7 @@ def flash_bwd(do, q, k, v, o, lse, causal: bool, scale: float, dq=None, dk=None,
     if dv is None:
         dv = torch.empty((B, Tk, Hkv, D), dtype=q.dtype, device=q.device)
     assert dk.stride() == dv.stride()
-    delta = torch.empty_like(lse)
+    delta = torch.empty((2, B, Hq, (Tq + 127) // 128 * 128), dtype=torch.float32, device=q.device)
     if not _strides_ok(do):
         do = do.contiguous()
     code = lib().tpb_flash_bwd_ex(
