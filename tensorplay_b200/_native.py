@@ -82,6 +82,7 @@ _KERNEL_SIGS = {
     "tpb_fp8_quant": [P, P, P, LL, I, I, I, P],
     "tpb_fp8_dequant": [P, P, P, LL, I, I, I, P],
     "tpb_embedding_fwd": [P, P, P, LL, I, LL, P],
+    "tpb_zero": [P, LL, P],
     "tpb_embedding_bwd": [P, P, P, LL, I, LL, I, P],
     "tpb_kv_append": [P, P, P, P, I, I, I, I, I, I, I, LL, LL, LL, LL, LL, LL, P],
     "tpb_nms": [P, P, I, F, P, P, P, P],

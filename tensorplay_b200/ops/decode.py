@@ -33,13 +33,20 @@ class _EmbeddingFn(torch.autograd.Function):
         if dst is not None:
             # engine-owned flat gradient: accumulate in place, nothing flows through autograd
             if not getattr(w, "_tpb_grad_written", False):
-                dst.zero_()
+                _zero_(dst)
                 w._tpb_grad_written = True
             embedding_backward_(dst, ids, dy)
             return None, None
-        dw = torch.zeros(ctx.wshape, dtype=ctx.wdtype, device=dy.device)
+        dw = _zero_(torch.empty(ctx.wshape, dtype=ctx.wdtype, device=dy.device))
         embedding_backward_(dw, ids, dy)
         return None, dw
+
+
+def _zero_(t: Tensor) -> Tensor:
+    if use_native(t) and t.is_contiguous():
+        _native.check(lib().tpb_zero(ptr(t), t.numel() * t.element_size(), stream_ptr()), "tpb_zero")
+        return t
+    return t.zero_()
 
 
 def embedding_forward(ids: Tensor, weight: Tensor) -> Tensor:
