@@ -329,6 +329,18 @@ __device__ __forceinline__ void mma_bf16_16816(float (&c)[4], uint32_t a0, uint3
       : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
+// (v & mask) | bits in one instruction: written with two literals it became two
+__device__ __forceinline__ uint32_t and_or(uint32_t v, uint32_t mask, uint32_t bits) {
+  uint32_t r;
+  asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(r) : "r"(v), "r"(mask), "r"(bits));
+  return r;
+}
+// A 2-byte load that stays where it is written and whose use may come much later
+__device__ __forceinline__ uint32_t ldg_u16(const void* p) {
+  uint16_t r;
+  asm volatile("ld.global.nc.u16 %0, [%1];" : "=h"(r) : "l"(p));
+  return r;
+}
 __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
   uint32_t r;
   asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
@@ -615,34 +627,55 @@ wq_gemv_mma_v2_kernel(const __nv_bfloat16* __restrict__ x, const uint8_t* __rest
     }
     xptr += KS * CH / 8;
   };
-  auto load_s = [&](int c, float (&sc)[TILES][2], float (&zs)[TILES][2]) {
+  // The 4-bit forms keep the raw 2-byte values until they are used: arithmetic on a loaded value makes the warp wait
+  // for the load on the spot. With and_or below, 5 x 28672 x 8192: 56.9 -> 45.1 us in groups of 128, 89.9 -> 80.8 us
+  // in groups of 32; 5 x 14336 x 4096 17.3 -> 14.0 us. The two forms that it does not help convert at once: 8 bits
+  // (62.9 us so, 63.4 late) and one tile with scales per weight (9.7, 10.0 at 5 x 4096 x 4096: registers).
+  constexpr bool kLate = BITS == 4 && (FOLD || TILES == 2);
+  auto load_s = [&](int c, uint32_t (&rs)[TILES][2], uint32_t (&rz)[TILES][2]) {
     if (!GROUPED) return;
     const int gi = (c * CH + t * KL) >> gshift;
 #pragma unroll
     for (int tl = 0; tl < TILES; ++tl)
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        float s = 1.f, z = 8.f;
-        if (c < n_chunks) {
-          s = __bfloat162float(scale[srow[tl][h] + gi]);
-          if (BITS == 4 && zero) z = __bfloat162float(zero[srow[tl][h] + gi]);
-        }
-        // 4-bit: the nibble goes to the top mantissa bits of 1.0 (v = 1 + code / 16) and one FMA
-        // gives (code - zp) * s = v * (16 s) - (16 + zp) * s, the constant exact to 2^-24 of 16 s
-        if (FOLD) {
-          sc[tl][h] = s;
-          zs[tl][h] = -(128.f + z);
+      for (int h = 0; h < 2; ++h)
+        if (kLate) {
+          if (c < n_chunks) {
+            rs[tl][h] = ldg_u16(scale + srow[tl][h] + gi);
+            if (zero) rz[tl][h] = ldg_u16(zero + srow[tl][h] + gi);
+          }
         } else {
-          sc[tl][h] = BITS == 4 ? 16.f * s : s;
-          zs[tl][h] = -(16.f + z) * s;
+          float s = 1.f, z = 8.f;
+          if (c < n_chunks) {
+            s = __bfloat162float(scale[srow[tl][h] + gi]);
+            if (BITS == 4 && zero) z = __bfloat162float(zero[srow[tl][h] + gi]);
+          }
+          // scaled as in the arithmetic below
+          rs[tl][h] = __float_as_uint(BITS == 4 ? 16.f * s : s);
+          rz[tl][h] = __float_as_uint(-(16.f + z) * s);
         }
-      }
   };
 
   int st_use = 0;
   // arithmetic of one chunk, with the registers that hold its x rows and scales
-  auto compute = [&](const uint32_t (&xw)[KL / 2], const float (&sc)[TILES][2], const float (&zs)[TILES][2]) {
+  auto compute = [&](const uint32_t (&xw)[KL / 2], const uint32_t (&rs)[TILES][2], const uint32_t (&rz)[TILES][2]) {
     cp_async_wait<S - 1>();  // this chunk's group has landed (S - 1 younger ones may be pending)
+    float sc[TILES][2], zs[TILES][2];
+#pragma unroll
+    for (int tl = 0; tl < TILES; ++tl)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        if (kLate) {
+          const float s = __uint_as_float(rs[tl][h] << 16), z = __uint_as_float(rz[tl][h] << 16);
+          // without FOLD the nibble goes to the top mantissa bits of 1.0 (v = 1 + code / 16) and one FMA
+          // gives (code - zp) * s = v * (16 s) - (16 + zp) * s, the constant exact to 2^-24 of 16 s
+          sc[tl][h] = FOLD ? s : 16.f * s;
+          zs[tl][h] = FOLD ? -(128.f + z) : -(16.f + z) * s;
+        } else {
+          sc[tl][h] = __uint_as_float(rs[tl][h]);
+          zs[tl][h] = __uint_as_float(rz[tl][h]);
+        }
+      }
     const uint4* st = my_ring + st_use * SV;
     st_use = st_use + 1 == S ? 0 : st_use + 1;
     if constexpr (FOLD) {
@@ -670,7 +703,7 @@ wq_gemv_mma_v2_kernel(const __nv_bfloat16* __restrict__ x, const uint8_t* __rest
 #pragma unroll
           for (int h = 0; h < 2; ++h)
 #pragma unroll
-            for (int j = 0; j < 4; ++j) a[h][j] = ((wv[h][i] >> (4 * j)) & 0x000F000Fu) | 0x43004300u;
+            for (int j = 0; j < 4; ++j) a[h][j] = and_or(wv[h][i] >> (4 * j), 0x000F000Fu, 0x43004300u);
           mma_bf16_16816(tmp, a[0][0], a[1][0], a[0][1], a[1][1], px[4 * i], px[4 * i + 1]);
           mma_bf16_16816(tmp, a[0][2], a[1][2], a[0][3], a[1][3], px[4 * i + 2], px[4 * i + 3]);
         }
@@ -729,7 +762,14 @@ wq_gemv_mma_v2_kernel(const __nv_bfloat16* __restrict__ x, const uint8_t* __rest
 #pragma unroll
   for (int s = 0; s < S - 1; ++s) issue_w();
   uint32_t xa[KL / 2], xb[KL / 2];
-  float sa[TILES][2], za[TILES][2], sb[TILES][2], zb[TILES][2];
+  uint32_t sa[TILES][2], za[TILES][2], sb[TILES][2], zb[TILES][2];
+#pragma unroll
+  for (int tl = 0; tl < TILES; ++tl)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      sa[tl][h] = sb[tl][h] = 0u;
+      za[tl][h] = zb[tl][h] = 0x4100u;  // zero point 8
+    }
   load_x(kw, xa);
   load_s(kw, sa, za);
   for (int c = kw; c < n_chunks; c += 2 * KS) {
@@ -766,6 +806,164 @@ wq_gemv_mma_v2_kernel(const __nv_bfloat16* __restrict__ x, const uint8_t* __rest
       y[(size_t)r * ldy + n] = __float2bfloat16(a);
     }
   }
+}
+
+// 4-bit GEMV with x in registers: groups of at least 128 k, 6144 < K <= 8192, at most 8 rows of x.
+// The form above reads a warp's slice of x again for each weight tile (2 KB of x for 2 KB of weights with two
+// tiles). Here a warp owns four chunks (512 k) for good and keeps their x fragments (64 registers) and per-chunk
+// sums of x (8) while the CTA walks over the row tiles of 16 output columns; a lane fetches the scale and zero
+// point of ONE chunk per weight row, a tile ahead, and the quad exchanges them. The warps meet in shared memory
+// once per tile, in two buffers, so that one barrier per tile is enough. Weights run through a per-warp cp.async
+// ring kX4Stages - 1 tiles (4 KB each) ahead. The arithmetic per chunk is that of the FOLD form above.
+// 5 x 28672 x 8192: 56.9 us before, 45.1 us with the form above as it is now, 38.6 us here (3.0 TB/s; ALU pipe 50 %
+// busy, then the chains of one tile's 32 MMAs: 16 warps are all that 64 registers of x leave room for).
+// Extracting two of the four nibbles of a half word with multiplies on the FMA pipe: 46.2 us.
+constexpr int kX4Stages = 3;
+constexpr int kX4Chunks = 4;           // chunks of 128 k per warp
+constexpr int kX4MaxWarps = 16;
+constexpr int kX4RedStride = 136;      // floats per warp: 8 modulo 32, so four warps' rows hit different banks
+constexpr int kX4WarpVecs = kX4Stages * kX4Chunks * 2 * 32;  // uint4 of ring per warp
+constexpr int kX4WarpBytes = kX4WarpVecs * 16 + 2 * kX4RedStride * 4;
+
+__global__ void __launch_bounds__(kX4MaxWarps * 32, 1)
+wq4_gemv_xreg_kernel(const __nv_bfloat16* __restrict__ x, const uint8_t* __restrict__ w,
+                     const __nv_bfloat16* __restrict__ scale, const __nv_bfloat16* __restrict__ zero,
+                     const __nv_bfloat16* __restrict__ bias, __nv_bfloat16* __restrict__ y, int M, int N, int K,
+                     int gshift, long long ldx, long long ldy) {
+  extern __shared__ uint4 gemv_ring[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int warps = blockDim.x >> 5;
+  uint4* ring = gemv_ring + (size_t)warp * kX4WarpVecs + lane;
+  float* red = reinterpret_cast<float*>(gemv_ring + (size_t)warps * kX4WarpVecs);  // [2][warps][kX4RedStride]
+  const int c0 = warp * kX4Chunks;
+  const int chunks = min(kX4Chunks, K / 128 - c0);  // of this warp: at least one
+  const int gpr = K >> gshift;
+  const size_t row_bytes = (size_t)K / 2;
+  const int tiles = (N + 15) / 16;
+
+  auto issue_w = [&](int tile, int stage) {
+    if (tile < tiles) {
+      const uint8_t* p0 = w + (size_t)min(tile * 16 + g, N - 1) * row_bytes + c0 * 64 + t * 16;
+      const uint8_t* p1 = w + (size_t)min(tile * 16 + g + 8, N - 1) * row_bytes + c0 * 64 + t * 16;
+      uint4* dst = ring + stage * (kX4Chunks * 2 * 32);
+#pragma unroll
+      for (int c = 0; c < kX4Chunks; ++c)
+        if (c < chunks) {
+          cp_async_16(dst + (2 * c) * 32, p0 + c * 64);
+          cp_async_16(dst + (2 * c + 1) * 32, p1 + c * 64);
+        }
+    }
+    cp_async_commit();  // also when there is nothing to request: the group count stays uniform
+  };
+  // scale and zero point of chunk c0 + t for the lane's two weight rows, as they are: any arithmetic on
+  // them here would make the warp wait for the load, a tile before it is needed
+  auto load_sz = [&](int tile, uint32_t (&rs)[2], uint32_t (&rz)[2]) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      if (tile < tiles && t < chunks) {
+        const size_t i = (size_t)min(tile * 16 + g + 8 * h, N - 1) * gpr + (((c0 + t) * 128) >> gshift);
+        rs[h] = ldg_u16(scale + i);
+        if (zero) rz[h] = ldg_u16(zero + i);
+      }
+    }
+  };
+
+  int tile = blockIdx.x;
+#pragma unroll
+  for (int s = 0; s < kX4Stages - 1; ++s) issue_w(tile + s * gridDim.x, s);
+  uint32_t rs[2] = {0u, 0u}, rz[2] = {0x4100u, 0x4100u};  // scale 0, zero point 8
+  load_sz(tile, rs, rz);
+
+  // x pairs (k, k + 4) of every run of 8 k, and each chunk's sum of x per column; all loads first
+  uint32_t px[kX4Chunks][16];
+  float xs[kX4Chunks][2];
+  {
+    const uint4* xp = reinterpret_cast<const uint4*>(x + (size_t)(g < M ? g : 0) * ldx + c0 * 128 + t * 32);
+#pragma unroll
+    for (int c = 0; c < kX4Chunks; ++c)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        uint4 v = make_uint4(0u, 0u, 0u, 0u);
+        if (g < M && c < chunks) v = __ldg(xp + c * 16 + i);
+        px[c][4 * i] = v.x; px[c][4 * i + 1] = v.y; px[c][4 * i + 2] = v.z; px[c][4 * i + 3] = v.w;
+      }
+#pragma unroll
+    for (int c = 0; c < kX4Chunks; ++c) {
+      float sum[4] = {0.f, 0.f, 0.f, 0.f};
+      constexpr uint32_t kOnes = 0x3F803F80u;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const uint32_t v0 = px[c][4 * i], v1 = px[c][4 * i + 1], v2 = px[c][4 * i + 2], v3 = px[c][4 * i + 3];
+        px[c][4 * i + 0] = __byte_perm(v0, v2, 0x5410);
+        px[c][4 * i + 1] = __byte_perm(v0, v2, 0x7632);
+        px[c][4 * i + 2] = __byte_perm(v1, v3, 0x5410);
+        px[c][4 * i + 3] = __byte_perm(v1, v3, 0x7632);
+        mma_bf16_16816(sum, kOnes, kOnes, kOnes, kOnes, px[c][4 * i], px[c][4 * i + 1]);
+        mma_bf16_16816(sum, kOnes, kOnes, kOnes, kOnes, px[c][4 * i + 2], px[c][4 * i + 3]);
+      }
+      xs[c][0] = sum[0];
+      xs[c][1] = sum[1];
+    }
+  }
+
+  int stage = 0, fill = kX4Stages - 1, buf = 0;
+  for (; tile < tiles; tile += gridDim.x) {
+    issue_w(tile + (kX4Stages - 1) * gridDim.x, fill);
+    fill = fill + 1 == kX4Stages ? 0 : fill + 1;
+    const uint32_t sz[2] = {rs[0] | (rz[0] << 16), rs[1] | (rz[1] << 16)};
+    load_sz(tile + gridDim.x, rs, rz);
+    cp_async_wait<kX4Stages - 1>();  // this tile's group has landed; a lane reads back its own pieces only
+    const uint4* st = ring + stage * (kX4Chunks * 2 * 32);
+    stage = stage + 1 == kX4Stages ? 0 : stage + 1;
+    float acc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int c = 0; c < kX4Chunks; ++c) {
+      if (c < chunks) {
+        const uint4 w0 = st[(2 * c) * 32], w1 = st[(2 * c + 1) * 32];
+        const uint32_t wv[2][4] = {{w0.x, w0.y, w0.z, w0.w}, {w1.x, w1.y, w1.z, w1.w}};
+        float tmp[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          uint32_t a[2][4];
+#pragma unroll
+          for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) a[h][j] = and_or(wv[h][i] >> (4 * j), 0x000F000Fu, 0x43004300u);
+          mma_bf16_16816(tmp, a[0][0], a[1][0], a[0][1], a[1][1], px[c][4 * i], px[c][4 * i + 1]);
+          mma_bf16_16816(tmp, a[0][2], a[1][2], a[0][3], a[1][3], px[c][4 * i + 2], px[c][4 * i + 3]);
+        }
+        // accumulator element ci: weight row g + 8 (ci / 2), x row 2 t + (ci & 1)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const uint32_t q = __shfl_sync(0xffffffffu, sz[h], (lane & 28) | c);
+          const float s = __uint_as_float(q << 16), z = -(128.f + __uint_as_float(q & 0xffff0000u));
+          acc[2 * h] = fmaf(s, fmaf(z, xs[c][0], tmp[2 * h]), acc[2 * h]);
+          acc[2 * h + 1] = fmaf(s, fmaf(z, xs[c][1], tmp[2 * h + 1]), acc[2 * h + 1]);
+        }
+      }
+    }
+    float* rb = red + (size_t)buf * warps * kX4RedStride;
+    buf ^= 1;
+    *reinterpret_cast<float4*>(rb + warp * kX4RedStride + lane * 4) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+    // the next tile writes the other buffer, and the one after it waits at the next barrier for these reads
+    __syncthreads();
+    for (int idx = threadIdx.x; idx < 512; idx += blockDim.x) {  // four lanes per output, whole warps
+      const int part = idx & 3, e = idx >> 2;
+      float a = 0.f;
+      for (int i = part; i < warps; i += 4) a += rb[i * kX4RedStride + e];
+      a += __shfl_xor_sync(0xffffffffu, a, 1);
+      a += __shfl_xor_sync(0xffffffffu, a, 2);
+      // element e = (lane l, register ci) = (column g + 8 * (ci / 2), row 2 t + (ci & 1))
+      const int l = e >> 2, ci = e & 3;
+      const int n = tile * 16 + (l >> 2) + ((ci & 2) ? 8 : 0);
+      const int r = 2 * (l & 3) + (ci & 1);
+      if (part == 0 && n < N && r < M) {
+        if (bias) a += __bfloat162float(bias[n]);
+        y[(size_t)r * ldy + n] = __float2bfloat16(a);
+      }
+    }
+  }
+  cp_async_wait<0>();
 }
 
 // ------------------------------------------------------------------ quantise / dequantise
@@ -1009,6 +1207,22 @@ int tpb_wq_gemv(const void* x, const void* w, const void* scale, const void* zer
         } else {
           // groups of at least one 128-k chunk: scale and zero point applied per chunk, not per weight
           const bool fold = gshift >= 7 && g_gemv_force_simt != 4;
+          // x in registers where its slices fill 13 to 16 warps: M = 5, K x N, us there / in the better form below:
+          // 6272 x 10000 15.6 / 18.9, 7680 x 8192 15.6 / 15.6, 8192 x 1024 6.7 / 11.5, 8192 x 28672 38.6 / 45.1;
+          // with 9 warps 4224 x 28672 28.5 / 25.1, with two row tiles of 8 warps 4096 x 14336 17.0 / 14.0
+          const int warps = (K / 128 + kX4Chunks - 1) / kX4Chunks;
+          if (fold && g_gemv_tiles == 0 && warps > 12 && warps <= kX4MaxWarps) {
+            const int row_tiles = (N + 15) / 16;
+            static bool opted_in = false;
+            if (!opted_in) {
+              cudaFuncSetAttribute(wq4_gemv_xreg_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   kX4MaxWarps * kX4WarpBytes);
+              opted_in = true;
+            }
+            wq4_gemv_xreg_kernel<<<row_tiles < sm_count() ? row_tiles : sm_count(), warps * 32, warps * kX4WarpBytes,
+                                   st>>>(xs, wp, sc, zp, bs, ys, rows, N, K, gshift, ldx, ldy);
+            continue;
+          }
           if (fold && tiles == 2) launch(wq_gemv_mma_v2_kernel<4, 2, 4, true, true>, GemvRing<2>::kBytes, 6);
           else if (fold) launch(wq_gemv_mma_v2_kernel<4, 1, 4, true, true>, GemvRing<1>::kBytes, 7);
           else if (tiles == 2) launch(wq_gemv_mma_v2_kernel<4, 2, 4, true>, GemvRing<2>::kBytes, 4);
