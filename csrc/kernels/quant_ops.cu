@@ -1142,7 +1142,7 @@ int tpb_gemm_i8(const void* A, const void* B, void* C, const float* a_scale, con
 }
 
 static int g_gemv_tiles = 0;       // 0: pick by N; 1 / 2: 16-column tiles per CTA of the MMA kernel
-static int g_gemv_force_simt = 0;  // 0 / 2: second MMA version (default); 1: always the CUDA-core kernel; 3: first MMA version; 4: second version with per-weight scaling for 4 bits too
+static int g_gemv_force_simt = 0;  // 0 / 2: second MMA version, or x in registers where the dispatch says so (default); 1: always the CUDA-core kernel; 3: first MMA version; 4: second version with per-weight scaling for 4 bits too
 // Tuning / comparison knobs of the weight-only GEMV (process-wide).
 int tpb_wq_gemv_config(int tiles, int force_simt) {
   g_gemv_tiles = (tiles == 1 || tiles == 2) ? tiles : 0;
