@@ -21,6 +21,17 @@ def _rows_view(x: torch.Tensor):
     return x2, H
 
 
+def _check_width(x, weight, bias=None, residual=None) -> None:
+    """The kernels take the width from ``x`` and read that much of every other operand: one that is shorter (an empty
+    placeholder of a sharded parameter, a weight of another width) would be read past its end."""
+    H = x.shape[-1]
+    if weight.numel() != H or (bias is not None and bias.numel() != H):
+        raise ValueError(f"norm: weight {tuple(weight.shape)}" + (f" / bias {tuple(bias.shape)}" if bias is not None else "")
+                         + f" does not match rows of {H}")
+    if residual is not None and (residual.shape[-1] != H or residual.numel() != x.numel()):
+        raise ValueError(f"norm: residual {tuple(residual.shape)} does not match {tuple(x.shape)}")
+
+
 def _native_ok(x, w):
     return x.is_cuda and x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and x.shape[-1] % 8 == 0
 
@@ -90,6 +101,7 @@ def rms_norm(x: torch.Tensor, weight: torch.Tensor, eps: float = 1e-5,
     that the add, the statistics and the scale cost one pass over HBM.
     """
     if _native_ok(x, weight) and use_native(x, weight):
+        _check_width(x, weight, None, residual)
         y, r = _RMSNormFn.apply(x, weight, eps, residual)
         return (y, r) if residual is not None else y
     h = x if residual is None else (x + residual)
@@ -137,5 +149,6 @@ class _LayerNormFn(torch.autograd.Function):
 def layer_norm(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] = None,
                eps: float = 1e-5) -> torch.Tensor:
     if _native_ok(x, weight) and use_native(x, weight):
+        _check_width(x, weight, bias)
         return _LayerNormFn.apply(x, weight, bias, eps)
     return torch.nn.functional.layer_norm(x, (x.shape[-1],), weight, bias, eps)

@@ -1,0 +1,38 @@
+"""Operands whose sizes do not belong together are refused on the host, before a kernel is given their addresses."""
+import pytest
+import torch
+
+import tensorplay_b200.ops as O
+from tensorplay_b200.ops import norm
+
+
+def _bf16(*shape):
+    return torch.zeros(shape, dtype=torch.bfloat16)
+
+
+@pytest.fixture
+def as_native(monkeypatch):
+    """CPU tensors take the native branch of the norms; a launch would fail the test."""
+    def no_launch(*a):
+        raise AssertionError("a kernel would have been launched")
+
+    monkeypatch.setattr(norm, "_native_ok", lambda x, w: True)
+    monkeypatch.setattr(norm, "use_native", lambda *t: True)
+    monkeypatch.setattr(norm, "lib", no_launch)
+
+
+@pytest.mark.parametrize("width", [0, 8, 32])
+def test_norm_weight_of_another_width(as_native, width):
+    x = _bf16(2, 3, 16)
+    with pytest.raises(ValueError):
+        O.rms_norm(x, _bf16(width))
+    with pytest.raises(ValueError):
+        O.layer_norm(x, _bf16(width), None)
+    with pytest.raises(ValueError):
+        O.layer_norm(x, _bf16(16), _bf16(width))
+
+
+@pytest.mark.parametrize("shape", [(1, 3, 16), (2, 3, 8), (2, 6, 16)])
+def test_norm_residual_of_another_shape(as_native, shape):
+    with pytest.raises(ValueError):
+        O.rms_norm(_bf16(2, 3, 16), _bf16(16), residual=_bf16(*shape))
