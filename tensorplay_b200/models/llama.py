@@ -104,9 +104,20 @@ class LlamaBlock(nn.Module):
         gu = ops.linear(h, self.w_gate_up)
         return x + ops.linear(ops.swiglu_packed(gu), self.w_down)
 
+    def _shapes_as_configured(self, x: Tensor, cos: Tensor, sin: Tensor) -> bool:
+        """Whether every operand has the shape that the native halves of the block read it with. They take all sizes from
+        ``cfg``; a pruned or widened weight, the empty placeholder of a sharded one or an input of another width goes
+        operator by operator, where sizes come from the tensors and a mismatch raises."""
+        cfg = self.cfg
+        H, I, A, D = cfg.hidden_size, cfg.ffn_size, cfg.num_heads * cfg.head_dim, cfg.head_dim
+        return (x.dim() == 3 and x.shape[2] == H and self.attn_norm.shape == (H,) and self.ffn_norm.shape == (H,)
+                and self.wqkv.shape == (A + 2 * cfg.num_kv_heads * D, H) and self.wo.shape == (H, A)
+                and self.w_gate_up.shape == (2 * I, H) and self.w_down.shape == (H, I)
+                and cos.dim() == 2 and cos.shape == sin.shape and cos.shape[1] == D // 2)
+
     def _plain_inference(self, x: Tensor, cos: Tensor, sin: Tensor) -> bool:
-        """Whether a forward pass with a cache may go to the native halves of the block: plain CUDA bf16 tensors, no
-        gradient, and nothing that watches or transforms single operators."""
+        """Whether a forward pass with a cache may go to the native halves of the block: plain CUDA bf16 tensors of the
+        configured shapes, no gradient, and nothing that watches or transforms single operators."""
         if torch.is_grad_enabled() or type(x) is not Tensor or not x.is_cuda or x.dtype != torch.bfloat16 \
                 or not x.is_contiguous() or x.data_ptr() % 16 or x.numel() == 0 or self.cfg.head_dim not in (64, 128):
             return False
@@ -123,7 +134,7 @@ class LlamaBlock(nn.Module):
             if type(t) is not Tensor or t.dtype != torch.float32 or t.device != dev or not t.is_contiguous() \
                     or t.data_ptr() % 16:
                 return False
-        return dev.index == torch._C._cuda_getDevice() and use_native(x)
+        return self._shapes_as_configured(x, cos, sin) and dev.index == torch._C._cuda_getDevice() and use_native(x)
 
     def _infer_cached(self, x: Tensor, cos: Tensor, sin: Tensor, position_ids: Optional[Tensor], cache) -> Tensor:
         """The block as two native calls around the cache and the attention. Of at most 128 rows the last product is

@@ -86,3 +86,29 @@ def test_pair_append_strides():
     kv_append_pair(cache[0], cache[1], k, v, 9)
     assert torch.equal(cache[0][:, :, 9:14], k) and torch.equal(cache[1][:, :, 9:14], v)
     assert cache[:, :, :, :9].abs().max() == 0 and cache[:, :, :, 14:].abs().max() == 0
+
+
+@pytest.mark.parametrize("ffn", [264, 392])
+def test_pruned_and_widened_ffn(ffn):
+    """A block whose FFN was replaced by one of another width than configured."""
+    m = _model()
+    with torch.no_grad():
+        for blk in m.layers:
+            blk.w_gate_up = torch.nn.Parameter(torch.randn(2 * ffn, 256, device=DEV).mul(0.02).bfloat16())
+            blk.w_down = torch.nn.Parameter(torch.randn(256, ffn, device=DEV).mul(0.02).bfloat16())
+    tok = torch.randint(0, 512, (2, 30), device=DEV)
+    fast = _run(m, tok, (29, 30), DynamicCache(), False)
+    slow = _run(m, tok, (29, 30), DynamicCache(), True)
+    O.check_status()
+    assert torch.equal(fast, slow)   # the same operators
+
+
+def test_wrong_sizes_raise():
+    m = _model()
+    blk, (cos, sin) = m.layers[0], m.rope_tables(16, torch.device(DEV))
+    with torch.no_grad():
+        with pytest.raises(ValueError):
+            blk(torch.zeros(1, 4, 264, device=DEV, dtype=torch.bfloat16), cos, sin, None, DynamicCache())
+        blk.attn_norm.data = torch.empty(0, device=DEV, dtype=torch.bfloat16)   # as a sharding engine leaves it
+        with pytest.raises(ValueError):
+            blk(torch.zeros(1, 4, 256, device=DEV, dtype=torch.bfloat16), cos, sin, None, DynamicCache())

@@ -3,6 +3,7 @@ import pytest
 import torch
 
 import tensorplay_b200.ops as O
+from tensorplay_b200.models.llama import LlamaBlock, LlamaConfig
 from tensorplay_b200.ops import norm
 
 
@@ -36,3 +37,19 @@ def test_norm_weight_of_another_width(as_native, width):
 def test_norm_residual_of_another_shape(as_native, shape):
     with pytest.raises(ValueError):
         O.rms_norm(_bf16(2, 3, 16), _bf16(16), residual=_bf16(*shape))
+
+
+@pytest.mark.parametrize("name,shape", [
+    (None, None), ("attn_norm", (0,)), ("wqkv", (0,)), ("ffn_norm", (72,)), ("wqkv", (5 * 16, 64)), ("wo", (64, 80)),
+    ("w_gate_up", (2 * 88, 64)), ("w_gate_up", (2 * 104, 64)), ("w_down", (64, 88)), ("x", (1, 4, 72)), ("x", (4, 64)),
+    ("cos", (32, 16)), ("sin", (31, 8))])
+def test_block_shapes(name, shape):
+    """Only a block whose every operand has the configured shape may go to the native halves."""
+    cfg = LlamaConfig.tiny(hidden_size=64, num_heads=4, num_kv_heads=2, head_dim=16, ffn_size=96)
+    block = LlamaBlock(cfg, dtype=torch.bfloat16)
+    ops = dict(x=_bf16(1, 4, 64), cos=torch.zeros(32, 8), sin=torch.zeros(32, 8))
+    if name in ops:
+        ops[name] = torch.zeros(shape, dtype=ops[name].dtype)
+    elif name:
+        getattr(block, name).data = _bf16(*shape)
+    assert block._shapes_as_configured(**ops) == (name is None)
