@@ -117,7 +117,9 @@ class LlamaBlock(nn.Module):
 
     def _plain_inference(self, x: Tensor, cos: Tensor, sin: Tensor) -> bool:
         """Whether a forward pass with a cache may go to the native halves of the block: plain CUDA bf16 tensors of the
-        configured shapes, no gradient, and nothing that watches or transforms single operators."""
+        configured shapes, no gradient, and nothing that watches, transforms or replaces single steps."""
+        if getattr(self._attend_cached, "__func__", None) is not LlamaBlock._attend_cached:
+            return False   # a subclass or an instance brings its own cached attention
         if torch.is_grad_enabled() or type(x) is not Tensor or not x.is_cuda or x.dtype != torch.bfloat16 \
                 or not x.is_contiguous() or x.data_ptr() % 16 or x.numel() == 0 or self.cfg.head_dim not in (64, 128):
             return False

@@ -112,3 +112,14 @@ def test_wrong_sizes_raise():
         blk.attn_norm.data = torch.empty(0, device=DEV, dtype=torch.bfloat16)   # as a sharding engine leaves it
         with pytest.raises(ValueError):
             blk(torch.zeros(1, 4, 256, device=DEV, dtype=torch.bfloat16), cos, sin, None, DynamicCache())
+
+
+def test_own_cached_attention_is_called():
+    m = _model()
+    calls = []
+    blk = m.layers[1]
+    own = blk._attend_cached
+    blk._attend_cached = lambda *a: calls.append(1) or own(*a)
+    tok = torch.randint(0, 512, (2, 9), device=DEV)
+    _run(m, tok, (8, 9), DynamicCache(), False)
+    assert len(calls) == 2

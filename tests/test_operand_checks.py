@@ -53,3 +53,22 @@ def test_block_shapes(name, shape):
     elif name:
         getattr(block, name).data = _bf16(*shape)
     assert block._shapes_as_configured(**ops) == (name is None)
+
+
+def test_own_cached_attention_is_kept(monkeypatch):
+    """A subclass or an instance with its own cached attention never goes to the native halves."""
+    class Block(LlamaBlock):
+        def _attend_cached(self, *a):
+            return super()._attend_cached(*a)
+
+    cfg = LlamaConfig.tiny(hidden_size=64, num_heads=4, num_kv_heads=2, head_dim=16, ffn_size=96)
+    replaced = LlamaBlock(cfg, dtype=torch.bfloat16)
+    replaced._attend_cached = lambda *a: None
+    x, cos = _bf16(1, 4, 64), torch.zeros(32, 8)
+    asked = []
+    monkeypatch.setattr(torch, "is_grad_enabled", lambda: asked.append(1) or True)   # the first question after the method
+    for block, goes_on in ((LlamaBlock(cfg, dtype=torch.bfloat16), True), (Block(cfg, dtype=torch.bfloat16), False),
+                           (replaced, False)):
+        asked.clear()
+        assert not block._plain_inference(x, cos, cos)
+        assert bool(asked) == goes_on
