@@ -18,6 +18,7 @@ from torch import Tensor, nn
 from .. import _native, ops
 from ..ops import _ckpt
 from ..ops._common import lib, status_word, stream_ptr, use_native
+from ..ops.rope import flat_positions
 
 
 @dataclass
@@ -145,10 +146,8 @@ class LlamaBlock(nn.Module):
         B, T, H = x.shape
         Hq, Hkv, D, I = cfg.num_heads, cfg.num_kv_heads, cfg.head_dim, cfg.ffn_size
         off = cache.get_seq_length(self.layer_idx)
-        pos = None
-        if position_ids is not None:
-            pos = position_ids.reshape(-1).to(torch.int64).contiguous()
-        elif off + T > cos.shape[0]:
+        pos = flat_positions(position_ids, B * T, x.device)
+        if pos is None and off + T > cos.shape[0]:
             raise IndexError(f"rotary tables of {cos.shape[0]} positions are too short for position {off + T - 1}")
         rows, tot, L = B * T, Hq + 2 * Hkv, lib()
         st, stream = status_word(x.device).data_ptr(), stream_ptr()

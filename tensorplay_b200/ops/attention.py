@@ -298,8 +298,9 @@ def qkv_attention(qkv: torch.Tensor, cos: Optional[torch.Tensor], sin: Optional[
     B, T, _ = qkv.shape
     native = (qkv.is_cuda and qkv.dtype == torch.bfloat16 and head_dim in (64, 128)
               and use_native(qkv))
-    pos = None if position_ids is None else position_ids.reshape(-1).to(torch.int64).contiguous()
     if native:
+        from .rope import flat_positions
+        pos = None if cos is None else flat_positions(position_ids, B * T, qkv.device)
         if not qkv.is_contiguous():
             qkv = qkv.contiguous()
         return _QKVAttnFn.apply(qkv, cos, sin, pos, num_heads, num_kv_heads, head_dim, causal, scale,

@@ -22,6 +22,16 @@ def rope_tables(max_pos: int, dim: int, theta: float = 10000.0, device=None,
     return ang.cos().float().contiguous(), ang.sin().float().contiguous()
 
 
+def flat_positions(position_ids: Optional[torch.Tensor], tokens: int, device) -> Optional[torch.Tensor]:
+    """``position_ids`` as the kernels read them: one int64 per token, contiguous, on the device of the tokens."""
+    if position_ids is None:
+        return None
+    if position_ids.numel() != tokens or position_ids.device != device:
+        raise ValueError(f"rope: position_ids {tuple(position_ids.shape)} on {position_ids.device} do not give one position "
+                         f"for each of {tokens} tokens on {device}")
+    return position_ids.reshape(-1).to(torch.int64).contiguous()
+
+
 def _rope_ref(x, cos, sin, pos, interleaved, sign):
     # x: [B, T, H, D]
     B, T, H, D = x.shape
@@ -120,9 +130,7 @@ def apply_rope(x: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor,
                inplace: bool = False) -> torch.Tensor:
     """Rotate ``x`` of shape ``[B, T, H, D]``; ``position_ids`` is ``[B, T]`` int64 or None."""
     if x.is_cuda and x.dtype == torch.bfloat16 and x.shape[-1] % 16 == 0 and use_native(x):
-        pos = None
-        if position_ids is not None:
-            pos = position_ids.reshape(-1).to(torch.int64).contiguous()
+        pos = flat_positions(position_ids, x.shape[0] * x.shape[1], x.device)
         needs_grad = x.requires_grad or torch.is_grad_enabled() and x.grad_fn is not None
         if not inplace:
             if needs_grad:

@@ -109,6 +109,9 @@ def test_wrong_sizes_raise():
     with torch.no_grad():
         with pytest.raises(ValueError):
             blk(torch.zeros(1, 4, 264, device=DEV, dtype=torch.bfloat16), cos, sin, None, DynamicCache())
+        for pos in (torch.arange(4, device=DEV).view(1, 4), torch.arange(8).view(2, 4)):   # one row for two, and on the host
+            with pytest.raises(ValueError):
+                blk(torch.zeros(2, 4, 256, device=DEV, dtype=torch.bfloat16), cos, sin, pos, DynamicCache())
         blk.attn_norm.data = torch.empty(0, device=DEV, dtype=torch.bfloat16)   # as a sharding engine leaves it
         with pytest.raises(ValueError):
             blk(torch.zeros(1, 4, 256, device=DEV, dtype=torch.bfloat16), cos, sin, None, DynamicCache())

@@ -4,7 +4,7 @@ import torch
 
 import tensorplay_b200.ops as O
 from tensorplay_b200.models.llama import LlamaBlock, LlamaConfig
-from tensorplay_b200.ops import norm
+from tensorplay_b200.ops import attention, norm, rope
 
 
 def _bf16(*shape):
@@ -72,3 +72,22 @@ def test_own_cached_attention_is_kept(monkeypatch):
         asked.clear()
         assert not block._plain_inference(x, cos, cos)
         assert bool(asked) == goes_on
+
+
+@pytest.mark.parametrize("pos", [torch.arange(6).view(1, 6), torch.arange(13), torch.zeros(2, 6, device="meta", dtype=torch.long)])
+def test_positions_that_do_not_fit(monkeypatch, pos):
+    """One position per token, on the tokens' device: the kernels read as many as there are tokens."""
+    def no_launch(*a):
+        raise AssertionError("a kernel would have been launched")
+
+    class OnGpu(torch.Tensor):   # a CPU tensor that takes the native branches
+        is_cuda = True
+
+    for module in (attention, rope):
+        monkeypatch.setattr(module, "use_native", lambda *t: True)
+        monkeypatch.setattr(module, "lib", no_launch)
+    cos = torch.zeros(32, 32)
+    with pytest.raises(ValueError):
+        O.apply_rope(_bf16(2, 6, 4, 64).as_subclass(OnGpu), cos, cos, pos)
+    with pytest.raises(ValueError):
+        O.qkv_attention(_bf16(2, 6, 4 * 64).as_subclass(OnGpu), cos, cos, pos, 2, 1, 64)
