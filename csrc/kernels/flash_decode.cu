@@ -223,15 +223,21 @@ flash_decode_kernel(const DecodeParams p) {
     const int rr = x / VEC, d = (x % VEC) * 4;
     const int r = rt * kDecRows + rr;
     if (r >= p.R) break;
+    // Whether this split holds a key of the row is asked of the bounds: a maximum of -inf may also mean scores that are
+    // all NaN, which have to reach the output, and V at keys that are masked for the row may hold anything.
+    const int at_q = r / p.group + p.Tk - p.Tq;
+    const int last = min(k_end - 1, p.causal ? at_q : p.Tk - 1);
+    const int first = max(split * p.keys_per_split, p.window > 0 ? at_q - p.window + 1 : 0);
     float M = -INFINITY;
 #pragma unroll
     for (int w = 0; w < kDecWarps; ++w) M = fmaxf(M, sm_m[w][rr]);
+    const float mu = M == -INFINITY ? 0.f : M;
     float L = 0.f;
     float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (M != -INFINITY) {
+    if (first <= last) {
 #pragma unroll
       for (int w = 0; w < kDecWarps; ++w) {
-        const float f = dec_exp2(sm_m[w][rr] - M);
+        const float f = dec_exp2(sm_m[w][rr] - mu);
         L += f * sm_l[w][rr];
         const float4 a = *reinterpret_cast<const float4*>(&sm_o[w][rr][d]);
         o.x += f * a.x; o.y += f * a.y; o.z += f * a.z; o.w += f * a.w;
@@ -239,7 +245,7 @@ flash_decode_kernel(const DecodeParams p) {
     }
     const float inv = L > 0.f ? 1.f / L : 0.f;
     o.x *= inv; o.y *= inv; o.z *= inv; o.w *= inv;
-    const float lse2 = L > 0.f ? M + log2f(L) : -INFINITY;
+    const float lse2 = L > 0.f ? M + log2f(L) : (L == 0.f || p.n_splits == 1 ? -INFINITY : L);   // NaN stays NaN in a partial row
     if (p.n_splits > 1) {
       const long long row = (long long)(b * p.Hkv + hk) * p.R + r;
       const long long at = (long long)split * p.B * p.Hkv * p.R + row;

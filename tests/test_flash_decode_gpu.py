@@ -74,3 +74,33 @@ def test_token_major_views_and_backward():
     (rg,) = torch.autograd.grad(r, ref_in, do.float())
     assert ((o.float() - r).norm() / r.norm()).item() < 6e-3
     assert ((g.float() - rg).norm() / rg.norm()).item() < 1.5e-2
+
+
+@pytest.mark.parametrize("Tk", [100, 4097])
+@pytest.mark.parametrize("case", ["query", "key", "many keys", "value", "overflow"])
+def test_nan_and_infinity_reach_the_output(Tk, case):
+    """A NaN query row, one NaN key, whole splits of them, a NaN value, scores of +inf; rows without a key stay zero."""
+    torch.manual_seed(Tk)
+    B, Tq, Hq, Hkv, D = 2, 4, 8, 4, 64
+    q, k, v = (torch.randn(B, T, H, D, device=DEV).bfloat16() for T, H in ((Tq, Hq), (Tk, Hkv), (Tk, Hkv)))
+    if case == "query":
+        q[1, 2, 3] = float("nan")
+    elif case == "key":
+        k[0, 7, 1, 5] = float("nan")
+    elif case == "many keys":
+        k[0, : Tk - 50, 2] = float("nan")
+    elif case == "value":
+        v[0, 7, 1] = float("nan")
+    else:
+        q[0, 1, 0], k[0, 9, 0] = 1e25, 1e25
+    assert _few_rows(q, k, v)
+    o, lse = flash_fwd(q, k, v, True, D ** -0.5)
+    ref = O.attention_reference(q.float(), k.float(), v.float(), True)
+    assert torch.equal(o.isnan(), ref.isnan()) and ref.isnan().any()
+    fin = ~ref.isnan()
+    assert (o.float() - ref)[fin].abs().max().item() < 6 * 2.0 ** -8
+    rows = ~ref.isnan().all(-1).transpose(1, 2)
+    assert lse[:, :, :Tq][rows].isfinite().all()
+    none, _ = flash_fwd(q, k[:, :2], v[:, :2], True, D ** -0.5)   # the first two queries have no key
+    assert (none[:, :2] == 0).all()
+
