@@ -100,9 +100,13 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
 
 
 def _bias_grad(dy: torch.Tensor) -> torch.Tensor:
-    """Column sums of ``dy [rows, N]`` in fp32, rounded once to its dtype."""
+    """Column sums of ``dy [rows, N]`` in fp32, rounded once to its dtype. A gradient that is differentiated again, batched
+    or traced stays with the operators, which autograd and the transforms can follow."""
     rows, N = dy.shape
-    if not (rows and N and dy.dtype == torch.bfloat16 and N % 8 == 0 and dy.data_ptr() % 16 == 0
+    followed = (type(dy) is not torch.Tensor or (dy.requires_grad and torch.is_grad_enabled())
+                or torch._C._are_functorch_transforms_active() or torch._C._functorch.is_legacy_batchedtensor(dy)
+                or torch._C._len_torch_dispatch_stack() or torch.autograd.forward_ad._current_level >= 0)
+    if followed or not (rows and N and dy.dtype == torch.bfloat16 and N % 8 == 0 and dy.data_ptr() % 16 == 0
             and dy.is_contiguous() and use_native(dy)):
         return dy.float().sum(0).to(dy.dtype)
     L = lib()
