@@ -118,7 +118,7 @@ def _load(name: str):
 
 # kernel launches issued by one call of each entry point (for launch accounting)
 _LAUNCHES = {"tpb_rmsnorm_bwd": 2, "tpb_layernorm_bwd": 2, "tpb_bias_grad": 2, "tpb_bias_grad_chunks": 0, "tpb_flash_decode_splits": 0, "tpb_block_pre": 3, "tpb_block_post": 5, "tpb_flash_bwd": 3, "tpb_rmsnorm_bwd_grid": 0,
-             "tpb_grouped_workspace_ints": 0, "tpb_adamw_set_overlap": 0, "tpb_flash_fwd_config": 0, "tpb_gemm_set_splitk_workspace": 0, "tpb_grouped_gemm": 2}
+             "tpb_grouped_workspace_ints": 0, "tpb_zero": 0, "tpb_adamw_set_overlap": 0, "tpb_flash_fwd_config": 0, "tpb_gemm_set_splitk_workspace": 0, "tpb_grouped_gemm": 2}
 launch_count = 0
 
 # FLOP accounting of the native kernels: the op wrappers report every launch's floating-point work here, and an

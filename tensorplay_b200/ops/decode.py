@@ -43,7 +43,10 @@ class _EmbeddingFn(torch.autograd.Function):
 
 
 def _zero_(t: Tensor) -> Tensor:
-    if use_native(t) and t.is_contiguous():
+    """Zeroes a buffer by a memset; a tensor without memory of its own (traced, fake) and one that a mode watches by the
+    operator."""
+    if type(t) in (Tensor, torch.nn.Parameter) and not torch._C._len_torch_dispatch_stack() and t.is_contiguous() \
+            and not torch._C._are_functorch_transforms_active() and use_native(t):
         _native.check(lib().tpb_zero(ptr(t), t.numel() * t.element_size(), stream_ptr()), "tpb_zero")
         return t
     return t.zero_()
