@@ -84,6 +84,13 @@ def embedding(ids: Tensor, weight: Tensor) -> Tensor:
     return embedding_forward(ids, weight)
 
 
+def _append_fits(cache: Tensor, new: Tensor, pos: int) -> None:
+    """The kernels write ``new`` [B, H, T, D] by the cache's strides: past its end where it is smaller."""
+    B, H, T, D = new.shape
+    if B > cache.shape[0] or H > cache.shape[1] or D > cache.shape[3] or pos < 0 or pos + T > cache.shape[2]:
+        raise ValueError(f"kv_append: {tuple(new.shape)} at token {pos} does not fit a cache of {tuple(cache.shape)}")
+
+
 def kv_append(cache: Tensor, new: Tensor, pos, block_table: Optional[Tensor] = None,
               block_size: int = 0) -> Tensor:
     """Write ``new`` [B, H, T, D] into a cache at token position ``pos`` (int, or int32 tensor [B]).
@@ -97,6 +104,8 @@ def kv_append(cache: Tensor, new: Tensor, pos, block_table: Optional[Tensor] = N
     if use_native(cache, new) and new.dtype == torch.bfloat16 and cache.dtype == torch.bfloat16 and D % 8 == 0 \
             and new.stride(3) == 1 and cache.stride(3) == 1 \
             and all(s % 8 == 0 for s in new.stride()[:3] + cache.stride()[:3]):
+        if block_table is None and pos_t is None:
+            _append_fits(cache, new, int(pos))
         bt = None if block_table is None else block_table.to(torch.int32).contiguous()
         pt = None if pos_t is None else pos_t.to(torch.int32).contiguous()
         _native.check(lib().tpb_kv_append(
@@ -123,6 +132,9 @@ def kv_append_pair(k_cache: Tensor, v_cache: Tensor, k: Tensor, v: Tensor, pos: 
             and ks[3] == vs[3] == cs[3] == 1 and not k.shape[3] % 8
             and not (ks[0] | ks[1] | ks[2] | vs[0] | vs[1] | vs[2] | cs[0] | cs[1] | cs[2]) % 8
             and not (k.data_ptr() | v.data_ptr() | k_cache.data_ptr() | v_cache.data_ptr()) % 16 and use_native(k, v, k_cache)):
+        _append_fits(k_cache, k, int(pos))
+        if v_cache.shape != k_cache.shape:
+            _append_fits(v_cache, v, int(pos))
         B, H, T, D = k.shape
         _native.check(lib().tpb_kv_append2(
             k.data_ptr(), v.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), int(pos), B, T, H, D, ks[0], ks[2], ks[1],

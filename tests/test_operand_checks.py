@@ -4,7 +4,7 @@ import torch
 
 import tensorplay_b200.ops as O
 from tensorplay_b200.models.llama import LlamaBlock, LlamaConfig
-from tensorplay_b200.ops import attention, norm, rope
+from tensorplay_b200.ops import attention, decode, norm, rope
 
 
 def _bf16(*shape):
@@ -91,3 +91,18 @@ def test_positions_that_do_not_fit(monkeypatch, pos):
         O.apply_rope(_bf16(2, 6, 4, 64).as_subclass(OnGpu), cos, cos, pos)
     with pytest.raises(ValueError):
         O.qkv_attention(_bf16(2, 6, 4 * 64).as_subclass(OnGpu), cos, cos, pos, 2, 1, 64)
+
+
+@pytest.mark.parametrize("shape,pos", [((3, 2, 1, 16), 0), ((2, 3, 1, 16), 0), ((2, 2, 3, 16), 6), ((2, 2, 1, 16), 8),
+                                       ((2, 2, 1, 24), 0), ((2, 2, 1, 16), -1)])
+def test_append_outside_of_a_cache(monkeypatch, shape, pos):
+    def no_launch(*a):
+        raise AssertionError("a kernel would have been launched")
+
+    monkeypatch.setattr(decode, "use_native", lambda *t: True)
+    monkeypatch.setattr(decode, "lib", no_launch)
+    cache, new = _bf16(2, 2, 8, 16), _bf16(*shape)
+    with pytest.raises(ValueError):
+        O.kv_append(cache, new, pos)
+    with pytest.raises(ValueError):
+        decode.kv_append_pair(cache, cache.clone(), new, new, pos)
