@@ -8,7 +8,9 @@
 //   * K and V go from global memory straight into the B fragments. The sum over d (and over keys) is free of order,
 //     so a lane takes whole 16-byte pieces of a row and the query fragments are permuted alike: no shared memory, no
 //     ldmatrix, 8 KB in flight per warp (one 16-key step of K and one of V ahead);
-//   * the keys are split over CTAs until the chip is full; partial sums stay fp32 and a second kernel merges them.
+//   * the keys are split over CTAs until the chip is full; partial sums stay fp32. Up to eight splits of a row tile are
+//     one cluster that merges them through distributed shared memory, in rank order; more go through memory and a
+//     second kernel.
 // The same case takes 117 us (4.6 TB/s).
 // Scores, running maximum, sums and output accumulate in fp32; probabilities are rounded to bf16 for the second
 // product, as in flash_fwd_kernel.
@@ -20,12 +22,13 @@ namespace tpb {
 constexpr int kDecWarps = 4;
 constexpr int kDecRows = 16;   // query rows per CTA
 constexpr int kDecKeys = 16;   // keys per warp and step
+constexpr int kDecCluster = 8; // splits that one cluster can hold (the portable size)
 
 struct DecodeParams {
   const __nv_bfloat16 *q, *k, *v;
   __nv_bfloat16* o;
   float* lse;
-  float* part_o;    // [n_splits][B * Hkv * R][D], null when n_splits == 1
+  float* part_o;    // [n_splits][B * Hkv * R][D]; null when n_splits == 1 or the splits of a row tile are one cluster
   float* part_lse;  // [n_splits][B * Hkv * R], log2 domain
   int B, Tq, Tk, Hq, Hkv, group, R, row_tiles, causal, window, lse_stride, n_splits, keys_per_split;
   float scale_log2e;
@@ -65,7 +68,7 @@ flash_decode_kernel(const DecodeParams p) {
   constexpr int NP = D / 32;   // 16-byte pieces of a K row per lane
   constexpr int VP = D / 64;   // 16-byte pieces of a V row per lane
   __shared__ float sm_o[kDecWarps][kDecRows][D];
-  __shared__ float sm_m[kDecWarps][kDecRows], sm_l[kDecWarps][kDecRows];
+  __shared__ float sm_m[kDecWarps][kDecRows], sm_l[kDecWarps][kDecRows], sm_lse[kDecRows];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int gq = lane >> 2, t = lane & 3;
   const int split = blockIdx.x, hk = blockIdx.y / p.row_tiles, rt = blockIdx.y % p.row_tiles, b = blockIdx.z;
@@ -219,6 +222,14 @@ flash_decode_kernel(const DecodeParams p) {
   }
   __syncthreads();
   constexpr int VEC = D / 4;   // float4 per row
+  auto store = [&](int r, int d, const float4& o, float lse2) {
+    const int tq = r / p.group, h = hk * p.group + r % p.group;
+    uint2 w;
+    w.x = dec_pack(o.x, o.y);
+    w.y = dec_pack(o.z, o.w);
+    *reinterpret_cast<uint2*>(p.o + b * p.o_batch + (long long)tq * p.o_tok + (long long)h * p.o_head + d) = w;
+    if (d == 0) p.lse[((long long)b * p.Hq + h) * p.lse_stride + tq] = lse2 * 0.6931471805599453f;
+  };
   for (int x = threadIdx.x; x < kDecRows * VEC; x += kDecWarps * 32) {
     const int rr = x / VEC, d = (x % VEC) * 4;
     const int r = rt * kDecRows + rr;
@@ -246,19 +257,51 @@ flash_decode_kernel(const DecodeParams p) {
     const float inv = L > 0.f ? 1.f / L : 0.f;
     o.x *= inv; o.y *= inv; o.z *= inv; o.w *= inv;
     const float lse2 = L > 0.f ? M + log2f(L) : (L == 0.f || p.n_splits == 1 ? -INFINITY : L);   // NaN stays NaN in a partial row
-    if (p.n_splits > 1) {
+    if (p.part_o) {
       const long long row = (long long)(b * p.Hkv + hk) * p.R + r;
       const long long at = (long long)split * p.B * p.Hkv * p.R + row;
       *reinterpret_cast<float4*>(p.part_o + at * D + d) = o;
       if (d == 0) p.part_lse[at] = lse2;
+    } else if (p.n_splits > 1) {
+      *reinterpret_cast<float4*>(&sm_o[0][rr][d]) = o;   // only this thread has read that place
+      if (d == 0) sm_lse[rr] = lse2;
     } else {
-      const int tq = r / p.group, h = hk * p.group + r % p.group;
-      uint2 w;
-      w.x = dec_pack(o.x, o.y);
-      w.y = dec_pack(o.z, o.w);
-      *reinterpret_cast<uint2*>(p.o + b * p.o_batch + (long long)tq * p.o_tok + (long long)h * p.o_head + d) = w;
-      if (d == 0) p.lse[((long long)b * p.Hq + h) * p.lse_stride + tq] = lse2 * 0.6931471805599453f;
+      store(r, d, o, lse2);
     }
+  }
+  if (p.n_splits > 1 && !p.part_o) {
+    // the splits are the CTAs of a cluster: each merges a slice of the rows, read in rank order
+    __syncthreads();
+    cluster_sync_all();
+    const int items = min(kDecRows, p.R - rt * kDecRows) * VEC;
+    const uint32_t o_sa = smem_u32(&sm_o[0][0][0]), l_sa = smem_u32(sm_lse);
+    for (int x = split * kDecWarps * 32 + threadIdx.x; x < items; x += p.n_splits * kDecWarps * 32) {
+      const int rr = x / VEC, d = (x % VEC) * 4;
+      float w[kDecCluster];
+      float4 v[kDecCluster];
+#pragma unroll
+      for (int s = 0; s < kDecCluster; ++s) {
+        w[s] = s < p.n_splits ? ld_cluster_f32(l_sa + rr * 4, s) : -INFINITY;
+        v[s] = s < p.n_splits ? ld_cluster_f4(o_sa + (rr * D + d) * 4, s) : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+      float M = -INFINITY;
+#pragma unroll
+      for (int s = 0; s < kDecCluster; ++s) M = fmaxf(M, w[s]);
+      const float mu = M == -INFINITY ? 0.f : M;
+      float den = 0.f;
+      float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int s = 0; s < kDecCluster; ++s) {
+        const float f = dec_exp2(w[s] - mu);
+        den += f;
+        o.x += f * v[s].x; o.y += f * v[s].y; o.z += f * v[s].z; o.w += f * v[s].w;
+      }
+      const float inv = den > 0.f ? 1.f / den : 0.f;
+      o.x *= inv; o.y *= inv; o.z *= inv; o.w *= inv;
+      store(rt * kDecRows + rr, d, o, den > 0.f ? M + log2f(den) : -INFINITY);
+    }
+    __syncthreads();
+    cluster_sync_all();   // nobody leaves while a peer may read its rows
   }
 }
 
@@ -308,15 +351,26 @@ flash_decode_merge_kernel(const DecodeParams p) {
     p.lse[((long long)b * p.Hq + h) * p.lse_stride + tq] = den > 0.f ? (M + log2f(den)) * 0.6931471805599453f : -INFINITY;
 }
 
-// Splits of the keys: the rounds of resident CTAs times the keys of one split is what a launch takes; a second kernel
-// and its partial rows cost about as much as 256 keys. Two CTAs of 128 threads fit an SM (registers).
-static int decode_splits(int B, int Hkv, int row_tiles, int Tk) {
-  const long long ctas = (long long)B * Hkv * row_tiles, slots = 2LL * sm_count();
+// Splits of the keys, by the time in ns that the launch takes. A CTA needs kKeyNs per key, more where several share an
+// SM (four of D = 64 fit by their registers, two of D = 128), kFullNs on a full chip, which for D = 128 is memory's rate,
+// and some 4 us from start to end. Splits that a cluster merges cost 1 us. More than kDecCluster of them need a second
+// kernel and scratch: 3 us + 60 ns a split on the device and 5 us on the host, which bounds a call over a short cache
+// (one token over 1000 keys: 32 us a call with one launch, 41 us with two). Measured, D x B x Hkv x Tk, splits: us:
+// 128 x 1 x 8 x 4096, 1: 76, 4: 22.8, 8: 13.8, by two kernels 16: 11.1; 128 x 16 x 8 x 4096, 1: 100, 2: 61, 4: 65, 8: 74;
+// 64 x 16 x 8 x 4096, 1: 66, 4: 29, 6: 37, 8: 32; 128 x 32 x 8 x 8192, 1: 222, 2: 227, 4: 236, 8: 255.
+static int decode_splits(int B, int Hkv, int row_tiles, int Tk, int D, int most) {
+  static const int kKeyNs[2][4] = {{11, 17, 21, 24}, {20, 27, 27, 27}}, kFullNs[2] = {24, 31};
+  const int fit = D == 64 ? 4 : 2;
+  const int* key_ns = kKeyNs[D == 64 ? 0 : 1];
+  const long long ctas = (long long)B * Hkv * row_tiles, sms = sm_count(), slots = fit * sms;
   int best = 1;
   long long best_cost = -1;
-  for (int n = 1; n <= 64 && (n == 1 || (Tk + n - 1) / n >= 128); ++n) {
-    const long long rounds = (ctas * n + slots - 1) / slots;
-    const long long cost = rounds * ((Tk + n - 1) / n + 64) + (n > 1 ? 256 : 0);
+  for (int n = 1; n <= most && (n == 1 || Tk / n >= 64); ++n) {
+    const long long keys = (Tk + n - 1) / n, full = ctas * n / slots, rest = ctas * n % slots;
+    long long cost = full * (keys * kFullNs[D == 64 ? 0 : 1] + 4000);
+    if (rest) cost += keys * key_ns[(rest + sms - 1) / sms - 1] + 4000;
+    if (n > kDecCluster) cost += 8000 + 60 * n;
+    else if (n > 1) cost += 1000;
     if (best_cost < 0 || cost < best_cost) { best = n; best_cost = cost; }
   }
   return best;
@@ -326,15 +380,17 @@ static int decode_splits(int B, int Hkv, int row_tiles, int Tk) {
 
 using namespace tpb;
 
-// Number of key splits tpb_flash_decode uses: with more than one, part_o holds n * B * Hq * Tq * D floats and part_lse
-// n * B * Hq * Tq.
-extern "C" int tpb_flash_decode_splits(int B, int Tq, int Tk, int Hq, int Hkv) {
+// Number of key splits to pass to tpb_flash_decode. Above tpb_flash_decode_cluster() of them part_o has to hold
+// n * B * Hq * Tq * D floats and part_lse n * B * Hq * Tq.
+extern "C" int tpb_flash_decode_cluster() { return kDecCluster; }
+extern "C" int tpb_flash_decode_splits(int B, int Tq, int Tk, int Hq, int Hkv, int D) {
   if (B <= 0 || Tq <= 0 || Tk <= 0 || Hkv <= 0) return 1;
   const int R = Tq * (Hq / Hkv);
-  return decode_splits(B, Hkv, (R + kDecRows - 1) / kDecRows, Tk);
+  return decode_splits(B, Hkv, (R + kDecRows - 1) / kDecRows, Tk, D, 64);
 }
 
-// Arguments as in tpb_flash_fwd_ex; lse [B, Hq, lse_stride].
+// Arguments as in tpb_flash_fwd_ex; lse [B, Hq, lse_stride]. n_splits 0: the best number that needs no part_o, which is
+// the best of all up to 2048 keys.
 extern "C" int tpb_flash_decode(const void* q, const void* k, const void* v, void* o, float* lse, float* part_o,
                                 float* part_lse, int B, int Tq, int Tk, int Hq, int Hkv, int D, long long q_tok,
                                 long long q_head, long long q_batch, long long k_tok, long long k_head,
@@ -343,16 +399,17 @@ extern "C" int tpb_flash_decode(const void* q, const void* k, const void* v, voi
                                 float scale, int window, int n_splits, void* stream) {
   TPB_NVTX("tpb_flash_decode");
   if (B <= 0 || Tq <= 0 || Hq <= 0) return 0;
-  if ((D != 64 && D != 128) || Hkv <= 0 || Hq % Hkv || Tk <= 0 || n_splits < 1 || B > 65535) return -2;
+  if ((D != 64 && D != 128) || Hkv <= 0 || Hq % Hkv || Tk <= 0 || n_splits < 0 || B > 65535) return -2;
   if ((q_tok | q_head | q_batch | k_tok | k_head | k_batch | v_tok | v_head | v_batch | o_tok | o_head | o_batch) % 8)
     return -2;
   if ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v) |
        reinterpret_cast<uintptr_t>(o)) & 15)
     return -2;
-  if (n_splits > 1 && (!part_o || !part_lse)) return -2;
+  if (n_splits > kDecCluster && (!part_o || !part_lse)) return -2;
+  if (n_splits == 0) n_splits = decode_splits(B, Hkv, (Tq * (Hq / Hkv) + kDecRows - 1) / kDecRows, Tk, D, kDecCluster);
   DecodeParams p;
   p.q = (const __nv_bfloat16*)q; p.k = (const __nv_bfloat16*)k; p.v = (const __nv_bfloat16*)v;
-  p.o = (__nv_bfloat16*)o; p.lse = lse; p.part_o = part_o; p.part_lse = part_lse;
+  p.o = (__nv_bfloat16*)o; p.lse = lse; p.part_o = n_splits > 1 ? part_o : nullptr; p.part_lse = part_lse;
   p.B = B; p.Tq = Tq; p.Tk = Tk; p.Hq = Hq; p.Hkv = Hkv; p.group = Hq / Hkv; p.R = Tq * p.group;
   p.row_tiles = (p.R + kDecRows - 1) / kDecRows;
   p.causal = causal; p.window = window > 0 ? window : 0; p.lse_stride = lse_stride; p.n_splits = n_splits;
@@ -363,9 +420,20 @@ extern "C" int tpb_flash_decode(const void* q, const void* k, const void* v, voi
   p.v_tok = v_tok; p.v_head = v_head; p.v_batch = v_batch; p.o_tok = o_tok; p.o_head = o_head; p.o_batch = o_batch;
   if ((long long)Hkv * p.row_tiles > 65535) return -2;
   const dim3 grid(n_splits, Hkv * p.row_tiles, B);
-  if (D == 128) flash_decode_kernel<128><<<grid, kDecWarps * 32, 0, (cudaStream_t)stream>>>(p);
-  else flash_decode_kernel<64><<<grid, kDecWarps * 32, 0, (cudaStream_t)stream>>>(p);
-  if (n_splits > 1) {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(kDecWarps * 32);
+  cfg.stream = (cudaStream_t)stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = n_splits > 1 && !p.part_o ? 1 : 0;
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = n_splits;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, D == 128 ? flash_decode_kernel<128> : flash_decode_kernel<64>, p);
+  if (e != cudaSuccess) return (int)e;
+  if (p.part_o) {
     const long long rows = (long long)B * Hkv * p.R;
     const unsigned blocks = (unsigned)((rows + 3) / 4);
     if (D == 128) flash_decode_merge_kernel<128><<<blocks, 128, 0, (cudaStream_t)stream>>>(p);

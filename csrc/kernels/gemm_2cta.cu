@@ -55,14 +55,6 @@ struct PairParams {
                      // 1 = operands of the k-block landed, 5 = its MMAs issued
 };
 
-__device__ __forceinline__ uint32_t cluster_ctarank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 // Arrive on the mbarrier at the same shared-memory offset in CTA `rank` of the cluster.
 __device__ __forceinline__ void mbar_arrive_remote(uint64_t* bar, uint32_t rank) {
   asm volatile(
@@ -552,23 +544,6 @@ struct PairSplitCfg {
   static constexpr int kLd = BN + 4;
   static_assert(128 * kLd * 4 <= PairCfg<BN>::kStages * PairCfg<BN>::kStageBytes, "the partial tile must fit the ring");
 };
-
-__device__ __forceinline__ uint32_t cluster_nctas() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ float4 ld_cluster_f4(uint32_t saddr, uint32_t rank) {
-  float4 v;
-  asm volatile(
-      "{\n\t.reg .b32 ra;\n\t"
-      "mapa.shared::cluster.u32 ra, %4, %5;\n\t"
-      "ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [ra];\n\t}"
-      : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
-      : "r"(saddr), "r"(rank)
-      : "memory");
-  return v;
-}
 
 template <int BN, bool A_MN, bool B_MN>
 __global__ void __launch_bounds__(kPairThreads, 1)

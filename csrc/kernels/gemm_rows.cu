@@ -39,31 +39,6 @@ struct RowsParams {
   unsigned long long wait_ns;
 };
 
-__device__ __forceinline__ uint32_t rows_rank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ uint32_t rows_size() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ void rows_cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ float4 rows_ld_remote(uint32_t saddr, uint32_t rank) {
-  float4 v;
-  asm volatile(
-      "{\n\t.reg .b32 ra;\n\t"
-      "mapa.shared::cluster.u32 ra, %4, %5;\n\t"
-      "ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [ra];\n\t}"
-      : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
-      : "r"(saddr), "r"(rank)
-      : "memory");
-  return v;
-}
-
 template <int NT, bool B_MN>
 __global__ void __launch_bounds__(kRowsThreads, 2)
 gemm_rows_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmA,
@@ -78,7 +53,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant_
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
   volatile uint32_t* abort_w = tmem_slot + 1;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int rank = (int)rows_rank(), csize = (int)rows_size();
+  const int rank = (int)cluster_ctarank(), csize = (int)cluster_nctas();
   const int tile = blockIdx.x / csize;
   const int n0 = tile * 128;
   const int k_blocks = (p.K + kRowsK - 1) / kRowsK;
@@ -183,7 +158,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant_
     while (globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
     __syncthreads();
   }
-  rows_cluster_sync();   // every partial tile of the cluster is in shared memory
+  cluster_sync_all();   // every partial tile of the cluster is in shared memory
   if (!*abort_w) {
     const uint32_t base = smem_u32(smem);
     for (int u = rank * kRowsThreads + (int)threadIdx.x; u < p.M * 32; u += csize * kRowsThreads) {
@@ -196,7 +171,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant_
         float4 t[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j)
-          t[j] = h0 + j < csize ? rows_ld_remote(at, h0 + j) : make_float4(0.f, 0.f, 0.f, 0.f);
+          t[j] = h0 + j < csize ? ld_cluster_f4(at, h0 + j) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
         for (int j = 0; j < 4; ++j) { acc.x += t[j].x; acc.y += t[j].y; acc.z += t[j].z; acc.w += t[j].w; }
       }
@@ -242,7 +217,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant_
       }
     }
   }
-  rows_cluster_sync();   // nobody leaves while a peer may read its tile
+  cluster_sync_all();   // nobody leaves while a peer may read its tile
   if (warp == 1) {
     tc_fence_after_sync();
     tmem_dealloc(tmem, Cfg::kTmemCols);

@@ -451,6 +451,44 @@ __host__ __device__ constexpr uint32_t make_idesc_i8(int m, int n) {
          ((uint32_t)(m >> 4) << 24);
 }
 
+// ---------------------------------------------------------------- thread-block clusters
+__device__ __forceinline__ uint32_t cluster_ctarank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ uint32_t cluster_nctas() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync_all() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// Value at the same shared-memory offset in CTA `rank` of the cluster.
+__device__ __forceinline__ float4 ld_cluster_f4(uint32_t saddr, uint32_t rank) {
+  float4 v;
+  asm volatile(
+      "{\n\t.reg .b32 ra;\n\t"
+      "mapa.shared::cluster.u32 ra, %4, %5;\n\t"
+      "ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [ra];\n\t}"
+      : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+      : "r"(saddr), "r"(rank)
+      : "memory");
+  return v;
+}
+__device__ __forceinline__ float ld_cluster_f32(uint32_t saddr, uint32_t rank) {
+  float v;
+  asm volatile(
+      "{\n\t.reg .b32 ra;\n\t"
+      "mapa.shared::cluster.u32 ra, %1, %2;\n\t"
+      "ld.shared::cluster.f32 %0, [ra];\n\t}"
+      : "=f"(v)
+      : "r"(saddr), "r"(rank)
+      : "memory");
+  return v;
+}
+
 // ---------------------------------------------------------------- GEMM epilogues
 // The bias of 32 consecutive output columns, shared by all rows a warp drains. Every lane reads the same
 // addresses, so the cost is the number of load instructions and their latency: four (bf16) or eight (fp32)

@@ -68,29 +68,32 @@ def _few_rows(q, k, v) -> bool:
     through the warp MMA. It reads them once per 16 rows while the 128-row tiles read them once per query head, and it
     splits the keys over the chip; at 64 rows (Tq = 8, groups of 8) the four reads through L2 are still half of those,
     and beyond 16 tokens the tensor-core tiles fill up."""
-    rows = q.shape[1] * (q.shape[2] // k.shape[2])
-    return (q.shape[1] <= 16 and rows <= 64 and q.shape[3] in (64, 128) and q.dtype == torch.bfloat16
-            and q.shape[2] % k.shape[2] == 0 and 0 < q.shape[0] <= 65535 and k.shape[2] * ((rows + 15) // 16) <= 65535
-            and rows > 0 and k.shape[1] > 0 and _strides_ok(q) and _strides_ok(k) and _strides_ok(v))
+    B, Tq, Hq, D = q.shape
+    Tk, Hkv = k.shape[1], k.shape[2]
+    rows = Tq * (Hq // Hkv)
+    return (Tq <= 16 and 0 < rows <= 64 and (D == 128 or D == 64) and q.dtype == torch.bfloat16 and Hq % Hkv == 0
+            and 0 < B <= 65535 and Hkv * ((rows + 15) // 16) <= 65535 and Tk > 0)
 
 
 def _flash_decode(q, k, v, o, lse, causal: bool, scale: float, window: int) -> None:
     B, Tq, Hq, D = q.shape
     Tk, Hkv = k.shape[1], k.shape[2]
     L = lib()
-    n = L.tpb_flash_decode_splits(B, Tq, Tk, Hq, Hkv)
-    part_o = part_lse = None
-    if n > 1:   # fp32 partial rows, merged by a second launch
-        part_o = torch.empty((n, B * Hq * Tq, D), dtype=torch.float32, device=q.device)
-        part_lse = torch.empty((n, B * Hq * Tq), dtype=torch.float32, device=q.device)
+    n = 0   # up to 2048 keys the launch picks its splits, which need no memory
+    part = part_lse = None
+    if Tk > 2048:
+        n = L.tpb_flash_decode_splits(B, Tq, Tk, Hq, Hkv, D)
+        if n > L.tpb_flash_decode_cluster():   # fp32 partial rows and their sums, merged by a second launch
+            rows = n * B * Hq * Tq
+            part = torch.empty(rows * (D + 1), dtype=torch.float32, device=q.device)
+            part_lse = part.data_ptr() + 4 * rows * D
+            _native.launch_count += 1
+    qs, ks, vs, os_ = q.stride(), k.stride(), v.stride(), o.stride()
     code = L.tpb_flash_decode(
-        q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr(), ptr(part_o), ptr(part_lse), B, Tq, Tk,
-        Hq, Hkv, D, q.stride(1), q.stride(2), q.stride(0), k.stride(1), k.stride(2), k.stride(0), v.stride(1),
-        v.stride(2), v.stride(0), o.stride(1), o.stride(2), o.stride(0), lse.shape[2], int(causal), float(scale),
-        int(window or 0), n, stream_ptr())
+        q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr(), ptr(part), part_lse, B, Tq, Tk, Hq, Hkv, D,
+        qs[1], qs[2], qs[0], ks[1], ks[2], ks[0], vs[1], vs[2], vs[0], os_[1], os_[2], os_[0], lse.shape[2], int(causal),
+        float(scale), int(window or 0), n, stream_ptr())
     _native.check(code, "tpb_flash_decode")
-    if n > 1:
-        _native.launch_count += 1
     if _native.flop_sinks:
         _native.add_flops("tpb.flash_attention_forward", 4 * B * Hq * Tq * Tk * D // (2 if causal and Tq == Tk else 1))
 

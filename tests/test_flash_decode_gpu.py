@@ -33,7 +33,10 @@ def _reference(q, k, v, causal, window):
 @pytest.mark.parametrize("B,Tq,Tk,Hq,Hkv,causal,window", [
     (1, 1, 1, 8, 8, True, 0),            # one key
     (2, 1, 63, 8, 2, True, 0),           # no split, ragged step
-    (1, 1, 4097, 32, 8, True, 0),        # many splits, one ragged key
+    (1, 1, 4097, 32, 8, True, 0),        # a full cluster of splits, one ragged key
+    (1, 1, 700, 16, 2, True, 0),         # a cluster, few keys each
+    (1, 2, 20001, 8, 2, True, 0),        # splits merged by a second launch
+    (1, 3, 30000, 8, 2, True, 5000),     # the same with a window: most splits have no key
     (3, 1, 1000, 16, 1, True, 0),        # a full 16-row tile
     (2, 3, 517, 24, 4, True, 0),         # 18 rows: two tiles, the second nearly empty
     (1, 8, 2051, 64, 8, True, 0),        # 64 rows
@@ -76,7 +79,7 @@ def test_token_major_views_and_backward():
     assert ((g.float() - rg).norm() / rg.norm()).item() < 1.5e-2
 
 
-@pytest.mark.parametrize("Tk", [100, 4097])
+@pytest.mark.parametrize("Tk", [100, 4097, 20001])   # one split, a cluster of them, two launches
 @pytest.mark.parametrize("case", ["query", "key", "many keys", "value", "overflow"])
 def test_nan_and_infinity_reach_the_output(Tk, case):
     """A NaN query row, one NaN key, whole splits of them, a NaN value, scores of +inf; rows without a key stay zero."""
@@ -104,3 +107,20 @@ def test_nan_and_infinity_reach_the_output(Tk, case):
     none, _ = flash_fwd(q, k[:, :2], v[:, :2], True, D ** -0.5)   # the first two queries have no key
     assert (none[:, :2] == 0).all()
 
+
+
+@pytest.mark.parametrize("n", range(1, 9))
+@pytest.mark.parametrize("D,Tk", [(64, 517), (128, 1030)])
+def test_every_cluster_size(n, D, Tk):
+    """Two row tiles, the second ragged, merged by clusters of any size, the last split short or empty."""
+    from tensorplay_b200.ops._common import lib, stream_ptr
+    torch.manual_seed(n)
+    B, Tq, Hq, Hkv = 2, 3, 12, 2
+    q, k, v = (torch.randn(B, T, H, D, device=DEV).bfloat16() for T, H in ((Tq, Hq), (Tk, Hkv), (Tk, Hkv)))
+    o, lse = torch.empty_like(q), torch.empty(B, Hq, 128, device=DEV)
+    strides = [t.stride(i) for t in (q, k, v, o) for i in (1, 2, 0)]
+    assert lib().tpb_flash_decode(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr(), None, None, B, Tq,
+                                  Tk, Hq, Hkv, D, *strides, 128, 1, D ** -0.5, 0, n, stream_ptr()) == 0
+    ref, rlse = _reference(q, k, v, True, 0)
+    assert (o.double() - ref).abs().max().item() < 6 * 2.0 ** -8
+    assert (lse[:, :, :Tq].double() - rlse).abs().max().item() < 2e-5 * rlse.abs().max().item()
