@@ -283,8 +283,22 @@ static int launch_rows(const CUtensorMap& tb, const CUtensorMap& ta, const RowsP
   return (int)cudaLaunchKernelEx(&cfg, gemm_rows_kernel<NT, B_MN>, tb, ta, p);
 }
 
-bool gemm_rows_takes(int M, int a_mn) {
-  return M <= 128 && !a_mn;
+// Which products of at most 128 rows go here; the others go to the persistent one-CTA kernel, which loads its next tile
+// under the stores of the last. What this kernel gains is the split of K over a cluster while there are fewer tiles
+// than CTAs that fit (two per SM), and the small column operand; what it pays is an epilogue of 3 us a round at 16 rows
+// and 9 us at 128, under which nothing is loaded. Measured on one B200, operands from memory, N x K: us here / there:
+//   M = 16: 14336 x 2048 15.0 / 17.3, 50304 x 768 20.4 / 21.4, 128256 x 2048 88 / 87
+//   M = 32: 28672 x 4096 41.2 / 45.1, 50304 x 768 22.3 / 21.4
+//   M = 64: 6144 x 1024 9.4 / 11.2, 14336 x 2048 18.5 / 16.6, 28672 x 4096 45.9 / 46.6, 128256 x 4096 182 / 176
+//   M = 128: 4096 x 1024 9.3 / 11.1, 4096 x 14336 32 / 70, 6144 x 1024 12.1 / 11.5, 50304 x 768 33.6 / 23.4
+// Between 5/8 and one tile per SM two CTAs share a tile, and half the k-blocks at twice the time each is no gain.
+bool gemm_rows_takes(int M, int N, int K, int a_mn) {
+  if (M > 128 || a_mn) return false;
+  if (M <= 16) return true;
+  const long long tiles = (N + 127) / 128, sms = sm_count();
+  if (M <= 32) return tiles <= 2 * sms;
+  if (M <= 64) return tiles <= 5 * sms / 8 || (tiles > sms && tiles <= 2 * sms);
+  return tiles <= 5 * sms / 8 && (K >= 2048 || tiles * M <= 36 * sms);
 }
 
 // Same contract as gemm_bf16_dispatch for the plain product with a K-major A of at most 128 rows.

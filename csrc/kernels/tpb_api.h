@@ -58,7 +58,7 @@ int gemm_bf16_dispatch(const void* A, const void* B, void* C, const void* bias, 
                        int rows_per_flag, uint32_t flag_want, int max_ctas, uint32_t* status,
                        cudaStream_t stream, const GemmFused* fused);
 // A K-major A of at most 128 rows (gemm_rows.cu): whether the product goes there, and the product.
-bool gemm_rows_takes(int M, int a_mn);
+bool gemm_rows_takes(int M, int N, int K, int a_mn);
 int gemm_rows_dispatch(const void* A, const void* B, void* C, const void* bias, int M, int N, int K, int lda, int ldb,
                        int ldc, int b_mn, int out_f32, int bias_f32, int accumulate, float alpha, uint32_t* status,
                        cudaStream_t stream);
