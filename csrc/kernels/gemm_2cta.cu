@@ -788,24 +788,25 @@ static int launch_pair_split(const CUtensorMap& ta, const CUtensorMap& tb, const
   return (int)cudaLaunchKernelEx(&cfg, gemm_pair_split_kernel<BN, A_MN, B_MN>, ta, tb, p);
 }
 
-// Whether a product with fewer tiles than one wave of CTA pairs goes to the split form, and with which tile width and
-// how many pairs per tile. Estimated times in units of 10 ns, from measurements on one B200: a k-block takes 0.44 us in
-// a 256 x 256 pair tile and 0.28 us in a 256 x 128 one, 0.55 and 0.33 us in the one-CTA tiles of 128 x 256 and
-// 128 x 128; a launch costs about 5 us beside its k-blocks and the cluster reduction 3 us a round.
-bool gemm_pair_split_plan(int M, int N, int K, int* bn, int* c) {
+// Whether a product with fewer tiles than one wave of CTA pairs goes to CTA pairs, with which tile width and how many
+// pairs per tile: the shortest of the estimated times, in units of 10 ns, which fit 345 products of 2 to 64 pair tiles
+// and K = 64 to 16384 in the three operand layouts within 6 % (rms). The pair kernel itself (256 columns, one pair)
+// takes 0.30 us a k-block, 3 us a round and 4.8 us; the split form 0.32 us a k-block and 10 us a round with 256 columns,
+// 0.26 and 8 us with 128, and 1.5 us. Over those products the choice takes 1.006 of the best of all forms on average
+// and nowhere more than the one-CTA kernel. 1024 x 4096 x 4096: one-CTA 31, pair 28, split over two pairs 43 us;
+// 768 x 768 x 16384: one-CTA 79, split over four pairs 29 us.
+bool gemm_pair_split_plan(int M, int N, int K, long long single, int* bn, int* c) {
   if (M <= 128 || N <= 64 || K <= 0) return false;
-  const long long kb = (K + kPairK - 1) / kPairK, sms = sm_count();
-  const long long tm1 = (M + 127) / 128;
-  const long long t256 = tm1 * ((N + 255) / 256), t128 = tm1 * ((N + 127) / 128);
-  const long long single = (t256 * 2 > sms ? (t256 + sms - 1) / sms * kb * 55 : (t128 + sms - 1) / sms * kb * 33) + 500;
-  long long best = single * 9 / 10;
+  const long long kb = (K + kPairK - 1) / kPairK, pairs = sm_count() / 2, tm = (M + kPairM - 1) / kPairM;
+  const long long whole = (tm * ((N + 255) / 256) + pairs - 1) / pairs * (30 * kb + 300) + 480;
+  long long best = single;
   bool found = false;
   for (int width = 256; width >= 128; width -= 128) {
-    const long long tiles = (long long)((M + kPairM - 1) / kPairM) * ((N + width - 1) / width);
-    for (int n = 1; n <= 4 && n <= kb; ++n) {
+    const long long tiles = tm * ((N + width - 1) / width);
+    for (int n = width == 256 ? 2 : 1; n <= 4 && n <= kb; ++n) {
       const int fit = width == 256 ? pair_split_resident<256>(n) : pair_split_resident<128>(n);
       if (fit <= 0) continue;
-      const long long cost = (tiles + fit - 1) / fit * ((kb + n - 1) / n * (width == 256 ? 44 : 28) + 300) + 500;
+      const long long cost = (tiles + fit - 1) / fit * ((kb + n - 1) / n * (width == 256 ? 32 : 26) + (width == 256 ? 1000 : 800)) + 150;
       if (cost < best) { best = cost; *bn = width; *c = n; found = true; }
     }
   }
@@ -813,6 +814,7 @@ bool gemm_pair_split_plan(int M, int N, int K, int* bn, int* c) {
 }
 
 int gemm_pair_split_dispatch(const void* A, const void* B, void* C, const void* bias, int M, int N, int K, int lda,
+  if (whole < best) { best = whole; *bn = 256; *c = 1; found = true; }
                              int ldb, int ldc, int a_mn, int b_mn, int out_f32, int bias_f32, int accumulate,
                              float alpha, uint32_t* status, cudaStream_t stream, int bn, int c) {
   if (M <= 0 || N <= 0) return 0;

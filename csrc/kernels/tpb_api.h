@@ -63,7 +63,8 @@ int gemm_rows_dispatch(const void* A, const void* B, void* C, const void* bias, 
                        int ldc, int b_mn, int out_f32, int bias_f32, int accumulate, float alpha, uint32_t* status,
                        cudaStream_t stream);
 // Few 256-row tiles with a long reduction (gemm_2cta.cu): whether and how the product is split, and the product.
-bool gemm_pair_split_plan(int M, int N, int K, int* bn, int* c);
+// `single` is the time of the one-CTA kernel in units of 10 ns; (256, 1) stands for the CTA-pair kernel itself.
+bool gemm_pair_split_plan(int M, int N, int K, long long single, int* bn, int* c);
 int gemm_pair_split_dispatch(const void* A, const void* B, void* C, const void* bias, int M, int N, int K, int lda,
                              int ldb, int ldc, int a_mn, int b_mn, int out_f32, int bias_f32, int accumulate,
                              float alpha, uint32_t* status, cudaStream_t stream, int bn, int c);

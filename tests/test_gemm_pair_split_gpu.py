@@ -38,3 +38,10 @@ def test_small_output_long_reduction(M, N, K, a_mn, b_mn):
                                 dict(bias=torch.bfloat16, accumulate=True), dict(out_dtype=torch.float32)])
 def test_epilogue(kw):
     _check(500, 1036, 8192, False, False, **kw)
+
+
+@pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, True)])
+@pytest.mark.parametrize("M,N,K", [(1000, 4096, 2048), (2500, 1032, 4096), (200, 14336, 512), (1024, 1024, 64)])
+def test_less_than_a_wave_of_pairs(M, N, K, a_mn, b_mn):
+    """Products that stay whole: on CTA pairs, or on single CTAs."""
+    _check(M, N, K, a_mn, b_mn)
