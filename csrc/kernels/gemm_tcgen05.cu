@@ -1025,15 +1025,16 @@ int gemm_bf16_dispatch(const void* A, const void* B, void* C, const void* bias, 
 // operands MN-major (weight gradients) the two kernels time the same in isolation, but the pair
 // kernel moves a third less through shared memory and the training step, which runs at the power
 // cap, is 1.2 % shorter with it. 0 = never.
-// Among those, the one-CTA kernel (128 x 256 tiles, one per SM) where it needs clearly fewer rounds: a round of either
-// kernel takes about the same time (256 x 256 on two SMs against 128 x 256 on one; the one-CTA kernel 5-12 % longer), and
-// a product whose rows just exceed a multiple of 256 pays a nearly empty row of pair tiles: M = 777, N = 14336 has 224
-// pair tiles, four rounds of 74, and 392 one-CTA tiles, three rounds of 148.
+// Among those, the one-CTA kernel (128 x 256 tiles, one per SM) where it needs fewer rounds by a quarter: a round takes it
+// 0.35 us a k-block where a pair takes 0.30 (256 x 256 on two SMs), and a product whose rows just exceed a multiple of 256
+// pays a nearly empty row of pair tiles. One-CTA / pair, us and rounds: 1100 x 4096 x 4096 29 / 46 (1, 2), 777 x 14336 x
+// 4096 92 / 102 (3, 4), 520 x 19000 x 768 27.6 / 28.5 (3, 4); 1100 x 19000 x 4096 159 / 157 (5, 6), 777 x 28672 x 4096
+// 192 / 183 (6, 7), 520 x 50304 x 4096 241 / 229 (7, 8).
 static int g_pair_min_tiles = 74;
 static bool single_has_fewer_rounds(int M, int N) {
   const long long sms = tpb::sm_count(), pairs = sms / 2;
   const long long tp = (long long)((M + 255) / 256) * ((N + 255) / 256), ts = (long long)((M + 127) / 128) * ((N + 255) / 256);
-  return ((ts + sms - 1) / sms) * 112 < ((tp + pairs - 1) / pairs) * 100;
+  return ((ts + sms - 1) / sms) * 124 < ((tp + pairs - 1) / pairs) * 100;
 }
 extern "C" void tpb_gemm_set_pair_min_tiles(int tiles) { g_pair_min_tiles = tiles; }
 
@@ -1094,8 +1095,8 @@ extern "C" int tpb_gemm_bf16(const void* A, const void* B, void* C, const void* 
                                      alpha, 0, status, static_cast<cudaStream_t>(stream));
     return tpb::gemm_pair_split_dispatch(A, B, C, bias, M, N, K, lda, ldb, ldc, a_mn, b_mn, out_f32, bias_f32, accumulate,
                                          alpha, status, static_cast<cudaStream_t>(stream), bn, c);
-  return tpb::gemm_bf16_dispatch(A, B, C, bias, M, N, K, lda, ldb, ldc, a_mn, b_mn, out_f32,
   }
+  return tpb::gemm_bf16_dispatch(A, B, C, bias, M, N, K, lda, ldb, ldc, a_mn, b_mn, out_f32,
                                  bias_f32, accumulate, alpha, nullptr, 0, 0, 0, status,
                                  static_cast<cudaStream_t>(stream), nullptr);
 }
