@@ -32,9 +32,8 @@ struct PairCfg {
   static constexpr int kBBytes = kHalfN * kPairK * 2;
   static constexpr int kStageBytes = kPairABytes + kBBytes;
   static constexpr int kStages = BN == 256 ? 6 : 8;
-  // staging of the bf16 epilogue: per warp 32 rows of 64 columns, padded to 144 bytes (conflict-free both ways)
-  static constexpr int kOutOff = kStages * kStageBytes + 512;
-  static constexpr int kSmem = kOutOff + 4 * 32 * 144 + 1024;
+  static constexpr int kOutOff = kStages * kStageBytes + 512;   // staging of the bf16 epilogue
+  static constexpr int kSmem = kOutOff + 4 * kDrainStage + 1024;
 };
 constexpr int kPairGroupM = 8;
 
@@ -308,12 +307,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     }
   } else {
     // ------------------------------------------------------------ epilogue (4 warps per CTA, own 128 rows)
-    // A lane holds 32 columns of one row. Stored from there, an instruction touches 32 rows by 16 bytes and takes 32
-    // passes of the load/store unit: 4096 of the ~6000 cycles that the MMAs of a tile take at K = 768. Plain bf16
-    // results therefore go through shared memory and leave as 4 rows by 128 contiguous bytes.
     const int q = warp & 3;
-    uint8_t* out_stage = smem + Cfg::kOutOff + q * (32 * 144);
-    const bool staged = !p.out_f32 && !p.accumulate && p.ldc % 8 == 0 && (reinterpret_cast<uintptr_t>(p.C) & 15) == 0;
+    uint8_t* out_stage = smem + Cfg::kOutOff + q * kDrainStage;
+    const bool plain = !p.out_f32 && !p.accumulate && p.ldc % 8 == 0 && (reinterpret_cast<uintptr_t>(p.C) & 15) == 0 &&
+                       !(p.bias && (p.bias_f32 || (reinterpret_cast<uintptr_t>(p.bias) & 15)));
     uint32_t lt = 0;
     for (int wi = 0; pair_work(sc, pair, wi, w); ++wi, ++lt) {
       int tm, tn;
@@ -358,18 +355,33 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         got = __all_sync(0xffffffffu, got);
         if (!got) { *abort_w = 1; break; }
       }
+      int c0 = 0;
+      if (plain && !sk_tile) {
+        const int row0 = tm * kPairM + (int)crank * 128 + q * 32, col0 = tn * kPairN;
+        c0 = drain_bf16(t_row, out_stage, reinterpret_cast<__nv_bfloat16*>(p.C) + (size_t)row0 * p.ldc + col0, p.ldc,
+                        p.M - row0, min(kPairN, p.N - col0), p.alpha,
+                        p.bias ? reinterpret_cast<const __nv_bfloat16*>(p.bias) + col0 : nullptr, lane);
+      }
 #pragma unroll 1
-      for (int c = 0; c < kPairN; c += 32) {
+      for (int c = c0; c < kPairN; c += 32) {
         const int col0 = tn * kPairN + c;
         if (col0 >= p.N) break;  // warp-uniform
         uint32_t r[32];
         tmem_ld_32x32b_x32(t_row + c, r);
-        Bias32 bias;
-        const bool bias_vec = bias32_vec_ok(p.bias, p.bias_f32, col0, p.N);
-        if (bias_vec) bias32_load(bias, p.bias, col0);
-        const bool stage_it = staged && (c & ~32) + tn * kPairN + 64 <= p.N;   // warp-uniform, both halves of 64 columns
+        const bool full_chunk = (col0 + 32 <= p.N);
+        uint8_t* crow_b = reinterpret_cast<uint8_t*>(p.C) + ((size_t)row * p.ldc + col0) * (p.out_f32 ? 4 : 2);
+        const bool vec = full_chunk && (reinterpret_cast<uintptr_t>(crow_b) & 15) == 0;
+        uint4 old[8];   // what is accumulated into, requested under the TMEM load (6144 x 4096 x 1032: 99.4 -> 73.0 us)
+        if (p.accumulate && vec && row < p.M) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) old[i] = reinterpret_cast<const uint4*>(crow_b)[i];
+          if (p.out_f32) {
+#pragma unroll
+            for (int i = 4; i < 8; ++i) old[i] = reinterpret_cast<const uint4*>(crow_b)[i];
+          }
+        }
         tmem_ld_wait();
-        if (row < p.M || stage_it) {
+        if (row < p.M) {
           float v[32];
 #pragma unroll
           for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
@@ -385,28 +397,17 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           }
 #pragma unroll
           for (int i = 0; i < 32; ++i) v[i] *= p.alpha;
-          const bool full_chunk = (col0 + 32 <= p.N);
-          if (bias_vec) bias32_add(v, bias);
-          else if (p.bias) bias32_add_any(v, p.bias, p.bias_f32, col0, p.N);
-          if (stage_it) {
-            uint8_t* srow = out_stage + lane * 144 + (c & 32) * 2;
-#pragma unroll
-            for (int i = 0; i < 32; i += 8) {
-              uint4 o;
-              __nv_bfloat162* ob2 = reinterpret_cast<__nv_bfloat162*>(&o);
-#pragma unroll
-              for (int j = 0; j < 4; ++j) ob2[j] = __floats2bfloat162_rn(v[i + 2 * j], v[i + 2 * j + 1]);
-              *reinterpret_cast<uint4*>(srow + i * 2) = o;
-            }
-          } else if (p.out_f32) {
-            float* crow = reinterpret_cast<float*>(p.C) + (size_t)row * p.ldc + col0;
-            if (full_chunk && ((reinterpret_cast<uintptr_t>(crow) & 15) == 0)) {
+          if (p.bias) bias32_apply(v, p.bias, p.bias_f32, col0, p.N);
+          if (p.out_f32) {
+            float* crow = reinterpret_cast<float*>(crow_b);
+            if (vec) {
 #pragma unroll
               for (int i = 0; i < 32; i += 4) {
                 float4 o = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
                 if (p.accumulate) {
-                  const float4 old = *reinterpret_cast<float4*>(crow + i);
-                  o.x += old.x; o.y += old.y; o.z += old.z; o.w += old.w;
+                  const uint4 u = old[i / 4];
+                  o.x += __uint_as_float(u.x); o.y += __uint_as_float(u.y);
+                  o.z += __uint_as_float(u.z); o.w += __uint_as_float(u.w);
                 }
                 *reinterpret_cast<float4*>(crow + i) = o;
               }
@@ -415,13 +416,12 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                 if (col0 + i < p.N) crow[i] = p.accumulate ? crow[i] + v[i] : v[i];
             }
           } else {
-            __nv_bfloat16* crow = reinterpret_cast<__nv_bfloat16*>(p.C) + (size_t)row * p.ldc + col0;
-            if (full_chunk && ((reinterpret_cast<uintptr_t>(crow) & 15) == 0)) {
+            __nv_bfloat16* crow = reinterpret_cast<__nv_bfloat16*>(crow_b);
+            if (vec) {
 #pragma unroll
               for (int i = 0; i < 32; i += 8) {
                 if (p.accumulate) {
-                  const uint4 old = *reinterpret_cast<uint4*>(crow + i);
-                  const __nv_bfloat162* ob = reinterpret_cast<const __nv_bfloat162*>(&old);
+                  const __nv_bfloat162* ob = reinterpret_cast<const __nv_bfloat162*>(&old[i / 8]);
 #pragma unroll
                   for (int j = 0; j < 4; ++j) {
                     const float2 f = __bfloat1622float2(ob[j]);
@@ -443,17 +443,6 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                 }
             }
           }
-        }
-        if (stage_it && (c & 32)) {
-          __syncwarp();
-          const int row8 = tm * kPairM + (int)crank * 128 + q * 32 + (lane >> 3);
-          __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(p.C) + (size_t)row8 * p.ldc + (col0 - 32) + (lane & 7) * 8;
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const uint4 val = *reinterpret_cast<const uint4*>(out_stage + (i * 4 + (lane >> 3)) * 144 + (lane & 7) * 16);
-            if (row8 + i * 4 < p.M) *reinterpret_cast<uint4*>(dst + (size_t)(i * 4) * p.ldc) = val;
-          }
-          __syncwarp();
         }
       }
       tc_fence_before_sync();
@@ -801,6 +790,7 @@ bool gemm_pair_split_plan(int M, int N, int K, long long single, int* bn, int* c
   const long long whole = (tm * ((N + 255) / 256) + pairs - 1) / pairs * (30 * kb + 300) + 480;
   long long best = single;
   bool found = false;
+  if (whole < best) { best = whole; *bn = 256; *c = 1; found = true; }
   for (int width = 256; width >= 128; width -= 128) {
     const long long tiles = tm * ((N + width - 1) / width);
     for (int n = width == 256 ? 2 : 1; n <= 4 && n <= kb; ++n) {
@@ -814,7 +804,6 @@ bool gemm_pair_split_plan(int M, int N, int K, long long single, int* bn, int* c
 }
 
 int gemm_pair_split_dispatch(const void* A, const void* B, void* C, const void* bias, int M, int N, int K, int lda,
-  if (whole < best) { best = whole; *bn = 256; *c = 1; found = true; }
                              int ldb, int ldc, int a_mn, int b_mn, int out_f32, int bias_f32, int accumulate,
                              float alpha, uint32_t* status, cudaStream_t stream, int bn, int c) {
   if (M <= 0 || N <= 0) return 0;

@@ -51,7 +51,7 @@ struct GemmCfg {
   // staging of the reduce-scatter epilogue: per epilogue warp 32 rows x 64 bf16 columns, rows padded
   // to 144 bytes (conflict-free 16-byte accesses both ways)
   static constexpr int kOutStageOff = kStages * kStageBytes + 256;
-  static constexpr int kOutStageBytes = 4 * 32 * 144;
+  static constexpr int kOutStageBytes = 4 * kDrainStage;
   static constexpr int kSmemBytes = kStages * kStageBytes + 1024 /*align*/ + 256 /*barriers*/ + kOutStageBytes;
   static constexpr int kTmemCols = 2 * BLOCK_N;  // double-buffered accumulator (256 or 512)
 };
@@ -470,8 +470,11 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   } else {
     // ------------------------------------------------------------ epilogue (4 warps)
     const int q = warp & 3;  // TMEM lane quarter this warp may read
-    uint8_t* out_stage = smem + Cfg::kOutStageOff + q * (32 * 144);
+    uint8_t* out_stage = smem + Cfg::kOutStageOff + q * kDrainStage;
     const bool rs_coalesce = p.rs_mode && (p.N % 64 == 0);
+    const bool plain = !p.rs_mode && !p.out_f32 && !p.accumulate && p.ldc % 8 == 0 &&
+                       (reinterpret_cast<uintptr_t>(p.C) & 15) == 0 &&
+                       !(p.bias && (p.bias_f32 || (reinterpret_cast<uintptr_t>(p.bias) & 15)));
     uint32_t lt = 0;
     for (int wi = 0; wi < n_items; ++wi, ++lt) {
       const WorkItem w = get_work(wi);
@@ -642,15 +645,19 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         got = __all_sync(0xffffffffu, got);
         if (!got) { *abort_w = 1; break; }
       }
+      int c0 = 0;
+      if (plain && !sk_tile) {
+        const int row0 = tm * kBlockM + q * 32, col0 = tn * BLOCK_N;
+        c0 = drain_bf16(t_row, out_stage, reinterpret_cast<__nv_bfloat16*>(p.C) + (size_t)row0 * p.ldc + col0, p.ldc,
+                        p.M - row0, min(BLOCK_N, p.N - col0), p.alpha,
+                        p.bias ? reinterpret_cast<const __nv_bfloat16*>(p.bias) + col0 : nullptr, lane);
+      }
 #pragma unroll 1
-      for (int c = 0; c < BLOCK_N; c += 32) {
+      for (int c = c0; c < BLOCK_N; c += 32) {
         const int col0 = tn * BLOCK_N + c;
         if (col0 >= p.N) break;  // warp-uniform
         uint32_t r[32];
         tmem_ld_32x32b_x32(t_row + c, r);
-        Bias32 bias;
-        const bool bias_vec = bias32_vec_ok(p.bias, p.bias_f32, col0, p.N);
-        if (bias_vec) bias32_load(bias, p.bias, col0);
         tmem_ld_wait();
         if (row < p.M) {
           float v[32];
@@ -669,8 +676,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 #pragma unroll
           for (int i = 0; i < 32; ++i) v[i] *= p.alpha;
           const bool full_chunk = (col0 + 32 <= p.N);
-          if (bias_vec) bias32_add(v, bias);
-          else if (p.bias) bias32_add_any(v, p.bias, p.bias_f32, col0, p.N);
+          if (p.bias) bias32_apply(v, p.bias, p.bias_f32, col0, p.N);
           if (p.rs_mode && rs_coalesce) {
             // bf16 partial into the warp's staging rows; flushed below in 128-byte row segments
             uint8_t* srow = out_stage + lane * 144 + (c & 32) * 2;

@@ -31,9 +31,8 @@ struct GCfg {
   static constexpr int kABytes = kGBlockM * kGBlockK * 2;
   static constexpr int kBBytes = BLOCK_N * kGBlockK * 2;
   static constexpr int kStageBytes = kABytes + kBBytes;
-  // staging of the bf16 epilogue: per warp 32 rows of 64 columns, padded to 144 bytes (conflict-free both ways)
-  static constexpr int kOutOff = kStages * kStageBytes + 256;
-  static constexpr int kSmemBytes = kOutOff + 4 * 32 * 144 + 1024;
+  static constexpr int kOutOff = kStages * kStageBytes + 256;   // staging of the bf16 epilogue
+  static constexpr int kSmemBytes = kOutOff + 4 * kDrainStage + 1024;
   static constexpr int kTmemCols = 2 * BLOCK_N;
 };
 
@@ -223,12 +222,10 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       }
     }
   } else {
-    // Plain bf16 results go through shared memory and leave as 4 rows by 128 contiguous bytes: stored from the lane that
-    // holds 32 columns of a row, an instruction touches 32 rows by 16 bytes, and a weight gradient over the ~256 rows of
-    // an expert has four k-blocks per tile to hide that behind.
+    // A weight gradient over the ~256 rows of an expert has four k-blocks per tile to hide its stores behind.
     const int q = warp & 3;
-    uint8_t* out_stage = smem + Cfg::kOutOff + q * (32 * 144);
-    const bool staged = !p.out_f32 && !p.accumulate && p.ldc % 8 == 0 && (p.mode == 0 || p.c_expert_stride % 8 == 0) &&
+    uint8_t* out_stage = smem + Cfg::kOutOff + q * kDrainStage;
+    const bool plain = !p.out_f32 && !p.accumulate && p.ldc % 8 == 0 && (p.mode == 0 || p.c_expert_stride % 8 == 0) &&
                         (reinterpret_cast<uintptr_t>(p.C) & 15) == 0;
     uint32_t lt = 0;
     for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
@@ -246,8 +243,15 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       const int row_lim = (p.mode == 0) ? p.offs[e + 1] : p.N;
       const int col_lim = (p.mode == 0) ? p.N : p.K;
       const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + as * BLOCK_N;
+      int c_done = 0;
+      if (plain && !empty_k) {
+        const int r0 = row0 + q * 32;
+        c_done = drain_bf16(t_row, out_stage, reinterpret_cast<__nv_bfloat16*>(p.C) +
+                            (p.mode == 0 ? (size_t)0 : (size_t)e * p.c_expert_stride) + (size_t)r0 * p.ldc + c0, p.ldc,
+                            row_lim - r0, min(BLOCK_N, col_lim - c0), 1.f, nullptr, lane);
+      }
 #pragma unroll 1
-      for (int c = 0; c < BLOCK_N; c += 32) {
+      for (int c = c_done; c < BLOCK_N; c += 32) {
         const int col0 = c0 + c;
         if (col0 >= col_lim) break;
         uint32_t r[32];
@@ -258,30 +262,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
 #pragma unroll
           for (int i = 0; i < 32; ++i) r[i] = 0;
         }
-        if (staged && (c0 + (c & ~32)) + 64 <= col_lim) {   // warp-uniform, both halves of 64 columns
-          uint8_t* srow = out_stage + lane * 144 + (c & 32) * 2;
-#pragma unroll
-          for (int i = 0; i < 32; i += 8) {
-            uint4 o;
-            __nv_bfloat162* ob2 = reinterpret_cast<__nv_bfloat162*>(&o);
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-              ob2[j] = __floats2bfloat162_rn(__uint_as_float(r[i + 2 * j]), __uint_as_float(r[i + 2 * j + 1]));
-            *reinterpret_cast<uint4*>(srow + i * 2) = o;
-          }
-          if (c & 32) {
-            __syncwarp();
-            const int row8 = row0 + q * 32 + (lane >> 3);
-            __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(p.C) + (p.mode == 0 ? (size_t)0 : (size_t)e * p.c_expert_stride) +
-                                 (size_t)row8 * p.ldc + (col0 - 32) + (lane & 7) * 8;
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-              const uint4 val = *reinterpret_cast<const uint4*>(out_stage + (i * 4 + (lane >> 3)) * 144 + (lane & 7) * 16);
-              if (row8 + i * 4 < row_lim) *reinterpret_cast<uint4*>(dst + (size_t)(i * 4) * p.ldc) = val;
-            }
-            __syncwarp();
-          }
-        } else if (row < row_lim) {
+        if (row < row_lim) {
           const bool full_chunk = col0 + 32 <= col_lim;
           const size_t base = (p.mode == 0) ? (size_t)row * p.ldc + col0
                                             : (size_t)e * p.c_expert_stride + (size_t)row * p.ldc + col0;

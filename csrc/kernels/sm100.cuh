@@ -534,4 +534,69 @@ __device__ __forceinline__ void bias32_add_any(float (&v)[32], const void* bias,
                        : __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(bias)[col0 + i]);
 }
 
+// The bias of a chunk of 32 columns in any of its forms.
+__device__ __forceinline__ void bias32_apply(float (&v)[32], const void* bias, int bias_f32, int col0, int N) {
+  if (bias32_vec_ok(bias, bias_f32, col0, N)) {
+    Bias32 b;
+    bias32_load(b, bias, col0);
+    bias32_add(v, b);
+  } else {
+    bias32_add_any(v, bias, bias_f32, col0, N);
+  }
+}
+
+// Plain bf16 results: 32 accumulator rows (the TMEM lanes of a warp) to `rows` valid rows of C, 64 columns at a time while
+// `cols` lasts; returns the columns done. c: first row and column, 16-byte aligned like every row; bias: null, or
+// 16-byte aligned bf16 at that column; stage: kDrainStage bytes of the warp's own.
+// A lane holds 32 columns of one row. Stored from there, an instruction touches 32 rows by 16 bytes and takes 32 passes
+// of the load/store unit, 4096 of the ~6000 cycles that the MMAs of a 256-row tile take at K = 768: the results go
+// through shared memory (144-byte rows, free of conflicts both ways) and leave as 4 rows by 128 contiguous bytes. Both
+// TMEM loads share one wait, and all of a chunk is read back before any of it is stored, which the compiler may not
+// arrange by itself (the two could alias). CTA-pair kernel, 4096 x 4096, K = 64 / 1032 / 4096: 21.7 / 32.8 / 115.8 us
+// with 32 columns at a time, 15.4 / 31.5 / 112.6 us so; stored from the lanes 21.1 / 35.3 / 119.5 us.
+constexpr int kDrainStage = 32 * 144;
+__device__ __forceinline__ int drain_bf16(uint32_t t_row, uint8_t* stage, __nv_bfloat16* c, size_t ldc, int rows, int cols,
+                                          float alpha, const void* bias, int lane) {
+  if (rows <= 0) return cols & ~63;
+  int done = 0;
+#pragma unroll 1
+  for (; done + 64 <= cols; done += 64) {
+    uint32_t r[2][32];
+    tmem_ld_32x32b_x32(t_row + done, r[0]);
+    tmem_ld_32x32b_x32(t_row + done + 32, r[1]);
+    Bias32 b[2];
+    if (bias) {
+      bias32_load(b[0], bias, done);
+      bias32_load(b[1], bias, done + 32);
+    }
+    tmem_ld_wait();
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      float v[32];
+#pragma unroll
+      for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[h][i]) * alpha;
+      if (bias) bias32_add(v, b[h]);
+#pragma unroll
+      for (int i = 0; i < 32; i += 8) {
+        uint4 o;
+        __nv_bfloat162* ob2 = reinterpret_cast<__nv_bfloat162*>(&o);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) ob2[j] = __floats2bfloat162_rn(v[i + 2 * j], v[i + 2 * j + 1]);
+        *reinterpret_cast<uint4*>(stage + lane * 144 + h * 64 + i * 2) = o;
+      }
+    }
+    __syncwarp();
+    uint4 val[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      val[i] = *reinterpret_cast<const uint4*>(stage + (i * 4 + (lane >> 3)) * 144 + (lane & 7) * 16);
+    __nv_bfloat16* dst = c + (size_t)(lane >> 3) * ldc + done + (lane & 7) * 8;
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      if (i * 4 + (lane >> 3) < rows) *reinterpret_cast<uint4*>(dst + (size_t)(i * 4) * ldc) = val[i];
+    __syncwarp();
+  }
+  return done;
+}
+
 }  // namespace tpb
