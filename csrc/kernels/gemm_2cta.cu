@@ -779,15 +779,15 @@ static int launch_pair_split(const CUtensorMap& ta, const CUtensorMap& tb, const
 
 // Whether a product with fewer tiles than one wave of CTA pairs goes to CTA pairs, with which tile width and how many
 // pairs per tile: the shortest of the estimated times, in units of 10 ns, which fit 345 products of 2 to 64 pair tiles
-// and K = 64 to 16384 in the three operand layouts within 6 % (rms). The pair kernel itself (256 columns, one pair)
-// takes 0.30 us a k-block, 3 us a round and 4.8 us; the split form 0.32 us a k-block and 10 us a round with 256 columns,
-// 0.26 and 8 us with 128, and 1.5 us. Over those products the choice takes 1.006 of the best of all forms on average
-// and nowhere more than the one-CTA kernel. 1024 x 4096 x 4096: one-CTA 31, pair 28, split over two pairs 43 us;
+// and K = 64 to 16384 in the three operand layouts within 7 % (rms). The pair kernel itself (256 columns, one pair)
+// takes 0.30 us a k-block, 1.9 us a round and 4.5 us; the split form 0.32 us a k-block and 10 us a round with 256
+// columns, 0.26 and 8 us with 128, and 1.5 us. Over those products the choice takes 1.005 of the best of all forms on
+// average and nowhere 6 % more than the one-CTA kernel. 1024 x 4096 x 4096: one-CTA 30, pair 27, over two pairs 44 us;
 // 768 x 768 x 16384: one-CTA 79, split over four pairs 29 us.
 bool gemm_pair_split_plan(int M, int N, int K, long long single, int* bn, int* c) {
   if (M <= 128 || N <= 64 || K <= 0) return false;
   const long long kb = (K + kPairK - 1) / kPairK, pairs = sm_count() / 2, tm = (M + kPairM - 1) / kPairM;
-  const long long whole = (tm * ((N + 255) / 256) + pairs - 1) / pairs * (30 * kb + 300) + 480;
+  const long long whole = (tm * ((N + 255) / 256) + pairs - 1) / pairs * (30 * kb + 190) + 450;
   long long best = single;
   bool found = false;
   if (whole < best) { best = whole; *bn = 256; *c = 1; found = true; }

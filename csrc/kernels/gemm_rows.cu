@@ -287,18 +287,16 @@ static int launch_rows(const CUtensorMap& tb, const CUtensorMap& ta, const RowsP
 // under the stores of the last. What this kernel gains is the split of K over a cluster while there are fewer tiles
 // than CTAs that fit (two per SM), and the small column operand; what it pays is an epilogue of 3 us a round at 16 rows
 // and 9 us at 128, under which nothing is loaded. Measured on one B200, operands from memory, N x K: us here / there:
-//   M = 16: 14336 x 2048 15.0 / 17.3, 50304 x 768 20.4 / 21.4, 128256 x 2048 88 / 87
-//   M = 32: 28672 x 4096 41.2 / 45.1, 50304 x 768 22.3 / 21.4
-//   M = 64: 6144 x 1024 9.4 / 11.2, 14336 x 2048 18.5 / 16.6, 28672 x 4096 45.9 / 46.6, 128256 x 4096 182 / 176
-//   M = 128: 4096 x 1024 9.3 / 11.1, 4096 x 14336 32 / 70, 6144 x 1024 12.1 / 11.5, 50304 x 768 33.6 / 23.4
+//   M = 16: 14336 x 2048 15.1 / 16.3, 50304 x 768 20.5 / 19.2, 128256 x 2048 89.9 / 87.2, 128256 x 4096 168.0 / 174.2
+//   M = 32: 4096 x 4096 11.2 / 23.5, 28672 x 4096 41.8 / 43.8, 50304 x 768 22.5 / 19.5
+//   M = 64: 6144 x 1024 9.4 / 10.0, 14336 x 2048 18.6 / 15.6, 28672 x 4096 46.3 / 45.3, 32000 x 1024 17.8 / 16.4
+//   M = 128: 4096 x 1024 9.3 / 10.0, 4096 x 14336 31.9 / 69.7, 6144 x 1024 12.1 / 10.4, 50304 x 768 33.7 / 21.4
 // Between 5/8 and one tile per SM two CTAs share a tile, and half the k-blocks at twice the time each is no gain.
 bool gemm_rows_takes(int M, int N, int K, int a_mn) {
   if (M > 128 || a_mn) return false;
-  if (M <= 16) return true;
   const long long tiles = (N + 127) / 128, sms = sm_count();
-  if (M <= 32) return tiles <= 2 * sms;
-  if (M <= 64) return tiles <= 5 * sms / 8 || (tiles > sms && tiles <= 2 * sms);
-  return tiles <= 5 * sms / 8 && (K >= 2048 || tiles * M <= 36 * sms);
+  if (M <= 32) return tiles <= 2 * sms || (M <= 16 && K >= 4096);
+  return tiles <= 5 * sms / 8 && (M <= 64 || K >= 2048 || tiles * M <= 28 * sms);
 }
 
 // Same contract as gemm_bf16_dispatch for the plain product with a K-major A of at most 128 rows.

@@ -950,17 +950,16 @@ static int pick_block_n(int M, int N, int K, bool splitk) {
   return cost(tiles256, 32) <= cost(tm * ((N + 127) / 128), 16) ? 256 : 128;
 }
 
-// Time of a plain product in this kernel in units of 10 ns, fitted within 6 % (rms) over 230 shapes of 2 to 73 pair tiles
-// and K = 64 to 16384: a round of tiles takes 0.35 us a k-block and 3.2 us with 256 columns, 0.29 and 3.1 us with 128.
-// With a split-K workspace the last round is as long as one split plus 4 us.
+// Time of a plain product in this kernel in units of 10 ns, fitted within 7 % (rms) over 230 shapes of 2 to 73 pair tiles
+// and K = 64 to 16384: a round of tiles takes 0.35 us a k-block and 1.5 us with 256 columns, 0.295 and 2.5 us with 128,
+// and the launch 4.6 and 2.5 us. With a split-K workspace the last round is as long as one split plus 4 us.
 static long long gemm_single_cost(int M, int N, int K) {
   const bool wide = pick_block_n(M, N, K, g_sk_ws != nullptr) == 256;
   const long long sms = sm_count(), tiles = (long long)((M + kBlockM - 1) / kBlockM) * ((N + (wide ? 255 : 127)) / (wide ? 256 : 128));
-  const int kb = (K + kBlockK - 1) / kBlockK, tail = (int)(tiles % sms), block = wide ? 35 : 29;
+  const int kb = (K + kBlockK - 1) / kBlockK, tail = (int)(tiles % sms);
   const int ns = g_sk_ws && tail ? tail_nsplit(tail, (int)sms, kb) : 1;
-  long long cost = tiles / sms * (block * kb + 320) + (wide ? 500 : 310);
-  if (tail) cost += (kb + ns - 1) / ns * block + 320 + (ns > 1 ? 400 : 0);
-  return cost;
+  auto round = [&](int k_blocks) { return wide ? 35LL * k_blocks + 150 : 295LL * k_blocks / 10 + 250; };
+  return tiles / sms * round(kb) + (tail ? round((kb + ns - 1) / ns) + (ns > 1 ? 400 : 0) : 0) + (wide ? 460 : 250);
 }
 
 int gemm_bf16_dispatch(const void* A, const void* B, void* C, const void* bias, int M, int N,

@@ -42,9 +42,8 @@ def test_few_rows_epilogue(M, N, K, kw):
     _check(M, N, K, False, False, **kw)
 
 
-@pytest.mark.parametrize("M,N,K", [(16, 40000, 72), (17, 37888, 136), (32, 37896, 136), (33, 11776, 192), (64, 11848, 192),
-                                   (64, 18952, 64), (48, 37896, 64), (65, 10368, 2048), (128, 5248, 64), (128, 5384, 64),
-                                   (128, 11848, 2048)])
+@pytest.mark.parametrize("M,N,K", [(16, 40000, 72), (1, 40000, 4096), (17, 37888, 136), (32, 37896, 136), (33, 11776, 192),
+                                   (64, 11848, 192), (65, 10368, 2048), (128, 4096, 64), (128, 4240, 64), (128, 11848, 2048)])
 def test_both_sides_of_the_choice(M, N, K):
     """Sizes on which the kernels of few and of more rows meet."""
     _check(M, N, K, False, M % 2 == 0)
