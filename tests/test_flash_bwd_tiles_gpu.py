@@ -12,7 +12,9 @@ DEV = "cuda"
 @pytest.mark.parametrize("B,Tq,Tk,Hq,Hkv,causal,window", [
     (1, 1, 1, 1, 1, True, 0), (2, 64, 64, 2, 2, True, 0), (1, 127, 127, 4, 2, True, 0), (1, 128, 128, 8, 1, True, 0),
     (2, 129, 129, 2, 1, True, 0), (1, 700, 700, 8, 2, True, 0), (1, 1500, 1500, 2, 2, False, 0), (1, 200, 513, 4, 1, True, 0),
-    (1, 300, 130, 2, 2, True, 0), (1, 1000, 1000, 4, 2, True, 65), (1, 900, 900, 2, 1, True, 257), (1, 77, 640, 2, 2, False, 0)])
+    (1, 300, 130, 2, 2, True, 0), (1, 1000, 1000, 4, 2, True, 65), (1, 900, 900, 2, 1, True, 257), (1, 77, 640, 2, 2, False, 0),
+    # streams long enough for 128-row tiles at head dimension 128, in one pass or both
+    (2, 1301, 1301, 4, 2, True, 0), (1, 1900, 1900, 2, 1, True, 700), (1, 33, 1500, 4, 1, True, 0), (1, 1500, 40, 2, 2, False, 0)])
 def test_gradients(D, B, Tq, Tk, Hq, Hkv, causal, window):
     torch.manual_seed(Tq + Tk)
     q = torch.randn(B, Tq, Hq, D, device=DEV).bfloat16().requires_grad_()
