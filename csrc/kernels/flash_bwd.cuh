@@ -53,6 +53,114 @@ __device__ __forceinline__ float bwd_exp2(float x) {
   return y;
 }
 
+// What a CTA works on: batch, head (KV head for dKV, query head for dQ) and first row of its stationary tile.
+// CTAs start in the order of their linear index; with a causal mask the tile index is the slowest coordinate, heaviest
+// tile first (key tile 0 for dK/dV, the last query tile for dQ), heads and batches the fastest, so that the light CTAs of
+// all heads fill the tail.
+struct BwdTile {
+  int b, hx, x0;
+};
+template <bool DKV>
+__device__ __forceinline__ BwdTile bwd_tile(const AttnBwdParams& p) {
+  int b = blockIdx.z, hx = blockIdx.y, xi = blockIdx.x;
+  if (p.causal) {
+    const int lin = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
+    const int hb = gridDim.y * gridDim.z;
+    xi = lin / hb;
+    hx = (lin % hb) % gridDim.y;
+    b = (lin % hb) / gridDim.y;
+  }
+  return {b, hx, ((DKV || !p.causal) ? xi : (int)gridDim.x - 1 - xi) * kStat};
+}
+
+// Streamed tiles of KS rows that the stationary tile at x0 may pair with: [first, first + count).
+template <bool DKV, int KS>
+__device__ __forceinline__ void bwd_stream(const AttnBwdParams& p, const BwdTile& t, int& first, int& count) {
+  const long long seg_base = (long long)t.b * p.Tq;
+  const int x0 = t.x0;
+  first = 0;
+  if (DKV) {
+    // queries of this key tile: from the first key's lower bound to the last key's upper bound
+    int q_hi = p.Tq;
+    const int k_last = min(x0 + kStat - 1, p.Tk - 1);
+    if (p.causal) {
+      const int qmin = x0 - p.kv_offset;
+      first = qmin > 0 ? qmin / KS : 0;
+    }
+    if (p.window > 0) q_hi = min(q_hi, k_last - p.kv_offset + p.window);
+    if (p.seg_start && x0 < p.Tk) first = max(first, p.seg_start[seg_base + x0] / KS);
+    if (p.seg_end && x0 < p.Tk) q_hi = min(q_hi, p.seg_end[seg_base + k_last]);
+    count = max((max(q_hi, 0) + KS - 1) / KS - first, 0);
+  } else {
+    // keys of this query tile: from the first query's lower bound to the last query's upper bound
+    int nkb = (p.Tk + KS - 1) / KS;
+    const int q_last = min(x0 + kStat - 1, p.Tq - 1);
+    if (p.causal) {
+      const int last_key = x0 + kStat - 1 + p.kv_offset;
+      nkb = min(nkb, last_key < 0 ? 0 : last_key / KS + 1);
+    }
+    if (p.seg_end && x0 < p.Tq) nkb = min(nkb, (p.seg_end[seg_base + q_last] + KS - 1) / KS);
+    int lo_first = 0;
+    if (p.window > 0) lo_first = max(lo_first, x0 + p.kv_offset - p.window + 1);
+    if (p.seg_start && x0 < p.Tq) lo_first = max(lo_first, p.seg_start[seg_base + x0]);
+    first = lo_first / KS;
+    count = max(nkb - first, 0);
+  }
+}
+
+// Streamed indices (queries for dKV, keys for dQ) that row xi (a key, a query) may pair with: [lo, hi).
+template <bool DKV>
+__device__ __forceinline__ void bwd_row_bounds(const AttnBwdParams& p, int b, int xi, int& lo, int& hi) {
+  const long long seg_base = (long long)b * p.Tq;
+  if (DKV) {
+    lo = (xi < p.Tk) ? (p.causal ? max(xi - p.kv_offset, 0) : 0) : 0x3fffffff;
+    hi = p.Tq;
+    if (p.window > 0) hi = min(hi, xi - p.kv_offset + p.window);
+  } else {
+    lo = 0;
+    hi = (xi < p.Tq) ? (p.causal ? min(p.Tk, xi + p.kv_offset + 1) : p.Tk) : 0;
+    if (p.window > 0) lo = max(lo, xi + p.kv_offset - p.window + 1);
+  }
+  if (xi < (DKV ? p.Tk : p.Tq)) {
+    if (p.seg_start) lo = max(lo, p.seg_start[seg_base + xi]);
+    if (p.seg_end) hi = min(hi, p.seg_end[seg_base + xi]);
+  }
+}
+
+// A warp's half of its accumulator rows (dV and dK, or dQ) to global memory; zeros where nothing was streamed.
+template <int D, bool DKV>
+__device__ __forceinline__ void bwd_store(const AttnBwdParams& p, const BwdTile& t, uint32_t t_acc0, uint32_t t_acc1, int xi,
+                                          int half, bool streamed) {
+  const long long obase = (long long)t.b * p.out_batch + (long long)xi * p.out_tok + (long long)t.hx * p.out_head;
+#pragma unroll 1
+  for (int a = DKV ? 0 : 1; a < 2; ++a) {
+    __nv_bfloat16* orow = (a == 0 ? p.out0 : p.out1) + obase;
+    const uint32_t t_acc = a == 0 ? t_acc0 : t_acc1;
+#pragma unroll 1
+    for (int c = half * (D / 64); c < (half + 1) * (D / 64); ++c) {
+      uint32_t o[32];
+      if (streamed) {
+        tmem_ld_32x32b_x32(t_acc + c * 32, o);
+        tmem_ld_wait();
+      } else {
+#pragma unroll
+        for (int i = 0; i < 32; ++i) o[i] = 0;
+      }
+      if (xi < (DKV ? p.Tk : p.Tq)) {
+#pragma unroll
+        for (int g = 0; g < 4; ++g) {
+          uint4 v;
+          __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&v);
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            h[i] = __floats2bfloat162_rn(__uint_as_float(o[g * 8 + 2 * i]), __uint_as_float(o[g * 8 + 2 * i + 1]));
+          *reinterpret_cast<uint4*>(orow + c * 32 + g * 8) = v;
+        }
+      }
+    }
+  }
+}
+
 // The wide form, by head dimension 128 (128-row streamed tiles) or 64 (64-row tiles, two CTAs per SM): rows of its
 // streamed tiles, and the launch of one pass.
 constexpr int bwd_wide_rows(int d) { return d; }

@@ -136,57 +136,11 @@ flash_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmX0, const __grid_con
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const int G = p.Hq / p.Hkv;
-  // CTAs start in the order of their linear index; with a causal mask the tile index is the slowest
-  // coordinate, heaviest tile first (key tile 0 for dK/dV, the last query tile for dQ), heads and
-  // batches the fastest, so that the light CTAs of all heads fill the tail.
-  int b = blockIdx.z;
-  int hx = blockIdx.y;  // DKV: kv head ; dQ: query head
-  int xi = blockIdx.x;
-  if (p.causal) {
-    const int lin = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
-    const int hb = gridDim.y * gridDim.z;
-    xi = lin / hb;
-    hx = (lin % hb) % gridDim.y;
-    b = (lin % hb) / gridDim.y;
-  }
-  const int xb = (DKV || !p.causal) ? xi : (gridDim.x - 1 - xi);
-  const int x0 = xb * kStat;  // first key (DKV) or first query (dQ) of this CTA
-
-  // iteration space over streamed tiles
-  int y_first = 0, y_count, n_it;
-  const long long seg_base = (long long)b * p.Tq;
-  if (DKV) {
-    // queries of this key tile: from the first key's lower bound to the last key's upper bound
-    int q_hi = p.Tq;
-    const int k_last = min(x0 + kStat - 1, p.Tk - 1);
-    if (p.causal) {
-      int qmin = x0 - p.kv_offset;
-      y_first = qmin > 0 ? qmin / kStream : 0;
-    }
-    if (p.window > 0) q_hi = min(q_hi, k_last - p.kv_offset + p.window);
-    if (p.seg_start && x0 < p.Tk) y_first = max(y_first, p.seg_start[seg_base + x0] / kStream);
-    if (p.seg_end && x0 < p.Tk) q_hi = min(q_hi, p.seg_end[seg_base + k_last]);
-    const int nqb = (max(q_hi, 0) + kStream - 1) / kStream;
-    y_count = nqb - y_first;
-    if (y_count < 0) y_count = 0;
-    n_it = y_count * G;
-  } else {
-    // keys of this query tile: from the first query's lower bound to the last query's upper bound
-    int nkb = (p.Tk + kStream - 1) / kStream;
-    const int q_last = min(x0 + kStat - 1, p.Tq - 1);
-    if (p.causal) {
-      int last_key = x0 + kStat - 1 + p.kv_offset;
-      int lim = last_key < 0 ? 0 : last_key / kStream + 1;
-      nkb = min(nkb, lim);
-    }
-    if (p.seg_end && x0 < p.Tq) nkb = min(nkb, (p.seg_end[seg_base + q_last] + kStream - 1) / kStream);
-    int lo_first = 0;
-    if (p.window > 0) lo_first = max(lo_first, x0 + p.kv_offset - p.window + 1);
-    if (p.seg_start && x0 < p.Tq) lo_first = max(lo_first, p.seg_start[seg_base + x0]);
-    y_first = lo_first / kStream;
-    y_count = max(nkb - y_first, 0);
-    n_it = y_count;
-  }
+  const BwdTile tile = bwd_tile<DKV>(p);
+  const int b = tile.b, hx = tile.hx, x0 = tile.x0;   // hx: KV head (DKV) or query head (dQ)
+  int y_first, y_count;
+  bwd_stream<DKV, kStream>(p, tile, y_first, y_count);
+  const int n_it = DKV ? y_count * G : y_count;
 
   if (threadIdx.x == 0) {
     *abort_w = 0;
@@ -344,25 +298,8 @@ flash_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmX0, const __grid_con
         delta_row = p.ndsc[o];
       }
     }
-    // streamed indices (queries for dKV, keys for dQ) that this row may pair with
     int y_lo, y_hi;
-    if (DKV) {
-      y_lo = (xi < p.Tk) ? (p.causal ? max(xi - p.kv_offset, 0) : 0) : 0x3fffffff;
-      y_hi = p.Tq;
-      if (p.window > 0) y_hi = min(y_hi, xi - p.kv_offset + p.window);
-      if (xi < p.Tk) {
-        if (p.seg_start) y_lo = max(y_lo, p.seg_start[seg_base + xi]);
-        if (p.seg_end) y_hi = min(y_hi, p.seg_end[seg_base + xi]);
-      }
-    } else {
-      y_lo = 0;
-      y_hi = (xi < p.Tq) ? (p.causal ? min(p.Tk, xi + p.kv_offset + 1) : p.Tk) : 0;
-      if (p.window > 0) y_lo = max(y_lo, xi + p.kv_offset - p.window + 1);
-      if (xi < p.Tq) {
-        if (p.seg_start) y_lo = max(y_lo, p.seg_start[seg_base + xi]);
-        if (p.seg_end) y_hi = min(y_hi, p.seg_end[seg_base + xi]);
-      }
-    }
+    bwd_row_bounds<DKV>(p, b, xi, y_lo, y_hi);
     bool ok = true;
     if (kXTmem && n_it > 0) {
       // one group of four warps per operand, a row per thread: 16-byte pieces of the 128-byte-swizzled tile to bf16 pairs
@@ -453,44 +390,7 @@ flash_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmX0, const __grid_con
     if (ok && n_it > 0) ok = mbar_wait_warp(acc_done, 0, wc, 8);
     if (ok) {
       tc_fence_after_sync();
-      const int t_lim = DKV ? p.Tk : p.Tq;
-      const long long obase = (long long)b * p.out_batch + (long long)xi * p.out_tok +
-                              (long long)hx * p.out_head;
-#pragma unroll 1
-      for (int a = DKV ? 0 : 1; a < 2; ++a) {
-        __nv_bfloat16* orow = (a == 0 ? p.out0 : p.out1) + obase;
-        const uint32_t t_acc = (a == 0 ? tmem_acc0 : tmem_acc1) + t_lane;
-#pragma unroll 1
-        for (int c = half * (D / 64); c < (half + 1) * (D / 64); ++c) {
-          uint32_t o[32];
-          if (n_it > 0) {
-            tmem_ld_32x32b_x32(t_acc + c * 32, o);
-            tmem_ld_wait();
-          } else {
-#pragma unroll
-            for (int i = 0; i < 32; ++i) o[i] = 0;
-          }
-          if (xi < t_lim) {
-#pragma unroll
-            for (int g = 0; g < 4; ++g) {
-              uint4 v;
-              __nv_bfloat162 t0 = __floats2bfloat162_rn(__uint_as_float(o[g * 8 + 0]),
-                                                        __uint_as_float(o[g * 8 + 1]));
-              __nv_bfloat162 t1 = __floats2bfloat162_rn(__uint_as_float(o[g * 8 + 2]),
-                                                        __uint_as_float(o[g * 8 + 3]));
-              __nv_bfloat162 t2 = __floats2bfloat162_rn(__uint_as_float(o[g * 8 + 4]),
-                                                        __uint_as_float(o[g * 8 + 5]));
-              __nv_bfloat162 t3 = __floats2bfloat162_rn(__uint_as_float(o[g * 8 + 6]),
-                                                        __uint_as_float(o[g * 8 + 7]));
-              v.x = *reinterpret_cast<uint32_t*>(&t0);
-              v.y = *reinterpret_cast<uint32_t*>(&t1);
-              v.z = *reinterpret_cast<uint32_t*>(&t2);
-              v.w = *reinterpret_cast<uint32_t*>(&t3);
-              *reinterpret_cast<uint4*>(orow + c * 32 + g * 8) = v;
-            }
-          }
-        }
-      }
+      bwd_store<D, DKV>(p, tile, tmem_acc0 + t_lane, tmem_acc1 + t_lane, xi, half, n_it > 0);
     }
   }
 
