@@ -668,59 +668,8 @@ gemm_pair_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
   cluster_sync_all();   // every partial tile is in shared memory, and the MMAs are done with the peers' operands
   if (!*abort_w) {
     const int row0 = tm * kPairM + half * 128;
-    const int rows = min(128, p.M - row0);
-    const uint32_t base = smem_u32(smem);
-    for (int u = pair * kPairThreads + (int)threadIdx.x; u < rows * (BN / 4); u += c * kPairThreads) {
-      const int r = u / (BN / 4), j4 = (u % (BN / 4)) * 4;
-      const int col = tn * BN + j4;
-      if (col >= p.N) continue;
-      const uint32_t at = base + (uint32_t)(r * LD + j4) * 4;
-      float4 t[4];
-#pragma unroll
-      for (int h = 0; h < 4; ++h) t[h] = h < c ? ld_cluster_f4(at, 2 * h + half) : make_float4(0.f, 0.f, 0.f, 0.f);
-      float v[4] = {t[0].x, t[0].y, t[0].z, t[0].w};
-#pragma unroll
-      for (int h = 1; h < 4; ++h) { v[0] += t[h].x; v[1] += t[h].y; v[2] += t[h].z; v[3] += t[h].w; }
-      const bool whole = col + 4 <= p.N;
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        v[i] *= p.alpha;
-        if (p.bias && col + i < p.N)
-          v[i] += p.bias_f32 ? reinterpret_cast<const float*>(p.bias)[col + i]
-                             : __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(p.bias)[col + i]);
-      }
-      const size_t off = (size_t)(row0 + r) * p.ldc + col;
-      if (p.out_f32) {
-        float* o = reinterpret_cast<float*>(p.C) + off;
-        if (whole && (reinterpret_cast<uintptr_t>(o) & 15) == 0) {
-          float4 w = make_float4(v[0], v[1], v[2], v[3]);
-          if (p.accumulate) {
-            const float4 old = *reinterpret_cast<const float4*>(o);
-            w.x += old.x; w.y += old.y; w.z += old.z; w.w += old.w;
-          }
-          *reinterpret_cast<float4*>(o) = w;
-        } else {
-          for (int i = 0; i < 4 && col + i < p.N; ++i) o[i] = p.accumulate ? o[i] + v[i] : v[i];
-        }
-      } else {
-        __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(p.C) + off;
-        if (whole && (reinterpret_cast<uintptr_t>(o) & 7) == 0) {
-          if (p.accumulate) {
-            const uint2 old = *reinterpret_cast<const uint2*>(o);
-            const float2 f0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&old.x));
-            const float2 f1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&old.y));
-            v[0] += f0.x; v[1] += f0.y; v[2] += f1.x; v[3] += f1.y;
-          }
-          uint2 w;
-          *reinterpret_cast<__nv_bfloat162*>(&w.x) = __floats2bfloat162_rn(v[0], v[1]);
-          *reinterpret_cast<__nv_bfloat162*>(&w.y) = __floats2bfloat162_rn(v[2], v[3]);
-          *reinterpret_cast<uint2*>(o) = w;
-        } else {
-          for (int i = 0; i < 4 && col + i < p.N; ++i)
-            o[i] = __float2bfloat16(p.accumulate ? __bfloat162float(o[i]) + v[i] : v[i]);
-        }
-      }
-    }
+    cluster_sum_store<BN, LD, 2, 4>({p.C, p.ldc, p.N, p.bias, p.bias_f32, p.out_f32, p.accumulate, p.alpha}, smem_u32(smem), row0,
+                                 min(128, p.M - row0), tn * BN, pair * kPairThreads + (int)threadIdx.x, c * kPairThreads, half, c);
   }
   cluster_sync_all();   // nobody leaves while a peer may read its tile
   if (warp == 1) {

@@ -159,64 +159,9 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant_
     __syncthreads();
   }
   cluster_sync_all();   // every partial tile of the cluster is in shared memory
-  if (!*abort_w) {
-    const uint32_t base = smem_u32(smem);
-    for (int u = rank * kRowsThreads + (int)threadIdx.x; u < p.M * 32; u += csize * kRowsThreads) {
-      const int r = u >> 5, c = (u & 31) * 4;   // row of C, column of the tile
-      const int col = n0 + c;
-      if (col >= p.N) continue;
-      const uint32_t at = base + (uint32_t)(r * 132 + c) * 4;
-      float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-      for (int h0 = 0; h0 < csize; h0 += 4) {
-        float4 t[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-          t[j] = h0 + j < csize ? ld_cluster_f4(at, h0 + j) : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) { acc.x += t[j].x; acc.y += t[j].y; acc.z += t[j].z; acc.w += t[j].w; }
-      }
-      float v[4] = {acc.x * p.alpha, acc.y * p.alpha, acc.z * p.alpha, acc.w * p.alpha};
-      const bool whole = col + 4 <= p.N;
-      if (p.bias) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-          if (col + i < p.N)
-            v[i] += p.bias_f32 ? reinterpret_cast<const float*>(p.bias)[col + i]
-                               : __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(p.bias)[col + i]);
-      }
-      const size_t off = (size_t)r * p.ldc + col;
-      if (p.out_f32) {
-        float* o = reinterpret_cast<float*>(p.C) + off;
-        if (whole && (reinterpret_cast<uintptr_t>(o) & 15) == 0) {
-          float4 w = make_float4(v[0], v[1], v[2], v[3]);
-          if (p.accumulate) {
-            const float4 old = *reinterpret_cast<const float4*>(o);
-            w.x += old.x; w.y += old.y; w.z += old.z; w.w += old.w;
-          }
-          *reinterpret_cast<float4*>(o) = w;
-        } else {
-          for (int i = 0; i < 4 && col + i < p.N; ++i) o[i] = p.accumulate ? o[i] + v[i] : v[i];
-        }
-      } else {
-        __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(p.C) + off;
-        if (whole && (reinterpret_cast<uintptr_t>(o) & 7) == 0) {
-          if (p.accumulate) {
-            const uint2 old = *reinterpret_cast<const uint2*>(o);
-            const float2 f0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&old.x));
-            const float2 f1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&old.y));
-            v[0] += f0.x; v[1] += f0.y; v[2] += f1.x; v[3] += f1.y;
-          }
-          uint2 w;
-          *reinterpret_cast<__nv_bfloat162*>(&w.x) = __floats2bfloat162_rn(v[0], v[1]);
-          *reinterpret_cast<__nv_bfloat162*>(&w.y) = __floats2bfloat162_rn(v[2], v[3]);
-          *reinterpret_cast<uint2*>(o) = w;
-        } else {
-          for (int i = 0; i < 4 && col + i < p.N; ++i)
-            o[i] = __float2bfloat16(p.accumulate ? __bfloat162float(o[i]) + v[i] : v[i]);
-        }
-      }
-    }
-  }
+  if (!*abort_w)
+    cluster_sum_store<128, 132, 1, 8>({p.C, p.ldc, p.N, p.bias, p.bias_f32, p.out_f32, p.accumulate, p.alpha}, smem_u32(smem), 0,
+                                   p.M, n0, rank * kRowsThreads + (int)threadIdx.x, csize * kRowsThreads, 0, csize);
   cluster_sync_all();   // nobody leaves while a peer may read its tile
   if (warp == 1) {
     tc_fence_after_sync();

@@ -658,6 +658,18 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         if (col0 >= p.N) break;  // warp-uniform
         uint32_t r[32];
         tmem_ld_32x32b_x32(t_row + c, r);
+        const bool full_chunk = (col0 + 32 <= p.N);
+        uint8_t* crow_b = reinterpret_cast<uint8_t*>(p.C) + ((size_t)row * p.ldc + col0) * (p.out_f32 ? 4 : 2);
+        const bool vec = full_chunk && (reinterpret_cast<uintptr_t>(crow_b) & 15) == 0;
+        uint4 old[8];   // what is accumulated into, requested under the TMEM load (2048 x 2048 x 768: 22.2 -> 17.5 us)
+        if (p.accumulate && vec && row < p.M) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) old[i] = reinterpret_cast<const uint4*>(crow_b)[i];
+          if (p.out_f32) {
+#pragma unroll
+            for (int i = 4; i < 8; ++i) old[i] = reinterpret_cast<const uint4*>(crow_b)[i];
+          }
+        }
         tmem_ld_wait();
         if (row < p.M) {
           float v[32];
@@ -675,7 +687,6 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           }
 #pragma unroll
           for (int i = 0; i < 32; ++i) v[i] *= p.alpha;
-          const bool full_chunk = (col0 + 32 <= p.N);
           if (p.bias) bias32_apply(v, p.bias, p.bias_f32, col0, p.N);
           if (p.rs_mode && rs_coalesce) {
             // bf16 partial into the warp's staging rows; flushed below in 128-byte row segments
@@ -709,14 +720,15 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                 if (col0 + i < p.N) crow[i] = __float2bfloat16(v[i]);
             }
           } else if (p.out_f32) {
-            float* crow = reinterpret_cast<float*>(p.C) + (size_t)row * p.ldc + col0;
-            if (full_chunk && ((reinterpret_cast<uintptr_t>(crow) & 15) == 0)) {
+            float* crow = reinterpret_cast<float*>(crow_b);
+            if (vec) {
 #pragma unroll
               for (int i = 0; i < 32; i += 4) {
                 float4 o = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
                 if (p.accumulate) {
-                  float4 old = *reinterpret_cast<float4*>(crow + i);
-                  o.x += old.x; o.y += old.y; o.z += old.z; o.w += old.w;
+                  const uint4 u = old[i / 4];
+                  o.x += __uint_as_float(u.x); o.y += __uint_as_float(u.y);
+                  o.z += __uint_as_float(u.z); o.w += __uint_as_float(u.w);
                 }
                 *reinterpret_cast<float4*>(crow + i) = o;
               }
@@ -725,17 +737,15 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                 if (col0 + i < p.N) crow[i] = p.accumulate ? crow[i] + v[i] : v[i];
             }
           } else {
-            __nv_bfloat16* crow =
-                reinterpret_cast<__nv_bfloat16*>(p.C) + (size_t)row * p.ldc + col0;
-            if (full_chunk && ((reinterpret_cast<uintptr_t>(crow) & 15) == 0)) {
+            __nv_bfloat16* crow = reinterpret_cast<__nv_bfloat16*>(crow_b);
+            if (vec) {
 #pragma unroll
               for (int i = 0; i < 32; i += 8) {
                 if (p.accumulate) {
-                  uint4 old = *reinterpret_cast<uint4*>(crow + i);
-                  const __nv_bfloat162* ob = reinterpret_cast<const __nv_bfloat162*>(&old);
+                  const __nv_bfloat162* ob = reinterpret_cast<const __nv_bfloat162*>(&old[i / 8]);
 #pragma unroll
                   for (int j = 0; j < 4; ++j) {
-                    float2 f = __bfloat1622float2(ob[j]);
+                    const float2 f = __bfloat1622float2(ob[j]);
                     v[i + 2 * j] += f.x;
                     v[i + 2 * j + 1] += f.y;
                   }
@@ -743,14 +753,13 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                 uint4 o;
                 __nv_bfloat162* ob2 = reinterpret_cast<__nv_bfloat162*>(&o);
 #pragma unroll
-                for (int j = 0; j < 4; ++j)
-                  ob2[j] = __floats2bfloat162_rn(v[i + 2 * j], v[i + 2 * j + 1]);
+                for (int j = 0; j < 4; ++j) ob2[j] = __floats2bfloat162_rn(v[i + 2 * j], v[i + 2 * j + 1]);
                 *reinterpret_cast<uint4*>(crow + i) = o;
               }
             } else {
               for (int i = 0; i < 32; ++i)
                 if (col0 + i < p.N) {
-                  float x = p.accumulate ? __bfloat162float(crow[i]) + v[i] : v[i];
+                  const float x = p.accumulate ? __bfloat162float(crow[i]) + v[i] : v[i];
                   crow[i] = __float2bfloat16(x);
                 }
             }

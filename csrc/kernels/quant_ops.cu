@@ -321,14 +321,7 @@ wq_gemv_kernel(const __nv_bfloat16* __restrict__ x, const uint8_t* __restrict__ 
 // lane (g, t) takes 16 consecutive bytes of weight rows g and g + 8 (16 or 32 k) and the matching
 // k of x row g: every global load is a full 16-byte vector and no shuffles are needed.
 // A CTA owns TILES x 16 output columns; its 8 warps split K and reduce through shared memory.
-__device__ __forceinline__ void mma_bf16_16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2,
-                                               uint32_t a3, uint32_t b0, uint32_t b1) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
-      "{%0,%1,%2,%3};\n"
-      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
+
 // (v & mask) | bits in one instruction: written with two literals it became two
 __device__ __forceinline__ uint32_t and_or(uint32_t v, uint32_t mask, uint32_t bits) {
   uint32_t r;

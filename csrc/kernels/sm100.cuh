@@ -489,7 +489,109 @@ __device__ __forceinline__ float ld_cluster_f32(uint32_t saddr, uint32_t rank) {
   return v;
 }
 
+// ---------------------------------------------------------------- warp MMA
+__device__ __forceinline__ void mma_bf16_16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
+                                               uint32_t b0, uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
+      "{%0, %1, %2, %3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
 // ---------------------------------------------------------------- GEMM epilogues
+// Where and how the sum of a split product leaves.
+struct SumStore {
+  void* C;
+  int ldc, N;
+  const void* bias;
+  int bias_f32, out_f32, accumulate;
+  float alpha;
+};
+// Sums the fp32 partial tiles of COLS columns (rows LD floats apart) that `parts` CTAs of a cluster hold at `base` in
+// their shared memory, CTAs rank0, rank0 + STEP, .., in that order, and stores the result: `rows` rows from (row0, col0)
+// on. Units of four columns are dealt out from u0 in steps of du. MOST: parts at most, all requested at once.
+template <int COLS, int LD, int STEP, int MOST>
+__device__ __forceinline__ void cluster_sum_store(const SumStore& p, uint32_t base, int row0, int rows, int col0, int u0,
+                                                  int du, int rank0, int parts) {
+  constexpr int UNITS = 2;   // in flight per thread
+  for (int u = u0; u < rows * (COLS / 4); u += UNITS * du) {
+    float4 t[UNITS][MOST];
+    uint4 old[UNITS];
+    uint8_t* o[UNITS];
+    int cols[UNITS];   // of a unit that exist: 0 to 4
+    bool vec[UNITS];
+#pragma unroll
+    for (int k = 0; k < UNITS; ++k) {
+      const int uk = u + k * du, r = uk / (COLS / 4), j4 = (uk % (COLS / 4)) * 4, col = col0 + j4;
+      cols[k] = r < rows ? max(0, min(4, p.N - col)) : 0;
+      o[k] = reinterpret_cast<uint8_t*>(p.C) + ((size_t)(row0 + r) * p.ldc + col) * (p.out_f32 ? 4 : 2);
+      vec[k] = cols[k] == 4 && (reinterpret_cast<uintptr_t>(o[k]) & (p.out_f32 ? 15 : 7)) == 0;
+      // what is accumulated into is requested with the partial sums, and converted only where it is used: the warp
+      // would wait for it here
+      old[k] = make_uint4(0u, 0u, 0u, 0u);
+      if (p.accumulate && vec[k]) {
+        if (p.out_f32) {
+          old[k] = *reinterpret_cast<const uint4*>(o[k]);
+        } else {
+          const uint2 w = *reinterpret_cast<const uint2*>(o[k]);
+          old[k].x = w.x;
+          old[k].y = w.y;
+        }
+      }
+      const uint32_t at = base + (uint32_t)(r * LD + j4) * 4;
+#pragma unroll
+      for (int h = 0; h < MOST; ++h)
+        t[k][h] = h < parts && cols[k] ? ld_cluster_f4(at, rank0 + STEP * h) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+#pragma unroll
+    for (int k = 0; k < UNITS; ++k) {
+      const int col = col0 + ((u + k * du) % (COLS / 4)) * 4;
+      float v[4] = {t[k][0].x, t[k][0].y, t[k][0].z, t[k][0].w};
+#pragma unroll
+      for (int h = 1; h < MOST; ++h) { v[0] += t[k][h].x; v[1] += t[k][h].y; v[2] += t[k][h].z; v[3] += t[k][h].w; }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        v[i] *= p.alpha;
+        if (p.bias && i < cols[k])
+          v[i] += p.bias_f32 ? reinterpret_cast<const float*>(p.bias)[col + i]
+                             : __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(p.bias)[col + i]);
+      }
+      if (p.accumulate) {
+        if (vec[k] && p.out_f32) {
+          v[0] += __uint_as_float(old[k].x); v[1] += __uint_as_float(old[k].y);
+          v[2] += __uint_as_float(old[k].z); v[3] += __uint_as_float(old[k].w);
+        } else if (vec[k]) {
+          const float2 f0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&old[k].x));
+          const float2 f1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&old[k].y));
+          v[0] += f0.x; v[1] += f0.y; v[2] += f1.x; v[3] += f1.y;
+        } else {
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            if (i < cols[k])
+              v[i] += p.out_f32 ? reinterpret_cast<const float*>(o[k])[i]
+                                : __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(o[k])[i]);
+        }
+      }
+      if (vec[k] && p.out_f32) {
+        *reinterpret_cast<float4*>(o[k]) = make_float4(v[0], v[1], v[2], v[3]);
+      } else if (vec[k]) {
+        uint2 w;
+        *reinterpret_cast<__nv_bfloat162*>(&w.x) = __floats2bfloat162_rn(v[0], v[1]);
+        *reinterpret_cast<__nv_bfloat162*>(&w.y) = __floats2bfloat162_rn(v[2], v[3]);
+        *reinterpret_cast<uint2*>(o[k]) = w;
+      } else {
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          if (i < cols[k]) {
+            if (p.out_f32) reinterpret_cast<float*>(o[k])[i] = v[i];
+            else reinterpret_cast<__nv_bfloat16*>(o[k])[i] = __float2bfloat16(v[i]);
+          }
+      }
+    }
+  }
+}
+
 // The bias of 32 consecutive output columns, shared by all rows a warp drains. Every lane reads the same
 // addresses, so the cost is the number of load instructions and their latency: four (bf16) or eight (fp32)
 // 16-byte loads, issued by the caller before it waits for its TMEM load. As 32 two-byte loads inside the

@@ -141,6 +141,7 @@ int tpb_flash_fwd(const void* q, const void* k, const void* v, void* o, float* l
                   long long o_head, long long o_batch, int lse_stride, int causal, float scale,
                   uint32_t* status, void* stream, const int* kv_len, int n_splits,
                   long long o_split_stride, long long lse_split_stride);
+// delta: scratch of two arrays [B, Hq, Tq rounded up to 128].
 int tpb_flash_bwd(const void* dout, const void* q, const void* k, const void* v, const void* o,
                   const float* lse, float* delta, void* dq, void* dk, void* dv, int B, int Tq,
                   int Tk, int Hq, int Hkv, int D, long long q_tok, long long q_head,
