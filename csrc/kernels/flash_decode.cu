@@ -11,7 +11,7 @@
 //   * the keys are split over CTAs until the chip is full; partial sums stay fp32. Up to eight splits of a row tile are
 //     one cluster that merges them through distributed shared memory, in rank order; more go through memory and a
 //     second kernel.
-// The same case takes 117 us (4.6 TB/s).
+// The same case takes 114 us (4.7 TB/s).
 // Scores, running maximum, sums and output accumulate in fp32; probabilities are rounded to bf16 for the second
 // product, as in flash_fwd_kernel.
 #include "sm100.cuh"
@@ -343,28 +343,63 @@ flash_decode_merge_kernel(const DecodeParams p) {
     p.lse[((long long)b * p.Hq + h) * p.lse_stride + tq] = den > 0.f ? (M + log2f(den)) * 0.6931471805599453f : -INFINITY;
 }
 
-// Splits of the keys, by the time in ns that the launch takes. A CTA needs kKeyNs per key, more where several share an
-// SM (four of D = 64 fit by their registers, two of D = 128), kFullNs on a full chip, which for D = 128 is memory's rate,
-// and some 4 us from start to end. Splits that a cluster merges cost 1 us. More than kDecCluster of them need a second
-// kernel and scratch: 3 us + 60 ns a split on the device and 5 us on the host, which bounds a call over a short cache
-// (one token over 1000 keys: 32 us a call with one launch, 41 us with two). Measured, D x B x Hkv x Tk, splits: us:
-// 128 x 1 x 8 x 4096, 1: 76, 4: 22.8, 8: 13.8, by two kernels 16: 11.1; 128 x 16 x 8 x 4096, 1: 100, 2: 61, 4: 65, 8: 74;
-// 64 x 16 x 8 x 4096, 1: 66, 4: 29, 6: 37, 8: 32; 128 x 32 x 8 x 8192, 1: 222, 2: 227, 4: 236, 8: 255.
-static int decode_splits(int B, int Hkv, int row_tiles, int Tk, int D, int most) {
-  static const int kKeyNs[2][4] = {{11, 17, 21, 24}, {20, 27, 27, 27}}, kFullNs[2] = {24, 31};
-  const int fit = D == 64 ? 4 : 2;
-  const int* key_ns = kKeyNs[D == 64 ? 0 : 1];
-  const long long ctas = (long long)B * Hkv * row_tiles, sms = sm_count(), slots = fit * sms;
-  int best = 1;
-  long long best_cost = -1;
-  for (int n = 1; n <= most && (n == 1 || Tk / n >= 64); ++n) {
-    const long long keys = (Tk + n - 1) / n, full = ctas * n / slots, rest = ctas * n % slots;
-    long long cost = full * (keys * kFullNs[D == 64 ? 0 : 1] + 4000);
-    if (rest) cost += keys * key_ns[(rest + sms - 1) / sms - 1] + 4000;
-    if (n > kDecCluster) cost += 8000 + 60 * n;
-    else if (n > 1) cost += 1000;
-    if (best_cost < 0 || cost < best_cost) { best = n; best_cost = cost; }
+// Clusters of n CTAs that fit the device at once, asked of the runtime once per size: the SMs of a GPC are not a multiple
+// of every n (32 clusters of 8 CTAs of D = 128 fit, 96 of 3 do not, although 296 CTAs do).
+static int decode_resident(int D, int n) {
+  static int resident[2][kDecCluster + 1] = {};
+  int& r = resident[D == 64 ? 0 : 1][n];
+  if (r == 0) {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = n;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.gridDim = dim3(n, 4 * sm_count());
+    cfg.blockDim = dim3(kDecWarps * 32);
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int fit = 0;
+    const cudaError_t e = D == 64 ? cudaOccupancyMaxActiveClusters(&fit, flash_decode_kernel<64>, &cfg)
+                                  : cudaOccupancyMaxActiveClusters(&fit, flash_decode_kernel<128>, &cfg);
+    r = e == cudaSuccess && fit > 0 ? fit : -1;
   }
+  return r;
+}
+
+// Splits of the keys and who merges them, by the time in ns that the launch takes: for each round of resident CTAs 1.8 us,
+// of clusters, which start together, 3.3 us, and kKeyNs per key of a CTA, more where several share an SM (four of D = 64
+// fit by their registers, two of D = 128), kFullNs on a full chip (some 5 TB/s). A cluster's merge costs 1 us; a second
+// kernel and scratch 3 us + 60 ns a split on the device and 5 us on the host, which bounds a call over a short cache (one
+// token over 1000 keys: 32 us a call with one launch, 41 us with two). Caches from memory, D x B x Hkv x Tk, splits: us
+// (9 and more by two kernels): 128 x 8 x 8 x 16381, 1: 396, 3: 152, 4: 119, 8: 124, 9: 114, 10: 143, 16: 126;
+// 128 x 12 x 8 x 8192, 3: 146, 4: 117, 5: 99, 6: 122, 9: 90; 128 x 32 x 8 x 8192, 1: 223, 2: 230, 8: 258; 64 x 8 x 8 x
+// 16381, 4: 78, 8: 53, 9: 51; 128 x 1 x 8 x 4096, 1: 76, 4: 23, 8: 14, 16: 11.
+struct DecodePlan {
+  int splits;
+  bool memory;   // merged by the second kernel
+};
+static DecodePlan decode_plan(int B, int Hkv, int row_tiles, int Tk, int D, bool memory) {
+  static const int kKeyNs[2][4] = {{14, 18, 20, 22}, {22, 27, 27, 27}}, kFullNs[2] = {22, 28};
+  const int fit = D == 64 ? 4 : 2, wide = D == 64 ? 0 : 1;
+  const long long tiles = (long long)B * Hkv * row_tiles, sms = sm_count();
+  DecodePlan best = {1, false};
+  long long best_cost = -1;
+  // units are what is scheduled, clusters of `ctas` or single CTAs
+  auto consider = [&](int n, bool mem, long long units, long long slots, int ctas) {
+    const long long keys = (Tk + n - 1) / n, full = units / slots, rest = units % slots, round = ctas > 1 ? 3300 : 1800;
+    long long cost = full * (keys * kFullNs[wide] + round);
+    if (rest) {
+      const long long per_sm = (rest * ctas + sms - 1) / sms;
+      cost += keys * kKeyNs[wide][(per_sm < fit ? per_sm : fit) - 1] + round;
+    }
+    cost += mem ? 8000 + 60 * n : (n > 1 ? 1000 : 0);
+    if (best_cost < 0 || cost < best_cost) { best = {n, mem}; best_cost = cost; }
+  };
+  consider(1, false, tiles, fit * sms, 1);
+  for (int n = 2; n <= kDecCluster && Tk / n >= 64; ++n)
+    if (decode_resident(D, n) > 0) consider(n, false, tiles, decode_resident(D, n), n);
+  for (int n = 2; memory && n <= 64 && Tk / n >= 64; ++n) consider(n, true, tiles * n, fit * sms, 1);
   return best;
 }
 
@@ -372,17 +407,16 @@ static int decode_splits(int B, int Hkv, int row_tiles, int Tk, int D, int most)
 
 using namespace tpb;
 
-// Number of key splits to pass to tpb_flash_decode. Above tpb_flash_decode_cluster() of them part_o has to hold
-// n * B * Hq * Tq * D floats and part_lse n * B * Hq * Tq.
-extern "C" int tpb_flash_decode_cluster() { return kDecCluster; }
+// 0 where tpb_flash_decode needs no memory for its splits (it then takes n_splits 0 and picks them itself, as it may
+// anyway up to 2048 keys); else their number n: part_o has to hold n * B * Hq * Tq * D floats, part_lse n * B * Hq * Tq.
 extern "C" int tpb_flash_decode_splits(int B, int Tq, int Tk, int Hq, int Hkv, int D) {
-  if (B <= 0 || Tq <= 0 || Tk <= 0 || Hkv <= 0) return 1;
-  const int R = Tq * (Hq / Hkv);
-  return decode_splits(B, Hkv, (R + kDecRows - 1) / kDecRows, Tk, D, 64);
+  if (B <= 0 || Tq <= 0 || Tk <= 0 || Hkv <= 0) return 0;
+  const DecodePlan plan = decode_plan(B, Hkv, (Tq * (Hq / Hkv) + kDecRows - 1) / kDecRows, Tk, D, true);
+  return plan.memory ? plan.splits : 0;
 }
 
-// Arguments as in tpb_flash_fwd_ex; lse [B, Hq, lse_stride]. n_splits 0: the best number that needs no part_o, which is
-// the best of all up to 2048 keys.
+// Arguments as in tpb_flash_fwd_ex; lse [B, Hq, lse_stride]. n_splits 0: the best number that needs no part_o. With
+// part_o the splits are merged by a second kernel, without (eight at most) by clusters.
 extern "C" int tpb_flash_decode(const void* q, const void* k, const void* v, void* o, float* lse, float* part_o,
                                 float* part_lse, int B, int Tq, int Tk, int Hq, int Hkv, int D, long long q_tok,
                                 long long q_head, long long q_batch, long long k_tok, long long k_head,
@@ -397,8 +431,11 @@ extern "C" int tpb_flash_decode(const void* q, const void* k, const void* v, voi
   if ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v) |
        reinterpret_cast<uintptr_t>(o)) & 15)
     return -2;
-  if (n_splits > kDecCluster && (!part_o || !part_lse)) return -2;
-  if (n_splits == 0) n_splits = decode_splits(B, Hkv, (Tq * (Hq / Hkv) + kDecRows - 1) / kDecRows, Tk, D, kDecCluster);
+  if ((n_splits > kDecCluster && !part_o) || (part_o && !part_lse)) return -2;
+  if (n_splits == 0) {
+    part_o = part_lse = nullptr;
+    n_splits = decode_plan(B, Hkv, (Tq * (Hq / Hkv) + kDecRows - 1) / kDecRows, Tk, D, false).splits;
+  }
   DecodeParams p;
   p.q = (const __nv_bfloat16*)q; p.k = (const __nv_bfloat16*)k; p.v = (const __nv_bfloat16*)v;
   p.o = (__nv_bfloat16*)o; p.lse = lse; p.part_o = n_splits > 1 ? part_o : nullptr; p.part_lse = part_lse;

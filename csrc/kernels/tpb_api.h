@@ -103,7 +103,6 @@ int tpb_block_pre(const void* x, const void* norm_w, float eps, const void* w_qk
 int tpb_block_post(const void* attn, const void* w_o, void* o, const void* x, const void* norm_w, float eps, void* x2,
                    void* h, const void* w_gu, void* gu, void* act, const void* w_down, void* y, int accumulate,
                    int rows, int hidden, int attn_width, int inter, uint32_t* status, void* stream);
-int tpb_flash_decode_cluster();
 int tpb_flash_decode_splits(int B, int Tq, int Tk, int Hq, int Hkv, int D);
 int tpb_flash_decode(const void* q, const void* k, const void* v, void* o, float* lse, float* part_o, float* part_lse,
                      int B, int Tq, int Tk, int Hq, int Hkv, int D, long long q_tok, long long q_head,

@@ -55,7 +55,6 @@ _KERNEL_SIGS = {
     "tpb_cross_entropy_bwd": [P, P, P, P, P, P, P, LL, I, LL, LL, P],
     "tpb_flash_fwd": [P, P, P, P, P, I, I, I, I, I, I] + [LL] * 12 + [I, I, F, P, P, P, I, LL, LL],
     "tpb_flash_fwd_ex": [P, P, P, P, P, I, I, I, I, I, I] + [LL] * 12 + [I, I, F, P, P, P, I, LL, LL, I, P, P],
-    "tpb_flash_decode_cluster": [],
     "tpb_flash_decode_splits": [I, I, I, I, I, I],
     "tpb_flash_decode": [P, P, P, P, P, P, P, I, I, I, I, I, I] + [LL] * 12 + [I, I, F, I, I, P],
     "tpb_flash_bwd_ex": [P] * 10 + [I, I, I, I, I, I] + [LL] * 21 + [I, I, F, P, P, I, P, P],
@@ -118,7 +117,7 @@ def _load(name: str):
 
 
 # kernel launches issued by one call of each entry point (for launch accounting)
-_LAUNCHES = {"tpb_rmsnorm_bwd": 2, "tpb_layernorm_bwd": 2, "tpb_bias_grad": 2, "tpb_bias_grad_chunks": 0, "tpb_flash_decode_splits": 0, "tpb_flash_decode_cluster": 0, "tpb_block_pre": 3, "tpb_block_post": 5, "tpb_flash_bwd": 3, "tpb_rmsnorm_bwd_grid": 0,
+_LAUNCHES = {"tpb_rmsnorm_bwd": 2, "tpb_layernorm_bwd": 2, "tpb_bias_grad": 2, "tpb_bias_grad_chunks": 0, "tpb_flash_decode_splits": 0, "tpb_block_pre": 3, "tpb_block_post": 5, "tpb_flash_bwd": 3, "tpb_rmsnorm_bwd_grid": 0,
              "tpb_grouped_workspace_ints": 0, "tpb_zero": 0, "tpb_adamw_set_overlap": 0, "tpb_flash_fwd_config": 0, "tpb_gemm_set_splitk_workspace": 0, "tpb_grouped_gemm": 2}
 launch_count = 0
 

@@ -83,7 +83,7 @@ def _flash_decode(q, k, v, o, lse, causal: bool, scale: float, window: int) -> N
     part = part_lse = None
     if Tk > 2048:
         n = L.tpb_flash_decode_splits(B, Tq, Tk, Hq, Hkv, D)
-        if n > L.tpb_flash_decode_cluster():   # fp32 partial rows and their sums, merged by a second launch
+        if n:   # fp32 partial rows and their sums, merged by a second launch
             rows = n * B * Hq * Tq
             part = torch.empty(rows * (D + 1), dtype=torch.float32, device=q.device)
             part_lse = part.data_ptr() + 4 * rows * D
