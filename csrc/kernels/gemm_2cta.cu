@@ -733,10 +733,10 @@ static int launch_pair_split(const CUtensorMap& ta, const CUtensorMap& tb, const
 // columns, 0.26 and 8 us with 128, and 1.5 us. Over those products the choice takes 1.005 of the best of all forms on
 // average and nowhere 6 % more than the one-CTA kernel. 1024 x 4096 x 4096: one-CTA 30, pair 27, over two pairs 44 us;
 // 768 x 768 x 16384: one-CTA 79, split over four pairs 29 us.
-bool gemm_pair_split_plan(int M, int N, int K, long long single, int* bn, int* c) {
+bool gemm_pair_split_plan(int M, int N, int K, long long single, long long store, int* bn, int* c) {
   if (M <= 128 || N <= 64 || K <= 0) return false;
   const long long kb = (K + kPairK - 1) / kPairK, pairs = sm_count() / 2, tm = (M + kPairM - 1) / kPairM;
-  const long long whole = (tm * ((N + 255) / 256) + pairs - 1) / pairs * (30 * kb + 190) + 450;
+  const long long whole = (tm * ((N + 255) / 256) + pairs - 1) / pairs * (30 * kb + 190 + 2 * store) + 450;
   long long best = single;
   bool found = false;
   if (whole < best) { best = whole; *bn = 256; *c = 1; found = true; }

@@ -236,12 +236,16 @@ static int launch_rows(const CUtensorMap& tb, const CUtensorMap& ta, const RowsP
 //   M = 32: 4096 x 4096 11.2 / 23.5, 28672 x 4096 41.8 / 43.8, 50304 x 768 22.5 / 19.5
 //   M = 64: 6144 x 1024 9.4 / 10.0, 14336 x 2048 18.6 / 15.6, 28672 x 4096 46.3 / 45.3, 32000 x 1024 17.8 / 16.4
 //   M = 128: 4096 x 1024 9.3 / 10.0, 4096 x 14336 31.9 / 69.7, 6144 x 1024 12.1 / 10.4, 50304 x 768 33.7 / 21.4
-// Between 5/8 and one tile per SM two CTAs share a tile, and half the k-blocks at twice the time each is no gain.
-bool gemm_rows_takes(int M, int N, int K, int a_mn) {
+// Lines in between: M = 64: 8192 x 2048 13.0 / 14.4, 11000 x 2048 18.3 / 16.5; M = 128: 6144 x 4096 21.2 / 23.9, 8192 x
+// 2048 15.8 / 14.4. With results that the other kernel stores from its lanes one by one (accumulated ones, fp32 with a
+// bias) more stay here: 32 x 50304 x 768 accumulated 25 / 28, fp32 with a bias 16 x 50304 x 768 18 / 23, 40 x 28672 x
+// 4096 46 / 50. A single row: 128256 x 2048 84 / 87, 50304 x 768 19.5 / 19.8, 128256 x 512 30 / 26.
+bool gemm_rows_takes(int M, int N, int K, int a_mn, bool slow_store) {
   if (M > 128 || a_mn) return false;
   const long long tiles = (N + 127) / 128, sms = sm_count();
-  if (M <= 32) return tiles <= 2 * sms || (M <= 16 && K >= 4096);
-  return tiles <= 5 * sms / 8 && (M <= 64 || K >= 2048 || tiles * M <= 28 * sms);
+  if (M <= 32) return tiles <= 2 * sms || slow_store || (M <= 16 && K >= 4096) || (M <= 4 && K >= 768);
+  if (M <= 64) return tiles <= sms / 2 || (slow_store && tiles > sms && tiles <= 2 * sms);
+  return tiles <= sms / 4 || (tiles <= sms / 3 && K >= 4096);
 }
 
 // Same contract as gemm_bf16_dispatch for the plain product with a K-major A of at most 128 rows.

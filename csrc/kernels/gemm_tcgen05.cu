@@ -961,13 +961,14 @@ static int pick_block_n(int M, int N, int K, bool splitk) {
 
 // Time of a plain product in this kernel in units of 10 ns, fitted within 7 % (rms) over 230 shapes of 2 to 73 pair tiles
 // and K = 64 to 16384: a round of tiles takes 0.35 us a k-block and 1.5 us with 256 columns, 0.295 and 2.5 us with 128,
-// and the launch 4.6 and 2.5 us. With a split-K workspace the last round is as long as one split plus 4 us.
-static long long gemm_single_cost(int M, int N, int K) {
+// and the launch 4.6 and 2.5 us. With a split-K workspace the last round is as long as one split plus 4 us. `store`: what
+// 128 columns that are not plain bf16 take longer, since a lane stores its own row.
+static long long gemm_single_cost(int M, int N, int K, long long store) {
   const bool wide = pick_block_n(M, N, K, g_sk_ws != nullptr) == 256;
   const long long sms = sm_count(), tiles = (long long)((M + kBlockM - 1) / kBlockM) * ((N + (wide ? 255 : 127)) / (wide ? 256 : 128));
   const int kb = (K + kBlockK - 1) / kBlockK, tail = (int)(tiles % sms);
   const int ns = g_sk_ws && tail ? tail_nsplit(tail, (int)sms, kb) : 1;
-  auto round = [&](int k_blocks) { return wide ? 35LL * k_blocks + 150 : 295LL * k_blocks / 10 + 250; };
+  auto round = [&](int k_blocks) { return wide ? 35LL * k_blocks + 150 + 2 * store : 295LL * k_blocks / 10 + 250 + store; };
   return tiles / sms * round(kb) + (tail ? round((kb + ns - 1) / ns) + (ns > 1 ? 400 : 0) : 0) + (wide ? 460 : 250);
 }
 
@@ -1092,7 +1093,7 @@ extern "C" int tpb_gemm_bf16(const void* A, const void* B, void* C, const void* 
                              int bias_f32, int accumulate, float alpha, uint32_t* status,
                              void* stream) {
   TPB_NVTX("tpb_gemm_bf16");
-  if (tpb::gemm_rows_takes(M, N, K, a_mn))
+  if (tpb::gemm_rows_takes(M, N, K, a_mn, accumulate || (out_f32 && bias)))
     return tpb::gemm_rows_dispatch(A, B, C, bias, M, N, K, lda, ldb, ldc, b_mn, out_f32, bias_f32, accumulate, alpha,
                                    status, static_cast<cudaStream_t>(stream));
   if (g_pair_min_tiles > 0 && (long long)((M + 255) / 256) * ((N + 255) / 256) >= g_pair_min_tiles) {
@@ -1102,8 +1103,10 @@ extern "C" int tpb_gemm_bf16(const void* A, const void* B, void* C, const void* 
     return tpb::gemm_pair_dispatch(A, B, C, bias, M, N, K, lda, ldb, ldc, a_mn, b_mn, out_f32, bias_f32,
                                    accumulate, alpha, 0, status, static_cast<cudaStream_t>(stream));
   }
+  // us that 128 columns take longer as fp32 or accumulated (256 x 1024 x 1032: 11.4 and 12.2 for 8.8) and as both (13.8)
+  const long long store = out_f32 && accumulate ? 500 : (out_f32 || accumulate ? 300 : 0);
   int bn, c;
-  if (g_pair_min_tiles > 0 && tpb::gemm_pair_split_plan(M, N, K, tpb::gemm_single_cost(M, N, K), &bn, &c)) {
+  if (g_pair_min_tiles > 0 && tpb::gemm_pair_split_plan(M, N, K, tpb::gemm_single_cost(M, N, K, store), store, &bn, &c)) {
     if (bn == 256 && c == 1)
       return tpb::gemm_pair_dispatch(A, B, C, bias, M, N, K, lda, ldb, ldc, a_mn, b_mn, out_f32, bias_f32, accumulate,
                                      alpha, 0, status, static_cast<cudaStream_t>(stream));

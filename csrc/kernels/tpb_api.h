@@ -58,13 +58,15 @@ int gemm_bf16_dispatch(const void* A, const void* B, void* C, const void* bias, 
                        int rows_per_flag, uint32_t flag_want, int max_ctas, uint32_t* status,
                        cudaStream_t stream, const GemmFused* fused);
 // A K-major A of at most 128 rows (gemm_rows.cu): whether the product goes there, and the product.
-bool gemm_rows_takes(int M, int N, int K, int a_mn);
+// slow_store: results that are accumulated, or fp32 with a bias.
+bool gemm_rows_takes(int M, int N, int K, int a_mn, bool slow_store);
 int gemm_rows_dispatch(const void* A, const void* B, void* C, const void* bias, int M, int N, int K, int lda, int ldb,
                        int ldc, int b_mn, int out_f32, int bias_f32, int accumulate, float alpha, uint32_t* status,
                        cudaStream_t stream);
 // Few 256-row tiles with a long reduction (gemm_2cta.cu): whether and how the product is split, and the product.
 // `single` is the time of the one-CTA kernel in units of 10 ns; (256, 1) stands for the CTA-pair kernel itself.
-bool gemm_pair_split_plan(int M, int N, int K, long long single, int* bn, int* c);
+// `store`: 10 ns that 128 columns which are not plain bf16 take longer.
+bool gemm_pair_split_plan(int M, int N, int K, long long single, long long store, int* bn, int* c);
 int gemm_pair_split_dispatch(const void* A, const void* B, void* C, const void* bias, int M, int N, int K, int lda,
                              int ldb, int ldc, int a_mn, int b_mn, int out_f32, int bias_f32, int accumulate,
                              float alpha, uint32_t* status, cudaStream_t stream, int bn, int c);

@@ -42,8 +42,13 @@ def test_few_rows_epilogue(M, N, K, kw):
     _check(M, N, K, False, False, **kw)
 
 
-@pytest.mark.parametrize("M,N,K", [(16, 40000, 72), (1, 40000, 4096), (17, 37888, 136), (32, 37896, 136), (33, 11776, 192),
-                                   (64, 11848, 192), (65, 10368, 2048), (128, 4096, 64), (128, 4240, 64), (128, 11848, 2048)])
+@pytest.mark.parametrize("M,N,K", [(16, 40000, 72), (1, 40000, 4096), (17, 37888, 136), (32, 37896, 136), (33, 9472, 192),
+                                   (64, 9480, 192), (65, 6272, 4096), (128, 4736, 64), (128, 4744, 64), (128, 6280, 4096)])
 def test_both_sides_of_the_choice(M, N, K):
     """Sizes on which the kernels of few and of more rows meet."""
     _check(M, N, K, False, M % 2 == 0)
+
+
+def test_choice_by_the_kind_of_result():
+    _check(32, 40000, 72, False, False, accumulate=True)
+    _check(16, 40000, 72, False, False, out_dtype=torch.float32, bias=torch.bfloat16)
