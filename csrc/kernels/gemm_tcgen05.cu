@@ -662,7 +662,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         uint8_t* crow_b = reinterpret_cast<uint8_t*>(p.C) + ((size_t)row * p.ldc + col0) * (p.out_f32 ? 4 : 2);
         const bool vec = full_chunk && (reinterpret_cast<uintptr_t>(crow_b) & 15) == 0;
         uint4 old[8];   // what is accumulated into, requested under the TMEM load (2048 x 2048 x 768: 22.2 -> 17.5 us)
-        if (p.accumulate && vec && row < p.M) {
+        if (p.accumulate && !p.rs_mode && vec && row < p.M) {
 #pragma unroll
           for (int i = 0; i < 4; ++i) old[i] = reinterpret_cast<const uint4*>(crow_b)[i];
           if (p.out_f32) {
