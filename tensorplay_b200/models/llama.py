@@ -105,16 +105,21 @@ class LlamaBlock(nn.Module):
         gu = ops.linear(h, self.w_gate_up)
         return x + ops.linear(ops.swiglu_packed(gu), self.w_down)
 
-    def _shapes_as_configured(self, x: Tensor, cos: Tensor, sin: Tensor) -> bool:
+    def _weights(self):
+        return self.attn_norm, self.ffn_norm, self.wqkv, self.wo, self.w_gate_up, self.w_down
+
+    def _shapes_as_configured(self, x: Tensor, cos: Tensor, sin: Tensor, weights=None) -> bool:
         """Whether every operand has the shape that the native halves of the block read it with. They take all sizes from
         ``cfg``; a pruned or widened weight, the empty placeholder of a sharded one or an input of another width goes
         operator by operator, where sizes come from the tensors and a mismatch raises."""
         cfg = self.cfg
-        H, I, A, D = cfg.hidden_size, cfg.ffn_size, cfg.num_heads * cfg.head_dim, cfg.head_dim
-        return (x.dim() == 3 and x.shape[2] == H and self.attn_norm.shape == (H,) and self.ffn_norm.shape == (H,)
-                and self.wqkv.shape == (A + 2 * cfg.num_kv_heads * D, H) and self.wo.shape == (H, A)
-                and self.w_gate_up.shape == (2 * I, H) and self.w_down.shape == (H, I)
-                and cos.dim() == 2 and cos.shape == sin.shape and cos.shape[1] == D // 2)
+        H, I, D = cfg.hidden_size, cfg.ffn_size, cfg.head_dim
+        A, table = cfg.num_heads * D, cos.shape
+        attn_norm, ffn_norm, wqkv, wo, w_gate_up, w_down = weights or self._weights()
+        return (x.dim() == 3 and x.shape[2] == H and attn_norm.shape == (H,) and ffn_norm.shape == (H,)
+                and wqkv.shape == (A + 2 * cfg.num_kv_heads * D, H) and wo.shape == (H, A)
+                and w_gate_up.shape == (2 * I, H) and w_down.shape == (H, I)
+                and len(table) == 2 and table[1] == D // 2 and sin.shape == table)
 
     def _plain_inference(self, x: Tensor, cos: Tensor, sin: Tensor) -> bool:
         """Whether a forward pass with a cache may go to the native halves of the block: plain CUDA bf16 tensors of the
@@ -122,22 +127,24 @@ class LlamaBlock(nn.Module):
         if getattr(self._attend_cached, "__func__", None) is not LlamaBlock._attend_cached:
             return False   # a subclass or an instance brings its own cached attention
         if torch.is_grad_enabled() or type(x) is not Tensor or not x.is_cuda or x.dtype != torch.bfloat16 \
-                or not x.is_contiguous() or x.data_ptr() % 16 or x.numel() == 0 or self.cfg.head_dim not in (64, 128):
+                or not x.is_contiguous() or x.data_ptr() % 16 or x.numel() == 0 or self.cfg.head_dim not in (64, 128) \
+                or self.cfg.hidden_size % 8 or self.cfg.ffn_size % 8:
             return False
         if _native.flop_sinks or _ckpt.active() or torch._C._are_functorch_transforms_active() \
                 or torch._C._len_torch_dispatch_stack() or torch._C._is_torch_function_mode_enabled() \
                 or torch.autograd.forward_ad._current_level >= 0 or torch.jit.is_tracing():
             return False
         dev = x.device
-        for w in (self.attn_norm, self.wqkv, self.wo, self.ffn_norm, self.w_gate_up, self.w_down):
+        weights = self._weights()
+        for w in weights:
             if type(w) is not nn.Parameter or w.dtype != torch.bfloat16 or w.device != dev or not w.is_contiguous() \
-                    or w.data_ptr() % 16 or w.shape[-1] % 8:
+                    or w.data_ptr() % 16:
                 return False
         for t in (cos, sin):
             if type(t) is not Tensor or t.dtype != torch.float32 or t.device != dev or not t.is_contiguous() \
                     or t.data_ptr() % 16:
                 return False
-        return self._shapes_as_configured(x, cos, sin) and dev.index == torch._C._cuda_getDevice() and use_native(x)
+        return self._shapes_as_configured(x, cos, sin, weights) and dev.index == torch._C._cuda_getDevice() and use_native(x)
 
     def _infer_cached(self, x: Tensor, cos: Tensor, sin: Tensor, position_ids: Optional[Tensor], cache) -> Tensor:
         """The block as two native calls around the cache and the attention. Of at most 128 rows the last product is

@@ -241,9 +241,9 @@ class _QKVAttnFn(torch.autograd.Function):
     """Flash attention on a packed QKV projection ``[B, T, (Hq + 2 Hkv) * D]``, with RoPE unless ``cos`` is None.
 
     Without rotation q, k and v are all read in place. Forward rotates q and k out of the packed buffer into a fresh
-    ``[B, T, Hq + Hkv, D]`` one with one launch (no copy before the rotation) and attends with v read in place from the packed buffer. Backward has the flash kernels
-    write dq, dk and dv straight into the slices of one packed gradient buffer and un-rotates
-    its q/k part in place, so that no concatenation or copy is needed around the projection.
+    ``[B, T, Hq + Hkv, D]`` one with one launch (no copy before the rotation) and attends with v read in place from the
+    packed buffer. Backward has the flash kernels write dq, dk and dv straight into the slices of one packed gradient
+    buffer and un-rotates its q/k part in place, so that no concatenation or copy is needed around the projection.
     """
 
     @staticmethod

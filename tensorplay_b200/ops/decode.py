@@ -86,8 +86,8 @@ def embedding(ids: Tensor, weight: Tensor) -> Tensor:
 
 def _append_fits(cache: Tensor, new: Tensor, pos: int) -> None:
     """The kernels write ``new`` [B, H, T, D] by the cache's strides: past its end where it is smaller."""
-    B, H, T, D = new.shape
-    if B > cache.shape[0] or H > cache.shape[1] or D > cache.shape[3] or pos < 0 or pos + T > cache.shape[2]:
+    (B, H, T, D), (cB, cH, cT, cD) = new.shape, cache.shape
+    if B > cB or H > cH or D > cD or pos < 0 or pos + T > cT:
         raise ValueError(f"kv_append: {tuple(new.shape)} at token {pos} does not fit a cache of {tuple(cache.shape)}")
 
 
