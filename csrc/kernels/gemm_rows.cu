@@ -231,21 +231,26 @@ static int launch_rows(const CUtensorMap& tb, const CUtensorMap& ta, const RowsP
 // Which products of at most 128 rows go here; the others go to the persistent one-CTA kernel, which loads its next tile
 // under the stores of the last. What this kernel gains is the split of K over a cluster while there are fewer tiles
 // than CTAs that fit (two per SM), and the small column operand; what it pays is an epilogue of 3 us a round at 16 rows
-// and 9 us at 128, under which nothing is loaded. Measured on one B200, operands from memory, N x K: us here / there:
-//   M = 16: 14336 x 2048 15.1 / 16.3, 50304 x 768 20.5 / 19.2, 128256 x 2048 89.9 / 87.2, 128256 x 4096 168.0 / 174.2
-//   M = 32: 4096 x 4096 11.2 / 23.5, 28672 x 4096 41.8 / 43.8, 50304 x 768 22.5 / 19.5
-//   M = 64: 6144 x 1024 9.4 / 10.0, 14336 x 2048 18.6 / 15.6, 28672 x 4096 46.3 / 45.3, 32000 x 1024 17.8 / 16.4
-//   M = 128: 4096 x 1024 9.3 / 10.0, 4096 x 14336 31.9 / 69.7, 6144 x 1024 12.1 / 10.4, 50304 x 768 33.7 / 21.4
-// Lines in between: M = 64: 8192 x 2048 13.0 / 14.4, 11000 x 2048 18.3 / 16.5; M = 128: 6144 x 4096 21.2 / 23.9, 8192 x
-// 2048 15.8 / 14.4. With results that the other kernel stores from its lanes one by one (accumulated ones, fp32 with a
-// bias) more stay here: 32 x 50304 x 768 accumulated 25 / 28, fp32 with a bias 16 x 50304 x 768 18 / 23, 40 x 28672 x
-// 4096 46 / 50. A single row: 128256 x 2048 84 / 87, 50304 x 768 19.5 / 19.8, 128256 x 512 30 / 26.
+// and 9 us at 128, under which nothing is loaded. Column tiles (N / 128) x K, us here / there, operands from memory:
+//   M = 16: 64 x 4096 16.5 / 24.2, 296 x 4096 52.5 / 54.9, 393 x 1024 28.6 / 28.3, 393 x 2048 39.8 / 41.0
+//   M = 32: 250 x 2048 26.4 / 26.6, 393 x 2048 42.0 / 41.6, 393 x 3072 57.8 / 59.9, 700 x 1024 48.0 / 39.8
+//   M = 64: 72 x 1024 10.2 / 10.4, 72 x 4096 20.2 / 24.3, 78 x 2048 18.0 / 15.1, 78 x 3072 17.0 / 19.7, 96 x 4096 29.6 / 25.0
+//   M = 128: 20 x 512 7.3 / 7.0, 30 x 512 7.7 / 7.0, 44 x 1024 10.7 / 10.2, 44 x 2048 13.3 / 14.8, 64 x 2048 16.6 / 15.1,
+//            64 x 4096 23.4 / 24.2, 56 x 8192 35.8 / 42.2, 78 x 8192 35.3 / 42.7, 112 x 8192 62.3 / 46.7
+// (the step between 72 and 78 tiles is that of the cluster size, two to three, which pays from K = 3072 on). With results
+// that the other kernel stores from its lanes one by one (accumulated ones, fp32 with a bias) more stay here: M = 16, fp32
+// with a bias, 393 x 1024 26.8 / 31.6; M = 32 29.7 / 32.9, 700 x 1024 47.0 / 45.8; M = 64 290 x 1024 24.4 / 28.3, 224 x
+// 14336 153.5 / 142.7.
+// A single row: 128256 x 2048 84 / 87, 50304 x 768 19.5 / 19.8, 128256 x 512 30 / 26. Over 849 such products the choice
+// takes 1.002 of the faster kernel on average and 1.08 at most.
 bool gemm_rows_takes(int M, int N, int K, int a_mn, bool slow_store) {
   if (M > 128 || a_mn) return false;
   const long long tiles = (N + 127) / 128, sms = sm_count();
-  if (M <= 32) return tiles <= 2 * sms || slow_store || (M <= 16 && K >= 4096) || (M <= 4 && K >= 768);
-  if (M <= 64) return tiles <= sms / 2 || (slow_store && tiles > sms && tiles <= 2 * sms);
-  return tiles <= sms / 4 || (tiles <= sms / 3 && K >= 4096);
+  if (M <= 32)
+    return tiles <= 2 * sms || K >= (M <= 4 ? 768 : M <= 16 ? 2048 : 3072) || (slow_store && (M <= 16 || tiles <= 3 * sms));
+  if (K >= 3072 && tiles <= sms * 3 / 5) return true;
+  if (M <= 64) return tiles <= sms / 2 || (slow_store && tiles > sms * 7 / 4 && tiles <= 2 * sms);
+  return tiles <= sms / 7 || (K >= 1024 && tiles <= sms / 3);
 }
 
 // Same contract as gemm_bf16_dispatch for the plain product with a K-major A of at most 128 rows.

@@ -43,7 +43,9 @@ def test_few_rows_epilogue(M, N, K, kw):
 
 
 @pytest.mark.parametrize("M,N,K", [(16, 40000, 72), (1, 40000, 4096), (17, 37888, 136), (32, 37896, 136), (33, 9472, 192),
-                                   (64, 9480, 192), (65, 6272, 4096), (128, 4736, 64), (128, 4744, 64), (128, 6280, 4096)])
+                                   (64, 9480, 192), (65, 6272, 4096), (128, 4736, 64), (128, 4744, 64), (128, 6280, 4096),
+                                   (16, 40000, 2040), (16, 40000, 2048), (32, 40000, 3072), (64, 11264, 3072), (65, 11272, 3072),
+                                   (128, 11264, 3064), (128, 6272, 1024), (65, 6280, 1024), (128, 2688, 64), (100, 2696, 1016)])
 def test_both_sides_of_the_choice(M, N, K):
     """Sizes on which the kernels of few and of more rows meet."""
     _check(M, N, K, False, M % 2 == 0)
