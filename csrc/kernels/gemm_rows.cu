@@ -237,20 +237,21 @@ static int launch_rows(const CUtensorMap& tb, const CUtensorMap& ta, const RowsP
 //   M = 64: 72 x 1024 10.2 / 10.4, 72 x 4096 20.2 / 24.3, 78 x 2048 18.0 / 15.1, 78 x 3072 17.0 / 19.7, 96 x 4096 29.6 / 25.0
 //   M = 128: 20 x 512 7.3 / 7.0, 30 x 512 7.7 / 7.0, 44 x 1024 10.7 / 10.2, 44 x 2048 13.3 / 14.8, 64 x 2048 16.6 / 15.1,
 //            64 x 4096 23.4 / 24.2, 56 x 8192 35.8 / 42.2, 78 x 8192 35.3 / 42.7, 112 x 8192 62.3 / 46.7
-// (the step between 72 and 78 tiles is that of the cluster size, two to three, which pays from K = 3072 on). With results
-// that the other kernel stores from its lanes one by one (accumulated ones, fp32 with a bias) more stay here: M = 16, fp32
-// with a bias, 393 x 1024 26.8 / 31.6; M = 32 29.7 / 32.9, 700 x 1024 47.0 / 45.8; M = 64 290 x 1024 24.4 / 28.3, 224 x
-// 14336 153.5 / 142.7.
-// A single row: 128256 x 2048 84 / 87, 50304 x 768 19.5 / 19.8, 128256 x 512 30 / 26. Over 849 such products the choice
-// takes 1.002 of the faster kernel on average and 1.08 at most.
-bool gemm_rows_takes(int M, int N, int K, int a_mn, bool slow_store) {
+// (the step between 72 and 78 tiles is that of the cluster size, two to three; M = 40 80 x 2560 14.3 / 17.4, M =
+// 128 27 x 768 7.9 / 8.3). With results that the other kernel stores from its lanes one by one more stay here (`store`: 1
+// accumulated, 2 fp32 with a bias). As 2: M = 16 393 x 1024 26.8 / 31.6, M = 32 29.7 / 32.9, 700 x 1024 47.0 / 45.8, M =
+// 64 148 x 1536 19.3 / 23.1, 224 x 14336 153.5 / 142.7, 290 x 1024 24.4 / 28.3, 393 x 14336 266.8 / 282.8.
+// A single row: 128256 x 2048 84 / 87, 50304 x 768 19.5 / 19.8, 128256 x 512 30 / 26. Over 1286 such products the choice
+// takes 1.003 of the faster kernel on average and 1.16 at most.
+bool gemm_rows_takes(int M, int N, int K, int a_mn, int store) {
   if (M > 128 || a_mn) return false;
   const long long tiles = (N + 127) / 128, sms = sm_count();
   if (M <= 32)
-    return tiles <= 2 * sms || K >= (M <= 4 ? 768 : M <= 16 ? 2048 : 3072) || (slow_store && (M <= 16 || tiles <= 3 * sms));
-  if (K >= 3072 && tiles <= sms * 3 / 5) return true;
-  if (M <= 64) return tiles <= sms / 2 || (slow_store && tiles > sms * 7 / 4 && tiles <= 2 * sms);
-  return tiles <= sms / 7 || (K >= 1024 && tiles <= sms / 3);
+    return tiles <= 2 * sms || K >= (M <= 4 ? 768 : M <= 16 ? 2048 : 3072) || (store && (M <= 16 || tiles <= 3 * sms));
+  if (K >= (M <= 100 ? 2560 : 3072) && tiles <= sms * 3 / 5) return true;
+  if (M <= 64)
+    return tiles <= sms / 2 || (store == 2 ? tiles >= sms : store && tiles > sms * 7 / 4 && tiles <= 2 * sms);
+  return tiles <= sms / 7 || (K >= (tiles <= sms / 4 ? 768 : 1024) && tiles <= sms / 3);
 }
 
 // Same contract as gemm_bf16_dispatch for the plain product with a K-major A of at most 128 rows.

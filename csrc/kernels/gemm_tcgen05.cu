@@ -1093,7 +1093,7 @@ extern "C" int tpb_gemm_bf16(const void* A, const void* B, void* C, const void* 
                              int bias_f32, int accumulate, float alpha, uint32_t* status,
                              void* stream) {
   TPB_NVTX("tpb_gemm_bf16");
-  if (tpb::gemm_rows_takes(M, N, K, a_mn, accumulate || (out_f32 && bias)))
+  if (tpb::gemm_rows_takes(M, N, K, a_mn, out_f32 && bias ? 2 : accumulate != 0))
     return tpb::gemm_rows_dispatch(A, B, C, bias, M, N, K, lda, ldb, ldc, b_mn, out_f32, bias_f32, accumulate, alpha,
                                    status, static_cast<cudaStream_t>(stream));
   if (g_pair_min_tiles > 0 && (long long)((M + 255) / 256) * ((N + 255) / 256) >= g_pair_min_tiles) {

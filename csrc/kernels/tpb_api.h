@@ -59,7 +59,7 @@ int gemm_bf16_dispatch(const void* A, const void* B, void* C, const void* bias, 
                        cudaStream_t stream, const GemmFused* fused);
 // A K-major A of at most 128 rows (gemm_rows.cu): whether the product goes there, and the product.
 // slow_store: results that are accumulated, or fp32 with a bias.
-bool gemm_rows_takes(int M, int N, int K, int a_mn, bool slow_store);
+bool gemm_rows_takes(int M, int N, int K, int a_mn, int store);
 int gemm_rows_dispatch(const void* A, const void* B, void* C, const void* bias, int M, int N, int K, int lda, int ldb,
                        int ldc, int b_mn, int out_f32, int bias_f32, int accumulate, float alpha, uint32_t* status,
                        cudaStream_t stream);

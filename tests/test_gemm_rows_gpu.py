@@ -52,5 +52,8 @@ def test_both_sides_of_the_choice(M, N, K):
 
 
 def test_choice_by_the_kind_of_result():
+    _check(40, 18944, 200, False, False, out_dtype=torch.float32, bias=torch.bfloat16)
+    _check(64, 18816, 200, False, False, out_dtype=torch.float32, bias=torch.bfloat16)
+    _check(64, 37888, 72, False, False, accumulate=True)
     _check(32, 40000, 72, False, False, accumulate=True)
     _check(16, 40000, 72, False, False, out_dtype=torch.float32, bias=torch.bfloat16)
