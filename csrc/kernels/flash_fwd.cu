@@ -1,14 +1,19 @@
 // Flash attention forward for sm_100a: GQA-native, causal or full, head_dim 64 / 128.
 //
-// One CTA handles two tiles of 128 queries of one query head in ping-pong. Warp 0 streams K/V
-// tiles with TMA through one ring, warp 1 issues tcgen05.mma: S_g = Q_g K^T into the TMEM region
-// of tile g and O_g += P_g V into a second region; each tile has four softmax warps with one
-// query row per thread: they read S from TMEM, keep the running max / sum in the exp2 domain,
-// write P (bf16 pairs) back over the S columns - the second MMA takes P as its A operand
-// straight from TMEM - rescale O in TMEM only when a row maximum grew by more than a factor of two, and
-// finally write O / LSE. While one tile is in its softmax the tensor pipe runs the other tile's
-// MMAs. K and V of a KV head are shared by the query heads of its group through L2, so GQA costs
+// One CTA handles a tile of 128 queries of one query head, and two CTAs share an SM. Warp 0 streams K/V tiles with TMA
+// through one ring, warp 1 issues tcgen05.mma: S = Q K^T into TMEM and O += P V into a second region; four softmax warps
+// with one query row per thread read S from TMEM, write P = exp2(..) (bf16 pairs) back over the S columns - the second MMA
+// takes P as its A operand straight from TMEM - keep the running sum, rescale O in TMEM only when a row outgrew its
+// reference maximum, and finally write O / LSE. A tile alternates between its softmax and its MMAs: while one CTA of an SM
+// is in the one, the tensor pipe runs the other CTA's MMAs. Start, end and the first, exposed loads of a CTA lie under the
+// other's work as well, which one CTA with two tiles in ping-pong (the form before) paid in full: 4.5 rounds of
+// iterations a CTA at T = 1024. K and V of a KV head are shared by the query heads of its group through L2, so GQA costs
 // no expanded K/V traffic.
+//
+// Bound by the special-function unit and the tensor pipe alternating within a tile; long sequences run at the power cap.
+// Against the form with two tiles and the maximum taken before the exponentials, 32/8 heads of 128, causal: T = 8190
+// 504 -> 492 us (1120 TFLOP/s), T = 2900 99.4 -> 87.2, 16 x 1000 268 -> 231; a window of 512 over 2 x 4096 (16/4 heads)
+// 93 -> 76; 12 heads of 64, 16 x 1024 95.4 -> 78.8.
 //
 // Counterpart in the reference: vendored FlashAttention-2 sm80 leaves
 // (p10/src/backend/cuda/transformers/flash/flash_fwd_kernel.h, AttentionKernels.cu:1782-1969),
@@ -20,10 +25,11 @@
 
 namespace tpb {
 
-constexpr int kAttnThreads = 320;  // TMA warp, MMA warp, 2 x 4 softmax warps (one group per query tile)
+constexpr int kAttnThreads = 192;  // TMA warp, MMA warp, 4 softmax warps
 constexpr int kBlockQ = 128;
-constexpr int kTilesQ = 2;  // query tiles per CTA, processed in ping-pong
 constexpr int kBlockKV = 128;
+constexpr int kFirstKeys = 96;  // keys of a tile whose P is handed over first
+constexpr int kFwdTmemCols = 256;  // S (P), O
 constexpr float kNegBig = -1.0e30f;
 
 struct AttnFwdParams {
@@ -55,14 +61,19 @@ struct AttnFwdParams {
 
 // Debug aid: cycle stamps of block (0,0,0), kept in shared memory while the kernel runs (a stamp
 // costs one shared store) and copied out at the end: trace[(who * 64 + it) * 8 + tag] = clock.
-//   who 0: MMA thread (tags 0/1: P half of tile 0/1 seen, 2/3: P complete, 4/5: S(j+1) issued)
-//   who 1/2: first softmax thread of tile 0/1 (tags 1: S seen, 2: S in registers, 3: maximum done,
-//            4: first half exponentiated, 5: first half handed over, 6: second half exponentiated,
-//            7: second half handed over)
+//   who 0: MMA thread (tags 0: first part of P seen, 2: P complete, 4: S(j+1) issued)
+//   who 1: first softmax thread (tags 1: S seen, 4: first 96 keys exponentiated, 5: handed over, 6: the others exponentiated,
+//          7: handed over)
 constexpr int kTraceIts = 64;
-constexpr int kTraceWords = 3 * kTraceIts * 8;
+constexpr int kTraceWords = 2 * kTraceIts * 8;
+// Only in the debug build: each stamp is a branch, which the compiler schedules nothing across.
+#ifdef TPB_KERNEL_DEBUG
+constexpr bool kFwdTrace = true;
+#else
+constexpr bool kFwdTrace = false;
+#endif
 __device__ __forceinline__ void fwd_trace(uint32_t* tr, int who, int tag, int it) {
-  if (tr && it < kTraceIts) tr[(who * kTraceIts + it) * 8 + tag] = (uint32_t)clock64();
+  if (kFwdTrace && tr && it < kTraceIts) tr[(who * kTraceIts + it) * 8 + tag] = (uint32_t)clock64();
 }
 
 __device__ __forceinline__ float fast_exp2(float x) {
@@ -116,11 +127,11 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
   return d;
 }
 
-// Maximum of one S row (raw scores): four chains of three-input maxima.
-__device__ __forceinline__ float row_max(const uint32_t (&sr)[128]) {
+// Maximum of 32 columns of one S row (raw scores): four chains of three-input maxima.
+__device__ __forceinline__ float row_max(const uint32_t (&sr)[32]) {
   float m0 = -INFINITY, m1 = -INFINITY, m2 = -INFINITY, m3 = -INFINITY;
 #pragma unroll
-  for (int i = 0; i < 128; i += 8) {
+  for (int i = 0; i < 32; i += 8) {
     m0 = max3(m0, __uint_as_float(sr[i]), __uint_as_float(sr[i + 1]));
     m1 = max3(m1, __uint_as_float(sr[i + 2]), __uint_as_float(sr[i + 3]));
     m2 = max3(m2, __uint_as_float(sr[i + 4]), __uint_as_float(sr[i + 5]));
@@ -133,10 +144,10 @@ __device__ __forceinline__ float row_max(const uint32_t (&sr)[128]) {
 // sequence, the left edge of a window or segment): it never raises the running maximum and its
 // exponential on the special-function unit is exactly zero, also for a row without any valid key
 // in this tile.
-__device__ __forceinline__ void row_mask(uint32_t (&sr)[128], int k0, int lo, int lim) {
+__device__ __forceinline__ void row_mask(uint32_t (&sr)[32], int k0, int lo, int lim) {
   const int a = lo - k0, b = lim - k0;   // valid columns: a <= i <= b
 #pragma unroll
-  for (int i = 0; i < 128; ++i) sr[i] = (i >= a && i <= b) ? sr[i] : 0xff800000u;
+  for (int i = 0; i < 32; ++i) sr[i] = (i >= a && i <= b) ? sr[i] : 0xff800000u;
 }
 
 // exp2 of a pair on the FMA pipe: floor by the magic-number add in round-down mode, cubic
@@ -159,15 +170,13 @@ __device__ __forceinline__ uint64_t exp2_poly2(uint64_t x) {
   return pk2u(p0 + (r0 << 23), p1 + (r1 << 23));
 }
 
-// One half of a row: columns [HALF * 64, HALF * 64 + 64) of sr become 32 bf16 pairs
-// P = exp2(S * scale - m) in sr[HALF * 32 ...] (in place: the pairs land where scores were already
-// consumed); the fp32 values are added into two packed accumulators. Of every four column pairs,
-// NPOLY take the polynomial, the rest the special-function unit.
-template <int HALF, int NPOLY>
-__device__ __forceinline__ void row_exp_half(uint32_t (&sr)[128], uint64_t sc, uint64_t nm, uint64_t& acc0,
-                                             uint64_t& acc1) {
+// 32 columns of a row become 16 bf16 pairs P = exp2(S * scale - m) in sr[0 .. 16) (in place: the pairs land where scores were
+// already consumed); the fp32 values are added into two packed accumulators. Of every four column pairs, NPOLY take the
+// polynomial, the rest the special-function unit.
+template <int NPOLY>
+__device__ __forceinline__ void row_exp(uint32_t (&sr)[32], uint64_t sc, uint64_t nm, uint64_t& acc0, uint64_t& acc1) {
 #pragma unroll
-  for (int i = HALF * 32; i < HALF * 32 + 32; ++i) {
+  for (int i = 0; i < 16; ++i) {
     const uint64_t x = fma2(pk2u(sr[2 * i], sr[2 * i + 1]), sc, nm);
     uint64_t e;
     if ((i & 3) < NPOLY) {
@@ -188,20 +197,20 @@ __device__ __forceinline__ void row_exp_half(uint32_t (&sr)[128], uint64_t sc, u
 template <int D>
 struct AttnSmem {
   static constexpr int kChunks = D / 64;
-  static constexpr int kQBytes = kBlockQ * D * 2;   // one Q tile
+  static constexpr int kQBytes = kBlockQ * D * 2;
   static constexpr int kKBytes = kBlockKV * D * 2;  // one K or V tile
-  static constexpr int kQOff = 0;                   // two Q tiles
+  static constexpr int kQOff = 0;
   // K and V tiles share one ring (K0 V0 K1 V1 ...)
-  static constexpr int kRing = D == 128 ? 4 : 6;
-  static constexpr int kKOff = kQOff + kTilesQ * kQBytes;
+  static constexpr int kRing = D == 128 ? 2 : 4;
+  static constexpr int kKOff = kQOff + kQBytes;
   static constexpr int kBarOff = kKOff + kRing * kKBytes;
   static constexpr int kTraceOff = kBarOff + 256;
-  static constexpr int kTotal = kTraceOff + kTraceWords * 4 + 1024;
-  static_assert(kTotal <= 227 * 1024, "attention forward exceeds the shared memory of one CTA");
+  static constexpr int kTotal = kTraceOff + (kFwdTrace ? kTraceWords * 4 : 0) + 1024;
+  static_assert(kFwdTrace || 2 * (kTotal + 1024) <= 228 * 1024, "two CTAs of the attention forward exceed an SM's shared memory");
 };
 
 template <int D, int NPOLY>
-__global__ void __launch_bounds__(kAttnThreads, 1)
+__global__ void __launch_bounds__(kAttnThreads, 2)
 flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                  const __grid_constant__ CUtensorMap tmV, const AttnFwdParams p) {
   using L = AttnSmem<D>;
@@ -213,11 +222,11 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   uint64_t* q_full = bars;              // 1
   uint64_t* kv_full = bars + 1;         // R
   uint64_t* kv_empty = kv_full + R;     // R
-  uint64_t* s_full = kv_empty + R;      // 2: S of tile g is complete (and so is every earlier MMA)
-  uint64_t* p_half = s_full + 2;        // 2 (128 arrivals): keys 0..63 of P of tile g are in TMEM (and O is rescaled)
-  uint64_t* p_full = p_half + 2;        // 2 (128 arrivals): all of P of tile g is in TMEM
-  uint64_t* o_done = p_full + 2;        // 2: last PV of tile g is complete
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_done + 2);
+  uint64_t* s_full = kv_empty + R;      // 1: S is complete (and so is every earlier MMA)
+  uint64_t* p_half = s_full + 1;        // 1 (one arrival per warp): the first kFirstKeys keys of P are in TMEM (and O is rescaled)
+  uint64_t* p_full = p_half + 1;        // 1 (one arrival per warp): all of P is in TMEM
+  uint64_t* o_done = p_full + 1;        // 1: the last PV is complete
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_done + 1);
   volatile uint32_t* abort_w = tmem_slot + 1;
 
   const int warp = threadIdx.x >> 5;
@@ -244,7 +253,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   }
   const int qb = p.causal ? (q_tiles - 1 - qt) : qt;  // heavy tiles first
   const int hk = h / (p.Hq / p.Hkv);
-  const int q0 = qb * (kTilesQ * kBlockQ);
+  const int q0 = qb * kBlockQ;
   const int Tk = p.kv_len ? min(p.Tk, *p.kv_len) : p.Tk;
   // first KV block of this CTA: the split's share, or the block of the smallest key that the CTA's
   // first query may attend (bounds grow with the query index, so later rows need no earlier key)
@@ -255,26 +264,21 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     if (p.seg_start) lo_first = max(lo_first, p.seg_start[(long long)b * p.Tq + q0]);
     j0 = lo_first / kBlockKV;
   }
-  // KV blocks needed by each of the two query tiles
-  int nkv_t[kTilesQ];
+  // KV blocks needed
   int nkv = 0;
-#pragma unroll
-  for (int g = 0; g < kTilesQ; ++g) {
-    int n = (Tk + kBlockKV - 1) / kBlockKV;
+  if (q0 < p.Tq) {
+    nkv = (Tk + kBlockKV - 1) / kBlockKV;
     if (p.causal) {
-      const int last_key = q0 + g * kBlockQ + kBlockQ - 1 + p.kv_offset;
-      n = last_key < 0 ? 0 : min(n, last_key / kBlockKV + 1);
+      const int last_key = q0 + kBlockQ - 1 + p.kv_offset;
+      nkv = last_key < 0 ? 0 : min(nkv, last_key / kBlockKV + 1);
     }
-    if (q0 + g * kBlockQ >= p.Tq) n = 0;  // tile past the end of the sequence
-    if (p.seg_end && n > 0) {
+    if (p.seg_end && nkv > 0) {
       // the tile's last query has the largest upper bound
-      const int qlast = min(q0 + g * kBlockQ + kBlockQ - 1, p.Tq - 1);
-      n = min(n, (p.seg_end[(long long)b * p.Tq + qlast] + kBlockKV - 1) / kBlockKV);
+      const int qlast = min(q0 + kBlockQ - 1, p.Tq - 1);
+      nkv = min(nkv, (p.seg_end[(long long)b * p.Tq + qlast] + kBlockKV - 1) / kBlockKV);
     }
-    if (n_splits > 1) n = max(0, min(n - j0, p.blocks_per_split));  // this split's share
-    else n = max(0, n - j0);
-    nkv_t[g] = n;
-    nkv = max(nkv, n);
+    if (n_splits > 1) nkv = max(0, min(nkv - j0, p.blocks_per_split));  // this split's share
+    else nkv = max(0, nkv - j0);
   }
 
   if (threadIdx.x == 0) {
@@ -284,19 +288,17 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       mbar_init(&kv_full[i], 1);
       mbar_init(&kv_empty[i], 1);
     }
-    for (int i = 0; i < kTilesQ; ++i) {
-      mbar_init(&s_full[i], 1);
-      mbar_init(&p_half[i], 128);
-      mbar_init(&p_full[i], 128);
-      mbar_init(&o_done[i], 1);
-    }
+    mbar_init(s_full, 1);
+    mbar_init(p_half, 4);
+    mbar_init(p_full, 4);
+    mbar_init(o_done, 1);
     fence_barrier_init();
     prefetch_tmap(&tmQ);
     prefetch_tmap(&tmK);
     prefetch_tmap(&tmV);
   }
   if (warp == 1) {
-    tmem_alloc(tmem_slot, 512);
+    tmem_alloc(tmem_slot, kFwdTmemCols);
     tmem_relinquish();
   }
   tc_fence_before_sync();
@@ -304,7 +306,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
   WaitCtx wc{abort_w, p.status, p.wait_ns};
-  uint32_t* trc = (p.trace && qt == 0 && h == 0 && b == 0)
+  uint32_t* trc = (kFwdTrace && p.trace && qt == 0 && h == 0 && b == 0)
                       ? reinterpret_cast<uint32_t*>(smem + L::kTraceOff) : nullptr;
   if (trc) {
     for (int i = threadIdx.x; i < kTraceWords; i += kAttnThreads) trc[i] = 0;
@@ -315,13 +317,10 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   if (warp == 0) {
     // ---------------------------------------------------------------- TMA producer
     if (lane == 0 && nkv > 0) {
-      mbar_arrive_expect_tx(q_full, kTilesQ * L::kQBytes);
+      mbar_arrive_expect_tx(q_full, L::kQBytes);
 #pragma unroll
-      for (int g = 0; g < kTilesQ; ++g)
-#pragma unroll
-        for (int c = 0; c < L::kChunks; ++c)
-          tma_load_4d(smem + L::kQOff + g * L::kQBytes + c * (kBlockQ * 128), &tmQ, q_full, c * 64, h,
-                      q0 + g * kBlockQ, b);
+      for (int c = 0; c < L::kChunks; ++c)
+        tma_load_4d(smem + L::kQOff + c * (kBlockQ * 128), &tmQ, q_full, c * 64, h, q0, b);
       for (int t = 0; t < 2 * nkv; ++t) {
         const int j = t >> 1;
         const int slot = t % R;
@@ -337,10 +336,8 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     }
   } else if (warp == 1) {
     // ---------------------------------------------------------------- MMA issuer
-    // Order on the tensor pipe: S0(0) S1(0) | PV0(0) S0(1) PV1(0) S1(1) | PV0(1) S0(2) ...
-    // While the softmax warps of one tile work, the pipe runs the other tile's MMAs. P(j) lives
-    // in the columns of S(j); S(j+1) is issued after PV(j) and the pipe executes in issue order,
-    // so the overwrite needs no barrier.
+    // P(j) lives in the columns of S(j); S(j+1) is issued after PV(j) and the pipe executes in issue order, so the overwrite
+    // needs no barrier.
     // The whole warp runs this loop with uniform control flow and one elected lane issues: operands of
     // tcgen05 instructions live in uniform registers, and inside a divergent `if (lane == 0)` region
     // every one of them would first be moved there from a vector register, which costs the issuing
@@ -353,192 +350,199 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       const uint32_t q_lo = smem_desc_lo(smem_u32(smem + L::kQOff), 16);
       const uint32_t k_lo = smem_desc_lo(smem_u32(smem + L::kKOff), 16);
       const uint32_t v_lo = smem_desc_lo(smem_u32(smem + L::kKOff), kBlockKV * 128);
-      auto issue_s = [&](int g, int j) {
+      auto issue_s = [&](int j) {
         const int slot = (2 * j) % R;
-        const uint32_t qb_lo = q_lo + g * (L::kQBytes >> 4);
         const uint32_t kb_lo = k_lo + slot * (L::kKBytes >> 4);
         if (elect_one()) {
 #pragma unroll
           for (int kk = 0; kk < D / 16; ++kk) {
             const uint32_t off = ((kk / 4) * (kBlockQ * 128) + (kk % 4) * 32) >> 4;
-            umma_f16_ss_w(tmem_base + g * 128, qb_lo + off, hi_k, kb_lo + off, hi_k, idesc_s, kk != 0);
+            umma_f16_ss_w(tmem_base, q_lo + off, hi_k, kb_lo + off, hi_k, idesc_s, kk != 0);
           }
-          umma_commit(&s_full[g]);
+          umma_commit(s_full);
+          umma_commit(&kv_empty[slot]);
         }
         __syncwarp();
       };
-      auto commit = [&](uint64_t* bar) {
-        if (elect_one()) umma_commit(bar);
+      // keys [FROM, TO) of P(j) V(j)
+      auto issue_pv = [&](int j, int slot, int from, int to) {
+        const uint32_t vb_lo = v_lo + slot * (L::kKBytes >> 4);
+        if (elect_one()) {
+#pragma unroll
+          for (int kk = from / 16; kk < to / 16; ++kk)
+            umma_f16_ts_w(tmem_base + 128, tmem_base + kk * 8, vb_lo + kk * (2048 >> 4), hi_k, idesc_o, (j | kk) != 0);
+          if (to == kBlockKV) {
+            umma_commit(&kv_empty[slot]);
+            if (j + 1 == nkv) umma_commit(o_done);
+          }
+        }
         __syncwarp();
       };
       bool ok = mbar_wait_warp(q_full, 0, wc, 5);
       if (ok) ok = mbar_wait_warp(&kv_full[0], 0, wc, 3);
       if (ok) {
         tc_fence_after_sync();
-#pragma unroll
-        for (int g = 0; g < kTilesQ; ++g)
-          if (nkv_t[g] > 0) issue_s(g, 0);
-        commit(&kv_empty[0]);
+        issue_s(0);
       }
       for (int j = 0; j < nkv && ok; ++j) {
-        const int vslot = (2 * j + 1) % R;
-        const uint32_t vph = ((2 * j + 1) / R) & 1;
-        const int kslot = (2 * j + 2) % R;
-        const uint32_t kph = ((2 * j + 2) / R) & 1;
-        const uint32_t vb_lo = v_lo + vslot * (L::kKBytes >> 4);
-        bool have_v = false, have_k = false;
-#pragma unroll
-        for (int g = 0; g < kTilesQ; ++g) {
-          if (j >= nkv_t[g]) continue;
-          // PV starts on the first 64 keys while the softmax warps still work on the other 64
-          if (!mbar_wait_warp(&p_half[g], j & 1, wc, 6)) { ok = false; break; }
-          if (lane == 0) fwd_trace(trc, 0, g, j);
-          if (!have_v) {
-            if (!mbar_wait_warp(&kv_full[vslot], vph, wc, 7)) { ok = false; break; }
-            have_v = true;
-          }
+        const int vslot = (2 * j + 1) % R, kslot = (2 * j + 2) % R;
+        // PV starts on the first keys while the softmax warps still work on the others
+        if (!mbar_wait_warp(p_half, j & 1, wc, 6)) break;
+        if (lane == 0) fwd_trace(trc, 0, 0, j);
+        if (!mbar_wait_warp(&kv_full[vslot], ((2 * j + 1) / R) & 1, wc, 7)) break;
+        tc_fence_after_sync();
+        issue_pv(j, vslot, 0, kFirstKeys);
+        if (!mbar_wait_warp(p_full, j & 1, wc, 11)) break;
+        if (lane == 0) fwd_trace(trc, 0, 2, j);
+        tc_fence_after_sync();
+        issue_pv(j, vslot, kFirstKeys, kBlockKV);
+        if (j + 1 < nkv) {
+          if (!mbar_wait_warp(&kv_full[kslot], ((2 * j + 2) / R) & 1, wc, 3)) break;
           tc_fence_after_sync();
-          if (elect_one()) {
-#pragma unroll
-            for (int kk = 0; kk < kBlockKV / 32; ++kk)
-              umma_f16_ts_w(tmem_base + 256 + g * 128, tmem_base + g * 128 + kk * 8, vb_lo + kk * (2048 >> 4), hi_k,
-                            idesc_o, (j | kk) != 0);
-          }
-          __syncwarp();
-          if (!mbar_wait_warp(&p_full[g], j & 1, wc, 11)) { ok = false; break; }
-          if (lane == 0) fwd_trace(trc, 0, 2 + g, j);
-          tc_fence_after_sync();
-          if (elect_one()) {
-#pragma unroll
-            for (int kk = kBlockKV / 32; kk < kBlockKV / 16; ++kk)
-              umma_f16_ts_w(tmem_base + 256 + g * 128, tmem_base + g * 128 + kk * 8, vb_lo + kk * (2048 >> 4), hi_k,
-                            idesc_o, 1);
-          }
-          __syncwarp();
-          if (j + 1 < nkv_t[g]) {
-            if (!have_k) {
-              if (!mbar_wait_warp(&kv_full[kslot], kph, wc, 3)) { ok = false; break; }
-              have_k = true;
-              tc_fence_after_sync();
-            }
-            if (g == 0 && lane == 0) fwd_trace(trc, 0, 6, j);
-            issue_s(g, j + 1);
-            if (g == 0 && lane == 0) fwd_trace(trc, 0, 7, j);
-            if (lane == 0) fwd_trace(trc, 0, 4 + g, j);
-          } else {
-            commit(&o_done[g]);
-          }
+          issue_s(j + 1);
+          if (lane == 0) fwd_trace(trc, 0, 4, j);
         }
-        if (!ok) break;
-        commit(&kv_empty[vslot]);
-        if (have_k) commit(&kv_empty[kslot]);
       }
     }
   } else {
     // ---------------------------------------------------------------- softmax / epilogue
-    // warps 2..5 own query tile 0, warps 6..9 tile 1; one query row per thread
-    const int g = (warp - 2) >> 2;
+    // one query row per thread
     const int qd = warp & 3;
     const int row = qd * 32 + lane;  // row inside the tile == TMEM lane
-    const int qi = q0 + g * kBlockQ + row;
-    const uint32_t t_s = tmem_base + ((uint32_t)(qd * 32) << 16) + g * 128;
-    const uint32_t t_o = tmem_base + ((uint32_t)(qd * 32) << 16) + 256 + g * 128;
-    const int my_nkv = nkv_t[g];
+    const int qi = q0 + row;
+    const uint32_t t_s = tmem_base + ((uint32_t)(qd * 32) << 16);
+    const uint32_t t_o = t_s + 128;
     int lim = p.causal ? min(qi + p.kv_offset, Tk - 1) : (Tk - 1);  // last valid key
     int lo = 0;                                                            // first valid key
     // largest lower / smallest upper bound among the tile's rows decide which KV blocks need the mask
     int lo_tile = 0, lim_tile = 0x3fffffff;
     if (p.window > 0) {
       lo = qi + p.kv_offset - p.window + 1;
-      lo_tile = q0 + g * kBlockQ + kBlockQ - 1 + p.kv_offset - p.window + 1;
+      lo_tile = q0 + kBlockQ - 1 + p.kv_offset - p.window + 1;
     }
     if (p.seg_start) {
       const long long base = (long long)b * p.Tq;
       lo = max(lo, p.seg_start[base + min(qi, p.Tq - 1)]);
-      lo_tile = max(lo_tile, p.seg_start[base + min(q0 + g * kBlockQ + kBlockQ - 1, p.Tq - 1)]);
+      lo_tile = max(lo_tile, p.seg_start[base + min(q0 + kBlockQ - 1, p.Tq - 1)]);
     }
     if (p.seg_end) {
       const long long base = (long long)b * p.Tq;
       lim = min(lim, p.seg_end[base + min(qi, p.Tq - 1)] - 1);
-      lim_tile = p.seg_end[base + min(q0 + g * kBlockQ, p.Tq - 1)] - 1;
+      lim_tile = p.seg_end[base + min(q0, p.Tq - 1)] - 1;
     }
     float m = kNegBig, l = 0.f;
     bool ok = true;
-    for (int j = 0; j < my_nkv; ++j) {
-      if (!mbar_wait_warp(&s_full[g], j & 1, wc, 8)) { ok = false; break; }
-      const bool tr = (threadIdx.x & 127) == 64;  // first thread of each tile's first softmax warp
-      if (tr) fwd_trace(trc, 1 + g, 1, j);
+    for (int j = 0; j < nkv; ++j) {
+      if (!mbar_wait_warp(s_full, j & 1, wc, 8)) { ok = false; break; }
+      uint32_t* tr = threadIdx.x == 64 ? trc : nullptr;  // first softmax thread
+      fwd_trace(tr, 1, 1, j);
       tc_fence_after_sync();
       const int k0 = (j0 + j) * kBlockKV;
-      const bool need_mask = (p.causal && (k0 + kBlockKV - 1 > q0 + g * kBlockQ + p.kv_offset)) ||
+      const bool need_mask = (p.causal && (k0 + kBlockKV - 1 > q0 + p.kv_offset)) ||
                              (k0 + kBlockKV > Tk) || (k0 < lo_tile) || (k0 + kBlockKV - 1 > lim_tile);
-      // the whole S row (128 fp32) in one TMEM round trip
-      uint32_t sr[128];
+      // P = exp2(S * scale - m) as bf16 pairs goes over the first 64 columns of S, the first 96 keys first; the row sum adds
+      // the fp32 values. m need not be the maximum, only so large that nothing overflows. One warp per scheduler works on
+      // a tile, so what it spends before its first exponential (loading 128 scores and taking their maximum: 500 of 1800
+      // cycles a tile) nothing else fills. So the exponentials start against the m so far, 32 keys at a time, each group
+      // loaded under those of the one before, and the maximum is not taken: a score that outgrew m shows in the sum, and
+      // only the keys that are handed over later are looked at themselves. The first tile, masked ones and, once more, a
+      // tile in which a row has to move its m take the maximum first.
+      const uint64_t sc2 = pk2(p.scale_log2e, p.scale_log2e);
+      uint64_t acc0, acc1;
+      uint32_t x[4][32];
+      float alpha = 1.f, s0, s1;
+      bool with_max = need_mask || j == 0;
+      while (true) {
+        if (with_max) {
+          float mx = -INFINITY;
+          tmem_ld_32x32b_x32(t_s, x[0]);
 #pragma unroll
-      for (int c = 0; c < 4; ++c) tmem_ld_32x32b_x32(t_s + c * 32, &sr[c * 32]);
-      tmem_ld_wait();
-      if (tr) fwd_trace(trc, 1 + g, 2, j);
-      if (need_mask) row_mask(sr, k0, lo, lim);
-      const float mx = fmaxf(m, row_max(sr) * p.scale_log2e);
-      // The reference maximum only moves when the row maximum grew by more than 2^4: until then
-      // P stays below 16 (harmless in bf16, whose error is relative) and O needs no rescale.
-      float alpha = 1.f;
-      if (mx - m > 4.f) {
-        alpha = fast_exp2(m - mx);
-        m = mx;
-      }
-      if (j > 0 && __any_sync(0xffffffffu, alpha != 1.f)) {
-        // every MMA issued before S(j), PV(j-1) included, completed before s_full fired
+          for (int c = 0; c < 4; ++c) {
+            tmem_ld_wait(x[c]);
+            if (c < 3) tmem_ld_32x32b_x32(t_s + (c + 1) * 32, x[c + 1]);
+            if (need_mask) row_mask(x[c], k0 + c * 32, lo, lim);
+            mx = fmaxf(mx, row_max(x[c]));
+          }
+          mx = fmaxf(m, mx * p.scale_log2e);
+          // m only moves when the row maximum grew by more than 2^4: until then P stays below 16 (harmless in bf16, whose
+          // error is relative) and O needs no rescale
+          if (mx - m > 4.f) {
+            alpha = fast_exp2(m - mx);
+            m = mx;
+          }
+          if (j > 0 && __any_sync(0xffffffffu, alpha != 1.f)) {
+            // every MMA issued before S(j), PV(j-1) included, completed before s_full fired
 #pragma unroll 1
-        for (int c = 0; c < D / 32; ++c) {
-          uint32_t o[32];
-          tmem_ld_32x32b_x32(t_o + c * 32, o);
-          tmem_ld_wait();
+            for (int c = 0; c < D / 32; ++c) {
+              tmem_ld_32x32b_x32(t_o + c * 32, x[0]);
+              tmem_ld_wait(x[0]);
 #pragma unroll
-          for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-          tmem_st_32x32b_x16(t_o + c * 32, &o[0]);
-          tmem_st_32x32b_x16(t_o + c * 32 + 16, &o[16]);
+              for (int i = 0; i < 32; ++i) x[0][i] = __float_as_uint(__uint_as_float(x[0][i]) * alpha);
+              tmem_st_32x32b_x16(t_o + c * 32, &x[0][0]);
+              tmem_st_32x32b_x16(t_o + c * 32 + 16, &x[0][16]);
+            }
+          }
         }
+        const uint64_t nm2 = pk2(-m, -m);
+        acc0 = acc1 = pk2(0.f, 0.f);
+        tmem_ld_32x32b_x32(t_s, x[0]);
+        if (need_mask) {
+          // (masked tiles stay on the special-function unit, whose exp2(-inf) is an exact zero)
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            tmem_ld_wait(x[c]);
+            if (c < 3) tmem_ld_32x32b_x32(t_s + (c + 1) * 32, x[c + 1]);
+            row_mask(x[c], k0 + c * 32, lo, lim);
+            if (c < 3) row_exp<0>(x[c], sc2, nm2, acc0, acc1);
+          }
+          break;
+        }
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          tmem_ld_wait(x[c]);
+          tmem_ld_32x32b_x32(t_s + (c + 1) * 32, x[c + 1]);
+          row_exp<NPOLY>(x[c], sc2, nm2, acc0, acc1);
+        }
+        tmem_ld_wait(x[3]);
+        if (with_max) break;
+        // 2^11: what 128 keys of 2^4 add up to, the bound of the other case (NaN fails, too)
+        upk2(add2(acc0, acc1), s0, s1);
+        const float late = row_max(x[3]) * p.scale_log2e - m;
+        if (__all_sync(0xffffffffu, s0 + s1 <= 2048.f && late <= 4.f)) break;
+        with_max = true;   // the scores are still in TMEM
       }
-      // P = exp2(S * scale - m) as bf16 pairs written over the first 64 columns of S, in two halves
-      // of 64 keys; the row sum adds the fp32 values
-      const uint64_t sc2 = pk2(p.scale_log2e, p.scale_log2e), nm2 = pk2(-m, -m);
-      uint64_t acc0 = pk2(0.f, 0.f), acc1 = acc0;
-      if (tr) fwd_trace(trc, 1 + g, 3, j);
-      // (masked tiles stay on the special-function unit, whose exp2(-inf) is an exact zero)
-      if (need_mask) row_exp_half<0, 0>(sr, sc2, nm2, acc0, acc1);
-      else row_exp_half<0, NPOLY>(sr, sc2, nm2, acc0, acc1);
-      if (tr) fwd_trace(trc, 1 + g, 4, j);
-      tmem_st_32x32b_x16(t_s, &sr[0]);
-      tmem_st_32x32b_x16(t_s + 16, &sr[16]);
+      fwd_trace(tr, 1, 4, j);
+#pragma unroll
+      for (int c = 0; c < 3; ++c) tmem_st_32x32b_x16(t_s + c * 16, x[c]);
       tmem_st_wait();
       tc_fence_before_sync();
-      mbar_arrive(&p_half[g]);
-      if (tr) fwd_trace(trc, 1 + g, 5, j);
-      if (need_mask) row_exp_half<1, 0>(sr, sc2, nm2, acc0, acc1);
-      else row_exp_half<1, NPOLY>(sr, sc2, nm2, acc0, acc1);
-      if (tr) fwd_trace(trc, 1 + g, 6, j);
-      tmem_st_32x32b_x16(t_s + 32, &sr[32]);
-      tmem_st_32x32b_x16(t_s + 48, &sr[48]);
-      float s0, s1;
+      __syncwarp();
+      if (lane == 0) mbar_arrive(p_half);   // one arrival per warp: 32 on one barrier are served one after the other
+      fwd_trace(tr, 1, 5, j);
+      const uint64_t nm2 = pk2(-m, -m);
+      if (need_mask) row_exp<0>(x[3], sc2, nm2, acc0, acc1);
+      else row_exp<NPOLY>(x[3], sc2, nm2, acc0, acc1);
+      tmem_st_32x32b_x16(t_s + 48, x[3]);
+      fwd_trace(tr, 1, 6, j);
       upk2(add2(acc0, acc1), s0, s1);
       l = l * alpha + (s0 + s1);
       tmem_st_wait();
       tc_fence_before_sync();
-      mbar_arrive(&p_full[g]);
-      if (tr) fwd_trace(trc, 1 + g, 7, j);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(p_full);
+      fwd_trace(tr, 1, 7, j);
     }
-    if (ok && my_nkv > 0) ok = mbar_wait_warp(&o_done[g], 0, wc, 10);
-    if ((threadIdx.x & 127) == 64) fwd_trace(trc, 0, 2 + g, 63);  // last PV of the tile complete
+    if (ok && nkv > 0) ok = mbar_wait_warp(o_done, 0, wc, 10);
+    if (threadIdx.x == 64) fwd_trace(trc, 0, 2, 63);  // last PV complete
     if (ok) {
       tc_fence_after_sync();
-      const float inv = (my_nkv > 0 && l > 0.f) ? 1.f / l : 0.f;
+      const float inv = (nkv > 0 && l > 0.f) ? 1.f / l : 0.f;
       __nv_bfloat16* orow = p.O + split * p.o_split_stride + (long long)b * p.o_batch_stride + (long long)qi * p.o_tok_stride +
                             (long long)h * p.o_head_stride;
 #pragma unroll 1
       for (int c = 0; c < D / 32; ++c) {
         uint32_t o[32];
-        if (my_nkv > 0) {
+        if (nkv > 0) {
           tmem_ld_32x32b_x32(t_o + c * 32, o);
           tmem_ld_wait();
         } else {
@@ -566,13 +570,13 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         }
       }
       if (qi < p.Tq && p.lse) {
-        float lse = (my_nkv > 0 && l > 0.f) ? (m + log2f(l)) * 0.6931471805599453f : -INFINITY;
+        float lse = (nkv > 0 && l > 0.f) ? (m + log2f(l)) * 0.6931471805599453f : -INFINITY;
         p.lse[split * p.lse_split_stride + ((long long)b * p.Hq + h) * p.lse_stride + qi] = lse;
       }
     }
   }
 
-  if ((threadIdx.x & 127) == 64 && warp >= 2) fwd_trace(trc, 0, 4 + ((warp - 2) >> 2), 63);  // output written
+  if (threadIdx.x == 64) fwd_trace(trc, 0, 4, 63);  // output written
   tc_fence_before_sync();
   __syncthreads();
   if (trc)
@@ -584,7 +588,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   }
   if (warp == 1) {
     tc_fence_after_sync();
-    tmem_dealloc(tmem_base, 512);
+    tmem_dealloc(tmem_base, kFwdTmemCols);
   }
 }
 
@@ -644,7 +648,7 @@ static int launch_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtens
     if (e != cudaSuccess) return (int)e;
     configured = true;
   }
-  dim3 grid(((p.Tq + kTilesQ * kBlockQ - 1) / (kTilesQ * kBlockQ)) * (p.n_splits > 1 ? p.n_splits : 1), p.Hq, p.B);
+  dim3 grid(((p.Tq + kBlockQ - 1) / kBlockQ) * (p.n_splits > 1 ? p.n_splits : 1), p.Hq, p.B);
   kern<<<grid, kAttnThreads, L::kTotal, stream>>>(tq, tk, tv, p);
   return (int)cudaGetLastError();
 }
@@ -695,9 +699,10 @@ static int g_fwd_npoly = 1;
 static unsigned long long* g_fwd_trace = nullptr;
 static int g_fwd_trace_cap = 0;
 
-// Debug aid: buf = device array of `cap` uint64 (3 * 64 * 8 are used). The next forward launches
+// Debug aid: buf = device array of `cap` uint64 (2 * 64 * 8 are used). The next forward launches
 // copy the cycle stamps of block (0,0,0) into it (layout at fwd_trace). Pass null to switch it off.
 extern "C" int tpb_flash_fwd_set_trace(unsigned long long* buf, int cap) {
+  if (!kFwdTrace && buf) return -2;   // debug build only
   g_fwd_trace = buf;
   g_fwd_trace_cap = cap;
   return 0;
@@ -752,9 +757,8 @@ extern "C" int tpb_flash_fwd_ex(const void* q, const void* k, const void* v, voi
       default: return launch_fwd<128, 0>(tq, tk, tv, p, (cudaStream_t)stream);
     }
   }
-  // head_dim 64 halves the tensor work per score, so the exponentials dominate: more of them
-  // go to the FMA pipe
-  return launch_fwd<64, 2>(tq, tk, tv, p, (cudaStream_t)stream);
+  // (two of four for head_dim 64: 86.4 against 84.8 us at 16 x 1024, 12 heads)
+  return launch_fwd<64, 1>(tq, tk, tv, p, (cudaStream_t)stream);
 }
 
 extern "C" int tpb_flash_fwd(const void* q, const void* k, const void* v, void* o, float* lse,
