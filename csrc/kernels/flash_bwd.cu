@@ -165,7 +165,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmX0, const __grid_constant
         const int s = it % kYStages;
         const uint32_t ph = (it / kYStages) & 1;
         if (!mbar_wait_relaxed(&y_empty[s], ph ^ 1, wc, 1)) break;
-        trace_pt(p, 0, it, 1);
+        trace_pt<DKV>(p, 0, it, 1);
         int hy, yb;
         if (DKV) { hy = hx * G + it / y_count; yb = y_first + it % y_count; }
         else { hy = hx / G; yb = y_first + it; }
@@ -204,7 +204,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmX0, const __grid_constant
         const uint32_t yph = (it / kYStages) & 1;
         const int s = it & 1;
         if (!mbar_wait_warp(&y_full[ys], yph, wc, 2)) return false;
-        if (lane == 0) trace_pt(p, 1, it, 1);
+        if (lane == 0) trace_pt<DKV>(p, 1, it, 1);
         // Slot s last held iteration it - 2: its S / dP were read by the P/dS warps before they
         // arrived on pds_full(it - 2), and its P / dS (same columns) are consumed by MMAs issued
         // earlier by this warp, which the tensor pipe executes in order before these.
@@ -237,7 +237,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmX0, const __grid_constant
         }
         const int s = it % kYStages;
         if (!mbar_wait_warp(pds_full, it & 1, wc, 5)) break;
-        if (lane == 0) trace_pt(p, 1, it, 3);
+        if (lane == 0) trace_pt<DKV>(p, 1, it, 3);
         tc_fence_after_sync();
         const uint32_t y0_lo = ym_lo + s * ((2 * L::kStreamBytes) >> 4);
         const uint32_t y1_lo = y0_lo + (L::kStreamBytes >> 4);
@@ -259,7 +259,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmX0, const __grid_constant
           if (it == n_it - 1) umma_commit(acc_done);
         }
         __syncwarp();
-        if (lane == 0) trace_pt(p, 1, it, 4);
+        if (lane == 0) trace_pt<DKV>(p, 1, it, 4);
       }
     }
   } else {
@@ -288,13 +288,13 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmX0, const __grid_constant
       else yb = y_first + it;
       const int y0i = yb * kStream + half * 32;  // first query (DKV) or key (dQ) of this warp's columns
       if (!mbar_wait_warp(&sdp_full[s], ph, wc, 6)) { ok = false; break; }
-      if (threadIdx.x == 64) trace_pt(p, 2, it, 1);
+      if (threadIdx.x == 64) trace_pt<DKV>(p, 2, it, 1);
       tc_fence_after_sync();
       uint32_t sr[32], dr[32];
       tmem_ld_32x32b_x32(tmem_base + t_lane + s * 128 + half * 32, sr);
       tmem_ld_32x32b_x32(tmem_base + t_lane + s * 128 + 64 + half * 32, dr);
       tmem_ld_wait();
-      if (threadIdx.x == 64) trace_pt(p, 2, it, 2);
+      if (threadIdx.x == 64) trace_pt<DKV>(p, 2, it, 2);
 
       // Valid streamed indices of this thread's row form one interval [lo, hi): tiles that lie
       // entirely inside it take the predicate-free path (warp-uniform choice).
@@ -309,7 +309,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmX0, const __grid_constant
       uint32_t pw[16], dw[16];
       if (need_mask) pds_math<DKV, true>(sr, dr, lse_sa, lse_row, delta_row, y0i, y_lo, y_hi, p.scale_log2e, p.scale, pw, dw);
       else pds_math<DKV, false>(sr, dr, lse_sa, lse_row, delta_row, y0i, y_lo, y_hi, p.scale_log2e, p.scale, pw, dw);
-      if (threadIdx.x == 64) trace_pt(p, 2, it, 3);
+      if (threadIdx.x == 64) trace_pt<DKV>(p, 2, it, 3);
       // P / dS (bf16 pairs) go back into this warp's own S / dP columns
       if (DKV) tmem_st_32x32b_x16(tmem_base + t_lane + s * 128 + half * 32, pw);
       tmem_st_32x32b_x16(tmem_base + t_lane + s * 128 + 64 + half * 32, dw);
@@ -317,7 +317,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmX0, const __grid_constant
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive(pds_full);   // one arrival per warp: 32 on one barrier are served one after the other
-      if (threadIdx.x == 64) trace_pt(p, 2, it, 5);
+      if (threadIdx.x == 64) trace_pt<DKV>(p, 2, it, 5);
     }
     if (ok && n_it > 0) ok = mbar_wait_warp(acc_done, 0, wc, 8);
     if (ok) {
@@ -388,7 +388,6 @@ attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __re
 }
 
 static unsigned long long* g_bwd_trace = nullptr;
-static int g_bwd_trace_cap = 0;
 
 template <int D, bool DKV>
 static int launch_bwd(const CUtensorMap& x0, const CUtensorMap& x1, const CUtensorMap& y0,
@@ -467,7 +466,7 @@ extern "C" int tpb_flash_bwd_ex(const void* dout, const void* q, const void* k, 
   p.kv_offset = Tk - Tq; p.scale = scale; p.scale_log2e = scale * 1.4426950408889634f;
   p.nlse2 = nlse2; p.ndsc = ndsc; p.stat_stride = stat_stride; p.status = status;
   p.wait_ns = kDefaultWaitNs;
-  p.trace = g_bwd_trace; p.trace_cap = g_bwd_trace_cap;
+  p.trace = g_bwd_trace;
   p.window = window > 0 ? window : 0; p.seg_start = seg_start; p.seg_end = seg_end;
   int r;
   // ---- dK / dV: [B, Tk, Hkv, D] by the dkv strides (dk and dv share them)
@@ -505,9 +504,6 @@ extern "C" int tpb_flash_bwd_ex(const void* dout, const void* q, const void* k, 
   return 0;
 }
 
-// Debug aid: buf = device array of 1 + 2 * cap uint64 (buf[0] = record count, zero it first). The
-// next backward launches record role / iteration / phase timestamps of block (0,0,0) of BOTH
-// passes into it. Pass null to switch tracing off.
 extern "C" int tpb_flash_bwd(const void* dout, const void* q, const void* k, const void* v,
                              const void* o, const float* lse, float* delta, void* dq, void* dk,
                              void* dv, int B, int Tq, int Tk, int Hq, int Hkv, int D,
@@ -526,8 +522,10 @@ extern "C" int tpb_flash_bwd(const void* dout, const void* q, const void* k, con
                           status, stream_, 0, nullptr, nullptr);
 }
 
+// Debug aid: buf = device array of `cap` uint64 (2 * 3 * 64 * 8 are needed). The next backward launches of the debug build
+// write the cycle stamps of block (0,0,0) of both passes into it (layout at trace_pt). Pass null to switch tracing off.
 extern "C" int tpb_flash_bwd_set_trace(unsigned long long* buf, int cap) {
+  if (buf && (!kBwdTrace || cap < kBwdTraceWords)) return -2;
   tpb::g_bwd_trace = buf;
-  tpb::g_bwd_trace_cap = cap;
   return 0;
 }

@@ -30,21 +30,22 @@ struct AttnBwdParams {
   long long out_tok, out_head, out_batch;
   uint32_t* status;
   unsigned long long wait_ns;
-  unsigned long long* trace;  // optional: timestamps of CTA (0,0,0), see tpb_flash_bwd_set_trace
-  int trace_cap;
+  unsigned long long* trace;  // optional: cycle stamps of CTA (0,0,0), see tpb_flash_bwd_set_trace
 };
 
-// Debug aid: records (role, iteration, phase, globaltimer) tuples of block (0,0,0).
-__device__ __forceinline__ void trace_pt(const AttnBwdParams& p, int role, int it, int phase) {
-  if (p.trace && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0) {
-    unsigned long long idx = atomicAdd(p.trace, 1ull);
-    if ((int)idx < p.trace_cap) {
-      unsigned long long t;
-      asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-      p.trace[1 + idx * 2] = ((unsigned long long)role << 48) | ((unsigned long long)(it & 0xffffff) << 16) | (unsigned)phase;
-      p.trace[2 + idx * 2] = t;
-    }
-  }
+// Debug aid: cycle stamps of block (0,0,0), trace[((pass * 3 + who) * 64 + it) * 8 + tag] with pass 0 = dKV, 1 = dQ and
+// who 0 = TMA warp, 1 = MMA warp, 2 = first P / dS thread. Only in the debug build: each stamp is a branch, which the
+// compiler schedules nothing across.
+#ifdef TPB_KERNEL_DEBUG
+constexpr bool kBwdTrace = true;
+#else
+constexpr bool kBwdTrace = false;
+#endif
+constexpr int kBwdTraceWords = 2 * 3 * 64 * 8;
+template <bool DKV>
+__device__ __forceinline__ void trace_pt(const AttnBwdParams& p, int who, int it, int tag) {
+  if (kBwdTrace && p.trace && it < 64 && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0)
+    p.trace[(((DKV ? 0 : 3) + who) * 64 + it) * 8 + tag] = clock64();
 }
 
 __device__ __forceinline__ float bwd_exp2(float x) {

@@ -44,21 +44,20 @@ struct WideSmem {
   static_assert(2 * kStatSlots + 1 >= kRing, "statistics would be overwritten while in use");
 };
 
-// P = exp2(S * scale_log2e - lse * log2e) of C columns of one row, in place (fp32). Straight-line code: the masked
+// P = exp2(S * scale_log2e - lse * log2e) of 32 columns of one row, in place (fp32). Straight-line code: the masked
 // variant selects, it never branches.
 //   DKV: per-column statistics of the streamed queries come from shared memory;
 //   dQ : the row's own statistics are in registers.
 // Both come negated and scaled from the pass that computes delta: scaling them here cost two of the ~eight instructions
 // per element of the dK/dV pass.
-template <bool DKV, bool MASKED, int C>
-__device__ __forceinline__ void p_math(uint32_t (&sr)[C], uint32_t stats_sa, float nlse2_row, int y0i, int y_lo,
-                                       int y_hi, float scale_log2e) {
+template <bool DKV, bool MASKED>
+__device__ __forceinline__ void p_math(uint32_t* sr, const float4* stats, float nlse2_row, int y0i, int y_lo, int y_hi,
+                                       float scale_log2e) {
   const float2 sc2 = make_float2(scale_log2e, scale_log2e);
 #pragma unroll
-  for (int c = 0; c < C; c += 4) {
+  for (int c = 0; c < 32; c += 4) {
     float4 l = make_float4(nlse2_row, nlse2_row, nlse2_row, nlse2_row);
-    if (DKV)
-      asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(l.x), "=f"(l.y), "=f"(l.z), "=f"(l.w) : "r"(stats_sa + c * 4));
+    if (DKV) l = stats[c / 4];
     const float2 lo = __ffma2_rn(make_float2(__uint_as_float(sr[c]), __uint_as_float(sr[c + 1])), sc2, make_float2(l.x, l.y));
     const float2 hi = __ffma2_rn(make_float2(__uint_as_float(sr[c + 2]), __uint_as_float(sr[c + 3])), sc2, make_float2(l.z, l.w));
     float e[4] = {bwd_exp2(lo.x), bwd_exp2(lo.y), bwd_exp2(hi.x), bwd_exp2(hi.y)};
@@ -193,7 +192,7 @@ flash_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmX0, const __grid_con
         const int it = t >> 1, s = t % R;
         const bool second = t & 1;   // Y1
         if (!mbar_wait_relaxed(&y_empty[s], ((t / R) & 1) ^ 1, wc, 1)) break;
-        trace_pt(p, 0, it, 1);
+        trace_pt<DKV>(p, 0, it, 1);
         int hy, yb;
         if (DKV) { hy = hx * G + it / y_count; yb = y_first + it % y_count; }
         else { hy = hx / G; yb = y_first + it; }
@@ -267,7 +266,7 @@ flash_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmX0, const __grid_con
       if (ok) ok = issue_in(0, 0) && issue_in(0, 1);
       for (int it = 0; it < n_it && ok; ++it) {
         if (!mbar_wait_warp(p_full, it & 1, wc, 5)) break;
-        if (lane == 0) trace_pt(p, 1, it, 3);
+        if (lane == 0) trace_pt<DKV>(p, 1, it, 3);
         tc_fence_after_sync();
         if (DKV) issue_acc(it, tmem_base, tmem_acc0, 1);                     // dV += P^T dO
         if (it + 1 < n_it && !issue_in(it + 1, 0)) break;
@@ -280,7 +279,7 @@ flash_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmX0, const __grid_con
           if (elect_one()) umma_commit(acc_done);
           __syncwarp();
         }
-        if (lane == 0) trace_pt(p, 1, it, 4);
+        if (lane == 0) trace_pt<DKV>(p, 1, it, 4);
       }
     }
   } else {
@@ -330,62 +329,76 @@ flash_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmX0, const __grid_con
       if (DKV) yb = y_first + it % y_count;
       else yb = y_first + it;
       const int y0i = yb * kStream + half * C;  // first query (DKV) or key (dQ) of this warp's columns
-      if (!mbar_wait_warp(s_full, it & 1, wc, 6)) { ok = false; break; }
-      if (threadIdx.x == 64) trace_pt(p, 2, it, 1);
       // Valid streamed indices of this thread's row form one interval [lo, hi): tiles that lie
       // entirely inside it take the predicate-free path (warp-uniform choice).
       const bool need_mask = __any_sync(0xffffffffu, (y0i < y_lo) || (y0i + C > y_hi));
       uint32_t lse_sa = 0;
+      float4 st[C / 4];
       if (DKV) {
         // the statistics landed with Y1 (the wait orders the read)
         const int t = 2 * it + 1;
         if (!mbar_wait_warp(&y_full[t % R], (t / R) & 1, wc, 9)) { ok = false; break; }
         lse_sa = smem_u32(smem + L::kStats) + ((it % L::kStatSlots) * 2 * kStream + half * C) * 4;
+#pragma unroll
+        for (int c = 0; c < C / 4; ++c)
+          asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(st[c].x), "=f"(st[c].y), "=f"(st[c].z), "=f"(st[c].w) : "r"(lse_sa + c * 16));
       }
+      if (!mbar_wait_warp(s_full, it & 1, wc, 6)) { ok = false; break; }
+      if (threadIdx.x == 64) trace_pt<DKV>(p, 2, it, 1);
       tc_fence_after_sync();
-      uint32_t sr[C];
+      // 32 columns at a time, the next ones loaded under the math of the ones before
+      uint32_t sr[C / 32][32], dr[C / 32][32];
+      tmem_ld_32x32b_x32(t_s, sr[0]);
 #pragma unroll
-      for (int q = 0; q < C / 32; ++q) tmem_ld_32x32b_x32(t_s + q * 32, &sr[q * 32]);
-      tmem_ld_wait();
-      if (threadIdx.x == 64) trace_pt(p, 2, it, 2);
-      if (need_mask) p_math<DKV, true>(sr, lse_sa, lse_row, y0i, y_lo, y_hi, p.scale_log2e);
-      else p_math<DKV, false>(sr, lse_sa, lse_row, y0i, y_lo, y_hi, p.scale_log2e);
-      if (DKV) {
-        // P (bf16 pairs) goes back over this warp's own S columns
-#pragma unroll
-        for (int q = 0; q < C / 32; ++q) {
+      for (int q = 0; q < C / 32; ++q) {
+        tmem_ld_wait(sr[q]);
+        if (q + 1 < C / 32) tmem_ld_32x32b_x32(t_s + (q + 1) * 32, sr[q + 1]);
+        if (!DKV && q + 1 == C / 32) {
+          // S was read: its columns are free for the next tile, whose product runs under this tile's exponentials
+          tc_fence_before_sync();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(p_full);   // one arrival per warp: 32 on one barrier are served one after the other
+        }
+        if (need_mask) p_math<DKV, true>(sr[q], st + q * 8, lse_row, y0i + q * 32, y_lo, y_hi, p.scale_log2e);
+        else p_math<DKV, false>(sr[q], st + q * 8, lse_row, y0i + q * 32, y_lo, y_hi, p.scale_log2e);
+        if (DKV) {
+          // P (bf16 pairs) goes back over this warp's own S columns
           uint32_t pw[16];
 #pragma unroll
           for (int i = 0; i < 16; ++i) {
-            __nv_bfloat162 h = __floats2bfloat162_rn(__uint_as_float(sr[q * 32 + 2 * i]), __uint_as_float(sr[q * 32 + 2 * i + 1]));
+            __nv_bfloat162 h = __floats2bfloat162_rn(__uint_as_float(sr[q][2 * i]), __uint_as_float(sr[q][2 * i + 1]));
             pw[i] = *reinterpret_cast<uint32_t*>(&h);
           }
           tmem_st_32x32b_x16(t_s + q * 16, pw);
         }
-        tmem_st_wait();
       }
-      tc_fence_before_sync();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(p_full);   // one arrival per warp: 32 on one barrier are served one after the other
-      if (threadIdx.x == 64) trace_pt(p, 2, it, 3);
+      if (DKV) {
+        tmem_st_wait();
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(p_full);
+      }
+      if (threadIdx.x == 64) trace_pt<DKV>(p, 2, it, 3);
       if (!mbar_wait_warp(dp_full, it & 1, wc, 11)) { ok = false; break; }
       tc_fence_after_sync();
+      if (threadIdx.x == 64) trace_pt<DKV>(p, 2, it, 4);
       // dS of 32 columns at a time goes over dP columns that were already read
+      tmem_ld_32x32b_x32(t_dp, dr[0]);
 #pragma unroll
       for (int q = 0; q < C / 32; ++q) {
-        uint32_t dr[32], dw[16];
-        tmem_ld_32x32b_x32(t_dp + q * 32, dr);
-        tmem_ld_wait();
+        uint32_t dw[16];
+        tmem_ld_wait(dr[q]);
+        if (q + 1 < C / 32) tmem_ld_32x32b_x32(t_dp + (q + 1) * 32, dr[q + 1]);
         const uint32_t d_sa = lse_sa + (kStream + q * 32) * 4;
-        if (need_mask) ds_math<DKV, true>(&sr[q * 32], dr, d_sa, delta_row, y0i + q * 32, y_lo, y_hi, p.scale, dw);
-        else ds_math<DKV, false>(&sr[q * 32], dr, d_sa, delta_row, y0i + q * 32, y_lo, y_hi, p.scale, dw);
+        if (need_mask) ds_math<DKV, true>(sr[q], dr[q], d_sa, delta_row, y0i + q * 32, y_lo, y_hi, p.scale, dw);
+        else ds_math<DKV, false>(sr[q], dr[q], d_sa, delta_row, y0i + q * 32, y_lo, y_hi, p.scale, dw);
         tmem_st_32x32b_x16(t_dp + q * 16, dw);
       }
       tmem_st_wait();
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive(ds_full);
-      if (threadIdx.x == 64) trace_pt(p, 2, it, 5);
+      if (threadIdx.x == 64) trace_pt<DKV>(p, 2, it, 5);
     }
     if (ok && n_it > 0) ok = mbar_wait_warp(acc_done, 0, wc, 8);
     if (ok) {
