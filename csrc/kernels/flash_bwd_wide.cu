@@ -5,7 +5,10 @@
 // P = exp2(..) and then dP into dS = P (dP - delta) * scale, each written as bf16 over the columns it came from, from
 // where the accumulating MMAs take it as their A operand. The products of two tiles interleave on the tensor pipe,
 //     dV(i)  S(i+1)  dK(i)  dP(i+1)      (dQ pass: S(i+1)  dQ(i)  dP(i+1)),
-// and the warps compute dS(i) under dV(i) and S(i+1), and P(i+1) under dK(i) and dP(i+1).
+// and the warps compute dS(i) under dV(i) and S(i+1), and P(i+1) under dK(i) and dP(i+1). The dQ pass has no P product: S(i+1)
+// is issued once S(i) is in registers and runs under P(i). The warps take 32 columns at a time and load the next ones under
+// the math of the ones before, and read the statistics for P while they wait for S. 32/8 heads, both passes: T = 8190 1765 ->
+// 1571 us, T = 4096 496 -> 439; D = 64, T = 8190 1307 -> 1132, 16 x 1024 tokens of 12 heads 222 -> 200.
 //
 // D = 128: TMEM (S, dP and two accumulators of 128 columns) has no room for two tiles unless they have 64 rows; with 128
 // rows there are half as many barriers and round trips. 32/8 heads: T = 4096 533 -> 478 us for both passes, T = 8190
