@@ -100,6 +100,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmX0, const __grid_constant
                  const AttnBwdParams p) {
   using L = BwdSmem<D>;
   extern __shared__ uint8_t smem_raw[];
+  bwd_overlap_start<DKV>();
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~uintptr_t(1023));
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::kBar);
@@ -337,6 +338,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmX0, const __grid_constant
     tc_fence_after_sync();
     tmem_dealloc(tmem_base, 512);
   }
+  bwd_overlap_end<DKV>();
 }
 
 // ndsc[b, h, t] = -scale * sum_d O[b, t, h, d] * dO[b, t, h, d] and nlse2[b, h, t] = -log2(e) * lse[b, h, t].
@@ -401,8 +403,7 @@ static int launch_bwd(const CUtensorMap& x0, const CUtensorMap& x1, const CUtens
     if (e != cudaSuccess) return (int)e;
     configured = true;
   }
-  kern<<<grid, kBwdThreads, L::kTotal, stream>>>(x0, x1, y0, y1, p);
-  return (int)cudaGetLastError();
+  return bwd_launch(kern, !DKV, grid, L::kTotal, stream, x0, x1, y0, y1, p);
 }
 
 }  // namespace tpb

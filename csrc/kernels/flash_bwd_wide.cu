@@ -115,10 +115,12 @@ flash_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmX0, const __grid_con
   // TMEM columns: S, dP, accumulators (and X0, X1 in the dQ pass of D = 128, which has one accumulator)
   constexpr int kTmemCols = 2 * kStream + 2 * D <= 256 ? 256 : 512;
   extern __shared__ uint8_t smem_raw[];
+  bwd_overlap_start<DKV>();
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~uintptr_t(1023));
   if (smem + L::kUsed > smem_raw + L::kTotal) {   // see WideSmem::kTotal; the same for every thread
     if (threadIdx.x == 0 && p.status) atomicCAS(p.status, 0u, kStatusBadArgs | (20u << 8));
+    bwd_overlap_end<DKV>();
     return;
   }
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::kBar);
@@ -421,6 +423,7 @@ flash_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmX0, const __grid_con
     tc_fence_after_sync();
     tmem_dealloc(tmem_base, kTmemCols);
   }
+  bwd_overlap_end<DKV>();
 }
 
 template <int D, bool DKV, int KS>
@@ -435,8 +438,7 @@ static int launch_wide(const CUtensorMap& x0, const CUtensorMap& x1, const CUten
     if (e != cudaSuccess) return (int)e;
     configured = true;
   }
-  kern<<<grid, kBwdThreads, L::kTotal, stream>>>(x0, x1, y0, y1, p);
-  return (int)cudaGetLastError();
+  return bwd_launch(kern, !DKV, grid, L::kTotal, stream, x0, x1, y0, y1, p);
 }
 
 int launch_bwd_wide(int D, bool dkv, const CUtensorMap& x0, const CUtensorMap& x1, const CUtensorMap& y0,
