@@ -8,10 +8,10 @@
 //     group happens inside the accumulator (no expanded K/V, no atomics).
 //   * dQ pass: a CTA owns 128 queries of one query head, keeps Q and dO resident and streams
 //     64-key tiles of K and V; dQ += dS K in TMEM (deterministic, no atomics).
-// Two forms share the passes. Here, for head dimension 64 with few CTAs and 128 with short streams: per streamed tile
-// S = X0 Y0^T and dP = X1 Y1^T go to TMEM (two tiles at a time), eight warps turn both into P and dS = P (dP - delta) * scale
-// in one step and write them as bf16 over the same columns, from where the accumulating MMAs take them. The other form,
-// for head dimension 128 with long streams and 64 with many CTAs, is in flash_bwd_wide.cu.
+// Two forms share the passes. Here, for head dimension 128 with short streams and the dKV pass of 64 with few CTAs: per
+// streamed tile S = X0 Y0^T and dP = X1 Y1^T go to TMEM (two tiles at a time), eight warps turn both into P and
+// dS = P (dP - delta) * scale in one step and write them as bf16 over the same columns, from where the accumulating MMAs
+// take them. The other form, head dimension 128 with long streams and otherwise for 64, is in flash_bwd_wide.cu.
 //
 // Counterpart in the reference: FlashAttention-2 sm80 backward
 // (p10/src/backend/cuda/transformers/AttentionKernels.cu:2286-2543), which has no GQA path
@@ -436,22 +436,26 @@ extern "C" int tpb_flash_bwd_ex(const void* dout, const void* q, const void* k, 
     return -2;
   const int stat_stride = (Tq + kStatPad - 1) / kStatPad * kStatPad;
   float *ndsc = delta, *nlse2 = delta + (size_t)B * Hq * stat_stride;
-  // Which form of a pass. D = 64 (dKV / dQ pass in us, this file's form against the wide one): 16 x 1024 tokens, 12 heads
-  // (1536 CTAs) 138 / 99 against 118 / 91; 8190 tokens, 32/8 heads (512 / 2048 CTAs) 733 / 610 against 853 / 553; 2 x 2048
-  // tokens, 16 heads (512 CTAs) 68 / 53 against 72 / 56; 8 x 309 tokens, 16/4 heads (96 / 384 CTAs) 22 / 17 against 32 / 18.
-  // Two CTAs per SM pay from some six CTAs per SM on.
-  // D = 128 (both passes): the 128-row streamed tiles of the wide form pay once a CTA streams some 576 rows; before that
-  // their padding and the tiles on a mask's edge cost more than the round trips they save. Causal, 16 heads, B x T: 512 x
-  // 17 (8 heads) 286 against 360 us, 64 x 129 227 / 258, 16 x 512 178 / 180, 8 x 1024 226 / 225, 4 x 2048 346 / 333, 2 x 4096
-  // 600 / 565; window 128 at 4096 131 / 138, 500 213 / 213, 1000 313 / 307. Packed segments say nothing of their lengths
-  // here: of 64 to 1000 tokens 103 to 237 us against 110 to 250.
+  // Which form of a pass (us, both passes).
+  // D = 64: the dQ pass always has the wide form. Its CTAs share an SM in pairs, so the dKV pass has it, too, once they do:
+  // with groups of query heads from some 2.3 CTAs per SM on (this file's form against the wide one; 32/8 heads: 2 x 2048
+  // tokens, 256 CTAs 181 / 192; 16 x 309, 384 CTAs 101 / 98; 8 x 1024, 512 CTAs 224 / 217), without groups, where the dQ pass
+  // has as many CTAs as long, from 1.2 on (12 heads: 2 x 1024, 192 CTAs 42.3 / 39.7; 2900, 276 CTAs 113 / 93; 16 x 1024 218 /
+  // 194; 32/8 heads, 2900, 184 CTAs 175 / 229).
+  // D = 128 (both passes): the 128-row streamed tiles of the wide form pay once a CTA streams some 400 rows; before that
+  // their padding and the tiles on a mask's edge cost more than the round trips they save. Causal, 32/8 heads, B x T: 4 x
+  // 300 46.6 / 51.2, 8 x 309 81 / 94, 500 48 / 47, 1000 79 / 73, 2900 256 / 227; 16/2 heads, 1000 137 / 123; 8 heads, 8 x
+  // 1024 114 / 114. A window has two edges: 300 at 2 x 3000 224 / 250, 500 at 4096 213 / 213. Packed segments say nothing of
+  // their lengths here: of 64 to 1000 tokens 103 to 237 us against 110 to 250.
   const double pairs = !causal ? (double)Tq * Tk
                        : Tk >= Tq ? (double)Tq * Tk - 0.5 * Tq * (Tq - 1.0) : 0.5 * Tk * (Tk + 1.0);
-  auto wide = [&](long long ctas, int rows) {   // rows: stationary ones of the pass; the others stream past them
-    if (D == 64) return ctas >= 6LL * sm_count();
-    double streamed = pairs / rows + 64;
-    if (window > 0 && streamed > window + 128) streamed = window + 128;
-    return !seg_start && !seg_end && streamed >= 576;
+  auto wide128 = [&](int rows) {   // rows: stationary ones of the pass; the others stream past them
+    double streamed = pairs / rows + 64, need = 400;
+    if (window > 0 && streamed > window + 128) {
+      streamed = window + 128;
+      need = 576;
+    }
+    return !seg_start && !seg_end && streamed >= need;
   };
   {
     if (reinterpret_cast<uintptr_t>(dout) & 15) return -2;
@@ -474,7 +478,7 @@ extern "C" int tpb_flash_bwd_ex(const void* dout, const void* q, const void* k, 
   {
     CUtensorMap tk, tv, tq, tdo;
     const dim3 grid((Tk + kStat - 1) / kStat, Hkv, B);
-    const bool w = wide((long long)grid.x * grid.y * grid.z, Tk);
+    const bool w = D == 64 ? 10LL * grid.x * grid.y * grid.z >= (Hq == Hkv ? 12LL : 23LL) * sm_count() : wide128(Tk);
     const int rows = w ? bwd_wide_rows(D) : kStream;
     if ((r = make_tmap_bthd(&tk, k, B, Tk, Hkv, D, k_tok, k_head, k_batch, kStat))) return r;
     if ((r = make_tmap_bthd(&tv, v, B, Tk, Hkv, D, v_tok, v_head, v_batch, kStat))) return r;
@@ -490,7 +494,7 @@ extern "C" int tpb_flash_bwd_ex(const void* dout, const void* q, const void* k, 
   {
     CUtensorMap tq, tdo, tk, tv;
     const dim3 grid((Tq + kStat - 1) / kStat, Hq, B);
-    const bool w = wide((long long)grid.x * grid.y * grid.z, Tq);
+    const bool w = D == 64 || wide128(Tq);
     const int rows = w ? bwd_wide_rows(D) : kStream;
     if ((r = make_tmap_bthd(&tq, q, B, Tq, Hq, D, q_tok, q_head, q_batch, kStat))) return r;
     if ((r = make_tmap_bthd(&tdo, dout, B, Tq, Hq, D, do_tok, do_head, do_batch, kStat))) return r;
@@ -499,7 +503,7 @@ extern "C" int tpb_flash_bwd_ex(const void* dout, const void* q, const void* k, 
     p.out0 = nullptr; p.out1 = (__nv_bfloat16*)dq;
     p.out_tok = dq_tok; p.out_head = dq_head; p.out_batch = dq_batch;
     r = w ? launch_bwd_wide(D, false, tq, tdo, tk, tv, p, grid, stream)
-          : D == 128 ? launch_bwd<128, false>(tq, tdo, tk, tv, p, grid, stream) : launch_bwd<64, false>(tq, tdo, tk, tv, p, grid, stream);
+          : launch_bwd<128, false>(tq, tdo, tk, tv, p, grid, stream);
     if (r) return r;
   }
   return 0;

@@ -1,5 +1,5 @@
 // Flash attention backward for sm_100a, the form with one tile of S and dP in TMEM: head dimension 128 with long streams,
-// and head dimension 64 where there are many CTAs (flash_bwd.cu has the choice and the other form).
+// and head dimension 64, but for a dKV pass of few CTAs (flash_bwd.cu has the choice and the other form).
 //
 // Two passes as described there. Per streamed tile: S = X0 Y0^T and dP = X1 Y1^T into TMEM; eight warps turn S into
 // P = exp2(..) and then dP into dS = P (dP - delta) * scale, each written as bf16 over the columns it came from, from
