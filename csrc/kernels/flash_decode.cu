@@ -5,13 +5,15 @@
 // and leave all but B * Hq CTAs idle: 437 us at B = 8, Tk = 16381, 32/8 heads of 128 (0.54 GB). Here
 //   * all query rows of a KV head form the 16-row operand of one warp MMA (m16n8k16), so K and V are read once per
 //     16 rows; with at most 16 rows there is no tile that would amortise TMEM and a shared-memory operand pipeline;
-//   * K and V go from global memory straight into the B fragments. The sum over d (and over keys) is free of order,
-//     so a lane takes whole 16-byte pieces of a row and the query fragments are permuted alike: no shared memory, no
-//     ldmatrix, 8 KB in flight per warp (one 16-key step of K and one of V ahead);
-//   * the keys are split over CTAs until the chip is full; partial sums stay fp32. Up to eight splits of a row tile are
-//     one cluster that merges them through distributed shared memory, in rank order; more go through memory and a
-//     second kernel.
-// The same case takes 114 us (4.7 TB/s).
+//   * a warp works on steps of 16 keys and copies its own later steps with cp.async into a ring of its own (no barrier
+//     between warps): K of a step is replaced once its scores are there, V once its product is. The chain of a step
+//     (scores, maximum, exponentials, second product) takes some 1 000 cycles in which a warp's registers cannot also
+//     be loading; with the fragments of the next step in registers (204 of them, eight warps per SM) warps spent 60 % of
+//     the time in that chain and 4.8 TB/s came in. The ring leaves room for twelve (D = 128) or sixteen warps;
+//   * the keys are split over CTAs; partial sums stay fp32. Up to eight splits of a row tile are one cluster that merges
+//     them through distributed shared memory, in rank order; more go through memory and a second kernel.
+// The same case takes 82 us (6.6 TB/s; 112 before the ring); 32 x 8000 keys 151 (6.9 TB/s; 215), 16 x 1006 keys 15.7
+// (20), D = 64 with 8 x 16381 keys 44 (52).
 // Scores, running maximum, sums and output accumulate in fp32; probabilities are rounded to bf16 for the second
 // product, as in flash_fwd_kernel.
 #include "sm100.cuh"
@@ -45,42 +47,43 @@ __device__ __forceinline__ uint32_t dec_pack(float lo, float hi) {
   asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(hi), "f"(lo));
   return d;
 }
-// K and V are read once: keep them from pushing the next layer's weights out of L1.
-__device__ __forceinline__ uint4 dec_ld(const __nv_bfloat16* p) {
-  uint4 r;
-  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
-               : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w)
-               : "l"(p));
-  return r;
+// 16 bytes to shared memory, zeros where `in` is false.
+__device__ __forceinline__ void dec_cp(uint32_t dst, const __nv_bfloat16* src, bool in) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(in ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void dec_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void dec_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+template <bool TRANS>
+__device__ __forceinline__ void dec_ldm(uint32_t (&r)[4], uint32_t a) {
+  if (TRANS)
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a) : "memory");
+  else
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a) : "memory");
+}
+
+constexpr int dec_stages(int d) { return d == 128 ? 2 : 3; }   // steps that a warp's ring holds
+constexpr int dec_ctas(int d) { return d == 128 ? 3 : 4; }     // CTAs that fit an SM
+constexpr int dec_smem(int d) {
+  const int ring = kDecWarps * dec_stages(d) * 2 * kDecKeys * d * 2, rows = kDecWarps * kDecRows * d * 4;
+  return ring > rows ? ring : rows;
 }
 
 template <int D>
-__global__ void __launch_bounds__(kDecWarps * 32)
+__global__ void __launch_bounds__(kDecWarps * 32, dec_ctas(D))
 flash_decode_kernel(const DecodeParams p) {
-  constexpr int NP = D / 32;   // 16-byte pieces of a K row per lane
-  constexpr int VP = D / 64;   // 16-byte pieces of a V row per lane
-  __shared__ float sm_o[kDecWarps][kDecRows][D];
+  constexpr int S = dec_stages(D);
+  constexpr int kTile = kDecKeys * D * 2;   // bytes of a step's K (or V) of a warp
+  extern __shared__ __align__(128) uint8_t dec_sm[];   // the warps' rings, later their partial rows
   __shared__ float sm_m[kDecWarps][kDecRows], sm_l[kDecWarps][kDecRows], sm_lse[kDecRows];
+  float (&sm_o)[kDecWarps][kDecRows][D] = *reinterpret_cast<float (*)[kDecWarps][kDecRows][D]>(dec_sm);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int gq = lane >> 2, t = lane & 3;
   const int split = blockIdx.x, hk = blockIdx.y / p.row_tiles, rt = blockIdx.y % p.row_tiles, b = blockIdx.z;
-
-  // this lane's two rows: r0 (fragment row gq) and r0 + 8
-  const int r0 = rt * kDecRows + gq;
-  int lim[2], low[2];
-  uint4 qf[2][NP];
-#pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    const int r = r0 + 8 * i;
-    const int tq = r / p.group, h = hk * p.group + r % p.group;
-    const bool in = r < p.R;
-    lim[i] = in ? (p.causal ? min(p.Tk - 1, tq + p.Tk - p.Tq) : p.Tk - 1) : -1;
-    low[i] = p.window > 0 ? tq + p.Tk - p.Tq - p.window + 1 : 0;
-    const __nv_bfloat16* qr = p.q + b * p.q_batch + (long long)tq * p.q_tok + (long long)h * p.q_head;
-#pragma unroll
-    for (int c = 0; c < NP; ++c)
-      qf[i][c] = in ? *reinterpret_cast<const uint4*>(qr + (t + 4 * c) * 8) : make_uint4(0, 0, 0, 0);
-  }
 
   int k_begin = split * p.keys_per_split;
   const int k_end = min(p.Tk, k_begin + p.keys_per_split);
@@ -89,72 +92,119 @@ flash_decode_kernel(const DecodeParams p) {
     const int first = (rt * kDecRows) / p.group + p.Tk - p.Tq - p.window + 1;
     if (first > k_begin) k_begin += (first - k_begin) / kDecKeys * kDecKeys;
   }
-  const __nv_bfloat16* kb = p.k + b * p.k_batch + (long long)hk * p.k_head;
-  const __nv_bfloat16* vb = p.v + b * p.v_batch + (long long)hk * p.v_head;
 
-  uint4 kf[2][NP], vf[4][VP];
-  auto load_k = [&](int base) {
-#pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      const int key = base + u * 8 + gq;
-#pragma unroll
-      for (int c = 0; c < NP; ++c)
-        kf[u][c] = key < k_end ? dec_ld(kb + (long long)key * p.k_tok + (t + 4 * c) * 8) : make_uint4(0, 0, 0, 0);
-    }
-  };
+  // A lane copies one 16-byte piece of every LR-th row. Pieces are swizzled by their row, so that the eight rows of a
+  // matrix lie in different banks.
+  constexpr int LR = 256 / D;   // rows per copy of a warp
+  const int piece = lane % (D / 8), row0 = lane / (D / 8);
+  const uint32_t ring = smem_u32(dec_sm) + warp * (S * 2 * kTile);
+  const __nv_bfloat16* kp = p.k + b * p.k_batch + (long long)hk * p.k_head + piece * 8;
+  const __nv_bfloat16* vp = p.v + b * p.v_batch + (long long)hk * p.v_head + piece * 8;
   // keys past the end are zero-filled: their probability is zero, but zero times whatever lies there need not be
-  auto load_v = [&](int base) {
+  auto load = [&](const __nv_bfloat16* src, long long tok, int base, uint32_t dst) {
+    if (base < k_end) {
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int key = base + (u >> 1) * 8 + 2 * t + (u & 1);
-#pragma unroll
-      for (int c = 0; c < VP; ++c)
-        vf[u][c] = key < k_end ? dec_ld(vb + (long long)key * p.v_tok + (gq + 8 * c) * 8) : make_uint4(0, 0, 0, 0);
+      for (int i = 0; i < kDecKeys / LR; ++i) {
+        const int r = row0 + i * LR, key = base + r;
+        dec_cp(dst + r * (D * 2) + ((piece ^ (r & 7)) << 4), src + (key < k_end ? key : 0) * tok, key < k_end);
+      }
     }
+    dec_commit();
   };
-
-  float acc[VP * 8][4];
+  constexpr int kStep = kDecWarps * kDecKeys;
+  const int base0 = k_begin + warp * kDecKeys;
 #pragma unroll
-  for (int n = 0; n < VP * 8; ++n)
+  for (int s = 0; s < S; ++s) {
+    load(kp, p.k_tok, base0 + s * kStep, ring + s * 2 * kTile);
+    load(vp, p.v_tok, base0 + s * kStep, ring + s * 2 * kTile + kTile);
+  }
+
+  // this lane's two rows: r0 (fragment row gq) and r0 + 8
+  const int r0 = rt * kDecRows + gq;
+  int lim[2], low[2], all_lim = p.Tk - 1, all_low = 0;   // of the lane's rows that exist
+  uint32_t qf[D / 16][4];
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const int r = r0 + 8 * i;
+    const int tq = r / p.group, h = hk * p.group + r % p.group;
+    const bool in = r < p.R;
+    lim[i] = in ? (p.causal ? min(p.Tk - 1, tq + p.Tk - p.Tq) : p.Tk - 1) : -1;
+    low[i] = p.window > 0 ? tq + p.Tk - p.Tq - p.window + 1 : 0;
+    if (in) { all_lim = min(all_lim, lim[i]); all_low = max(all_low, low[i]); }
+    const __nv_bfloat16* qr = p.q + b * p.q_batch + (long long)tq * p.q_tok + (long long)h * p.q_head;
+#pragma unroll
+    for (int c = 0; c < D / 16; ++c)
+#pragma unroll
+      for (int e = 0; e < 2; ++e)
+        qf[c][i + 2 * e] = in ? *reinterpret_cast<const uint32_t*>(qr + c * 16 + e * 8 + 2 * t) : 0u;
+  }
+  // steps that lie inside every row's bounds take the path without masks (rows past the last one are not stored)
+#pragma unroll
+  for (int o = 4; o < 32; o <<= 1) {
+    all_lim = min(all_lim, __shfl_xor_sync(0xffffffffu, all_lim, o));
+    all_low = max(all_low, __shfl_xor_sync(0xffffffffu, all_low, o));
+  }
+  all_lim = min(all_lim, k_end - 1);
+
+  float acc[D / 8][4];
+#pragma unroll
+  for (int n = 0; n < D / 8; ++n)
 #pragma unroll
     for (int j = 0; j < 4; ++j) acc[n][j] = 0.f;
   float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
 
-  int base = k_begin + warp * kDecKeys;
-  if (base < k_end) {
-    load_k(base);
-    load_v(base);
-  }
-  for (; base < k_end; base += kDecWarps * kDecKeys) {
-    const int next = base + kDecWarps * kDecKeys;
-    float s[2][4];
+  // rows and piece halves of this lane's matrix addresses: K matrices (8 keys x 8 of d) side by side along d, V ones
+  // (transposed) two key halves by two along d
+  const int krow = lane & 7, kpc = lane >> 3;
+  const int vrow = lane & 15, vpc = lane >> 4;
+  int slot = 0;
+  for (int base = base0; base < k_end; base += kStep) {
+    const uint32_t sk = ring + slot * 2 * kTile, sv = sk + kTile;
+    dec_wait<2 * S - 1>();
+    __syncwarp();
+    float s[2][4], s2[2][4];
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
 #pragma unroll
-      for (int j = 0; j < 4; ++j) s[u][j] = 0.f;
+      for (int j = 0; j < 4; ++j) s[u][j] = s2[u][j] = 0.f;
 #pragma unroll
-      for (int c = 0; c < NP; ++c) {
-        mma_bf16_16816(s[u], qf[0][c].x, qf[1][c].x, qf[0][c].y, qf[1][c].y, kf[u][c].x, kf[u][c].y);
-        mma_bf16_16816(s[u], qf[0][c].z, qf[1][c].z, qf[0][c].w, qf[1][c].w, kf[u][c].z, kf[u][c].w);
+      for (int c = 0; c < D / 32; ++c) {
+        uint32_t kf[4];
+        dec_ldm<false>(kf, sk + (u * 8 + krow) * (D * 2) + (((c * 4 + kpc) ^ krow) << 4));
+        mma_bf16_16816(s[u], qf[2 * c][0], qf[2 * c][1], qf[2 * c][2], qf[2 * c][3], kf[0], kf[1]);
+        mma_bf16_16816(s2[u], qf[2 * c + 1][0], qf[2 * c + 1][1], qf[2 * c + 1][2], qf[2 * c + 1][3], kf[2], kf[3]);
       }
     }
-    if (next < k_end) load_k(next);
+    __syncwarp();   // every lane has read K
+    load(kp, p.k_tok, base + S * kStep, sk);
     // s[u][2 i + j]: row i, key base + 8 u + 2 t + j
     float mx[2] = {-INFINITY, -INFINITY};
+    const bool inside = base >= all_low && base + kDecKeys - 1 <= all_lim;
 #pragma unroll
     for (int u = 0; u < 2; ++u)
 #pragma unroll
       for (int i = 0; i < 2; ++i)
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
-          const int key = base + u * 8 + 2 * t + j;
           float& x = s[u][2 * i + j];
-          x = (key <= lim[i] && key >= low[i] && key < k_end) ? x * p.scale_log2e : -INFINITY;
-          mx[i] = fmaxf(mx[i], x);
+          x = (x + s2[u][2 * i + j]) * p.scale_log2e;
         }
+    if (!inside) {
+#pragma unroll
+      for (int u = 0; u < 2; ++u)
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+          for (int j = 0; j < 2; ++j) {
+            const int key = base + u * 8 + 2 * t + j;
+            float& x = s[u][2 * i + j];
+            x = (key <= lim[i] && key >= low[i] && key < k_end) ? x : -INFINITY;
+          }
+    }
     float alpha[2], mu[2];
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
+      mx[i] = fmaxf(fmaxf(s[0][2 * i], s[0][2 * i + 1]), fmaxf(s[1][2 * i], s[1][2 * i + 1]));
       mx[i] = fmaxf(mx[i], __shfl_xor_sync(0xffffffffu, mx[i], 1));
       mx[i] = fmaxf(mx[i], __shfl_xor_sync(0xffffffffu, mx[i], 2));
       const float mn = fmaxf(m[i], mx[i]);
@@ -165,7 +215,7 @@ flash_decode_kernel(const DecodeParams p) {
     }
     if (__any_sync(0xffffffffu, alpha[0] != 1.f || alpha[1] != 1.f)) {
 #pragma unroll
-      for (int n = 0; n < VP * 8; ++n) {
+      for (int n = 0; n < D / 8; ++n) {
         acc[n][0] *= alpha[0]; acc[n][1] *= alpha[0];
         acc[n][2] *= alpha[1]; acc[n][3] *= alpha[1];
       }
@@ -179,21 +229,21 @@ flash_decode_kernel(const DecodeParams p) {
         l[i] += e0 + e1;
         pa[2 * u + i] = dec_pack(e0, e1);
       }
+    dec_wait<2 * S - 1>();
+    __syncwarp();
 #pragma unroll
-    for (int c = 0; c < VP; ++c) {
-      const uint32_t* w0 = reinterpret_cast<const uint32_t*>(&vf[0][c]);
-      const uint32_t* w1 = reinterpret_cast<const uint32_t*>(&vf[1][c]);
-      const uint32_t* w2 = reinterpret_cast<const uint32_t*>(&vf[2][c]);
-      const uint32_t* w3 = reinterpret_cast<const uint32_t*>(&vf[3][c]);
-#pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        const uint32_t sel = (e & 1) ? 0x7632u : 0x5410u;
-        mma_bf16_16816(acc[c * 8 + e], pa[0], pa[1], pa[2], pa[3], __byte_perm(w0[e >> 1], w1[e >> 1], sel),
-                       __byte_perm(w2[e >> 1], w3[e >> 1], sel));
-      }
+    for (int c = 0; c < D / 16; ++c) {
+      uint32_t vf[4];
+      dec_ldm<true>(vf, sv + vrow * (D * 2) + (((c * 2 + vpc) ^ (vrow & 7)) << 4));
+      mma_bf16_16816(acc[2 * c], pa[0], pa[1], pa[2], pa[3], vf[0], vf[1]);
+      mma_bf16_16816(acc[2 * c + 1], pa[0], pa[1], pa[2], pa[3], vf[2], vf[3]);
     }
-    if (next < k_end) load_v(next);
+    __syncwarp();   // every lane has read V
+    load(vp, p.v_tok, base + S * kStep, sv);
+    slot = slot + 1 == S ? 0 : slot + 1;
   }
+  dec_wait<0>();
+  __syncthreads();   // the rings become the partial rows
 
   // ---- the four warps' partial rows
 #pragma unroll
@@ -202,15 +252,8 @@ flash_decode_kernel(const DecodeParams p) {
     l[i] += __shfl_xor_sync(0xffffffffu, l[i], 2);
     if (t == 0) { sm_m[warp][gq + 8 * i] = m[i]; sm_l[warp][gq + 8 * i] = l[i]; }
 #pragma unroll
-    for (int c = 0; c < VP; ++c)
-#pragma unroll
-      for (int j = 0; j < 2; ++j) {
-        float* dst = &sm_o[warp][gq + 8 * i][(2 * t + j + 8 * c) * 8];
-        *reinterpret_cast<float4*>(dst) = make_float4(acc[c * 8][2 * i + j], acc[c * 8 + 1][2 * i + j],
-                                                      acc[c * 8 + 2][2 * i + j], acc[c * 8 + 3][2 * i + j]);
-        *reinterpret_cast<float4*>(dst + 4) = make_float4(acc[c * 8 + 4][2 * i + j], acc[c * 8 + 5][2 * i + j],
-                                                          acc[c * 8 + 6][2 * i + j], acc[c * 8 + 7][2 * i + j]);
-      }
+    for (int n = 0; n < D / 8; ++n)
+      *reinterpret_cast<float2*>(&sm_o[warp][gq + 8 * i][n * 8 + 2 * t]) = make_float2(acc[n][2 * i], acc[n][2 * i + 1]);
   }
   __syncthreads();
   constexpr int VEC = D / 4;   // float4 per row
@@ -343,6 +386,18 @@ flash_decode_merge_kernel(const DecodeParams p) {
     p.lse[((long long)b * p.Hq + h) * p.lse_stride + tq] = den > 0.f ? (M + log2f(den)) * 0.6931471805599453f : -INFINITY;
 }
 
+// Once per head dimension: more shared memory than a launch gets unasked.
+static cudaError_t decode_configure(int D) {
+  static bool configured[2] = {};
+  bool& done = configured[D == 64 ? 0 : 1];
+  if (done) return cudaSuccess;
+  const cudaError_t e =
+      D == 64 ? cudaFuncSetAttribute(flash_decode_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, dec_smem(64))
+              : cudaFuncSetAttribute(flash_decode_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, dec_smem(128));
+  done = e == cudaSuccess;
+  return e;
+}
+
 // Clusters of n CTAs that fit the device at once, asked of the runtime once per size: the SMs of a GPC are not a multiple
 // of every n (32 clusters of 8 CTAs of D = 128 fit, 96 of 3 do not, although 296 CTAs do).
 static int decode_resident(int D, int n) {
@@ -357,9 +412,11 @@ static int decode_resident(int D, int n) {
     attr[0].val.clusterDim.z = 1;
     cfg.gridDim = dim3(n, 4 * sm_count());
     cfg.blockDim = dim3(kDecWarps * 32);
+    cfg.dynamicSmemBytes = dec_smem(D);
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     int fit = 0;
+    decode_configure(D);
     const cudaError_t e = D == 64 ? cudaOccupancyMaxActiveClusters(&fit, flash_decode_kernel<64>, &cfg)
                                   : cudaOccupancyMaxActiveClusters(&fit, flash_decode_kernel<128>, &cfg);
     r = e == cudaSuccess && fit > 0 ? fit : -1;
@@ -367,33 +424,39 @@ static int decode_resident(int D, int n) {
   return r;
 }
 
-// Splits of the keys and who merges them, by the time in ns that the launch takes: for each round of resident CTAs 1.8 us,
-// of clusters, which start together, 3.3 us, and kKeyNs per key of a CTA, more where several share an SM (four of D = 64
-// fit by their registers, two of D = 128), kFullNs on a full chip (some 5 TB/s). A cluster's merge costs 1 us; a second
-// kernel and scratch 3 us + 60 ns a split on the device and 5 us on the host, which bounds a call over a short cache (one
-// token over 1000 keys: 32 us a call with one launch, 41 us with two). Caches from memory, D x B x Hkv x Tk, splits: us
-// (9 and more by two kernels): 128 x 8 x 8 x 16381, 1: 396, 3: 152, 4: 119, 8: 124, 9: 114, 10: 143, 16: 126;
-// 128 x 12 x 8 x 8192, 3: 146, 4: 117, 5: 99, 6: 122, 9: 90; 128 x 32 x 8 x 8192, 1: 223, 2: 230, 8: 258; 64 x 8 x 8 x
-// 16381, 4: 78, 8: 53, 9: 51; 128 x 1 x 8 x 4096, 1: 76, 4: 23, 8: 14, 16: 11.
+// Splits of the keys and who merges them, by the time in ns that the launch takes. What resident CTAs take is what memory
+// takes (7 TB/s; the row tiles of a head share its reads) or the keys of one times kKeyNs, which grows with the CTAs per
+// SM: one alone reads 49 (D = 128) or 37 (64) GB/s and keeps an SM's share of the memory busy by itself. Clusters are not
+// spread evenly: at 0.87 of an SM each, some SMs have two CTAs. A launch costs 4 us, each further round 1.8 us and a tail of
+// 4 ns a key; a cluster's merge 1 us; a second kernel and scratch 4 us + 60 ns a split on the device and 5 us on the host,
+// which bounds a call over a short cache. Measured, D x B x Hkv x Tk, splits: us (m: by two kernels): 128 x 8 x 8 x 16381,
+// 1: 177, 2: 94, 3: 87, 4: 82, 5: 92, 8: 105, m9: 100, m12: 87; 128 x 32 x 8 x 8000, 1: 151, 2: 192, 3: 162, 8: 170;
+// 128 x 3 x 16 x 5000, 1: 57, 3: 30, 5: 24, 8: 25; 128 x 1 x 8 x 32768, 8: 49, m16: 30, m32: 29; 128 x 1 x 8 x 4096, 1: 47,
+// 4: 16, 8: 11, m16: 10; 64 x 8 x 8 x 16381, 1: 115, 2: 62, 4: 44, 7: 51, 8: 47; 64 x 32 x 8 x 8000, 1: 80, 2: 89, 3: 97.
 struct DecodePlan {
   int splits;
   bool memory;   // merged by the second kernel
 };
 static DecodePlan decode_plan(int B, int Hkv, int row_tiles, int Tk, int D, bool memory) {
-  static const int kKeyNs[2][4] = {{14, 18, 20, 22}, {22, 27, 27, 27}}, kFullNs[2] = {22, 28};
-  const int fit = D == 64 ? 4 : 2, wide = D == 64 ? 0 : 1;
+  static const double kKeyNs[2][4] = {{7.0, 9.1, 13.0, 21.0}, {10.5, 15.0, 26.0, 26.0}};
+  const int fit = dec_ctas(D), wide = D == 64 ? 0 : 1;
   const long long tiles = (long long)B * Hkv * row_tiles, sms = sm_count();
+  const double read_ns = 4.0 * D / 7000.0 / row_tiles;   // of a key of a CTA
   DecodePlan best = {1, false};
-  long long best_cost = -1;
+  double best_cost = -1;
   // units are what is scheduled, clusters of `ctas` or single CTAs
   auto consider = [&](int n, bool mem, long long units, long long slots, int ctas) {
-    const long long keys = (Tk + n - 1) / n, full = units / slots, rest = units % slots, round = ctas > 1 ? 3300 : 1800;
-    long long cost = full * (keys * kFullNs[wide] + round);
-    if (rest) {
-      const long long per_sm = (rest * ctas + sms - 1) / sms;
-      cost += keys * kKeyNs[wide][(per_sm < fit ? per_sm : fit) - 1] + round;
-    }
-    cost += mem ? 8000 + 60 * n : (n > 1 ? 1000 : 0);
+    const double keys = (double)((Tk + n - 1) / n);
+    auto round = [&](double running) {   // CTAs
+      const double per_sm = running * (ctas > 1 ? 1.15 : 1.0) / (double)sms;
+      const int at = per_sm <= 1 ? 0 : per_sm <= 2 ? 1 : per_sm <= 3 || fit == 3 ? 2 : 3;
+      const double read = running * read_ns, chain = kKeyNs[wide][at];
+      return keys * (read > chain ? read : chain);
+    };
+    const long long full = units / slots, rest = units % slots, rounds = full + (rest > 0);
+    double cost = full * round((double)(slots * ctas)) + (rest ? round((double)(rest * ctas)) : 0) + 4000 + 1800.0 * (rounds - 1);
+    if (rounds > 1) cost += 4 * keys;
+    cost += mem ? 9000 + 60 * n : (n > 1 ? 1000 : 0);
     if (best_cost < 0 || cost < best_cost) { best = {n, mem}; best_cost = cost; }
   };
   consider(1, false, tiles, fit * sms, 1);
@@ -453,6 +516,7 @@ extern "C" int tpb_flash_decode(const void* q, const void* k, const void* v, voi
   cudaLaunchAttribute attr[1];
   cfg.gridDim = grid;
   cfg.blockDim = dim3(kDecWarps * 32);
+  cfg.dynamicSmemBytes = dec_smem(D);
   cfg.stream = (cudaStream_t)stream;
   cfg.attrs = attr;
   cfg.numAttrs = n_splits > 1 && !p.part_o ? 1 : 0;
@@ -460,7 +524,9 @@ extern "C" int tpb_flash_decode(const void* q, const void* k, const void* v, voi
   attr[0].val.clusterDim.x = n_splits;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, D == 128 ? flash_decode_kernel<128> : flash_decode_kernel<64>, p);
+  cudaError_t e = decode_configure(D);
+  if (e != cudaSuccess) return (int)e;
+  e = cudaLaunchKernelEx(&cfg, D == 128 ? flash_decode_kernel<128> : flash_decode_kernel<64>, p);
   if (e != cudaSuccess) return (int)e;
   if (p.part_o) {
     const long long rows = (long long)B * Hkv * p.R;
