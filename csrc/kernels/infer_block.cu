@@ -44,3 +44,64 @@ extern "C" int tpb_block_post(const void* attn, const void* w_o, void* o, const 
   return tpb_gemm_bf16(act, w_down, y, nullptr, rows, hidden, inter, inter, inter, hidden, 0, 0, 0, 0, accumulate, 1.f,
                        status, stream);
 }
+
+// A forward pass of a whole decoder over a few rows (at most 128) with contiguous caches [B, Hkv, capacity, D]: embedding,
+// layers, final norm and logits by the launches that the pass makes operator by operator, issued by one call. A step of a
+// small model has some 25 kernels of 2-7 us, which the operators' Python takes three times as long to issue (one sequence,
+// 2 layers of 1024, a prompt of 37 tokens and 8 steps: 3160 us operator by operator, of which kernels 1000).
+// a: the words below, then 9 per layer.
+enum LlamaWord {
+  kLwTokens, kLwEmbed, kLwFinalNorm, kLwHead, kLwLogits, kLwCos, kLwSin, kLwPos, kLwStatus, kLwScratch, kLwPart, kLwPartLse,
+  kLwLse, kLwLseStride, kLwSplits, kLwFewRows, kLwBatch, kLwT, kLwPast, kLwHidden, kLwHq, kLwHkv, kLwD, kLwInter, kLwVocab,
+  kLwLayers, kLwHeader
+};
+enum LayerWord { kLyAttnNorm, kLyQkv, kLyO, kLyFfnNorm, kLyGateUp, kLyDown, kLyK, kLyV, kLyCap, kLyWords };
+
+// bf16 elements of scratch for `rows` rows: two residual streams, h, o, qkv, qk, attention, gate / up, activation.
+extern "C" long long tpb_llama_cached_scratch(int rows, int hidden, int Hq, int Hkv, int D, int inter) {
+  return (long long)rows * (4LL * hidden + (Hq + 2LL * Hkv) * D + (Hq + (long long)Hkv) * D + (long long)Hq * D + 3LL * inter);
+}
+
+extern "C" int tpb_llama_cached(const long long* a, float eps, float scale, void* stream) {
+  TPB_NVTX("tpb_llama_cached");
+  const int B = (int)a[kLwBatch], T = (int)a[kLwT], H = (int)a[kLwHidden], Hq = (int)a[kLwHq], Hkv = (int)a[kLwHkv];
+  const int D = (int)a[kLwD], I = (int)a[kLwInter], V = (int)a[kLwVocab], layers = (int)a[kLwLayers], rows = B * T;
+  const long long past = a[kLwPast];
+  const int Tk = (int)past + T, tot = Hq + 2 * Hkv;
+  if (rows <= 0 || rows > 128 || layers < 0) return -2;
+  auto in = [&](long long w) { return reinterpret_cast<const void*>(w); };
+  auto out = [&](long long w) { return reinterpret_cast<void*>(w); };
+  uint32_t* status = reinterpret_cast<uint32_t*>(a[kLwStatus]);
+  const float *cos_t = reinterpret_cast<const float*>(a[kLwCos]), *sin_t = reinterpret_cast<const float*>(a[kLwSin]);
+  const long long* pos = reinterpret_cast<const long long*>(a[kLwPos]);
+  float* lse = reinterpret_cast<float*>(a[kLwLse]);
+  __nv_bfloat16* next = reinterpret_cast<__nv_bfloat16*>(a[kLwScratch]);
+  auto take = [&](long long n) { __nv_bfloat16* p = next; next += rows * n; return p; };
+  __nv_bfloat16 *x = take(H), *x2 = take(H), *h = take(H), *o = take(H), *qkv = take((long long)tot * D);
+  __nv_bfloat16 *qk = take((long long)(Hq + Hkv) * D), *attn = take((long long)Hq * D), *gu = take(2LL * I), *act = take(I);
+  TPB_TRY(tpb_embedding_fwd(reinterpret_cast<const long long*>(a[kLwTokens]), in(a[kLwEmbed]), x, rows, H, V, stream));
+  for (int l = 0; l < layers; ++l) {
+    const long long* w = a + kLwHeader + l * kLyWords;
+    TPB_TRY(tpb_block_pre(x, in(w[kLyAttnNorm]), eps, in(w[kLyQkv]), h, qkv, qk, cos_t, sin_t, pos, past, rows, T, H, Hq, Hkv,
+                          D, status, stream));
+    const long long cap = w[kLyCap], qt = (long long)(Hq + Hkv) * D, vt = (long long)tot * D;   // token strides
+    TPB_TRY(tpb_kv_append2(qk + (long long)Hq * D, qkv + (long long)(Hq + Hkv) * D, out(w[kLyK]), out(w[kLyV]), (int)past, B,
+                           T, Hkv, D, T * qt, qt, D, T * vt, vt, D, Hkv * cap * D, D, cap * D, stream));
+    if (a[kLwFewRows])
+      TPB_TRY(tpb_flash_decode(qk, in(w[kLyK]), in(w[kLyV]), attn, lse, reinterpret_cast<float*>(a[kLwPart]),
+                               reinterpret_cast<float*>(a[kLwPartLse]), B, T, Tk, Hq, Hkv, D, qt, D, T * qt, D, cap * D,
+                               Hkv * cap * D, D, cap * D, Hkv * cap * D, (long long)Hq * D, D, (long long)T * Hq * D,
+                               (int)a[kLwLseStride], 1, scale, 0, (int)a[kLwSplits], stream));
+    else
+      TPB_TRY(tpb_flash_fwd_ex(qk, in(w[kLyK]), in(w[kLyV]), attn, lse, B, T, Tk, Hq, Hkv, D, qt, D, T * qt, D, cap * D,
+                               Hkv * cap * D, D, cap * D, Hkv * cap * D, (long long)Hq * D, D, (long long)T * Hq * D,
+                               (int)a[kLwLseStride], 1, scale, status, stream, nullptr, 1, 0, 0, 0, nullptr, nullptr));
+    TPB_TRY(tpb_block_post(attn, in(w[kLyO]), o, x, in(w[kLyFfnNorm]), eps, x2, h, in(w[kLyGateUp]), gu, act, in(w[kLyDown]),
+                           x2, 1, rows, H, Hq * D, I, status, stream));
+    __nv_bfloat16* t = x;
+    x = x2;
+    x2 = t;
+  }
+  TPB_TRY(tpb_rmsnorm_fwd(x, nullptr, in(a[kLwFinalNorm]), h, nullptr, nullptr, rows, H, H, H, eps, stream));
+  return tpb_gemm_bf16(h, in(a[kLwHead]), out(a[kLwLogits]), nullptr, rows, V, H, H, H, V, 0, 0, 0, 0, 0, 1.f, status, stream);
+}

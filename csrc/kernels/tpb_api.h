@@ -99,6 +99,17 @@ int tpb_layernorm_bwd(const void* dy, const void* x, const void* w, const float*
                       const float* rstd, void* dx, float* dw_part, float* db_part, float* dw_f32,
                       void* dw_bf16, float* db_f32, void* db_bf16, int accumulate, int rows, int H,
                       void* stream);
+int tpb_embedding_fwd(const long long* ids, const void* table, void* out, long long n, int H, long long V, void* stream);
+int tpb_kv_append2(const void* k, const void* v, void* k_cache, void* v_cache, int pos0, int B, int T, int H, int D,
+                   long long k_b, long long k_t, long long k_h, long long v_b, long long v_t, long long v_h, long long c_b,
+                   long long c_t, long long c_h, void* stream);
+int tpb_flash_fwd_ex(const void* q, const void* k, const void* v, void* o, float* lse, int B, int Tq, int Tk, int Hq,
+                     int Hkv, int D, long long q_tok, long long q_head, long long q_batch, long long k_tok, long long k_head,
+                     long long k_batch, long long v_tok, long long v_head, long long v_batch, long long o_tok,
+                     long long o_head, long long o_batch, int lse_stride, int causal, float scale, uint32_t* status,
+                     void* stream, const int* kv_len, int n_splits, long long o_split_stride, long long lse_split_stride,
+                     int window, const int* seg_start, const int* seg_end);
+int tpb_llama_cached(const long long* a, float eps, float scale, void* stream);
 int tpb_block_pre(const void* x, const void* norm_w, float eps, const void* w_qkv, void* h, void* qkv, void* qk,
                   const float* cos_t, const float* sin_t, const long long* pos, long long pos0, int rows, int T,
                   int hidden, int Hq, int Hkv, int D, uint32_t* status, void* stream);

@@ -90,6 +90,8 @@ _KERNEL_SIGS = {
     "tpb_roi_align_bwd": [P, P, P, I, I, I, I, I, I, I, I, F, I, I, P],
     "tpb_kv_append2": [P, P, P, P, I, I, I, I, I, LL, LL, LL, LL, LL, LL, LL, LL, LL, P],
     "tpb_block_pre": [P, P, F, P, P, P, P, P, P, P, LL, I, I, I, I, I, I, P, P],
+    "tpb_llama_cached": [P, F, F, P],
+    "tpb_llama_cached_scratch": [I] * 6,
     "tpb_block_post": [P, P, P, P, P, F, P, P, P, P, P, P, P, I, I, I, I, I, P, P],
     "tpb_decode_qkv_prep": [P, P, P, P, P, P, P, I, I, I, I, I, I, LL, LL, LL, LL, P],
     "tpb_sample": [P, P, P, P, I, I, LL, I, F, I, F, P],
@@ -117,7 +119,7 @@ def _load(name: str):
 
 
 # kernel launches issued by one call of each entry point (for launch accounting)
-_LAUNCHES = {"tpb_rmsnorm_bwd": 2, "tpb_layernorm_bwd": 2, "tpb_bias_grad": 2, "tpb_bias_grad_chunks": 0, "tpb_flash_decode_splits": 0, "tpb_block_pre": 3, "tpb_block_post": 5, "tpb_flash_bwd": 3, "tpb_rmsnorm_bwd_grid": 0,
+_LAUNCHES = {"tpb_rmsnorm_bwd": 2, "tpb_layernorm_bwd": 2, "tpb_bias_grad": 2, "tpb_bias_grad_chunks": 0, "tpb_flash_decode_splits": 0, "tpb_block_pre": 3, "tpb_block_post": 5, "tpb_llama_cached": 0, "tpb_llama_cached_scratch": 0, "tpb_flash_bwd": 3, "tpb_rmsnorm_bwd_grid": 0,
              "tpb_grouped_workspace_ints": 0, "tpb_zero": 0, "tpb_adamw_set_overlap": 0, "tpb_flash_fwd_config": 0, "tpb_gemm_set_splitk_workspace": 0, "tpb_grouped_gemm": 2}
 launch_count = 0
 

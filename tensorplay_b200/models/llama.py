@@ -9,15 +9,21 @@ modern_block.py:29-103).
 """
 from __future__ import annotations
 
+import math
+from array import array
 from dataclasses import dataclass
 from typing import Optional
 
 import torch
 from torch import Tensor, nn
 
+from torch.nn.modules import module as _nn_module
+
 from .. import _native, ops
+from ..nn.cache import DynamicCache, StaticCache
 from ..ops import _ckpt
 from ..ops._common import lib, status_word, stream_ptr, use_native
+from ..ops.attention import few_rows_sizes
 from ..ops.rope import flat_positions
 
 
@@ -66,6 +72,19 @@ class LlamaConfig:
         fwd = 2.0 * mm + 2.0 * 2 * self.num_layers * self.num_heads * self.head_dim * seq_len / 2
         mult = 1.0 + (2.0 if backward else 0.0) + (1.0 if recompute else 0.0)
         return fwd * mult
+
+
+def _watched() -> bool:
+    """Whether something watches, transforms or replaces single operators."""
+    return bool(_native.flop_sinks or _ckpt.active() or torch._C._are_functorch_transforms_active()
+                or torch._C._len_torch_dispatch_stack() or torch._C._is_torch_function_mode_enabled()
+                or torch.autograd.forward_ad._current_level >= 0 or torch.jit.is_tracing())
+
+
+def _plain(w, shape, dev) -> bool:
+    """A bf16 parameter that a kernel may read by its address."""
+    return type(w) is nn.Parameter and w.dtype is torch.bfloat16 and w.device == dev and w.shape == shape \
+        and w.is_contiguous() and not w.data_ptr() % 16
 
 
 class LlamaBlock(nn.Module):
@@ -130,9 +149,7 @@ class LlamaBlock(nn.Module):
                 or not x.is_contiguous() or x.data_ptr() % 16 or x.numel() == 0 or self.cfg.head_dim not in (64, 128) \
                 or self.cfg.hidden_size % 8 or self.cfg.ffn_size % 8:
             return False
-        if _native.flop_sinks or _ckpt.active() or torch._C._are_functorch_transforms_active() \
-                or torch._C._len_torch_dispatch_stack() or torch._C._is_torch_function_mode_enabled() \
-                or torch.autograd.forward_ad._current_level >= 0 or torch.jit.is_tracing():
+        if _watched():
             return False
         dev = x.device
         weights = self._weights()
@@ -252,12 +269,124 @@ class Llama(nn.Module):
     def forward(self, tokens: Tensor, targets: Optional[Tensor] = None,
                 position_ids: Optional[Tensor] = None, past_key_values=None) -> Tensor:
         B, T = tokens.shape
+        if past_key_values is not None and targets is None and 0 < B * T <= 128:
+            logits = self._infer_cached(tokens, position_ids, past_key_values)
+            if logits is not None:
+                return logits
         off = past_key_values.get_seq_length(0) if past_key_values is not None else 0
         cos, sin = self.rope_tables(off + T, tokens.device)
         x = self.embed_tokens(tokens)
         for layer in self.layers:
             x = layer(x, cos, sin, position_ids, past_key_values)
         return self.head(x, targets)
+
+
+    def _plain_layers(self, dev):
+        """Addresses of the layers' weights, six per layer, or None where a layer is not a plain one: another class or
+        configuration, a method of its own, a hook, a weight that is not a bf16 parameter of the configured shape."""
+        cfg = self.cfg
+        H, I, A = cfg.hidden_size, cfg.ffn_size, cfg.num_heads * cfg.head_dim
+        shapes = (("attn_norm", (H,)), ("wqkv", (A + 2 * cfg.num_kv_heads * cfg.head_dim, H)), ("wo", (H, A)),
+                  ("ffn_norm", (H,)), ("w_gate_up", (2 * I, H)), ("w_down", (H, I)))
+        found = []
+        for i, layer in enumerate(self.layers):
+            if type(layer) is not LlamaBlock or layer.cfg is not cfg or layer.layer_idx != i or layer._forward_hooks \
+                    or layer._forward_pre_hooks or layer._compiled_call_impl is not None \
+                    or not _BLOCK_METHODS.isdisjoint(layer.__dict__):
+                return None
+            own = layer._parameters
+            for name, shape in shapes:
+                w = own.get(name)
+                if not _plain(w, shape, dev):
+                    return None
+                found.append(w.data_ptr())
+        return found
+
+    def _infer_cached(self, tokens: Tensor, position_ids: Optional[Tensor], cache) -> Optional[Tensor]:
+        """The logits of a few rows over a contiguous cache by one native call, which launches what the pass launches operator
+        by operator; None where the model, its layers or the cache are not plain ones or something looks on."""
+        cfg = self.cfg
+        H, Hq, Hkv, D, I, V = cfg.hidden_size, cfg.num_heads, cfg.num_kv_heads, cfg.head_dim, cfg.ffn_size, cfg.vocab_size
+        kind = type(cache)
+        if type(self) is not Llama or (kind is not DynamicCache and kind is not StaticCache) or torch.is_grad_enabled() \
+                or type(tokens) is not Tensor or not tokens.is_cuda or tokens.dtype is not torch.int64 \
+                or D not in (64, 128) or H % 8 or I % 8 or V % 8 or Hq % Hkv or _watched() \
+                or type(self.layers) is not nn.ModuleList or _methods() != _METHODS \
+                or not _MODEL_METHODS.isdisjoint(self.__dict__) or not _CACHE_METHODS.isdisjoint(cache.__dict__) \
+                or _nn_module._global_forward_hooks or _nn_module._global_forward_pre_hooks:
+            return None
+        dev = tokens.device
+        if dev.index != torch._C._cuda_getDevice() or not use_native(tokens):
+            return None
+        own = self._parameters
+        embed, final_norm = own.get("embed"), own.get("final_norm")
+        head = own.get("lm_head")
+        if head is None and self.lm_head is None:
+            head = embed
+        if not (_plain(embed, (V, H), dev) and _plain(final_norm, (H,), dev) and _plain(head, (V, H), dev)):
+            return None
+        weights = self._plain_layers(dev)
+        if weights is None:
+            return None
+        B, T = tokens.shape
+        tokens = tokens.contiguous()
+        n_layers, rows = len(self.layers), B * T
+        past = cache.get_seq_length(0)
+        kv_shape = (B, Hkv, T, D)
+        for i in range(n_layers):
+            buf, vbuf = cache._k.get(i), cache._v.get(i)
+            if cache._len.get(i, 0) != past or (buf is not None and not (
+                    type(buf) is type(vbuf) is Tensor and buf.dtype is vbuf.dtype is torch.bfloat16 and buf.device == dev
+                    and vbuf.device == dev and buf.shape == vbuf.shape and buf.shape[0] == B and buf.shape[1] == Hkv
+                    and buf.shape[3] == D and buf.is_contiguous() and vbuf.is_contiguous())):
+                return None
+        cos, sin = self.rope_tables(past + T, dev)
+        for t in (cos, sin):
+            if type(t) is not Tensor or t.dtype is not torch.float32 or t.device != dev or not t.is_contiguous() \
+                    or t.data_ptr() % 16 or t.dim() != 2 or t.shape[1] != D // 2 or t.shape != cos.shape:
+                return None
+        pos = flat_positions(position_ids, rows, dev)
+        L, Tk = lib(), past + T
+        logits = embed.new_empty(B, T, V)
+        scratch = logits.new_empty(L.tpb_llama_cached_scratch(rows, H, Hq, Hkv, D, I))
+        few = few_rows_sizes(B, T, Tk, Hq, Hkv, D)
+        splits = L.tpb_flash_decode_splits(B, T, Tk, Hq, Hkv, D) if few and Tk > 2048 else 0
+        lse_stride = (T + 127) // 128 * 128
+        part_rows = splits * B * Hq * T   # fp32 partial rows and their sums, as the operator's
+        stats = torch.empty(B * Hq * lse_stride + part_rows * (D + 1), dtype=torch.float32, device=dev)
+        lse = stats.data_ptr()
+        part = lse + 4 * B * Hq * lse_stride if splits else 0
+        words = array("q", (
+            tokens.data_ptr(), embed.data_ptr(), final_norm.data_ptr(), head.data_ptr(), logits.data_ptr(), cos.data_ptr(),
+            sin.data_ptr(), 0 if pos is None else pos.data_ptr(), status_word(dev).data_ptr(), scratch.data_ptr(), part,
+            part + 4 * part_rows * D if splits else 0, lse, lse_stride, splits, int(few), B, T, past, H, Hq, Hkv, D, I, V,
+            n_layers))
+        for i in range(n_layers):
+            cache.room(kv_shape, kv_shape, logits, logits, i)
+            k = cache._k[i]
+            words.extend(weights[6 * i:6 * i + 6])
+            words.extend((k.data_ptr(), cache._v[i].data_ptr(), k.shape[2]))
+        _native.check(L.tpb_llama_cached(words.buffer_info()[0], cfg.rms_eps, 1.0 / math.sqrt(D), stream_ptr()),
+                      "tpb_llama_cached")
+        _native.launch_count += 3 + n_layers * (10 + (splits > 0))
+        for i in range(n_layers):
+            cache.advance(T, i)
+        return logits
+
+
+# What a pass operator by operator calls: where one of these was replaced, on a class or on an instance, it is called.
+_MODEL_METHODS = frozenset(("embed_tokens", "head", "rope_tables"))
+_BLOCK_METHODS = frozenset(("forward", "_attend_cached", "_infer_cached", "_plain_inference"))
+_CACHE_METHODS = frozenset(("update", "get_seq_length"))
+
+
+def _methods():
+    return (Llama.embed_tokens, Llama.head, LlamaBlock.__call__, LlamaBlock.forward, LlamaBlock._attend_cached,
+            LlamaBlock._infer_cached, DynamicCache.update, DynamicCache.get_seq_length, StaticCache.update,
+            StaticCache.get_seq_length, ops.embedding, ops.rms_norm, ops.linear, ops.flash_attention)
+
+
+_METHODS = _methods()
 
 
 def _embedding(tokens: Tensor, weight: Tensor) -> Tensor:

@@ -29,18 +29,28 @@ class DynamicCache(Cache):
         self._v: Dict[int, Tensor] = {}
         self._len: Dict[int, int] = {}
 
-    def update(self, key, value, layer_idx: int = 0):
+    def room(self, kshape, vshape, key: Tensor, value: Tensor, layer_idx: int = 0) -> int:
+        """Makes room in a layer's buffers for keys and values ``[B, H, T, D]`` of these shapes, in dtype and device of
+        ``key`` and ``value``, after the tokens they hold; returns the number of those. What is written there counts from :meth:`advance` on."""
         n = self._len.get(layer_idx, 0)
-        t = key.shape[2]
+        t = kshape[2]
         buf = self._k.get(layer_idx)
-        if buf is None or buf.shape[2] < n + t or buf.shape[0] != key.shape[0]:
+        if buf is None or buf.shape[2] < n + t or buf.shape[0] != kshape[0]:
             cap = max(2 * (n + t), 64)
-            nk = key.new_empty(key.shape[0], key.shape[1], cap, key.shape[3])
-            nv = value.new_empty(value.shape[0], value.shape[1], cap, value.shape[3])
+            nk = key.new_empty(kshape[0], kshape[1], cap, kshape[3])
+            nv = value.new_empty(vshape[0], vshape[1], cap, vshape[3])
             if buf is not None and n:
                 nk[:, :, :n] = buf[:, :, :n]
                 nv[:, :, :n] = self._v[layer_idx][:, :, :n]
             self._k[layer_idx], self._v[layer_idx] = nk, nv
+        return n
+
+    def advance(self, t: int, layer_idx: int = 0) -> None:
+        self._len[layer_idx] = self._len.get(layer_idx, 0) + t
+
+    def update(self, key, value, layer_idx: int = 0):
+        n = self.room(key.shape, value.shape, key, value, layer_idx)
+        t = key.shape[2]
         if key.is_cuda and key.dtype == torch.bfloat16:
             kv_append_pair(self._k[layer_idx], self._v[layer_idx], key, value, n)
         else:
@@ -62,15 +72,24 @@ class StaticCache(Cache):
         self._v: Dict[int, Tensor] = {}
         self._len: Dict[int, int] = {}
 
-    def update(self, key, value, layer_idx: int = 0):
+    def room(self, kshape, vshape, key: Tensor, value: Tensor, layer_idx: int = 0) -> int:
+        """As :meth:`DynamicCache.room`."""
         n = self._len.get(layer_idx, 0)
-        t = key.shape[2]
+        t = kshape[2]
         if n + t > self.max_seq_len:
             raise ValueError(f"StaticCache overflow: {n + t} > {self.max_seq_len}")
         if layer_idx not in self._k:
-            shape = (key.shape[0], key.shape[1], self.max_seq_len, key.shape[3])
+            shape = (kshape[0], kshape[1], self.max_seq_len, kshape[3])
             self._k[layer_idx] = key.new_zeros(shape)
             self._v[layer_idx] = value.new_zeros(shape)
+        return n
+
+    def advance(self, t: int, layer_idx: int = 0) -> None:
+        self._len[layer_idx] = self._len.get(layer_idx, 0) + t
+
+    def update(self, key, value, layer_idx: int = 0):
+        n = self.room(key.shape, value.shape, key, value, layer_idx)
+        t = key.shape[2]
         if key.is_cuda and key.dtype == torch.bfloat16:
             kv_append_pair(self._k[layer_idx], self._v[layer_idx], key, value, n)
         else:

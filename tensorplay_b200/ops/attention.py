@@ -69,9 +69,12 @@ def _few_rows(q, k, v) -> bool:
     splits the keys over the chip; at 64 rows (Tq = 8, groups of 8) the four reads through L2 are still half of those,
     and beyond 16 tokens the tensor-core tiles fill up."""
     B, Tq, Hq, D = q.shape
-    Tk, Hkv = k.shape[1], k.shape[2]
+    return q.dtype == torch.bfloat16 and few_rows_sizes(B, Tq, k.shape[1], Hq, k.shape[2], D)
+
+
+def few_rows_sizes(B: int, Tq: int, Tk: int, Hq: int, Hkv: int, D: int) -> bool:
     rows = Tq * (Hq // Hkv)
-    return (Tq <= 16 and 0 < rows <= 64 and (D == 128 or D == 64) and q.dtype == torch.bfloat16 and Hq % Hkv == 0
+    return (Tq <= 16 and 0 < rows <= 64 and (D == 128 or D == 64) and Hq % Hkv == 0
             and 0 < B <= 65535 and Hkv * ((rows + 15) // 16) <= 65535 and Tk > 0)
 
 
