@@ -18,6 +18,7 @@ embedding_fwd_kernel(const long long* __restrict__ ids, const __nv_bfloat16* __r
                      __nv_bfloat16* __restrict__ out, long long n, int H, long long V) {
   const int vec_per_row = H / 8;
   const long long total = n * vec_per_row;
+  chain_next();
   for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < total; i += (long long)gridDim.x * 256) {
     const long long r = i / vec_per_row;
     const int c = (int)(i - r * vec_per_row);
@@ -68,6 +69,8 @@ struct KvAppendParams {
 // blockIdx.y selects one of two appends (keys and values of a step in one launch).
 __global__ void __launch_bounds__(256) kv_append_kernel(const KvAppendParams p0, const KvAppendParams p1) {
   const KvAppendParams& p = blockIdx.y ? p1 : p0;
+  chain_next();
+  chain_wait();
   const int vec = p.D / 8;
   const long long total = (long long)p.B * p.T * p.H * vec;
   for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < total; i += (long long)gridDim.x * 256) {
@@ -87,7 +90,7 @@ __global__ void __launch_bounds__(256) kv_append_kernel(const KvAppendParams p0,
     } else {
       off = (long long)b * p.d_b + (long long)at * p.d_t;
     }
-    const uint4 v = *(reinterpret_cast<const uint4*>(p.src + b * p.s_b + t * p.s_t + h * p.s_h) + c);
+    const uint4 v = chain_ld(reinterpret_cast<const uint4*>(p.src + b * p.s_b + t * p.s_t + h * p.s_h) + c);
     *(reinterpret_cast<uint4*>(p.dst + off + h * p.d_h) + c) = v;
   }
 }
@@ -390,8 +393,7 @@ static int kv_append_params(KvAppendParams* out, const void* src, void* dst, con
 static int kv_append_launch(const KvAppendParams& a, const KvAppendParams& b, int n, void* stream) {
   const long long total = (long long)a.B * a.T * a.H * (a.D / 8);
   const int grid = (int)((total + 255) / 256 < 148 * 16 ? (total + 255) / 256 : 148 * 16);
-  kv_append_kernel<<<dim3(grid, n), 256, 0, static_cast<cudaStream_t>(stream)>>>(a, b);
-  return (int)cudaGetLastError();
+  return (int)launch_chained(kv_append_kernel, dim3(grid, n), 256, static_cast<cudaStream_t>(stream), a, b);
 }
 
 // Keys and values of the same shape into contiguous caches of the same strides at token pos0, in one launch.

@@ -85,6 +85,8 @@ flash_decode_kernel(const DecodeParams p) {
   const int gq = lane >> 2, t = lane & 3;
   const int split = blockIdx.x, hk = blockIdx.y / p.row_tiles, rt = blockIdx.y % p.row_tiles, b = blockIdx.z;
 
+  chain_next();
+  chain_wait();
   int k_begin = split * p.keys_per_split;
   const int k_end = min(p.Tk, k_begin + p.keys_per_split);
   if (p.window > 0) {
@@ -513,17 +515,22 @@ extern "C" int tpb_flash_decode(const void* q, const void* k, const void* v, voi
   if ((long long)Hkv * p.row_tiles > 65535) return -2;
   const dim3 grid(n_splits, Hkv * p.row_tiles, B);
   cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   cfg.gridDim = grid;
   cfg.blockDim = dim3(kDecWarps * 32);
   cfg.dynamicSmemBytes = dec_smem(D);
   cfg.stream = (cudaStream_t)stream;
   cfg.attrs = attr;
-  cfg.numAttrs = n_splits > 1 && !p.part_o ? 1 : 0;
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = n_splits;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
+  if (t_chained) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (n_splits > 1 && !p.part_o) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+    attr[cfg.numAttrs].val.clusterDim.x = n_splits;
+    attr[cfg.numAttrs].val.clusterDim.y = 1;
+    attr[cfg.numAttrs++].val.clusterDim.z = 1;
+  }
   cudaError_t e = decode_configure(D);
   if (e != cudaSuccess) return (int)e;
   e = cudaLaunchKernelEx(&cfg, D == 128 ? flash_decode_kernel<128> : flash_decode_kernel<64>, p);

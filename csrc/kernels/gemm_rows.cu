@@ -61,6 +61,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant_
   const int kb0 = rank * per + min(rank, rem);
   const int n_kb = per + (rank < rem ? 1 : 0);   // the host keeps csize <= k_blocks
 
+  chain_next();
   if (threadIdx.x == 0) {
     *abort_w = 0;
     for (int i = 0; i < S; ++i) {
@@ -84,12 +85,9 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant_
 
   if (warp == 0) {
     if (lane == 0) {
-      for (int it = 0; it < n_kb; ++it) {
-        const int s = it % S;
-        if (!mbar_wait_relaxed(&empty[s], ((it / S) & 1) ^ 1, wc, 1)) break;
+      auto load_b = [&](int it) {
+        const int s = it % S, k = (kb0 + it) * kRowsK;
         uint8_t* sp = smem + s * Cfg::kStageBytes;
-        uint8_t* sq = sp + kRowsBBytes;
-        const int k = (kb0 + it) * kRowsK;
         mbar_arrive_expect_tx(&full[s], Cfg::kStageBytes);
         if (!B_MN) {
           tma_load_2d(sp, &tmB, &full[s], k, n0);
@@ -97,12 +95,25 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant_
 #pragma unroll
           for (int c = 0; c < 2; ++c) tma_load_2d(sp + c * (kRowsK * 128), &tmB, &full[s], n0 + c * 64, k);
         }
-        tma_load_2d(sq, &tmA, &full[s], k, 0);
+      };
+      // In a chain the weights are nobody's output: a ring of them is requested while the kernel before still runs.
+      const int ahead = min(S, n_kb);
+      for (int it = 0; it < ahead; ++it) load_b(it);
+      chain_wait();
+      for (int it = 0; it < n_kb; ++it) {
+        const int s = it % S;
+        if (it >= ahead) {
+          if (!mbar_wait_relaxed(&empty[s], ((it / S) & 1) ^ 1, wc, 1)) break;
+          load_b(it);
+        }
+        tma_load_2d(smem + s * Cfg::kStageBytes + kRowsBBytes, &tmA, &full[s], (kb0 + it) * kRowsK, 0);
       }
     }
+    chain_wait();
     __syncwarp();
   } else if (warp == 1) {
     // warp-uniform control flow, one elected lane issues (tcgen05 operands live in uniform registers)
+    chain_wait();
     constexpr uint32_t idesc = make_idesc_f16(128, NT, 1, B_MN ? 1 : 0, 0);
     constexpr uint32_t hi = smem_desc_hi(1024);
     const uint32_t p_lo0 = smem_desc_lo(smem_u32(smem), B_MN ? kRowsK * 128 : 16);
@@ -126,6 +137,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant_
   } else {
     // drain the accumulator into the ring (every load has landed and every MMA has read it once `done` completes)
     const int q = warp & 3;
+    chain_wait();
     if (mbar_wait_warp(done, 0, wc, 3)) {
       tc_fence_after_sync();
       const int row = q * 32 + lane;
@@ -221,10 +233,15 @@ template <int NT, bool B_MN>
 static int launch_rows(const CUtensorMap& tb, const CUtensorMap& ta, const RowsParams& p, cudaStream_t stream) {
   const int tiles = (p.N + 127) / 128;
   cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   cudaError_t e = rows_config<NT, B_MN>(&cfg, attr, rows_cluster<NT, B_MN>(tiles, (p.K + kRowsK - 1) / kRowsK), tiles);
   if (e != cudaSuccess) return (int)e;
   cfg.stream = stream;
+  if (t_chained) {
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.numAttrs = 2;
+  }
   return (int)cudaLaunchKernelEx(&cfg, gemm_rows_kernel<NT, B_MN>, tb, ta, p);
 }
 

@@ -6,6 +6,16 @@
 #include "sm100.cuh"
 #include "tpb_api.h"
 
+namespace tpb {
+thread_local bool t_chained = false;
+namespace {
+struct Chain {   // the launches of this thread follow one another early, until the end of the scope
+  Chain() { t_chained = true; }
+  ~Chain() { t_chained = false; }
+};
+}  // namespace
+}  // namespace tpb
+
 #define TPB_TRY(call)          \
   do {                         \
     const int r_ = (call);     \
@@ -80,6 +90,10 @@ extern "C" int tpb_llama_cached(const long long* a, float eps, float scale, void
   __nv_bfloat16 *x = take(H), *x2 = take(H), *h = take(H), *o = take(H), *qkv = take((long long)tot * D);
   __nv_bfloat16 *qk = take((long long)(Hq + Hkv) * D), *attn = take((long long)Hq * D), *gu = take(2LL * I), *act = take(I);
   TPB_TRY(tpb_embedding_fwd(reinterpret_cast<const long long*>(a[kLwTokens]), in(a[kLwEmbed]), x, rows, H, V, stream));
+  // From here on each kernel starts while the one before still runs, and the products request their weights meanwhile. The
+  // kernels without a part in this (products of more rows, prompts' attention) are launched and waited for as usual.
+  // The pass of the figures above took 1340 us with launches that wait for one another, 955 so, of which the host 950.
+  const tpb::Chain chain;
   for (int l = 0; l < layers; ++l) {
     const long long* w = a + kLwHeader + l * kLyWords;
     TPB_TRY(tpb_block_pre(x, in(w[kLyAttnNorm]), eps, in(w[kLyQkv]), h, qkv, qk, cos_t, sin_t, pos, past, rows, T, H, Hq, Hkv,

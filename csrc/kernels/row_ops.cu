@@ -107,8 +107,9 @@ template <int TPR, int VPT>
 constexpr int fold_floats() { return TPR == kRowThreads ? 4 : kRowThreads * VPT * 8; }
 
 // ------------------------------------------------------------------ RMSNorm forward
-// y = (x [+ res]) * rstd * w ; optionally writes the summed residual stream back (res_out).
-template <int TPR, int VPT>
+// y = (x [+ res]) * rstd * w ; optionally writes the summed residual stream back (res_out). Many rows outside of a chain keep
+// the read-only loads, which the compiler orders more freely (30001 rows of 768 18.7 us against 20.6).
+template <int TPR, int VPT, bool CHAINED>
 __global__ void __launch_bounds__(kRowThreads)
 rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ res,
                    const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y,
@@ -118,6 +119,15 @@ rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
   constexpr int RPB = kRowThreads / TPR;
   const int t = threadIdx.x % TPR;
   const int nvec = H / 8;
+  if (CHAINED) {
+    chain_next();
+    chain_wait();
+  }
+  auto load = [](const __nv_bfloat16* p, int v) {
+    const uint4* q = reinterpret_cast<const uint4*>(p) + v;
+    if constexpr (CHAINED) return chain_ld(q);
+    else return *q;
+  };
   for (long long row0 = (long long)blockIdx.x * RPB; row0 < rows; row0 += (long long)gridDim.x * RPB) {
     const long long row = row0 + threadIdx.x / TPR;
     const bool live = row < rows;
@@ -127,12 +137,12 @@ rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
     for (int i = 0; i < VPT; ++i) {
       int v = t + i * TPR;
       if (live && v < nvec) {
-        uint4 a = reinterpret_cast<const uint4*>(x + row * x_stride)[v];
+        uint4 a = load(x + row * x_stride, v);
         float f[8];
         unpack8(a, f);
         if (res) {
           float g[8];
-          unpack8(reinterpret_cast<const uint4*>(res + row * (long long)H)[v], g);
+          unpack8(load(res + row * (long long)H, v), g);
 #pragma unroll
           for (int j = 0; j < 8; ++j) f[j] += g[j];
           a = pack8(f);
@@ -470,6 +480,8 @@ rope_kernel(const __nv_bfloat16* x, __nv_bfloat16* y, const float* __restrict__ 
   const int vec_per_head = half / 8;  // NeoX: 8 pairs per thread from both halves
   const Idx idx = (Idx)blockIdx.x * 256 + threadIdx.x;
   const Idx total = (Idx)tokens * heads * vec_per_head;
+  chain_next();
+  chain_wait();
   if (idx >= total) return;
   const Idx th = idx / (Idx)vec_per_head;
   const int v = (int)(idx - th * vec_per_head);
@@ -482,8 +494,8 @@ rope_kernel(const __nv_bfloat16* x, __nv_bfloat16* y, const float* __restrict__ 
   const float* c = cos_t + p * half;
   const float* s = sin_t + p * half;
   if (!interleaved) {
-    uint4 a = reinterpret_cast<const uint4*>(base)[v];
-    uint4 b = reinterpret_cast<const uint4*>(base + half)[v];
+    uint4 a = chain_ld(reinterpret_cast<const uint4*>(base) + v);
+    uint4 b = chain_ld(reinterpret_cast<const uint4*>(base + half) + v);
     float af[8], bf[8], oa[8], ob[8];
     unpack8(a, af);
     unpack8(b, bf);
@@ -505,7 +517,7 @@ rope_kernel(const __nv_bfloat16* x, __nv_bfloat16* y, const float* __restrict__ 
     // 16 consecutive elements = 8 (even, odd) pairs: two vectors per thread
 #pragma unroll
     for (int q = 0; q < 2; ++q) {
-      uint4 a = reinterpret_cast<const uint4*>(base)[v * 2 + q];
+      uint4 a = chain_ld(reinterpret_cast<const uint4*>(base) + v * 2 + q);
       float f[8], o[8];
       unpack8(a, f);
 #pragma unroll
@@ -532,6 +544,8 @@ swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gate, const __nv_bfloat16* _
                   __nv_bfloat16* __restrict__ out, long long rows, int I, long long in_stride,
                   const int* __restrict__ rows_dev) {
   const Idx nvec = I / 8;
+  chain_next();
+  chain_wait();
   if (rows_dev) rows = min(rows, (long long)*rows_dev);  // row count known only on the device (ragged buffers)
   const Idx total = (Idx)rows * nvec;
   const Idx i0 = (Idx)blockIdx.x * (256 * kActVecs) + threadIdx.x;
@@ -542,8 +556,8 @@ swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gate, const __nv_bfloat16* _
     if (idx >= total) break;
     const Idx r = idx / nvec;
     const int v = (int)(idx - r * nvec);
-    gv[k] = reinterpret_cast<const uint4*>(gate + (long long)r * in_stride)[v];
-    uv[k] = reinterpret_cast<const uint4*>(up + (long long)r * in_stride)[v];
+    gv[k] = chain_ld(reinterpret_cast<const uint4*>(gate + (long long)r * in_stride) + v);
+    uv[k] = chain_ld(reinterpret_cast<const uint4*>(up + (long long)r * in_stride) + v);
   }
 #pragma unroll
   for (int k = 0; k < kActVecs; ++k) {
@@ -849,11 +863,13 @@ extern "C" int tpb_rmsnorm_fwd(const void* x, const void* res, const void* w, vo
   if (rows <= 0) return 0;
   int tpr = pick_tpr(H);
   int grid = ((long long)rows + kRowThreads / tpr - 1) / (kRowThreads / tpr);
-  TPB_ROW_SWITCH(tpr, pick_vpt(H, tpr), (rmsnorm_fwd_kernel<TPR, VPT><<<grid, kRowThreads, 0, (cudaStream_t)stream>>>(
+  cudaError_t e = cudaSuccess;
+  TPB_ROW_SWITCH(tpr, pick_vpt(H, tpr), (e = launch_chained(
+                          t_chained ? rmsnorm_fwd_kernel<TPR, VPT, true> : rmsnorm_fwd_kernel<TPR, VPT, false>, dim3(grid), kRowThreads, (cudaStream_t)stream,
                           (const __nv_bfloat16*)x, (const __nv_bfloat16*)res,
                           (const __nv_bfloat16*)w, (__nv_bfloat16*)y, (__nv_bfloat16*)res_out, rstd,
                           rows, H, x_stride, y_stride, eps)));
-  return (int)cudaGetLastError();
+  return (int)e;
 }
 
 extern "C" int tpb_rmsnorm_bwd_grid(int rows, int H) {
@@ -946,10 +962,9 @@ extern "C" int tpb_rope_out(const void* x, void* y, const float* cos_t, const fl
   if (total <= 0) return 0;
   int grid = (int)((total + 255) / 256);
   auto kern = total < 0x7ff00000LL ? rope_kernel<unsigned> : rope_kernel<unsigned long long>;
-  kern<<<grid, 256, 0, (cudaStream_t)stream>>>(
+  return (int)launch_chained(kern, dim3(grid), 256, (cudaStream_t)stream,
       (const __nv_bfloat16*)x, (__nv_bfloat16*)y, cos_t, sin_t, pos, tokens, heads, D, tok_stride,
       head_stride, y_tok_stride, y_head_stride, seq_len, interleaved, backward ? -1.f : 1.f);
-  return (int)cudaGetLastError();
 }
 extern "C" int tpb_rope(void* x, const float* cos_t, const float* sin_t, const long long* pos,
                         long long tokens, int heads, int D, long long tok_stride,
@@ -970,10 +985,9 @@ extern "C" int tpb_swiglu_fwd_n(const void* gate, const void* up, void* out, lon
   long long total = rows * (I / 8);
   if (total <= 0) return 0;
   auto kern = total < 0x7ff00000LL ? swiglu_fwd_kernel<unsigned> : swiglu_fwd_kernel<unsigned long long>;
-  kern<<<(unsigned)((total + 256 * kActVecs - 1) / (256 * kActVecs)), 256, 0, (cudaStream_t)stream>>>(
+  return (int)launch_chained(kern, dim3((unsigned)((total + 256 * kActVecs - 1) / (256 * kActVecs))), 256, (cudaStream_t)stream,
       (const __nv_bfloat16*)gate, (const __nv_bfloat16*)up, (__nv_bfloat16*)out, rows, I,
       in_stride, rows_dev);
-  return (int)cudaGetLastError();
 }
 extern "C" int tpb_swiglu_fwd(const void* gate, const void* up, void* out, long long rows, int I,
                               long long in_stride, void* stream) {

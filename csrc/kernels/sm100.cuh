@@ -128,6 +128,36 @@ __device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
   return ok != 0;
 }
 
+// ---------------------------------------------------------------- launches that start early
+// A chain of launches (see launch_chained) starts each kernel while the one before still runs. A kernel of a chain calls
+// chain_next() at its start, which lets the next one's CTAs in as soon as all of its own have started, and chain_wait()
+// in every thread before it touches what an earlier kernel of the chain reads or writes; what no kernel of the chain
+// writes (weights, tables) it may load before. It then reads with chain_ld: a read-only load may be moved above the wait.
+__device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ uint4 chain_ld(const void* p) {
+  uint4 r;
+  asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(p));
+  return r;
+}
+
+// Host side: whether the launches of this thread belong to a chain whose first kernel was launched; set for the extent of a
+// native call that issues a chain.
+extern thread_local bool t_chained;
+template <typename... Params, typename... Args>
+inline cudaError_t launch_chained(void (*kern)(Params...), dim3 grid, int threads, cudaStream_t stream, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.stream = stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = t_chained ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kern, static_cast<Params>(args)...);
+}
+
 // Shared per-CTA abort word + global status word used by all bounded waits.
 struct WaitCtx {
   volatile uint32_t* abort_smem;  // set to 1 once any wait in the CTA gave up

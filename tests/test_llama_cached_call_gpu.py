@@ -137,3 +137,36 @@ def test_full_static_cache_raises():
         with pytest.raises(ValueError):
             m(tok[:, 8:].contiguous(), past_key_values=cache)
     assert cache.get_seq_length(0) == 8
+
+
+@pytest.mark.parametrize("B", [1, 5, 40])
+def test_chained_launches_repeat(B):
+    """Kernels of the call start before the ones they depend on have ended: many steps, back to back, bit by bit."""
+    m = _model(64, max_seq_len=256)
+    tok = torch.randint(0, 520, (B, 70), device=DEV)
+    cuts = tuple(range(3, 71))
+    fast = [_run(m, tok, cuts, DynamicCache()) for _ in range(3)]
+    m.layers[0].register_forward_hook(lambda *a: None)
+    slow = _run(m, tok, cuts, DynamicCache())
+    O.check_status()
+    for run in fast:
+        for f, s in zip(run, slow):
+            assert torch.equal(f, s)
+
+
+def test_capture():
+    m, cache = _model(128, max_seq_len=256), StaticCache(64)
+    tok = torch.randint(0, 520, (3, 21), device=DEV)
+    want = _run(m, tok, (20, 21), cache)[1].clone()
+    with torch.no_grad():
+        for i in range(2):
+            cache._len[i] = 20
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            got = m(tok[:, 20:], past_key_values=cache)
+        for _ in range(3):
+            got.zero_()
+            graph.replay()
+            torch.cuda.synchronize()
+            assert torch.equal(got, want)
+    O.check_status()
