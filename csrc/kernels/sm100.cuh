@@ -221,6 +221,11 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, c
   return __all_sync(0xffffffffu, ok);
 }
 
+__device__ __forceinline__ bool mbar_wait_relaxed_warp(uint64_t* bar, uint32_t parity, const WaitCtx& w, uint32_t where) {
+  bool ok = mbar_wait_relaxed(bar, parity, w, where);
+  return __all_sync(0xffffffffu, ok);
+}
+
 // Bounded wait on a 32-bit flag in global (possibly peer) memory reaching >= want.
 __device__ __forceinline__ uint32_t ld_acquire_sys(const uint32_t* p) {
   uint32_t v;

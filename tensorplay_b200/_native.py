@@ -74,6 +74,8 @@ _KERNEL_SIGS = {
     "tpb_clip_coef": [P, F, P, P, P],
     "tpb_gemm_i8": [P, P, P, P, P, P, I, I, I, I, I, I, P, P],
     "tpb_wq_gemv": [P, P, P, P, P, P, I, I, I, I, I, LL, LL, P],
+    "tpb_wq_gemm_pays": [I] * 5,
+    "tpb_wq_gemm": [P, P, P, P, P, P, I, I, I, I, I, LL, LL, P, P],
     "tpb_wq_gemv_config": [I, I],
     "tpb_lif_fwd": [P, P, P, P, I, LL, F, F, F, I, P],
     "tpb_lif_bwd": [P, P, P, P, I, LL, F, F, F, F, I, I, P],
@@ -119,7 +121,7 @@ def _load(name: str):
 
 
 # kernel launches issued by one call of each entry point (for launch accounting)
-_LAUNCHES = {"tpb_rmsnorm_bwd": 2, "tpb_layernorm_bwd": 2, "tpb_bias_grad": 2, "tpb_bias_grad_chunks": 0, "tpb_flash_decode_splits": 0, "tpb_block_pre": 3, "tpb_block_post": 5, "tpb_llama_cached": 0, "tpb_llama_cached_scratch": 0, "tpb_flash_bwd": 3, "tpb_rmsnorm_bwd_grid": 0,
+_LAUNCHES = {"tpb_rmsnorm_bwd": 2, "tpb_layernorm_bwd": 2, "tpb_bias_grad": 2, "tpb_bias_grad_chunks": 0, "tpb_flash_decode_splits": 0, "tpb_block_pre": 3, "tpb_block_post": 5, "tpb_llama_cached": 0, "tpb_llama_cached_scratch": 0, "tpb_wq_gemm_pays": 0, "tpb_flash_bwd": 3, "tpb_rmsnorm_bwd_grid": 0,
              "tpb_grouped_workspace_ints": 0, "tpb_zero": 0, "tpb_adamw_set_overlap": 0, "tpb_flash_fwd_config": 0, "tpb_gemm_set_splitk_workspace": 0, "tpb_grouped_gemm": 2}
 launch_count = 0
 

@@ -21,8 +21,7 @@ from torch.nn.modules import module as _nn_module
 
 from .. import _native, ops
 from ..nn.cache import DynamicCache, StaticCache
-from ..ops import _ckpt
-from ..ops._common import lib, status_word, stream_ptr, use_native
+from ..ops._common import lib, status_word, stream_ptr, use_native, watched
 from ..ops.attention import few_rows_sizes
 from ..ops.rope import flat_positions
 
@@ -72,13 +71,6 @@ class LlamaConfig:
         fwd = 2.0 * mm + 2.0 * 2 * self.num_layers * self.num_heads * self.head_dim * seq_len / 2
         mult = 1.0 + (2.0 if backward else 0.0) + (1.0 if recompute else 0.0)
         return fwd * mult
-
-
-def _watched() -> bool:
-    """Whether something watches, transforms or replaces single operators."""
-    return bool(_native.flop_sinks or _ckpt.active() or torch._C._are_functorch_transforms_active()
-                or torch._C._len_torch_dispatch_stack() or torch._C._is_torch_function_mode_enabled()
-                or torch.autograd.forward_ad._current_level >= 0 or torch.jit.is_tracing())
 
 
 def _plain(w, shape, dev) -> bool:
@@ -149,7 +141,7 @@ class LlamaBlock(nn.Module):
                 or not x.is_contiguous() or x.data_ptr() % 16 or x.numel() == 0 or self.cfg.head_dim not in (64, 128) \
                 or self.cfg.hidden_size % 8 or self.cfg.ffn_size % 8:
             return False
-        if _watched():
+        if watched():
             return False
         dev = x.device
         weights = self._weights()
@@ -310,7 +302,7 @@ class Llama(nn.Module):
         kind = type(cache)
         if type(self) is not Llama or (kind is not DynamicCache and kind is not StaticCache) or torch.is_grad_enabled() \
                 or type(tokens) is not Tensor or not tokens.is_cuda or tokens.dtype is not torch.int64 \
-                or D not in (64, 128) or H % 8 or I % 8 or V % 8 or Hq % Hkv or _watched() \
+                or D not in (64, 128) or H % 8 or I % 8 or V % 8 or Hq % Hkv or watched() \
                 or type(self.layers) is not nn.ModuleList or _methods() != _METHODS \
                 or not _MODEL_METHODS.isdisjoint(self.__dict__) or not _CACHE_METHODS.isdisjoint(cache.__dict__) \
                 or _nn_module._global_forward_hooks or _nn_module._global_forward_pre_hooks:

@@ -4,6 +4,7 @@ from __future__ import annotations
 import torch
 
 from .. import _native
+from . import _ckpt
 
 
 def use_native(*tensors: torch.Tensor) -> bool:
@@ -29,6 +30,13 @@ def stream_ptr() -> int:
     """Handle of the current stream of the current device (without building a ``torch.cuda.Stream``: 0.3 instead of
     2.5 us, paid by every launch)."""
     return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+
+
+def watched() -> bool:
+    """Whether something watches, transforms or replaces single operators."""
+    return bool(_native.flop_sinks or _ckpt.active() or torch._C._are_functorch_transforms_active()
+                or torch._C._len_torch_dispatch_stack() or torch._C._is_torch_function_mode_enabled()
+                or torch.autograd.forward_ad._current_level >= 0 or torch.jit.is_tracing())
 
 
 def ptr(t):

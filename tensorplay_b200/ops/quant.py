@@ -13,7 +13,7 @@ import torch
 from torch import Tensor
 
 from .. import _native
-from ._common import lib, ptr, status_word, stream_ptr, use_native
+from ._common import lib, ptr, status_word, stream_ptr, use_native, watched
 
 _FP8 = {torch.float8_e4m3fn: 0, torch.float8_e5m2: 1}
 _FP8_MAX = {torch.float8_e4m3fn: 448.0, torch.float8_e5m2: 57344.0}
@@ -110,12 +110,23 @@ def dequantize_weight(q: Tensor, scale: Tensor, zero: Optional[Tensor] = None, b
 
 def weight_only_linear(x: Tensor, q: Tensor, scale: Tensor, zero: Optional[Tensor] = None,
                        bias: Optional[Tensor] = None, bits: int = 8, group_size: int = 0) -> Tensor:
-    """``x @ dequant(q).T + bias``. Up to 16 rows of ``x`` (decode) stream the packed weights once in
-    a GEMV kernel; larger inputs dequantise and use the bf16 tensor-core GEMM."""
+    """``x @ dequant(q).T + bias``. Up to 16 rows of ``x`` (decode) stream the packed weights once per 8 rows in a GEMV
+    kernel; more go, where that is faster, through a tensor-core kernel that converts the weights on their way, and
+    otherwise dequantise and use the bf16 GEMM."""
     from .gemm import linear
     K = x.shape[-1]
     x2 = x.reshape(-1, K)
     M, N = x2.shape[0], q.shape[0]
+    if M > 16 and _converts_on_the_way(x2, q, scale, zero, bias, N, K, bits, group_size):
+        if x2.stride(1) != 1 or x2.stride(0) % 8 or x2.data_ptr() % 16:
+            x2 = x2.contiguous()
+        y = torch.empty(M, N, dtype=torch.bfloat16, device=x.device)
+        sc, qc = scale.to(torch.bfloat16).contiguous(), q.contiguous()
+        z = None if zero is None else zero.to(torch.bfloat16).contiguous()
+        b = None if bias is None else bias.detach().contiguous()
+        _native.check(lib().tpb_wq_gemm(ptr(x2), ptr(qc), ptr(sc), ptr(z), ptr(b), ptr(y), M, N, K, bits, group_size,
+                                        x2.stride(0), N, status_word(x.device).data_ptr(), stream_ptr()), "tpb_wq_gemm")
+        return y.view(*x.shape[:-1], N)
     if (use_native(x2, q) and x2.dtype == torch.bfloat16 and M <= 16 and K % 16 == 0
             and (group_size % 16 == 0 if group_size > 0 else bits == 8)):
         if x2.stride(1) != 1 or x2.stride(0) % 8:
@@ -129,6 +140,19 @@ def weight_only_linear(x: Tensor, q: Tensor, scale: Tensor, zero: Optional[Tenso
         return y.view(*x.shape[:-1], N)
     w = dequantize_weight(q, scale, zero, bits, group_size)
     return linear(x, w.to(x.dtype), bias)
+
+
+def _converts_on_the_way(x2, q, scale, zero, bias, N: int, K: int, bits: int, group_size: int) -> bool:
+    """Plain operands of a product without gradients, of the sizes that the kernel takes and is the fastest for."""
+    if type(x2) is not Tensor or x2.dtype != torch.bfloat16 or not use_native(x2, q, scale) \
+            or q.shape != (N, K * bits // 8) or q.dtype not in (torch.uint8, torch.int8) or q.data_ptr() % 16 \
+            or (zero is not None and not zero.is_cuda) or scale.numel() != N * (K // group_size if group_size > 0 else 1) \
+            or (zero is not None and zero.numel() != scale.numel()) \
+            or (bias is not None and (bias.dtype != torch.bfloat16 or not bias.is_cuda or bias.shape != (N,))):
+        return False
+    if torch.is_grad_enabled() and (x2.requires_grad or (bias is not None and bias.requires_grad)):
+        return False
+    return not watched() and bool(lib().tpb_wq_gemm_pays(x2.shape[0], N, K, bits, group_size))
 
 
 def gemv_config(tiles: int = 0, force_simt: bool = False, version: int = 2, fold: bool = True) -> None:
