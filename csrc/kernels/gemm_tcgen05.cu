@@ -390,7 +390,6 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         int tm, tn;
         tile_coords(tile, tiles_m, tiles_n, tm, tn);
         tm = (tm + p.tile_m_shift) % tiles_m;
-      tn = (tn + p.tile_n_shift) % tiles_n;
         tn = (tn + p.tile_n_shift) % tiles_n;
         if (p.ag_operand) {
           ok = ag_wait_rows(p, p.ag_operand == 1 ? tm * kBlockM : tn * BLOCK_N,
