@@ -225,7 +225,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer (every CTA, own halves)
-    if (lane == 0) {
+    // (warp-uniform control flow, one elected lane issues: operands of the copies live in uniform registers, too)
+    {
       uint32_t it = 0;
       bool ok = true;
       for (int wi = 0; ok && pair_work(sc, pair, wi, w); ++wi) {
@@ -236,31 +237,34 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         for (int kb = w.kb0; kb < w.kb1; ++kb, ++it) {
           const int s = it % kPairStages;
           const uint32_t ph = (it / kPairStages) & 1;
-          if (!mbar_wait_relaxed(&empty[s], ph ^ 1, wc, 1)) { ok = false; break; }
-          pair_stamp(p, pair, crank ? 3 : 0, it);
-          uint8_t* sa = smem + s * kPairStageBytes;
-          uint8_t* sb = sa + kPairABytes;
-          if (crank == 0) mbar_arrive_expect_tx(&full[s], 2 * kPairStageBytes);
-          const uint32_t fb = mapa_u32(&full[s], 0);
-          if (!A_MN) {
-            tma_load_2d_pair(sa, &tmA, fb, kb * kPairK, row0);
-          } else {
+          if (!mbar_wait_relaxed_warp(&empty[s], ph ^ 1, wc, 1)) { ok = false; break; }
+          if (elect_one()) {
+            pair_stamp(p, pair, crank ? 3 : 0, it);
+            uint8_t* sa = smem + s * kPairStageBytes;
+            uint8_t* sb = sa + kPairABytes;
+            if (crank == 0) mbar_arrive_expect_tx(&full[s], 2 * kPairStageBytes);
+            const uint32_t fb = mapa_u32(&full[s], 0);
+            if (!A_MN) {
+              tma_load_2d_pair(sa, &tmA, fb, kb * kPairK, row0);
+            } else {
 #pragma unroll
-            for (int c = 0; c < 2; ++c) tma_load_2d_pair(sa + c * (kPairK * 128), &tmA, fb, row0 + c * 64, kb * kPairK);
-          }
-          if (!B_MN) {
-            tma_load_2d_pair(sb, &tmB, fb, kb * kPairK, col0);
-          } else {
+              for (int c = 0; c < 2; ++c) tma_load_2d_pair(sa + c * (kPairK * 128), &tmA, fb, row0 + c * 64, kb * kPairK);
+            }
+            if (!B_MN) {
+              tma_load_2d_pair(sb, &tmB, fb, kb * kPairK, col0);
+            } else {
 #pragma unroll
-            for (int c = 0; c < Cfg::kHalfN / 64; ++c) tma_load_2d_pair(sb + c * (kPairK * 128), &tmB, fb, col0 + c * 64, kb * kPairK);
+              for (int c = 0; c < Cfg::kHalfN / 64; ++c) tma_load_2d_pair(sb + c * (kPairK * 128), &tmB, fb, col0 + c * 64, kb * kPairK);
+            }
           }
+          __syncwarp();
         }
       }
       // Tail: the leader's last commits arrive on this CTA's `empty` barriers from the other SM;
       // wait for them so that none lands after this CTA has left.
       for (int i = 0; i < kPairStages && ok; ++i, ++it) {
         if (it < (uint32_t)kPairStages) continue;  // this slot was never filled
-        ok = mbar_wait_relaxed(&empty[it % kPairStages], ((it / kPairStages) & 1) ^ 1, wc, 7);
+        ok = mbar_wait_relaxed_warp(&empty[it % kPairStages], ((it / kPairStages) & 1) ^ 1, wc, 7);
       }
     }
   } else if (warp == 1) {
@@ -583,35 +587,38 @@ gemm_pair_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
   WaitCtx wc{abort_w, p.status, p.wait_ns};
 
   if (warp == 0) {
-    if (lane == 0) {
+    {   // (warp-uniform control flow, one elected lane issues)
       const int row0 = tm * kPairM + half * 128, col0 = tn * BN + half * Cfg::kHalfN;
       bool ok = true;
       for (int it = 0; it < n_kb; ++it) {
         const int s = it % S;
-        if (!mbar_wait_relaxed(&empty[s], ((it / S) & 1) ^ 1, wc, 1)) { ok = false; break; }
-        uint8_t* sa = smem + s * Cfg::kStageBytes;
-        uint8_t* sb = sa + kPairABytes;
-        const int k = (kb0 + it) * kPairK;
-        if (half == 0) mbar_arrive_expect_tx(&full[s], 2 * Cfg::kStageBytes);
-        const uint32_t fb = mapa_u32(&full[s], lead);
-        if (!A_MN) {
-          tma_load_2d_pair(sa, &tmA, fb, k, row0);
-        } else {
+        if (!mbar_wait_relaxed_warp(&empty[s], ((it / S) & 1) ^ 1, wc, 1)) { ok = false; break; }
+        if (elect_one()) {
+          uint8_t* sa = smem + s * Cfg::kStageBytes;
+          uint8_t* sb = sa + kPairABytes;
+          const int k = (kb0 + it) * kPairK;
+          if (half == 0) mbar_arrive_expect_tx(&full[s], 2 * Cfg::kStageBytes);
+          const uint32_t fb = mapa_u32(&full[s], lead);
+          if (!A_MN) {
+            tma_load_2d_pair(sa, &tmA, fb, k, row0);
+          } else {
 #pragma unroll
-          for (int j = 0; j < 2; ++j) tma_load_2d_pair(sa + j * (kPairK * 128), &tmA, fb, row0 + j * 64, k);
-        }
-        if (!B_MN) {
-          tma_load_2d_pair(sb, &tmB, fb, k, col0);
-        } else {
+            for (int j = 0; j < 2; ++j) tma_load_2d_pair(sa + j * (kPairK * 128), &tmA, fb, row0 + j * 64, k);
+          }
+          if (!B_MN) {
+            tma_load_2d_pair(sb, &tmB, fb, k, col0);
+          } else {
 #pragma unroll
-          for (int j = 0; j < Cfg::kHalfN / 64; ++j)
-            tma_load_2d_pair(sb + j * (kPairK * 128), &tmB, fb, col0 + j * 64, k);
+            for (int j = 0; j < Cfg::kHalfN / 64; ++j)
+              tma_load_2d_pair(sb + j * (kPairK * 128), &tmB, fb, col0 + j * 64, k);
+          }
         }
+        __syncwarp();
       }
       // the last commits of every slot arrive on this CTA's `empty` barriers, from the other SM for the peer
       for (int it = n_kb; it < n_kb + S && ok; ++it) {
         if (it < S) continue;   // this slot was never filled
-        ok = mbar_wait_relaxed(&empty[it % S], ((it / S) & 1) ^ 1, wc, 7);
+        ok = mbar_wait_relaxed_warp(&empty[it % S], ((it / S) & 1) ^ 1, wc, 7);
       }
     }
     __syncwarp();

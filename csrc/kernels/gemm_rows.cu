@@ -84,33 +84,34 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant_
   WaitCtx wc{abort_w, p.status, p.wait_ns};
 
   if (warp == 0) {
-    if (lane == 0) {
-      auto load_b = [&](int it) {
-        const int s = it % S, k = (kb0 + it) * kRowsK;
-        uint8_t* sp = smem + s * Cfg::kStageBytes;
-        mbar_arrive_expect_tx(&full[s], Cfg::kStageBytes);
-        if (!B_MN) {
-          tma_load_2d(sp, &tmB, &full[s], k, n0);
-        } else {
+    // (warp-uniform control flow, one elected lane issues)
+    auto load_b = [&](int it) {
+      const int s = it % S, k = (kb0 + it) * kRowsK;
+      uint8_t* sp = smem + s * Cfg::kStageBytes;
+      mbar_arrive_expect_tx(&full[s], Cfg::kStageBytes);
+      if (!B_MN) {
+        tma_load_2d(sp, &tmB, &full[s], k, n0);
+      } else {
 #pragma unroll
-          for (int c = 0; c < 2; ++c) tma_load_2d(sp + c * (kRowsK * 128), &tmB, &full[s], n0 + c * 64, k);
-        }
-      };
-      // In a chain the weights are nobody's output: a ring of them is requested while the kernel before still runs.
-      const int ahead = min(S, n_kb);
-      for (int it = 0; it < ahead; ++it) load_b(it);
-      chain_wait();
-      for (int it = 0; it < n_kb; ++it) {
-        const int s = it % S;
-        if (it >= ahead) {
-          if (!mbar_wait_relaxed(&empty[s], ((it / S) & 1) ^ 1, wc, 1)) break;
-          load_b(it);
-        }
-        tma_load_2d(smem + s * Cfg::kStageBytes + kRowsBBytes, &tmA, &full[s], (kb0 + it) * kRowsK, 0);
+        for (int c = 0; c < 2; ++c) tma_load_2d(sp + c * (kRowsK * 128), &tmB, &full[s], n0 + c * 64, k);
       }
+    };
+    // In a chain the weights are nobody's output: a ring of them is requested while the kernel before still runs.
+    const int ahead = min(S, n_kb);
+    for (int it = 0; it < ahead; ++it) {
+      if (elect_one()) load_b(it);
+      __syncwarp();
     }
     chain_wait();
-    __syncwarp();
+    for (int it = 0; it < n_kb; ++it) {
+      const int s = it % S;
+      if (it >= ahead && !mbar_wait_relaxed_warp(&empty[s], ((it / S) & 1) ^ 1, wc, 1)) break;
+      if (elect_one()) {
+        if (it >= ahead) load_b(it);
+        tma_load_2d(smem + s * Cfg::kStageBytes + kRowsBBytes, &tmA, &full[s], (kb0 + it) * kRowsK, 0);
+      }
+      __syncwarp();
+    }
   } else if (warp == 1) {
     // warp-uniform control flow, one elected lane issues (tcgen05 operands live in uniform registers)
     chain_wait();

@@ -381,7 +381,11 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    // warp-uniform control flow, one elected lane issues: operands of the copies live in uniform registers, too, and from a
+    // branch of lane 0 a copy takes more than twice as long to issue (87 against 34 cycles), which bounds the products whose
+    // operands take four to six copies a k-block: dW of 768 x 768 over 16384 rows 32.7 -> 25.4 us in this kernel's and the
+    // pairs' form, of 3072 x 768 84 -> 68, of 1536 x 1024 over 2472 rows 18.4 -> 16.4; the others keep their times
+    {
       uint32_t it = 0;
       bool ok = true;
       for (int wi = 0; wi < n_items && ok; ++wi) {
@@ -394,13 +398,14 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         if (p.ag_operand) {
           ok = ag_wait_rows(p, p.ag_operand == 1 ? tm * kBlockM : tn * BLOCK_N,
                             p.ag_operand == 1 ? min(tm * kBlockM + kBlockM, p.M) : min(tn * BLOCK_N + BLOCK_N, p.N));
+          ok = __all_sync(0xffffffffu, ok);
           if (!ok) { *abort_w = 1; break; }
         }
         if (p.b_flags) {
           int r0 = tn * BLOCK_N;
           int r1 = min(r0 + BLOCK_N, p.N) - 1;
           for (int f = r0 / p.rows_per_flag; f <= r1 / p.rows_per_flag && ok; ++f) {
-            ok = flag_wait_ge(p.b_flags + f, p.flag_want, false, p.status, p.wait_ns, 10);
+            ok = __all_sync(0xffffffffu, flag_wait_ge(p.b_flags + f, p.flag_want, false, p.status, p.wait_ns, 10));
             if (!ok) *abort_w = 1;
           }
           if (!ok) break;
@@ -410,60 +415,68 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         for (int kb = w.kb0; kb < w.kb1; ++kb, ++it) {
           int s = it % Cfg::kStages;
           uint32_t ph = (it / Cfg::kStages) & 1;
-          if (!mbar_wait(&empty[s], ph ^ 1, wc, 1)) { ok = false; break; }
-          uint8_t* sa = smem + s * Cfg::kStageBytes;
-          uint8_t* sb = sa + Cfg::kABytes;
-          mbar_arrive_expect_tx(&full[s], A_MN ? Cfg::kStageBytes : p.a_box_rows * (kBlockK * 2) + Cfg::kBBytes);
-          if (!A_MN) {
-            tma_load_2d(sa, &tmA, &full[s], kb * kBlockK, tm * kBlockM);
-          } else {
+          if (!mbar_wait_warp(&empty[s], ph ^ 1, wc, 1)) { ok = false; break; }
+          if (elect_one()) {
+            uint8_t* sa = smem + s * Cfg::kStageBytes;
+            uint8_t* sb = sa + Cfg::kABytes;
+            mbar_arrive_expect_tx(&full[s], A_MN ? Cfg::kStageBytes : p.a_box_rows * (kBlockK * 2) + Cfg::kBBytes);
+            if (!A_MN) {
+              tma_load_2d(sa, &tmA, &full[s], kb * kBlockK, tm * kBlockM);
+            } else {
 #pragma unroll
-            for (int c = 0; c < kBlockM / 64; ++c)
-              tma_load_2d(sa + c * (kBlockK * 128), &tmA, &full[s], tm * kBlockM + c * 64,
-                          kb * kBlockK);
-          }
-          if (!B_MN) {
-            tma_load_2d(sb, &tmB, &full[s], kb * kBlockK, tn * BLOCK_N);
-          } else {
+              for (int c = 0; c < kBlockM / 64; ++c)
+                tma_load_2d(sa + c * (kBlockK * 128), &tmA, &full[s], tm * kBlockM + c * 64,
+                            kb * kBlockK);
+            }
+            if (!B_MN) {
+              tma_load_2d(sb, &tmB, &full[s], kb * kBlockK, tn * BLOCK_N);
+            } else {
 #pragma unroll
-            for (int c = 0; c < BLOCK_N / 64; ++c)
-              tma_load_2d(sb + c * (kBlockK * 128), &tmB, &full[s], tn * BLOCK_N + c * 64,
-                          kb * kBlockK);
+              for (int c = 0; c < BLOCK_N / 64; ++c)
+                tma_load_2d(sb + c * (kBlockK * 128), &tmB, &full[s], tn * BLOCK_N + c * 64,
+                            kb * kBlockK);
+            }
           }
+          __syncwarp();
         }
       }
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      constexpr uint32_t idesc = make_idesc_f16(kBlockM, BLOCK_N, 1, A_MN ? 1 : 0, B_MN ? 1 : 0);
-      uint32_t it = 0, lt = 0;
-      bool ok = true;
-      for (int wi = 0; wi < n_items && ok; ++wi, ++lt) {
-        const WorkItem w = get_work(wi);
-        int as = lt & 1;
-        uint32_t aph = (lt >> 1) & 1;
-        if (!mbar_wait(&tempty[as], aph ^ 1, wc, 2)) break;
+    // (warp-uniform control flow, one elected lane issues: tcgen05 operands live in uniform registers)
+    constexpr uint32_t idesc = make_idesc_f16(kBlockM, BLOCK_N, 1, A_MN ? 1 : 0, B_MN ? 1 : 0);
+    constexpr uint32_t hi = smem_desc_hi(1024);
+    const uint32_t a_lo0 = smem_desc_lo(smem_u32(smem), A_MN ? kBlockK * 128 : 16);
+    const uint32_t b_lo0 = smem_desc_lo(smem_u32(smem + Cfg::kABytes), B_MN ? kBlockK * 128 : 16);
+    uint32_t it = 0, lt = 0;
+    bool ok = true;
+    for (int wi = 0; wi < n_items && ok; ++wi, ++lt) {
+      const WorkItem w = get_work(wi);
+      const int as = lt & 1;
+      const uint32_t aph = (lt >> 1) & 1;
+      if (!mbar_wait_warp(&tempty[as], aph ^ 1, wc, 2)) break;
+      tc_fence_after_sync();
+      const uint32_t d_tmem = tmem_base + as * BLOCK_N;
+      for (int kb = w.kb0; kb < w.kb1; ++kb, ++it) {
+        const int s = it % Cfg::kStages;
+        const uint32_t ph = (it / Cfg::kStages) & 1;
+        if (!mbar_wait_warp(&full[s], ph, wc, 3)) { ok = false; break; }
         tc_fence_after_sync();
-        uint32_t d_tmem = tmem_base + as * BLOCK_N;
-        for (int kb = w.kb0; kb < w.kb1; ++kb, ++it) {
-          int s = it % Cfg::kStages;
-          uint32_t ph = (it / Cfg::kStages) & 1;
-          if (!mbar_wait(&full[s], ph, wc, 3)) { ok = false; break; }
-          tc_fence_after_sync();
-          uint32_t sa = smem_u32(smem + s * Cfg::kStageBytes);
-          uint32_t sb = sa + Cfg::kABytes;
+        const uint32_t a_lo = a_lo0 + s * (Cfg::kStageBytes >> 4), b_lo = b_lo0 + s * (Cfg::kStageBytes >> 4);
+        if (elect_one()) {
 #pragma unroll
           for (int j = 0; j < kBlockK / kUmmaK; ++j) {
-            uint64_t da = A_MN ? make_smem_desc_sw128(sa + j * 2048, kBlockK * 128, 1024)
-                               : make_smem_desc_sw128(sa + j * 32, 16, 1024);
-            uint64_t db = B_MN ? make_smem_desc_sw128(sb + j * 2048, kBlockK * 128, 1024)
-                               : make_smem_desc_sw128(sb + j * 32, 16, 1024);
-            umma_f16_ss(d_tmem, da, db, idesc, (kb != w.kb0) || (j != 0));
+            const uint32_t ao = A_MN ? j * (2048 >> 4) : j * (32 >> 4);
+            const uint32_t bo = B_MN ? j * (2048 >> 4) : j * (32 >> 4);
+            umma_f16_ss_w(d_tmem, a_lo + ao, hi, b_lo + bo, hi, idesc, (kb != w.kb0) || (j != 0));
           }
           umma_commit(&empty[s]);
         }
-        if (ok) umma_commit(&tfull[as]);
+        __syncwarp();
+      }
+      if (ok) {
+        if (elect_one()) umma_commit(&tfull[as]);
+        __syncwarp();
       }
     }
   } else {

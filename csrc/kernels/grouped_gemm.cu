@@ -147,7 +147,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   };
 
   if (warp == 0) {
-    if (lane == 0) {
+    {   // (warp-uniform control flow, one elected lane issues: operands of the copies live in uniform registers, too)
       uint32_t it = 0;
       bool ok = true;
       for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
@@ -156,28 +156,31 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         for (int kb = kb0; kb < kb1; ++kb, ++it) {
           const int s = it % Cfg::kStages;
           const uint32_t ph = (it / Cfg::kStages) & 1;
-          if (!mbar_wait(&empty[s], ph ^ 1, wc, 1)) { ok = false; break; }
-          uint8_t* sa = smem + s * Cfg::kStageBytes;
-          uint8_t* sb = sa + Cfg::kABytes;
-          mbar_arrive_expect_tx(&full[s], Cfg::kStageBytes);
-          if (p.mode == 0) {
-            tma_load_2d(sa, &tmA, &full[s], kb * kGBlockK, row0);
-            if (!B_MN) {
-              tma_load_3d(sb, &tmB, &full[s], kb * kGBlockK, c0, e);
+          if (!mbar_wait_warp(&empty[s], ph ^ 1, wc, 1)) { ok = false; break; }
+          if (elect_one()) {
+            uint8_t* sa = smem + s * Cfg::kStageBytes;
+            uint8_t* sb = sa + Cfg::kABytes;
+            mbar_arrive_expect_tx(&full[s], Cfg::kStageBytes);
+            if (p.mode == 0) {
+              tma_load_2d(sa, &tmA, &full[s], kb * kGBlockK, row0);
+              if (!B_MN) {
+                tma_load_3d(sb, &tmB, &full[s], kb * kGBlockK, c0, e);
+              } else {
+#pragma unroll
+                for (int c = 0; c < BLOCK_N / 64; ++c)
+                  tma_load_3d(sb + c * (kGBlockK * 128), &tmB, &full[s], c0 + c * 64, kb * kGBlockK, e);
+              }
             } else {
+              // A = dY^T: MN-major operand from dY [rows, N] ; B = X^T from X [rows, K]
+#pragma unroll
+              for (int c = 0; c < kGBlockM / 64; ++c)
+                tma_load_2d(sa + c * (kGBlockK * 128), &tmA, &full[s], row0 + c * 64, kb * kGBlockK);
 #pragma unroll
               for (int c = 0; c < BLOCK_N / 64; ++c)
-                tma_load_3d(sb + c * (kGBlockK * 128), &tmB, &full[s], c0 + c * 64, kb * kGBlockK, e);
+                tma_load_2d(sb + c * (kGBlockK * 128), &tmB, &full[s], c0 + c * 64, kb * kGBlockK);
             }
-          } else {
-            // A = dY^T: MN-major operand from dY [rows, N] ; B = X^T from X [rows, K]
-#pragma unroll
-            for (int c = 0; c < kGBlockM / 64; ++c)
-              tma_load_2d(sa + c * (kGBlockK * 128), &tmA, &full[s], row0 + c * 64, kb * kGBlockK);
-#pragma unroll
-            for (int c = 0; c < BLOCK_N / 64; ++c)
-              tma_load_2d(sb + c * (kGBlockK * 128), &tmB, &full[s], c0 + c * 64, kb * kGBlockK);
           }
+          __syncwarp();
         }
       }
     }
