@@ -12,8 +12,8 @@
 //
 // Bound by the special-function unit and the tensor pipe alternating within a tile; long sequences run at the power cap.
 // Against the form with two tiles and the maximum taken before the exponentials, 32/8 heads of 128, causal: T = 8190
-// 504 -> 492 us (1120 TFLOP/s), T = 2900 99.4 -> 87.2, 16 x 1000 268 -> 231; a window of 512 over 2 x 4096 (16/4 heads)
-// 93 -> 76; 12 heads of 64, 16 x 1024 95.4 -> 78.8.
+// 523 -> 515 us (both at the power cap, runs of one differ by 15), T = 4096 163 -> 156, T = 2900 99 -> 89.4, 16 x 1000
+// 269 -> 227; a window of 512 over 2 x 4096 (16/4 heads) 93 -> 77; 12 heads of 64, 16 x 1024 95.8 -> 79.5.
 //
 // Counterpart in the reference: vendored FlashAttention-2 sm80 leaves
 // (p10/src/backend/cuda/transformers/flash/flash_fwd_kernel.h, AttentionKernels.cu:1782-1969),
@@ -152,7 +152,9 @@ __device__ __forceinline__ void row_mask(uint32_t (&sr)[32], int k0, int lo, int
 
 // exp2 of a pair on the FMA pipe: floor by the magic-number add in round-down mode, cubic
 // polynomial on the fraction (relative error 1e-4, below the bf16 rounding of P), exponent added
-// as an integer. The special-function unit delivers 16 exp2 per cycle and SM while the tensor pipe
+// as an integer. Below -127 the result is 2^-127; from 128 on the sum leaves the exponent field and the result is anything,
+// a small number of either sign among others, so that who does not know the maximum has to look at x.
+// The special-function unit delivers 16 exp2 per cycle and SM while the tensor pipe
 // needs 16 per cycle for 128-wide head dimensions, so a share of the row goes this way.
 __device__ __forceinline__ uint64_t exp2_poly2(uint64_t x) {
   float x0, x1;
@@ -172,18 +174,20 @@ __device__ __forceinline__ uint64_t exp2_poly2(uint64_t x) {
 
 // 32 columns of a row become 16 bf16 pairs P = exp2(S * scale - m) in sr[0 .. 16) (in place: the pairs land where scores were
 // already consumed); the fp32 values are added into two packed accumulators. Of every four column pairs, NPOLY take the
-// polynomial, the rest the special-function unit.
+// polynomial, the rest the special-function unit. poly_max: the largest exponent that the polynomial was given.
 template <int NPOLY>
-__device__ __forceinline__ void row_exp(uint32_t (&sr)[32], uint64_t sc, uint64_t nm, uint64_t& acc0, uint64_t& acc1) {
+__device__ __forceinline__ void row_exp(uint32_t (&sr)[32], uint64_t sc, uint64_t nm, uint64_t& acc0, uint64_t& acc1,
+                                        float& poly_max) {
 #pragma unroll
   for (int i = 0; i < 16; ++i) {
     const uint64_t x = fma2(pk2u(sr[2 * i], sr[2 * i + 1]), sc, nm);
+    float x0, x1;
+    upk2(x, x0, x1);
     uint64_t e;
     if ((i & 3) < NPOLY) {
+      poly_max = max3(poly_max, x0, x1);
       e = exp2_poly2(x);
     } else {
-      float x0, x1;
-      upk2(x, x0, x1);
       e = pk2(fast_exp2(x0), fast_exp2(x1));
     }
     if (i & 1) acc1 = add2(acc1, e);
@@ -444,13 +448,15 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       // the fp32 values. m need not be the maximum, only so large that nothing overflows. One warp per scheduler works on
       // a tile, so what it spends before its first exponential (loading 128 scores and taking their maximum: 500 of 1800
       // cycles a tile) nothing else fills. So the exponentials start against the m so far, 32 keys at a time, each group
-      // loaded under those of the one before, and the maximum is not taken: a score that outgrew m shows in the sum, and
-      // only the keys that are handed over later are looked at themselves. The first tile, masked ones and, once more, a
-      // tile in which a row has to move its m take the maximum first.
+      // loaded under those of the one before, and the maximum is not taken: a score that outgrew m shows in the sum, where
+      // its exponential came from the special-function unit, which saturates; what went to the polynomial, which wraps, and
+      // the keys that are handed over later are looked at themselves. (The maximum of the polynomial's exponents took no
+      // time at T = 1000 to 4096; bounding them by 127 instead, so that they show in the sum, 1 to 3 %.) The first tile,
+      // masked ones and, once more, a tile in which a row has to move its m take the maximum first.
       const uint64_t sc2 = pk2(p.scale_log2e, p.scale_log2e);
       uint64_t acc0, acc1;
       uint32_t x[4][32];
-      float alpha = 1.f, s0, s1;
+      float alpha = 1.f, s0, s1, poly_max = -INFINITY;
       bool with_max = need_mask || j == 0;
       while (true) {
         if (with_max) {
@@ -493,7 +499,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             tmem_ld_wait(x[c]);
             if (c < 3) tmem_ld_32x32b_x32(t_s + (c + 1) * 32, x[c + 1]);
             row_mask(x[c], k0 + c * 32, lo, lim);
-            if (c < 3) row_exp<0>(x[c], sc2, nm2, acc0, acc1);
+            if (c < 3) row_exp<0>(x[c], sc2, nm2, acc0, acc1, poly_max);
           }
           break;
         }
@@ -501,14 +507,14 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         for (int c = 0; c < 3; ++c) {
           tmem_ld_wait(x[c]);
           tmem_ld_32x32b_x32(t_s + (c + 1) * 32, x[c + 1]);
-          row_exp<NPOLY>(x[c], sc2, nm2, acc0, acc1);
+          row_exp<NPOLY>(x[c], sc2, nm2, acc0, acc1, poly_max);
         }
         tmem_ld_wait(x[3]);
         if (with_max) break;
-        // 2^11: what 128 keys of 2^4 add up to, the bound of the other case (NaN fails, too)
+        // 2^11: what 128 keys of 2^4 add up to, the bound of the other case (NaN fails, too); no exponential alone exceeds it
         upk2(add2(acc0, acc1), s0, s1);
         const float late = row_max(x[3]) * p.scale_log2e - m;
-        if (__all_sync(0xffffffffu, s0 + s1 <= 2048.f && late <= 4.f)) break;
+        if (__all_sync(0xffffffffu, s0 + s1 <= 2048.f && poly_max <= 11.f && late <= 4.f)) break;
         with_max = true;   // the scores are still in TMEM
       }
       fwd_trace(tr, 1, 4, j);
@@ -520,8 +526,8 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       if (lane == 0) mbar_arrive(p_half);   // one arrival per warp: 32 on one barrier are served one after the other
       fwd_trace(tr, 1, 5, j);
       const uint64_t nm2 = pk2(-m, -m);
-      if (need_mask) row_exp<0>(x[3], sc2, nm2, acc0, acc1);
-      else row_exp<NPOLY>(x[3], sc2, nm2, acc0, acc1);
+      if (need_mask) row_exp<0>(x[3], sc2, nm2, acc0, acc1, poly_max);
+      else row_exp<NPOLY>(x[3], sc2, nm2, acc0, acc1, poly_max);
       tmem_st_32x32b_x16(t_s + 48, x[3]);
       fwd_trace(tr, 1, 6, j);
       upk2(add2(acc0, acc1), s0, s1);
