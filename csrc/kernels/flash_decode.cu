@@ -388,24 +388,18 @@ flash_decode_merge_kernel(const DecodeParams p) {
     p.lse[((long long)b * p.Hq + h) * p.lse_stride + tq] = den > 0.f ? (M + log2f(den)) * 0.6931471805599453f : -INFINITY;
 }
 
-// Once per head dimension: more shared memory than a launch gets unasked.
+// More shared memory than a launch gets unasked.
 static cudaError_t decode_configure(int D) {
-  static bool configured[2] = {};
-  bool& done = configured[D == 64 ? 0 : 1];
-  if (done) return cudaSuccess;
-  const cudaError_t e =
-      D == 64 ? cudaFuncSetAttribute(flash_decode_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, dec_smem(64))
-              : cudaFuncSetAttribute(flash_decode_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, dec_smem(128));
-  done = e == cudaSuccess;
-  return e;
+  static PerDevice done[2];
+  return D == 64 ? allow_smem(done[0], flash_decode_kernel<64>, dec_smem(64))
+                 : allow_smem(done[1], flash_decode_kernel<128>, dec_smem(128));
 }
 
-// Clusters of n CTAs that fit the device at once, asked of the runtime once per size: the SMs of a GPC are not a multiple
-// of every n (32 clusters of 8 CTAs of D = 128 fit, 96 of 3 do not, although 296 CTAs do).
+// Clusters of n CTAs that fit the device at once, asked of the runtime once per size and device: the SMs of a GPC are not a
+// multiple of every n (32 clusters of 8 CTAs of D = 128 fit, 96 of 3 do not, although 296 CTAs do).
 static int decode_resident(int D, int n) {
-  static int resident[2][kDecCluster + 1] = {};
-  int& r = resident[D == 64 ? 0 : 1][n];
-  if (r == 0) {
+  static PerDevice resident[2][kDecCluster + 1];
+  return resident[D == 64 ? 0 : 1][n].get([&] {
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -421,9 +415,8 @@ static int decode_resident(int D, int n) {
     decode_configure(D);
     const cudaError_t e = D == 64 ? cudaOccupancyMaxActiveClusters(&fit, flash_decode_kernel<64>, &cfg)
                                   : cudaOccupancyMaxActiveClusters(&fit, flash_decode_kernel<128>, &cfg);
-    r = e == cudaSuccess && fit > 0 ? fit : -1;
-  }
-  return r;
+    return e == cudaSuccess && fit > 0 ? fit : -1;
+  });
 }
 
 // Splits of the keys and who merges them, by the time in ns that the launch takes. What resident CTAs take is what memory

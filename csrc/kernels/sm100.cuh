@@ -12,6 +12,8 @@
 #include <stdint.h>
 #include <nvtx3/nvToolsExt.h>
 
+#include <atomic>
+
 namespace tpb {
 
 // NVTX ranges around the host side of every launching entry point, off unless tpb_nvtx_enable(1)
@@ -139,6 +141,35 @@ __device__ __forceinline__ uint4 chain_ld(const void* p) {
   uint4 r;
   asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(p));
   return r;
+}
+
+// Host side: a value for each device of the process. What the runtime keeps per device (a kernel's shared-memory limit) or
+// answers for one (how many clusters fit) is set or asked once on each; a process may launch on several, from several threads.
+// 0 means not yet; devices past the last slot are set and asked on every call.
+struct PerDevice {
+  static constexpr int kDevices = 64;
+  std::atomic<int> v[kDevices];
+  template <typename F>
+  int get(F&& ask) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kDevices) return ask();
+    int r = v[dev].load(std::memory_order_acquire);
+    if (r == 0) {
+      r = ask();
+      v[dev].store(r, std::memory_order_release);
+    }
+    return r;
+  }
+};
+// `kern` may have `bytes` of dynamic shared memory on the current device from then on.
+template <typename K>
+inline cudaError_t allow_smem(PerDevice& done, K kern, int bytes) {
+  cudaError_t e = cudaSuccess;
+  done.get([&] {
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    return e == cudaSuccess ? 1 : 0;   // a failure is tried again
+  });
+  return e;
 }
 
 // Host side: whether the launches of this thread belong to a chain whose first kernel was launched; set for the extent of a

@@ -1,0 +1,70 @@
+"""The host side of native launches in a process with several devices: what the runtime keeps or answers per device is set and
+asked on each. Against a stand-in for the CUDA runtime, in a child process without a GPU."""
+import os
+import shutil
+import subprocess
+import sys
+import textwrap
+from pathlib import Path
+
+import pytest
+
+from tensorplay_b200 import _build
+
+ROOT = Path(__file__).resolve().parent.parent
+pytestmark = pytest.mark.skipif(shutil.which("g++") is None, reason="needs a C++ compiler")
+
+
+@pytest.fixture(scope="module")
+def child(tmp_path_factory):
+    """Runs code over ``L`` (the kernel library) and ``F`` (the stand-in); returns what it prints."""
+    built = _build.LIBDIR / "libtpb200.so"
+    if not built.exists():
+        _build.build_kernels()
+    work = tmp_path_factory.mktemp("fake")
+    lib = work / "libfake.so"
+    subprocess.run(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-I", str(_build._cuda_home() / "include"),
+                    str(ROOT / "tests" / "cpp" / "fake_cuda_runtime.cpp"), "-o", str(lib)], check=True)
+    head = textwrap.dedent(f"""
+        import ctypes
+        from ctypes import c_void_p as P, c_int as I, c_longlong as LL, c_float as FL
+        F = ctypes.CDLL({str(lib)!r})
+        L = ctypes.CDLL({str(built)!r})
+        def decode(D, B=1, Tk=64, splits=0):
+            a = P(4096)
+            s = LL(8 * D)
+            return L.tpb_flash_decode(a, a, a, a, a, None, None, I(B), I(1), I(Tk), I(8), I(8), I(D), *[s] * 12, I(128), I(1), FL(1.0),
+                                      I(0), I(splits), None)
+    """)
+
+    def run(code):
+        out = subprocess.run([sys.executable, "-c", head + textwrap.dedent(code)], capture_output=True, text=True, timeout=120,
+                             env=dict(os.environ, LD_PRELOAD=str(lib), LD_LIBRARY_PATH=str(_build._cuda_home() / "lib64")))
+        assert out.returncode == 0, out.stdout + out.stderr
+        return out.stdout.split()
+
+    return run
+
+
+@pytest.mark.parametrize("D", [64, 128])
+def test_few_row_attention_on_every_device(child, D):
+    assert child(f"""
+        for d in (0, 1, 7, 0):
+            F.fake_set_device(d)
+            print(decode({D}))
+    """) == ["0"] * 4
+
+
+@pytest.mark.parametrize("D", [64, 128])
+def test_splits_by_the_device_at_hand(child, D):
+    """Two devices that hold different numbers of clusters: each gets the splits that it gets as the first one."""
+    code = f"""
+        F.fake_set_clusters(0, 40)
+        F.fake_set_clusters(1, 1)
+        for d in %s:
+            F.fake_set_device(d)
+            assert decode({D}, 8, 2000) == 0
+            print(F.fake_last_grid_x())
+    """
+    both = child(code % "(0, 1)")
+    assert both == child(code % "(0,)") + child(code % "(1,)") and both[0] != both[1]
