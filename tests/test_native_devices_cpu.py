@@ -68,3 +68,13 @@ def test_splits_by_the_device_at_hand(child, D):
     """
     both = child(code % "(0, 1)")
     assert both == child(code % "(0,)") + child(code % "(1,)") and both[0] != both[1]
+
+
+@pytest.mark.parametrize("bits,group", [(4, 128), (8, 0)])
+def test_packed_weights_on_every_device(child, bits, group):
+    assert child(f"""
+        a = P(4096)
+        for d in (0, 1, 63, 64, 0):
+            F.fake_set_device(d)
+            print(L.tpb_wq_gemm(a, a, a, None, None, a, I(64), I(256), I(512), I({bits}), I({group}), LL(512), LL(256), None, None))
+    """) == ["0"] * 5
