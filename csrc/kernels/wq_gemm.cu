@@ -337,13 +337,13 @@ int launch_wq_gemm(const CUtensorMap& tw, const CUtensorMap& tx, const WqGemmPar
 }
 
 // Rows of x per tile, by rounds of tiles times what a k-block takes (measured: 0.45 us at 16 rows, 0.51 at 64, 0.66 at 128, 0.69
-// at 176); also that time for one k-block of all tiles.
+// at 176); also that time for one k-block of all tiles. Tried are the twelve sizes there are, the larger one first where two cost
+// the same: trying every number of row tiles, M / 16 of them, took 20 us of the host at 65536 rows, twice a call.
 int wq_pick_nt(int M, int n_tiles, double* us) {
   int best = 0;
-  for (int t = (M + kWqMaxNT - 1) / kWqMaxNT; t <= (M + 15) / 16; ++t) {
-    const int nt = ((M + t - 1) / t + 15) / 16 * 16;
-    if (nt > kWqMaxNT) continue;
-    const long long tiles = (long long)n_tiles * ((M + nt - 1) / nt), rounds = (tiles + sm_count() - 1) / sm_count();
+  for (int nt = kWqMaxNT; nt >= 16; nt -= 16) {
+    if (nt > 16 && nt - 16 >= M) continue;   // no row in its last 16
+    const long long tiles = (long long)n_tiles * ((M + (long long)nt - 1) / nt), rounds = (tiles + sm_count() - 1) / sm_count();
     const double cost = rounds * (0.42 + 0.0016 * nt);
     if (!best || cost < *us) { best = nt; *us = cost; }
   }

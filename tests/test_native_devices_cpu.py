@@ -78,3 +78,47 @@ def test_packed_weights_on_every_device(child, bits, group):
             F.fake_set_device(d)
             print(L.tpb_wq_gemm(a, a, a, None, None, a, I(64), I(256), I(512), I({bits}), I({group}), LL(512), LL(256), None, None))
     """) == ["0"] * 5
+
+
+def test_packed_weights_host_time_of_many_rows(child):
+    """What is asked on every call of more rows than the GEMV takes is answered in the same time for any number of rows."""
+    few, many = (float(t) for t in child("""
+        import time
+        for M in (1000, 1 << 30):
+            best = 1.0
+            for _ in range(5):
+                t = time.perf_counter()
+                L.tpb_wq_gemm_pays(I(M), I(14336), I(4096), I(4), I(128))
+                best = min(best, time.perf_counter() - t)
+            print(best)
+    """))
+    assert many < 20 * few + 1e-4   # by the number of row tiles it is a million times
+
+
+def test_packed_weights_tile_rows(child):
+    """The tiles that a launch takes are the cheapest of those with any number of row tiles: its grid says how many there are."""
+    SMS = 148
+    rows = [1, 5, 16, 17, 31, 32, 33, 48, 49, 100, 128, 129, 191, 192, 193, 200, 333, 384, 385, 512, 577, 777, 1000, 1024, 3000]
+    widths = [8, 136, 1000, 4096, 14336, 28672]
+    got = child(f"""
+        a = P(4096)
+        for N in {widths}:
+            for M in {rows}:
+                assert L.tpb_wq_gemm(a, a, a, None, None, a, I(M), I(N), I(256), I(4), I(128), LL(256), LL(N), None, None) == 0
+                print(F.fake_last_grid_x())
+    """)
+    want = []
+    for N in widths:
+        for M in rows:
+            best = None
+            n_tiles = (N + 127) // 128
+            for t in range((M + 191) // 192, (M + 15) // 16 + 1):
+                nt = ((M + t - 1) // t + 15) // 16 * 16
+                if nt > 192:
+                    continue
+                tiles = n_tiles * ((M + nt - 1) // nt)
+                cost = (tiles + SMS - 1) // SMS * (0.42 + 0.0016 * nt)
+                if best is None or cost < best[0]:
+                    best = (cost, tiles)
+            want.append(str(min(best[1], SMS)))
+    assert got == want
