@@ -335,11 +335,16 @@ class Llama(nn.Module):
         cos, sin = self.rope_tables(past + T, dev)
         for t in (cos, sin):
             if type(t) is not Tensor or t.dtype is not torch.float32 or t.device != dev or not t.is_contiguous() \
-                    or t.data_ptr() % 16 or t.dim() != 2 or t.shape[1] != D // 2 or t.shape != cos.shape:
+                    or t.data_ptr() % 16 or t.dim() != 2 or t.shape[1] != D // 2 or t.shape != cos.shape \
+                    or (position_ids is None and t.shape[0] < past + T):
                 return None
         pos = flat_positions(position_ids, rows, dev)
         L, Tk = lib(), past + T
         logits = embed.new_empty(B, T, V)
+        for i in range(n_layers):
+            cache.room(kv_shape, kv_shape, logits, logits, i)
+            if cache._k[i].shape[2] < Tk:   # buffers of before the cache was allowed more: the append layer by layer refuses
+                return None
         scratch = logits.new_empty(L.tpb_llama_cached_scratch(rows, H, Hq, Hkv, D, I))
         few = few_rows_sizes(B, T, Tk, Hq, Hkv, D)
         splits = L.tpb_flash_decode_splits(B, T, Tk, Hq, Hkv, D) if few and Tk > 2048 else 0
@@ -354,7 +359,6 @@ class Llama(nn.Module):
             part + 4 * part_rows * D if splits else 0, lse, lse_stride, splits, int(few), B, T, past, H, Hq, Hkv, D, I, V,
             n_layers))
         for i in range(n_layers):
-            cache.room(kv_shape, kv_shape, logits, logits, i)
             k = cache._k[i]
             words.extend(weights[6 * i:6 * i + 6])
             words.extend((k.data_ptr(), cache._v[i].data_ptr(), k.shape[2]))
