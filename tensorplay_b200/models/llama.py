@@ -372,13 +372,15 @@ class Llama(nn.Module):
 
 # What a pass operator by operator calls: where one of these was replaced, on a class or on an instance, it is called.
 _MODEL_METHODS = frozenset(("embed_tokens", "head", "rope_tables"))
-_BLOCK_METHODS = frozenset(("forward", "_attend_cached", "_infer_cached", "_plain_inference"))
+_BLOCK_METHODS = frozenset(("forward", "_attend_cached", "_infer_cached", "_plain_inference", "_weights",
+                            "_shapes_as_configured"))
 _CACHE_METHODS = frozenset(("update", "get_seq_length"))
 
 
 def _methods():
     return (Llama.embed_tokens, Llama.head, LlamaBlock.__call__, LlamaBlock.forward, LlamaBlock._attend_cached,
-            LlamaBlock._infer_cached, DynamicCache.update, DynamicCache.get_seq_length, StaticCache.update,
+            LlamaBlock._infer_cached, LlamaBlock._plain_inference, LlamaBlock._weights, LlamaBlock._shapes_as_configured,
+            DynamicCache.update, DynamicCache.get_seq_length, StaticCache.update,
             StaticCache.get_seq_length, ops.embedding, ops.rms_norm, ops.linear, ops.flash_attention)
 
 

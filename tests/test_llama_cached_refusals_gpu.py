@@ -5,7 +5,7 @@ import torch
 
 import tensorplay_b200.ops as O
 from tensorplay_b200 import _native
-from tensorplay_b200.models.llama import Llama, LlamaConfig
+from tensorplay_b200.models.llama import Llama, LlamaBlock, LlamaConfig
 from tensorplay_b200.nn.cache import DynamicCache, StaticCache
 
 pytestmark = pytest.mark.gpu
@@ -55,3 +55,69 @@ def test_buffers_that_did_not_grow_with_the_limit(seen):
     with pytest.raises(ValueError):
         _pass(m, tok[:, 8:].contiguous(), cache)
     assert seen == [1] and cache.get_seq_length(0) == 8
+
+
+@pytest.mark.parametrize("name", ["_plain_inference", "_weights", "_shapes_as_configured", "_attend_cached", "_infer_cached"])
+def test_replaced_on_the_block_class(monkeypatch, seen, name):
+    """What the pass layer by layer asks of a block is asked where the class has another one."""
+    m, own = _model(), []
+    f = getattr(LlamaBlock, name)
+    monkeypatch.setattr(LlamaBlock, name, lambda *a: own.append(1) or f(*a))
+    if name == "_attend_cached":   # of a block that goes operator by operator
+        monkeypatch.setattr(LlamaBlock, "_plain_inference", lambda *a: False)
+    tok = torch.randint(0, 520, (2, 9), device=DEV)
+    _pass(m, tok, DynamicCache())
+    assert own == [1, 1] and not seen
+
+
+def test_operators_of_a_block_that_says_it_is_not_plain(monkeypatch, seen):
+    m, own = _model(), []
+    monkeypatch.setattr(LlamaBlock, "_plain_inference", lambda *a: False)
+    for name in ("apply_rope", "swiglu_packed"):
+        f = getattr(O, name)
+        monkeypatch.setattr(O, name, lambda *a, f=f, name=name: own.append(name) or f(*a))
+    _pass(m, torch.randint(0, 520, (2, 9), device=DEV), DynamicCache())
+    assert own == ["apply_rope", "swiglu_packed"] * 2 and not seen
+
+
+def _both(m, call):
+    """``call`` on the model as it is and with a hook that sends it layer by layer: two results or two refusals."""
+    out = []
+    for hook in (False, True):
+        handle = m.layers[0].register_forward_hook(lambda *a: None) if hook else None
+        try:
+            out.append(call())
+        except Exception as e:
+            out.append((type(e), str(e)))
+        if handle is not None:
+            handle.remove()
+    return out
+
+
+def test_norm_weight_of_another_type(seen):
+    m = _model()
+    m.final_norm = torch.nn.Parameter(m.final_norm.detach().float())
+    tok = torch.randint(0, 520, (2, 9), device=DEV)
+    a, b = _both(m, lambda: _pass(m, tok, DynamicCache()))
+    assert not seen and (torch.equal(a, b) if isinstance(a, torch.Tensor) else a == b)
+
+
+def test_weight_of_other_strides(seen):
+    m = _model()
+    m.layers[1].wo = torch.nn.Parameter(m.layers[1].wo.detach().t().contiguous().t())
+    tok = torch.randint(0, 520, (2, 9), device=DEV)
+    a, b = _both(m, lambda: _pass(m, tok, DynamicCache()))
+    assert not seen and torch.equal(a, b)
+
+
+def test_with_gradients(seen):
+    m = _model()
+    tok = torch.randint(0, 520, (2, 8), device=DEV)
+
+    def call():
+        m.zero_grad(set_to_none=True)
+        m(tok, past_key_values=DynamicCache()).float().square().sum().backward()
+        return [p.grad for p in m.parameters()]
+
+    a, b = _both(m, call)
+    assert not seen and len(a) == 15 and all(torch.equal(x, y) and x.abs().sum() > 0 for x, y in zip(a, b))
