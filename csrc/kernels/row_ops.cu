@@ -668,6 +668,7 @@ __global__ void gelu_bwd_kernel(const __nv_bfloat16* __restrict__ dy,
 // With the loss's reduction, 16384 x 50257 / 4096 x 128256 / 4000 x 8000 took 428 / 238 / 81 us with 512 threads and one
 // logit at a time; two at a time 368 / 204 / 73, and with 256 threads 298 / 194 / 56. Requesting the next round ahead costs
 // half of the resident warps: 459 / 257 / 91.
+// Few long rows leave SMs with one block or two, and a block's rounds are what takes the time: 512 threads (ce_threads).
 // Two fp32 numbers in a register pair: one instruction adds or multiplies both.
 __device__ __forceinline__ unsigned long long pack2(float x, float y) {
   return ((unsigned long long)__float_as_uint(y) << 32) | __float_as_uint(x);
@@ -704,8 +705,8 @@ __device__ __forceinline__ unsigned long long exp8_sum(const uint4& u, unsigned 
   }
   return acc;
 }
-constexpr int kCeThreads = 256;
 constexpr int kCeVec = 4;
+template <int kCeThreads>
 __global__ void __launch_bounds__(kCeThreads)
 cross_entropy_kernel(const __nv_bfloat16* __restrict__ logits, const long long* __restrict__ target,
                      float* __restrict__ loss, float* __restrict__ lse_out,
@@ -1069,15 +1070,24 @@ extern "C" int tpb_gelu_bwd(const void* dy, const void* x, void* dx, long long n
   return (int)cudaGetLastError();
 }
 
+// Threads of a block, by the rows that an SM has at once and the rounds of 256 threads that a row takes (8192 logits each). us with
+// 256 / 512: 64 x 128256 18.2 / 12.3, 296 x 128256 21.2 / 17.8, 900 x 128256 48.5 / 46.5, 2400 x 128256 98 / 105; 148 x 50304
+// 9.7 / 7.9, 296 x 50304 10.9 / 10.6, 592 x 50304 14.8 / 17.6; 148 x 32000 6.7 / 5.9, 200 x 32000 7.4 / 7.5; 64 x 8000 2.7 / 3.1.
+static int ce_threads(long long rows, int V) {
+  const long long sms = sm_count();
+  return (rows <= sms && V > 2 * 8192) || (rows <= 2 * sms && V > 5 * 8192) ? 512 : 256;
+}
+
 extern "C" int tpb_cross_entropy(const void* logits, const long long* target, float* loss,
                                  float* lse, void* dlogits, long long rows, int V, long long stride,
                                  long long ignore_index, float gscale, void* stream) {
   TPB_NVTX("tpb_cross_entropy");
   if (stride % 8) return -2;
   if (rows <= 0) return 0;
-  cross_entropy_kernel<<<(unsigned)rows, kCeThreads, 0, (cudaStream_t)stream>>>(
-      (const __nv_bfloat16*)logits, target, loss, lse, (__nv_bfloat16*)dlogits, V, stride,
-      ignore_index, gscale);
+  const int threads = ce_threads(rows, V);
+  auto kern = threads == 512 ? cross_entropy_kernel<512> : cross_entropy_kernel<256>;
+  kern<<<(unsigned)rows, threads, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)logits, target, loss, lse,
+                                                             (__nv_bfloat16*)dlogits, V, stride, ignore_index, gscale);
   return (int)cudaGetLastError();
 }
 
