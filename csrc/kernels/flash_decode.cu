@@ -15,7 +15,8 @@
 // The same case takes 82 us (6.6 TB/s; 112 before the ring); 32 x 8000 keys 151 (6.9 TB/s; 215), 16 x 1006 keys 15.7
 // (20), D = 64 with 8 x 16381 keys 44 (52).
 // Scores, running maximum, sums and output accumulate in fp32; probabilities are rounded to bf16 for the second
-// product, as in flash_fwd_kernel.
+// product, as in flash_fwd_kernel. With at most eight rows to a KV head the other eight rows of the operand carry what that
+// rounding cuts off (FINE).
 #include "sm100.cuh"
 #include "tpb_api.h"
 
@@ -73,10 +74,16 @@ constexpr int dec_smem(int d) {
   return ring > rows ? ring : rows;
 }
 
-template <int D>
+// FINE: at most eight rows. The operand's rows 8..15 are then nobody's; in the second product they hold P - bf16(P) of rows 0..7,
+// and their sums are added in the end. The largest probability of a warp's keys is exactly one and has no rounding error, so
+// that the error grew with longer runs of keys to a warp: of the norm, against 64 bits, 2.21e-3 at 8 x 16381 keys, 32/8 heads of
+// 128 (2.16e-3 in twice as many parts), 1.66e-3 so, which is the rounding of the result. It saves the exponentials of the rows that
+// are not there: the same case 82.3 -> 81.6 us, 16 x 1006 keys 15.9 -> 15.3, one sequence of 9000 18.1 -> 17.6.
+template <int D, bool FINE>
 __global__ void __launch_bounds__(kDecWarps * 32, dec_ctas(D))
 flash_decode_kernel(const DecodeParams p) {
   constexpr int S = dec_stages(D);
+  constexpr int NR = FINE ? 1 : 2;          // rows of a lane
   constexpr int kTile = kDecKeys * D * 2;   // bytes of a step's K (or V) of a warp
   extern __shared__ __align__(128) uint8_t dec_sm[];   // the warps' rings, later their partial rows
   __shared__ float sm_m[kDecWarps][kDecRows], sm_l[kDecWarps][kDecRows], sm_lse[kDecRows];
@@ -185,7 +192,7 @@ flash_decode_kernel(const DecodeParams p) {
 #pragma unroll
     for (int u = 0; u < 2; ++u)
 #pragma unroll
-      for (int i = 0; i < 2; ++i)
+      for (int i = 0; i < NR; ++i)
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
           float& x = s[u][2 * i + j];
@@ -195,7 +202,7 @@ flash_decode_kernel(const DecodeParams p) {
 #pragma unroll
       for (int u = 0; u < 2; ++u)
 #pragma unroll
-        for (int i = 0; i < 2; ++i)
+        for (int i = 0; i < NR; ++i)
 #pragma unroll
           for (int j = 0; j < 2; ++j) {
             const int key = base + u * 8 + 2 * t + j;
@@ -205,7 +212,7 @@ flash_decode_kernel(const DecodeParams p) {
     }
     float alpha[2], mu[2];
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
+    for (int i = 0; i < NR; ++i) {
       mx[i] = fmaxf(fmaxf(s[0][2 * i], s[0][2 * i + 1]), fmaxf(s[1][2 * i], s[1][2 * i + 1]));
       mx[i] = fmaxf(mx[i], __shfl_xor_sync(0xffffffffu, mx[i], 1));
       mx[i] = fmaxf(mx[i], __shfl_xor_sync(0xffffffffu, mx[i], 2));
@@ -215,6 +222,7 @@ flash_decode_kernel(const DecodeParams p) {
       m[i] = mn;
       l[i] *= alpha[i];
     }
+    if (FINE) alpha[1] = alpha[0];
     if (__any_sync(0xffffffffu, alpha[0] != 1.f || alpha[1] != 1.f)) {
 #pragma unroll
       for (int n = 0; n < D / 8; ++n) {
@@ -226,10 +234,12 @@ flash_decode_kernel(const DecodeParams p) {
 #pragma unroll
     for (int u = 0; u < 2; ++u)
 #pragma unroll
-      for (int i = 0; i < 2; ++i) {
+      for (int i = 0; i < NR; ++i) {
         const float e0 = dec_exp2(s[u][2 * i] - mu[i]), e1 = dec_exp2(s[u][2 * i + 1] - mu[i]);
         l[i] += e0 + e1;
-        pa[2 * u + i] = dec_pack(e0, e1);
+        const uint32_t w = dec_pack(e0, e1);
+        pa[2 * u + i] = w;
+        if (FINE) pa[2 * u + 1] = dec_pack(e0 - __uint_as_float(w << 16), e1 - __uint_as_float(w & 0xffff0000u));
       }
     dec_wait<2 * S - 1>();
     __syncwarp();
@@ -249,13 +259,19 @@ flash_decode_kernel(const DecodeParams p) {
 
   // ---- the four warps' partial rows
 #pragma unroll
-  for (int i = 0; i < 2; ++i) {
+  for (int i = 0; i < NR; ++i) {
     l[i] += __shfl_xor_sync(0xffffffffu, l[i], 1);
     l[i] += __shfl_xor_sync(0xffffffffu, l[i], 2);
     if (t == 0) { sm_m[warp][gq + 8 * i] = m[i]; sm_l[warp][gq + 8 * i] = l[i]; }
 #pragma unroll
-    for (int n = 0; n < D / 8; ++n)
-      *reinterpret_cast<float2*>(&sm_o[warp][gq + 8 * i][n * 8 + 2 * t]) = make_float2(acc[n][2 * i], acc[n][2 * i + 1]);
+    for (int n = 0; n < D / 8; ++n) {
+      float2 v = make_float2(acc[n][2 * i], acc[n][2 * i + 1]);
+      if (FINE) {   // an infinite V gives infinities of either sign in the second part
+        if (fabsf(v.x) < INFINITY) v.x += acc[n][2];
+        if (fabsf(v.y) < INFINITY) v.y += acc[n][3];
+      }
+      *reinterpret_cast<float2*>(&sm_o[warp][gq + 8 * i][n * 8 + 2 * t]) = v;
+    }
   }
   __syncthreads();
   constexpr int VEC = D / 4;   // float4 per row
@@ -388,15 +404,20 @@ flash_decode_merge_kernel(const DecodeParams p) {
     p.lse[((long long)b * p.Hq + h) * p.lse_stride + tq] = den > 0.f ? (M + log2f(den)) * 0.6931471805599453f : -INFINITY;
 }
 
+typedef void (*DecodeKernel)(DecodeParams);
+static DecodeKernel decode_kernel(int D, bool fine) {
+  return D == 64 ? (fine ? flash_decode_kernel<64, true> : flash_decode_kernel<64, false>)
+                 : (fine ? flash_decode_kernel<128, true> : flash_decode_kernel<128, false>);
+}
+
 // More shared memory than a launch gets unasked.
-static cudaError_t decode_configure(int D) {
-  static PerDevice done[2];
-  return D == 64 ? allow_smem(done[0], flash_decode_kernel<64>, dec_smem(64))
-                 : allow_smem(done[1], flash_decode_kernel<128>, dec_smem(128));
+static cudaError_t decode_configure(int D, bool fine) {
+  static PerDevice done[2][2];
+  return allow_smem(done[D == 64 ? 0 : 1][fine], decode_kernel(D, fine), dec_smem(D));
 }
 
 // Clusters of n CTAs that fit the device at once, asked of the runtime once per size and device: the SMs of a GPC are not a
-// multiple of every n (32 clusters of 8 CTAs of D = 128 fit, 96 of 3 do not, although 296 CTAs do).
+// multiple of every n (48 clusters of 8 CTAs of D = 128 fit, 142 of 3, although 444 CTAs do). Both forms take the same room.
 static int decode_resident(int D, int n) {
   static PerDevice resident[2][kDecCluster + 1];
   return resident[D == 64 ? 0 : 1][n].get([&] {
@@ -412,9 +433,8 @@ static int decode_resident(int D, int n) {
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     int fit = 0;
-    decode_configure(D);
-    const cudaError_t e = D == 64 ? cudaOccupancyMaxActiveClusters(&fit, flash_decode_kernel<64>, &cfg)
-                                  : cudaOccupancyMaxActiveClusters(&fit, flash_decode_kernel<128>, &cfg);
+    decode_configure(D, false);
+    const cudaError_t e = cudaOccupancyMaxActiveClusters(&fit, decode_kernel(D, false), &cfg);
     return e == cudaSuccess && fit > 0 ? fit : -1;
   });
 }
@@ -524,9 +544,10 @@ extern "C" int tpb_flash_decode(const void* q, const void* k, const void* v, voi
     attr[cfg.numAttrs].val.clusterDim.y = 1;
     attr[cfg.numAttrs++].val.clusterDim.z = 1;
   }
-  cudaError_t e = decode_configure(D);
+  const bool fine = p.R <= 8;
+  cudaError_t e = decode_configure(D, fine);
   if (e != cudaSuccess) return (int)e;
-  e = cudaLaunchKernelEx(&cfg, D == 128 ? flash_decode_kernel<128> : flash_decode_kernel<64>, p);
+  e = cudaLaunchKernelEx(&cfg, decode_kernel(D, fine), p);
   if (e != cudaSuccess) return (int)e;
   if (p.part_o) {
     const long long rows = (long long)B * Hkv * p.R;
