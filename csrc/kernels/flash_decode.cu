@@ -443,11 +443,14 @@ static int decode_resident(int D, int n) {
 // takes (7 TB/s; the row tiles of a head share its reads) or the keys of one times kKeyNs, which grows with the CTAs per
 // SM: one alone reads 49 (D = 128) or 37 (64) GB/s and keeps an SM's share of the memory busy by itself. Clusters are not
 // spread evenly: at 0.87 of an SM each, some SMs have two CTAs. A launch costs 4 us, each further round 1.8 us and a tail of
-// 4 ns a key; a cluster's merge 1 us; a second kernel and scratch 4 us + 60 ns a split on the device and 5 us on the host,
-// which bounds a call over a short cache. Measured, D x B x Hkv x Tk, splits: us (m: by two kernels): 128 x 8 x 8 x 16381,
-// 1: 177, 2: 94, 3: 87, 4: 82, 5: 92, 8: 105, m9: 100, m12: 87; 128 x 32 x 8 x 8000, 1: 151, 2: 192, 3: 162, 8: 170;
-// 128 x 3 x 16 x 5000, 1: 57, 3: 30, 5: 24, 8: 25; 128 x 1 x 8 x 32768, 8: 49, m16: 30, m32: 29; 128 x 1 x 8 x 4096, 1: 47,
-// 4: 16, 8: 11, m16: 10; 64 x 8 x 8 x 16381, 1: 115, 2: 62, 4: 44, 7: 51, 8: 47; 64 x 32 x 8 x 8000, 1: 80, 2: 89, 3: 97.
+// 4 ns a key; a cluster's merge 1 us; a second kernel and scratch 3 us + 60 ns a split. The 5 us that they cost on the host are
+// not counted: a launch that is waited for the host takes those whatever it does, and up to some 4000 keys the clusters are ahead
+// anyway. (Counted, one sequence of 9000 keys and one KV head took 17.8 us for 11.6, two of 30000 and eight 56.8 for 44.7.)
+// Measured, D x B x Hkv x Tk, splits: us (m: by two kernels): 128 x 8 x 8 x 16381, 1: 177, 2: 94, 3: 87, 4: 82, 5: 92, 8: 105,
+// m9: 100, m12: 87; 128 x 32 x 8 x 8000, 1: 151, 2: 192, 3: 162, 8: 170; 128 x 3 x 16 x 5000, 1: 57, 3: 30, 5: 24, 8: 25;
+// 128 x 1 x 8 x 3000, 8: 9.5, m16: 10.0; x 5500, 8: 13.0, m16: 12.0; x 10000, 8: 19.0, m16: 14.7; x 30000, 8: 44.8, m32: 27.3;
+// 128 x 1 x 1 x 3000, 8: 8.7, m16: 8.2; x 7500, 8: 14.9, m40: 10.2; 64 x 1 x 8 x 5500, 8: 9.6, m16: 9.8; x 14000, 8: 16.6,
+// m32: 12.9; 64 x 8 x 8 x 16381, 1: 115, 2: 62, 4: 44, 7: 51, 8: 47; 64 x 32 x 8 x 8000, 1: 80, 2: 89, 3: 97.
 struct DecodePlan {
   int splits;
   bool memory;   // merged by the second kernel
@@ -471,7 +474,7 @@ static DecodePlan decode_plan(int B, int Hkv, int row_tiles, int Tk, int D, bool
     const long long full = units / slots, rest = units % slots, rounds = full + (rest > 0);
     double cost = full * round((double)(slots * ctas)) + (rest ? round((double)(rest * ctas)) : 0) + 4000 + 1800.0 * (rounds - 1);
     if (rounds > 1) cost += 4 * keys;
-    cost += mem ? 9000 + 60 * n : (n > 1 ? 1000 : 0);
+    cost += mem ? 3000 + 60 * n : (n > 1 ? 1000 : 0);
     if (best_cost < 0 || cost < best_cost) { best = {n, mem}; best_cost = cost; }
   };
   consider(1, false, tiles, fit * sms, 1);

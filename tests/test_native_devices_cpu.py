@@ -70,6 +70,16 @@ def test_splits_by_the_device_at_hand(child, D):
     assert both == child(code % "(0,)") + child(code % "(1,)") and both[0] != both[1]
 
 
+@pytest.mark.parametrize("D", [64, 128])
+def test_long_caches_of_few_heads_take_two_launches(child, D):
+    """Where eight CTAs to a head are few for the keys; a short cache stays one launch."""
+    assert child(f"""
+        F.fake_set_clusters(0, 48)
+        for B, Hkv, Tk in ((1, 1, 9000), (1, 2, 9000), (1, 8, 14000), (2, 8, 30000), (1, 1, 2100), (1, 8, 3000), (8, 8, 16381)):
+            print(int(L.tpb_flash_decode_splits(I(B), I(1), I(Tk), I(4 * Hkv), I(Hkv), I({D})) > 8))
+    """) == list("1111000")
+
+
 @pytest.mark.parametrize("bits,group", [(4, 128), (8, 0)])
 def test_packed_weights_on_every_device(child, bits, group):
     assert child(f"""
