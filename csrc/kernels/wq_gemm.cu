@@ -363,15 +363,19 @@ using namespace tpb;
 
 // Whether tpb_wq_gemm takes this product and is the fastest way to it. Up to 16 rows belong to the GEMV, which does not round
 // the weights (9 x 28672 x 8192 77 us there, 61 here). The other way: a pass that converts the weights (two launches, 5 TB/s
-// of packed and bf16 bytes) and the bf16 product (6 TB/s of weights or 1.1 PFLOP/s, 1.5 from 1024 rows on). us there / here,
-// 4 bits: 17 x 4096 x 4096 18 / 18, 200 x 1024 x 1024 12 / 9, 1024 x 28672 x 8192 445 / 430, 4096 x 14336 x 4096 351 / 449.
+// of packed and bf16 bytes) and the bf16 product (6 TB/s of weights or 1.1 PFLOP/s, 1.5 from 1024 rows on); of that 0.81 for few
+// rows, where the product finds the weights in L2 and splits K: up to 40 rows, or 128 of 8 bits. us there / here, 4 bits: 17 x
+// 4096 x 4096 18 / 18, 22 x 1280 x 1536 8.7 / 8.9, 27 x 7560 x 1280 13.5 / 9.1, 200 x 1024 x 1024 12 / 9, 1024 x 28672 x 8192
+// 445 / 430, 4096 x 14336 x 4096 351 / 449; 8 bits: 35 x 2216 x 1664 10.0 / 10.2, 73 x 2152 x 3200 13.5 / 15.4, 87 x 3800 x 2816
+// 16.7 / 15.0, 128 x 4096 x 4096 20.8 / 19.9.
 extern "C" int tpb_wq_gemm_pays(int M, int N, int K, int bits, int group) {
   if (M <= 16 || N <= 0 || K <= 0 || !wq_gemm_fits(N, K, bits, group)) return 0;
   double us = 0;
   wq_pick_nt(M, (N + 127) / 128, &us);
-  const double here = 4 + us * (K / 128), weights = (double)N * K, packed = weights * bits / 8;
+  const double here = 4.3 + us * (K / 128), weights = (double)N * K, packed = weights * bits / 8;
   const double read = weights * 2 / 6e6, math = 2.0 * M * weights / (M < 1024 ? 1.1e9 : 1.5e9);
-  return here < 9 + (packed + 2 * weights) / 5e6 + (read > math ? read : math);
+  const double there = 9 + (packed + 2 * weights) / 5e6 + (read > math ? read : math);
+  return here < (M <= 40 || (M <= 128 && bits == 8) ? 0.81 : 1.0) * there;
 }
 
 // Arguments as tpb_wq_gemv, any number of rows; K a multiple of 128, one scale per row (8 bits, group 0) or groups of 128 times

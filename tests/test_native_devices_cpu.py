@@ -132,3 +132,15 @@ def test_packed_weights_tile_rows(child):
                     best = (cost, tiles)
             want.append(str(min(best[1], SMS)))
     assert got == want
+
+
+def test_packed_weights_where_it_pays(child):
+    """Sizes at which one of the two ways was measured to be the faster by more than runs differ."""
+    here = [(56, 1656, 1280, 8), (20, 4336, 1152, 4), (27, 7560, 1280, 4), (79, 6336, 1152, 4), (87, 3800, 2816, 8), (128, 4096, 4096, 8),
+            (22, 10568, 3968, 8), (111, 18568, 7424, 8), (513, 1880, 1792, 4), (777, 14336, 4096, 4), (552, 27880, 2688, 8)]
+    there = [(73, 2152, 3200, 8), (35, 2216, 1664, 8), (21, 2136, 3200, 4), (4096, 14336, 4096, 4)]
+    got = child(f"""
+        for M, N, K, bits in {here + there}:
+            print(L.tpb_wq_gemm_pays(I(M), I(N), I(K), I(bits), I(128 if bits == 4 else 0)))
+    """)
+    assert got == ["1"] * len(here) + ["0"] * len(there)
