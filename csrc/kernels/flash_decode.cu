@@ -411,16 +411,16 @@ static DecodeKernel decode_kernel(int D, bool fine) {
 }
 
 // More shared memory than a launch gets unasked.
-static cudaError_t decode_configure(int D, bool fine) {
+static cudaError_t decode_configure(int dev, int D, bool fine) {
   static PerDevice done[2][2];
-  return allow_smem(done[D == 64 ? 0 : 1][fine], decode_kernel(D, fine), dec_smem(D));
+  return allow_smem(done[D == 64 ? 0 : 1][fine], dev, decode_kernel(D, fine), dec_smem(D));
 }
 
 // Clusters of n CTAs that fit the device at once, asked of the runtime once per size and device: the SMs of a GPC are not a
 // multiple of every n (48 clusters of 8 CTAs of D = 128 fit, 142 of 3, although 444 CTAs do). Both forms take the same room.
-static int decode_resident(int D, int n) {
+static int decode_resident(int dev, int D, int n) {
   static PerDevice resident[2][kDecCluster + 1];
-  return resident[D == 64 ? 0 : 1][n].get([&] {
+  return resident[D == 64 ? 0 : 1][n].get(dev, [&] {
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -433,7 +433,7 @@ static int decode_resident(int D, int n) {
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     int fit = 0;
-    decode_configure(D, false);
+    decode_configure(dev, D, false);
     const cudaError_t e = cudaOccupancyMaxActiveClusters(&fit, decode_kernel(D, false), &cfg);
     return e == cudaSuccess && fit > 0 ? fit : -1;
   });
@@ -455,7 +455,7 @@ struct DecodePlan {
   int splits;
   bool memory;   // merged by the second kernel
 };
-static DecodePlan decode_plan(int B, int Hkv, int row_tiles, int Tk, int D, bool memory) {
+static DecodePlan decode_plan(int dev, int B, int Hkv, int row_tiles, int Tk, int D, bool memory) {
   static const double kKeyNs[2][4] = {{7.0, 9.1, 13.0, 21.0}, {10.5, 15.0, 26.0, 26.0}};
   const int fit = dec_ctas(D), wide = D == 64 ? 0 : 1;
   const long long tiles = (long long)B * Hkv * row_tiles, sms = sm_count();
@@ -478,8 +478,10 @@ static DecodePlan decode_plan(int B, int Hkv, int row_tiles, int Tk, int D, bool
     if (best_cost < 0 || cost < best_cost) { best = {n, mem}; best_cost = cost; }
   };
   consider(1, false, tiles, fit * sms, 1);
-  for (int n = 2; n <= kDecCluster && Tk / n >= 64; ++n)
-    if (decode_resident(D, n) > 0) consider(n, false, tiles, decode_resident(D, n), n);
+  for (int n = 2; n <= kDecCluster && Tk / n >= 64; ++n) {
+    const int clusters = decode_resident(dev, D, n);
+    if (clusters > 0) consider(n, false, tiles, clusters, n);
+  }
   for (int n = 2; memory && n <= 64 && Tk / n >= 64; ++n) consider(n, true, tiles * n, fit * sms, 1);
   return best;
 }
@@ -492,7 +494,7 @@ using namespace tpb;
 // anyway up to 2048 keys); else their number n: part_o has to hold n * B * Hq * Tq * D floats, part_lse n * B * Hq * Tq.
 extern "C" int tpb_flash_decode_splits(int B, int Tq, int Tk, int Hq, int Hkv, int D) {
   if (B <= 0 || Tq <= 0 || Tk <= 0 || Hkv <= 0) return 0;
-  const DecodePlan plan = decode_plan(B, Hkv, (Tq * (Hq / Hkv) + kDecRows - 1) / kDecRows, Tk, D, true);
+  const DecodePlan plan = decode_plan(current_device(), B, Hkv, (Tq * (Hq / Hkv) + kDecRows - 1) / kDecRows, Tk, D, true);
   return plan.memory ? plan.splits : 0;
 }
 
@@ -513,9 +515,10 @@ extern "C" int tpb_flash_decode(const void* q, const void* k, const void* v, voi
        reinterpret_cast<uintptr_t>(o)) & 15)
     return -2;
   if ((n_splits > kDecCluster && !part_o) || (part_o && !part_lse)) return -2;
+  const int dev = current_device();
   if (n_splits == 0) {
     part_o = part_lse = nullptr;
-    n_splits = decode_plan(B, Hkv, (Tq * (Hq / Hkv) + kDecRows - 1) / kDecRows, Tk, D, false).splits;
+    n_splits = decode_plan(dev, B, Hkv, (Tq * (Hq / Hkv) + kDecRows - 1) / kDecRows, Tk, D, false).splits;
   }
   DecodeParams p;
   p.q = (const __nv_bfloat16*)q; p.k = (const __nv_bfloat16*)k; p.v = (const __nv_bfloat16*)v;
@@ -548,7 +551,7 @@ extern "C" int tpb_flash_decode(const void* q, const void* k, const void* v, voi
     attr[cfg.numAttrs++].val.clusterDim.z = 1;
   }
   const bool fine = p.R <= 8;
-  cudaError_t e = decode_configure(D, fine);
+  cudaError_t e = decode_configure(dev, D, fine);
   if (e != cudaSuccess) return (int)e;
   e = cudaLaunchKernelEx(&cfg, decode_kernel(D, fine), p);
   if (e != cudaSuccess) return (int)e;

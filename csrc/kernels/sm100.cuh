@@ -146,13 +146,16 @@ __device__ __forceinline__ uint4 chain_ld(const void* p) {
 // Host side: a value for each device of the process. What the runtime keeps per device (a kernel's shared-memory limit) or
 // answers for one (how many clusters fit) is set or asked once on each; a process may launch on several, from several threads.
 // 0 means not yet; devices past the last slot are set and asked on every call.
+inline int current_device() {
+  int dev = 0;
+  return cudaGetDevice(&dev) == cudaSuccess ? dev : -1;
+}
 struct PerDevice {
   static constexpr int kDevices = 64;
   std::atomic<int> v[kDevices];
   template <typename F>
-  int get(F&& ask) {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kDevices) return ask();
+  int get(int dev, F&& ask) {
+    if (dev < 0 || dev >= kDevices) return ask();
     int r = v[dev].load(std::memory_order_acquire);
     if (r == 0) {
       r = ask();
@@ -161,11 +164,11 @@ struct PerDevice {
     return r;
   }
 };
-// `kern` may have `bytes` of dynamic shared memory on the current device from then on.
+// `kern` may have `bytes` of dynamic shared memory on the current device `dev` from then on.
 template <typename K>
-inline cudaError_t allow_smem(PerDevice& done, K kern, int bytes) {
+inline cudaError_t allow_smem(PerDevice& done, int dev, K kern, int bytes) {
   cudaError_t e = cudaSuccess;
-  done.get([&] {
+  done.get(dev, [&] {
     e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     return e == cudaSuccess ? 1 : 0;   // a failure is tried again
   });

@@ -328,7 +328,7 @@ constexpr int wq_smem(int bits, int nt, int w_stages, int x_stages) {
 template <int BITS>
 int launch_wq_gemm(const CUtensorMap& tw, const CUtensorMap& tx, const WqGemmParams& p, cudaStream_t stream) {
   static PerDevice done;
-  const cudaError_t e = allow_smem(done, wq_gemm_kernel<BITS>, 227 * 1024);
+  const cudaError_t e = allow_smem(done, current_device(), wq_gemm_kernel<BITS>, 227 * 1024);
   if (e != cudaSuccess) return (int)e;
   const int tiles = p.n_tiles * p.m_tiles;
   wq_gemm_kernel<BITS><<<tiles < sm_count() ? tiles : sm_count(), kWqThreads, wq_smem(BITS, p.NT, p.w_stages, p.x_stages), stream>>>(

@@ -341,10 +341,6 @@ class Llama(nn.Module):
         pos = flat_positions(position_ids, rows, dev)
         L, Tk = lib(), past + T
         logits = embed.new_empty(B, T, V)
-        for i in range(n_layers):
-            cache.room(kv_shape, kv_shape, logits, logits, i)
-            if cache._k[i].shape[2] < Tk:   # buffers of before the cache was allowed more: the append layer by layer refuses
-                return None
         scratch = logits.new_empty(L.tpb_llama_cached_scratch(rows, H, Hq, Hkv, D, I))
         few = few_rows_sizes(B, T, Tk, Hq, Hkv, D)
         splits = L.tpb_flash_decode_splits(B, T, Tk, Hq, Hkv, D) if few and Tk > 2048 else 0
@@ -359,9 +355,13 @@ class Llama(nn.Module):
             part + 4 * part_rows * D if splits else 0, lse, lse_stride, splits, int(few), B, T, past, H, Hq, Hkv, D, I, V,
             n_layers))
         for i in range(n_layers):
+            cache.room(kv_shape, kv_shape, logits, logits, i)
             k = cache._k[i]
+            room = k.shape[2]
+            if room < Tk:   # buffers of before the cache was allowed more: the append layer by layer refuses
+                return None
             words.extend(weights[6 * i:6 * i + 6])
-            words.extend((k.data_ptr(), cache._v[i].data_ptr(), k.shape[2]))
+            words.extend((k.data_ptr(), cache._v[i].data_ptr(), room))
         _native.check(L.tpb_llama_cached(words.buffer_info()[0], cfg.rms_eps, 1.0 / math.sqrt(D), stream_ptr()),
                       "tpb_llama_cached")
         _native.launch_count += 3 + n_layers * (10 + (splits > 0))
