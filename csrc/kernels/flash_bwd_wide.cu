@@ -7,15 +7,16 @@
 //     dV(i)  S(i+1)  dK(i)  dP(i+1)      (dQ pass: S(i+1)  dQ(i)  dP(i+1)),
 // and the warps compute dS(i) under dV(i) and S(i+1), and P(i+1) under dK(i) and dP(i+1). The dQ pass has no P product: S(i+1)
 // is issued once S(i) is in registers and runs under P(i). The warps take 32 columns at a time and load the next ones under
-// the math of the ones before, and read the statistics for P while they wait for S. 32/8 heads, both passes: T = 8190 1765 ->
-// 1571 us, T = 4096 496 -> 439; D = 64, T = 8190 1307 -> 1132, 16 x 1024 tokens of 12 heads 222 -> 200.
+// the math of the ones before, and read the statistics for P while they wait for S. With that and the passes overlapping
+// (flash_bwd.cuh), in turn on one GPU, 32/8 heads, both passes: T = 8190 1910 -> 1706 us (at the power cap), T = 4096 514 -> 459;
+// D = 64, T = 8190 1303 -> 1157, 16 x 1024 tokens of 12 heads 216 -> 188.
 //
 // D = 128: TMEM (S, dP and two accumulators of 128 columns) has no room for two tiles unless they have 64 rows; with 128
-// rows there are half as many barriers and round trips. 32/8 heads: T = 4096 533 -> 478 us for both passes, T = 8190
-// 1845 -> 1687 us; the chip then runs at its power cap (1.7 GHz), at about 0.6 of what the MMAs alone would take.
+// rows there are half as many barriers and round trips (a tenth of the time at T = 4096 and 8190 when it was taken); the
+// chip then runs at its power cap (1.7 GHz), at about 0.6 of what the MMAs alone would take.
 // D = 64: 64-row tiles fit half of TMEM and of shared memory, so that two CTAs share an SM: starting and finishing a CTA
 // takes about as long as the eight iterations it has at T = 1024, and one CTA's start, end and waits lie under the
-// other's work (16 x 1024 tokens, 12 heads: 236 -> 209 us for both passes).
+// other's work (a ninth of the time at 16 x 1024 tokens of 12 heads when it was taken).
 #include "flash_bwd.cuh"
 #include "tpb_api.h"
 

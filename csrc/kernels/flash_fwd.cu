@@ -152,7 +152,7 @@ __device__ __forceinline__ void row_mask(uint32_t (&sr)[32], int k0, int lo, int
 
 // exp2 of a pair on the FMA pipe: floor by the magic-number add in round-down mode, cubic
 // polynomial on the fraction (relative error 1e-4, below the bf16 rounding of P), exponent added
-// as an integer. Below -127 the result is 2^-127; from 128 on the sum leaves the exponent field and the result is anything,
+// as an integer: the emulation that FlashAttention-4 published, with its coefficients. Below -127 the result is 2^-127; from 128 on the sum leaves the exponent field and the result is anything,
 // a small number of either sign among others, so that who does not know the maximum has to look at x.
 // The special-function unit delivers 16 exp2 per cycle and SM while the tensor pipe
 // needs 16 per cycle for 128-wide head dimensions, so a share of the row goes this way.
